@@ -374,10 +374,10 @@ class StepPool {
   explicit StepPool(int n) {
     int dev = 0;
     SBP_CUDA(cudaGetDevice(&dev));
-    double2* logt = Context::primary().logt;
-    for (int i = 0; i < n; ++i) std::thread([this, i, dev, logt] { worker(i, dev, logt); }).detach();
+    double2* xlogxt = Context::primary().xlogxt;
+    for (int i = 0; i < n; ++i) std::thread([this, i, dev, xlogxt] { worker(i, dev, xlogxt); }).detach();
   }
-  void worker(int i, int dev, double2* logt) {
+  void worker(int i, int dev, double2* xlogxt) {
     Context* ctx = nullptr;
     unsigned long long seen = 0;
     for (;;) {
@@ -390,7 +390,7 @@ class StepPool {
       try {
         if (!ctx) {
           SBP_CUDA(cudaSetDevice(dev));
-          ctx = Context::create(logt);
+          ctx = Context::create(xlogxt);
           Context::current() = ctx;
         }
         for (;;) {

@@ -94,28 +94,19 @@ __device__ __forceinline__ double dxlogx(double a, double b) {
   return (a - b) * log(sa) + b * log1p((sa - sb) / sb);
 }
 
-// g(a) - g(b) for integer counts a, b >= 0 as (a - b) log a + b log(a / b), from a table of
-// log(x) = hi + lo (lo carries the bits below hi's last place):
-//  - a close to b (128 |a - b| <= b, b > 0): log(a / b) = 2 atanh(z), z = (a - b) / (a + b), by its
-//    Taylor series 2 (z + z^3/3 + z^5/5 + z^7/7), |z| <= 1/255, which keeps the relative
-//    accuracy that a difference of two table logs would lose;
-//  - otherwise log(a / b) = (hi_a - hi_b) + (lo_a - lo_b).
-// A zero side uses log 1 = 0, which leaves the other side's g term.  Counts beyond the table
-// go through dxlogx.
-constexpr int kLogTable = 1 << 20;
-__device__ __forceinline__ double dxlogx_int(const double2* __restrict__ logt, int a, int b) {
-  if (a < kLogTable && b < kLogTable) {
-    const int d = a - b;
-    const double2 la = __ldg(logt + (a > 0 ? a : 1));
-    double lab;
-    if (b > 0 && 128LL * (d < 0 ? -(long long)d : (long long)d) <= (long long)b) {
-      const double z = (double)d / ((double)a + (double)b), w = z * z;
-      lab = 2.0 * z + 2.0 * z * w * (1.0 / 3.0 + w * (1.0 / 5.0 + w * (1.0 / 7.0)));
-    } else {
-      const double2 lb = __ldg(logt + (b > 0 ? b : 1));
-      lab = (la.x - lb.x) + (la.y - lb.y);
-    }
-    return (double)d * (la.x + la.y) + (double)b * lab;
+// g(a) - g(b) for integer counts a, b >= 0 from a table of g(x) = hi + lo (hi = g rounded, lo the
+// rest, about 104 bits in all; g(0) = g(1) = 0): (hi_a - hi_b) + (lo_a - lo_b).  hi_a - hi_b is
+// exact when the two are within a factor of two (Sterbenz) and otherwise within half an ulp of a
+// difference of the size of the larger, so the result keeps a relative error near 2^-53 whether
+// the counts are close or not (measured worst 1.9e-16; the (a - b) log a + b log(a / b) form
+// from a table of logs that it replaced: 3e-16).  Two loads and three additions: that form's
+// division, series and two-sided branch were most of the FP64 instructions of a visit.  Counts
+// beyond the table go through dxlogx.
+constexpr int kXlogxTable = 1 << 20;
+__device__ __forceinline__ double dxlogx_int(const double2* __restrict__ gt, int a, int b) {
+  if ((unsigned)a < (unsigned)kXlogxTable && (unsigned)b < (unsigned)kXlogxTable) {
+    const double2 ga = __ldg(gt + a), gb = __ldg(gt + b);
+    return (ga.x - gb.x) + (ga.y - gb.y);
   }
   return dxlogx((double)a, (double)b);
 }
@@ -186,7 +177,7 @@ struct BlockView {
   int* d_out;             // [B]
   int* d_in;              // [B]
   int* d;                 // [B] block degrees as the reference maintains them
-  const double2* logt;    // [kLogTable] log(x) = hi + lo for integer x (entry 0 unused)
+  const double2* xlogxt;  // [kXlogxTable] x log x = hi + lo for integer x
 };
 
 // Walk values row[0..n) ascending and return the first index whose running sum exceeds
@@ -646,28 +637,21 @@ __device__ __forceinline__ void prefetch_nb(const BlockView& bm, int r, const Wa
   p->din_r = ldi<ST>(bm.d_in + r);
 }
 
-// Position of the n-th (0-based) set bit of m; requires n < popc(m).
-__device__ __forceinline__ int nth_set_bit(unsigned m, int n) {
-  int pos = 0;
-#pragma unroll
-  for (int w = 16; w > 0; w >>= 1) {
-    const int c = __popc(m & ((1u << w) - 1u));
-    if (n >= c) {
-      n -= c;
-      m >>= w;
-      pos += w;
-    }
-  }
-  return pos;
+// Above this |delta-MDL| the zero snap (below) cannot apply, whatever the integer scale T of the
+// changed cells and degrees is: every changed cell lies in a row or column of r or s, so T is at
+// most six times the block degrees of r and s plus four times the vertex's.
+__device__ __forceinline__ bool maybe_zero_delta(double dS, int dout_r, int dout_s, int din_r, int din_s, int k,
+                                                 double log_E) {
+  const double bound = 6.0 * ((double)dout_r + (double)dout_s + (double)din_r + (double)din_s) + 4.0 * (double)k + 4.0;
+  return fabs(dS) <= 0x1p-40 * bound * log_E;
 }
 
 // Delta-MDL of moving v from r to s (s != r) against the current state, with the gathered
 // table of v's neighbour blocks, and the reference's Hastings correction (*H).
 //  - One load round over the distinct neighbour blocks (lane i: table entries i, i+32, ...)
-//    gives the Hastings sums and the changed cells.
-//  - The FP64 terms are then spread over the warp one term per lane: the eight corner-cell
-//    and degree terms, and two cells per (neighbour block, direction) pair that changes:
-//    (r,u) and (s,u) for v's out-edges to u, (u,r) and (u,s) for its in-edges from u.
+//    gives the Hastings sums and the changed cells; the lane that loaded a cell adds its FP64
+//    term: (r,u) and (s,u) for v's out-edges to u, (u,r) and (u,s) for its in-edges from u.
+//  - Eight lanes add the corner-cell and degree terms.
 //  - The double count of a present net-zero (r,s) / (s,r) Delta cell is added by the lanes
 //    that hold it, and only then.
 // Every lane returns the same values.
@@ -689,84 +673,51 @@ __device__ __forceinline__ double move_delta(const GraphView& g, const BlockView
   const int kin_self = k_in + self;
 
   double fwd = 0.0, bwd = 0.0, dS = 0.0;
-  long long T = 0;   // integer scale of the changed cells and degrees (zero snap below)
   const int n = *t.nlist;
-  for (int base = 0; base < n; base += kWarp) {
-    const int i = base + lane;
-    int M_su = 0, M_us = 0, M_ru = 0, M_ur = 0, co_c = 0, ci_c = 0;
-    if (i < n) {
-      int u, co, ci, du;
-      if (pre && base == 0) {
-        u = pre->u;
-        co = pre->co;
-        ci = pre->ci;
-        M_ru = pre->M_ru;
-        M_ur = pre->M_ur;
-        du = pre->du;
-      } else {
-        const int h = t.list[i];
-        u = t.keys[h];
-        co = t.cout[h];
-        ci = t.cin[h];
-        M_ru = bm_get<ST>(bm, r, u);
-        M_ur = bm_getT<ST>(bm, r, u);
-        du = ldi<ST>(bm.d + u);
-      }
-      M_su = bm_get<ST>(bm, s, u);
-      M_us = bm_getT<ST>(bm, s, u);
-      const bool is_r = (u == r), is_s = (u == s), corner = is_r || is_s;
-      const double c = (double)(co + ci + (is_r ? self : 0));
-      const double inv_u = 1.0 / ((double)du + (double)B);   // a non-corner block's degree is unchanged
-      fwd += c * (M_su + M_us + 1.0) * inv_u;
-      const double bw = is_r ? (double)(M_rr + d_rr) + (double)(M_rr + d_rr) + 1.0
-                      : is_s ? (double)(M_rs + d_rs) + (double)(M_sr + d_sr) + 1.0
-                             : (double)(M_ru - co) + (double)(M_ur - ci) + 1.0;
-      const int nd = is_r ? (dout_r - k_out) + (din_r - k_in) - (M_rr + d_rr)
-                   : is_s ? (dout_s + k_out) + (din_s + k_in) - (M_ss + d_ss) : du;
-      bwd += c * bw * (corner ? 1.0 / ((double)nd + (double)B) : inv_u);
-      // changed non-corner cells (r,u) (s,u) (u,r) (u,s); corner cells are terms 0-3 below
-      co_c = corner ? 0 : co;
-      ci_c = corner ? 0 : ci;
-      T += (co_c ? 2LL * (M_ru + M_su) : 0LL) + (ci_c ? 2LL * (M_ur + M_us) : 0LL);
+  for (int i = lane; i < n; i += kWarp) {
+    int u, co, ci, du, M_ru, M_ur;
+    if (pre && i < kWarp) {
+      u = pre->u;
+      co = pre->co;
+      ci = pre->ci;
+      M_ru = pre->M_ru;
+      M_ur = pre->M_ur;
+      du = pre->du;
+    } else {
+      const int h = t.list[i];
+      u = t.keys[h];
+      co = t.cout[h];
+      ci = t.cin[h];
+      M_ru = bm_get<ST>(bm, r, u);
+      M_ur = bm_getT<ST>(bm, r, u);
+      du = ldi<ST>(bm.d + u);
     }
-    const unsigned m_out = __ballot_sync(kFull, co_c != 0), m_in = __ballot_sync(kFull, ci_c != 0);
-    const int n_out = __popc(m_out), n_terms_cells = 2 * (n_out + __popc(m_in));
-    const int extra = base == 0 ? 8 : 0;   // corner-cell and degree terms, once
-    const int n_terms = extra + n_terms_cells;
-    for (int q0 = 0; q0 < n_terms; q0 += kWarp) {
-      const int q = q0 + lane;
-      const int cell = q - extra;
-      const int pair = cell >> 1;
-      const bool is_cell = q >= extra && q < n_terms;
-      const bool out_pair = pair < n_out;
-      const int owner = !is_cell ? lane : out_pair ? nth_set_bit(m_out, pair) : nth_set_bit(m_in, pair - n_out);
-      const int x_ru = __shfl_sync(kFull, M_ru, owner), x_su = __shfl_sync(kFull, M_su, owner);
-      const int x_ur = __shfl_sync(kFull, M_ur, owner), x_us = __shfl_sync(kFull, M_us, owner);
-      const int x_co = __shfl_sync(kFull, co_c, owner), x_ci = __shfl_sync(kFull, ci_c, owner);
-      int a = 0, d = 0;
-      double sign = 1.0;
-      if (is_cell) {
-        const bool s_side = cell & 1;
-        a = out_pair ? (s_side ? x_su : x_ru) : (s_side ? x_us : x_ur);
-        const int m = out_pair ? x_co : x_ci;
-        d = s_side ? m : -m;
-      } else if (q < extra) {
-        // corner cells (r,r) (r,s) (s,r) (s,s), then the out- and in-degrees of r and s
-        a = q == 0 ? M_rr : q == 1 ? M_rs : q == 2 ? M_sr : q == 3 ? M_ss
-          : q == 4 ? dout_r : q == 5 ? dout_s : q == 6 ? din_r : din_s;
-        d = q == 0 ? d_rr : q == 1 ? d_rs : q == 2 ? d_sr : q == 3 ? d_ss
-          : q == 4 ? -k_out : q == 5 ? k_out : q == 6 ? -kin_self : kin_self;
-        sign = q < 4 ? 1.0 : -1.0;
-      }
-      if (d) dS += sign * dxlogx_int(bm.logt, a, a + d);
+    const int M_su = bm_get<ST>(bm, s, u), M_us = bm_getT<ST>(bm, s, u);
+    const bool is_r = (u == r), is_s = (u == s);
+    const double c = (double)(co + ci + (is_r ? self : 0));
+    double inv = 1.0 / ((double)du + (double)B);   // a non-corner block's degree is unchanged
+    fwd += c * (M_su + M_us + 1.0) * inv;
+    if (is_r || is_s) {
+      const int nd = is_r ? (dout_r - k_out) + (din_r - k_in) - (M_rr + d_rr)
+                          : (dout_s + k_out) + (din_s + k_in) - (M_ss + d_ss);
+      const double bw = is_r ? (double)(M_rr + d_rr) + (double)(M_rr + d_rr) + 1.0
+                             : (double)(M_rs + d_rs) + (double)(M_sr + d_sr) + 1.0;
+      bwd += c * bw * (1.0 / ((double)nd + (double)B));
+    } else {   // changed non-corner cells (r,u) (s,u) (u,r) (u,s); the corner cells are added below
+      bwd += c * ((double)(M_ru - co) + (double)(M_ur - ci) + 1.0) * inv;
+      if (co) dS += dxlogx_int(bm.xlogxt, M_ru, M_ru - co) + dxlogx_int(bm.xlogxt, M_su, M_su + co);
+      if (ci) dS += dxlogx_int(bm.xlogxt, M_ur, M_ur - ci) + dxlogx_int(bm.xlogxt, M_us, M_us + ci);
     }
   }
-  if (lane < 8) {
-    const int ca = lane == 0 ? M_rr : lane == 1 ? M_rs : lane == 2 ? M_sr : lane == 3 ? M_ss
-                 : lane == 4 ? dout_r : lane == 5 ? dout_s : lane == 6 ? din_r : din_s;
-    const int cd = lane == 0 ? d_rr : lane == 1 ? d_rs : lane == 2 ? d_sr : lane == 3 ? d_ss
-                 : lane == 4 ? -k_out : lane == 5 ? k_out : lane == 6 ? -kin_self : kin_self;
-    T += lane < 4 ? (cd ? 2LL * ca + cd : 0LL) : 2LL * ca;
+  if (lane < 8) {   // corner cells (r,r) (r,s) (s,r) (s,s), then the out- and in-degrees of r and s
+    const int a = lane == 0 ? M_rr : lane == 1 ? M_rs : lane == 2 ? M_sr : lane == 3 ? M_ss
+                : lane == 4 ? dout_r : lane == 5 ? dout_s : lane == 6 ? din_r : din_s;
+    const int d = lane == 0 ? d_rr : lane == 1 ? d_rs : lane == 2 ? d_sr : lane == 3 ? d_ss
+                : lane == 4 ? -k_out : lane == 5 ? k_out : lane == 6 ? -kin_self : kin_self;
+    if (d) {
+      const double x = dxlogx_int(bm.xlogxt, a, a + d);
+      dS += lane < 4 ? x : -x;
+    }
   }
   {
     // the double count of a present net-zero (r,s) / (s,r) Delta cell (lanes 8 and 9)
@@ -782,11 +733,28 @@ __device__ __forceinline__ double move_delta(const GraphView& g, const BlockView
   fwd = warp_sum(fwd);
   bwd = warp_sum(bwd);
   dS = warp_sum(dS);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) T += __shfl_xor_sync(kFull, T, o);
   // A mathematically zero change reads as exactly 0 whatever the summation order: the
-  // Metropolis-Hastings early stop tests `delta == 0.0` (src/finetune.cpp:147).
-  if (fabs(dS) <= 0x1p-40 * (double)T * g.log_E) dS = 0.0;
+  // Metropolis-Hastings early stop tests `delta == 0.0` (src/finetune.cpp:147).  T, the integer
+  // scale of the snap, takes a second pass over the cells and is formed only when it can matter.
+  if (maybe_zero_delta(dS, dout_r, dout_s, din_r, din_s, k_out + k_in, g.log_E)) {   // warp-uniform
+    long long T = 0;
+    for (int i = lane; i < n; i += kWarp) {
+      const int h = t.list[i];
+      const int u = t.keys[h];
+      if (u == r || u == s) continue;
+      if (t.cout[h]) T += 2LL * (bm_get<ST>(bm, r, u) + bm_get<ST>(bm, s, u));
+      if (t.cin[h]) T += 2LL * (bm_getT<ST>(bm, r, u) + bm_getT<ST>(bm, s, u));
+    }
+    if (lane < 8) {
+      const int a = lane == 0 ? M_rr : lane == 1 ? M_rs : lane == 2 ? M_sr : lane == 3 ? M_ss
+                  : lane == 4 ? dout_r : lane == 5 ? dout_s : lane == 6 ? din_r : din_s;
+      const int d = lane == 0 ? d_rr : lane == 1 ? d_rs : lane == 2 ? d_sr : lane == 3 ? d_ss : 0;
+      T += lane < 4 ? (d ? 2LL * a + d : 0LL) : 2LL * a;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) T += __shfl_xor_sync(kFull, T, o);
+    if (fabs(dS) <= 0x1p-40 * (double)T * g.log_E) dS = 0.0;
+  }
   *H = bwd / fwd;
   return dS;
 }

@@ -242,28 +242,9 @@ struct DevBuf {
 // ------------------------------------------------------------------------------------------
 // Process-wide context: one stream, the device status word, counters and readback buffers.
 // ------------------------------------------------------------------------------------------
-// log(x) for the integers 1 <= x < kLogTable as a pair of doubles (hi = log x rounded, lo = the
-// rest), from the host's long-double log (64-bit mantissa): the vertex-move delta-MDL takes
-// g(a) - g(b), g(x) = x log x, of integer counts from it (dxlogx_int in sbp_device.cuh).
-inline double2* make_log_table() {
-  std::vector<double2> h(kLogTable);
-  h[0] = make_double2(0.0, 0.0);
-  const int nt = 8;
-  std::vector<std::thread> th;
-  for (int t = 0; t < nt; ++t)
-    th.emplace_back([&h, t, nt] {
-      for (int x = 1 + t; x < kLogTable; x += nt) {
-        const long double l = logl((long double)x);
-        const double hi = (double)l;
-        h[x] = make_double2(hi, (double)(l - (long double)hi));
-      }
-    });
-  for (auto& t : th) t.join();
-  double2* d = nullptr;
-  SBP_CUDA(cudaMalloc(&d, sizeof(double2) * kLogTable));
-  SBP_CUDA(cudaMemcpy(d, h.data(), sizeof(double2) * kLogTable, cudaMemcpyHostToDevice));
-  return d;
-}
+// x log x of the integers 0 <= x < kXlogxTable as a pair of doubles (dxlogx_int), computed on the
+// device in double-double arithmetic (k_xlogx_table).
+double2* make_xlogx_table(cudaStream_t stream);
 
 struct Context {
   cudaStream_t stream = nullptr;
@@ -274,12 +255,12 @@ struct Context {
   double* scalar = nullptr;              // MDL result
   double* mh_out = nullptr;              // MH sweep outputs [4]
   unsigned* done = nullptr;              // CTAs finished in the current k_mdl launch (0 between launches)
-  double2* logt = nullptr;               // [kLogTable] log(x) as hi + lo doubles (entry 0 unused)
+  double2* xlogxt = nullptr;             // [kXlogxTable] x log x as hi + lo doubles
   int npartial = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
-  // A context: its own stream and scratch; the log table is shared when given.
-  static Context* create(double2* logt) {
+  // A context: its own stream and scratch; the x log x table is shared when given.
+  static Context* create(double2* xlogxt) {
     auto* c = new Context();
     SBP_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     int dev = 0;
@@ -296,7 +277,7 @@ struct Context {
     SBP_CUDA(cudaMemset(c->done, 0, sizeof(unsigned)));
     SBP_CUDA(cudaEventCreate(&c->ev0));
     SBP_CUDA(cudaEventCreate(&c->ev1));
-    c->logt = logt ? logt : make_log_table();
+    c->xlogxt = xlogxt ? xlogxt : make_xlogx_table(c->stream);
     return c;
   }
   // The process's context: every entry point runs on it.
@@ -316,7 +297,7 @@ struct Context {
   // partitioner's merges while its sweep kernel runs).
   static Context& secondary() {
     static Context* ctx = nullptr;
-    if (!ctx) ctx = create(primary().logt);
+    if (!ctx) ctx = create(primary().xlogxt);
     return *ctx;
   }
   // The calling thread's current context: the primary one unless a ContextScope is open.
@@ -586,7 +567,7 @@ struct SbpBlockmodel {
     v.d_out = d_out.p;
     v.d_in = d_in.p;
     v.d = d.p;
-    v.logt = Context::get().logt;
+    v.xlogxt = Context::get().xlogxt;
     return v;
   }
 

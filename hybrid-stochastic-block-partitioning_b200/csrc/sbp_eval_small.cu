@@ -318,7 +318,6 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
   const bool active = valid && s != r;
   // 3. delta-MDL and the Hastings correction of the move r -> s
   double fwd = 0.0, bwd = 0.0, dS = 0.0;
-  long long Tz = 0;
   int co_r = 0, ci_r = 0, co_s = 0, ci_s = 0;
   int M_rr = 0, M_rs = 0, M_sr = 0, M_ss = 0, dout_r = 0, dout_s = 0, din_r = 0, din_s = 0;
   if (active) {
@@ -367,12 +366,10 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       bwd += c * bw * (corner ? 1.0 / ((double)nd + (double)B) : inv_u);
       if (!corner) {   // cells (r,u) (s,u) for out-edges to u, (u,r) (u,s) for in-edges
         if (co) {
-          dS += dxlogx_int(bm.logt, M_ru, M_ru - co) + dxlogx_int(bm.logt, M_su, M_su + co);
-          Tz += 2LL * (M_ru + M_su);
+          dS += dxlogx_int(bm.xlogxt, M_ru, M_ru - co) + dxlogx_int(bm.xlogxt, M_su, M_su + co);
         }
         if (ci) {
-          dS += dxlogx_int(bm.logt, M_ur, M_ur - ci) + dxlogx_int(bm.logt, M_us, M_us + ci);
-          Tz += 2LL * (M_ur + M_us);
+          dS += dxlogx_int(bm.xlogxt, M_ur, M_ur - ci) + dxlogx_int(bm.xlogxt, M_us, M_us + ci);
         }
       }
     }
@@ -384,8 +381,7 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
                   : q == 4 ? dout_r : q == 5 ? dout_s : q == 6 ? din_r : din_s;
       const int d = q == 0 ? d_rr : q == 1 ? d_rs : q == 2 ? d_sr : q == 3 ? d_ss
                   : q == 4 ? -k_out : q == 5 ? k_out : q == 6 ? -kin_self : kin_self;
-      if (d) dS += (q < 4 ? 1.0 : -1.0) * dxlogx_int(bm.logt, a, a + d);
-      Tz += q < 4 ? (d ? 2LL * a + d : 0LL) : 2LL * a;
+      if (d) dS += (q < 4 ? 1.0 : -1.0) * dxlogx_int(bm.xlogxt, a, a + d);
     }
     // the double count of a present net-zero (r,s) / (s,r) Delta cell
     if (gl == 0 && (co_s > 0 || ci_r > 0) && d_rs == 0 && M_rs > 0)
@@ -396,9 +392,29 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
   fwd = group_sum<G>(fwd);
   bwd = group_sum<G>(bwd);
   dS = group_sum<G>(dS);
-  Tz = group_sum_ll<G>(Tz);
+  const bool snap = active && maybe_zero_delta(dS, dout_r, dout_s, din_r, din_s, k, g.log_E);
+  if (__any_sync(kFull, snap)) {   // the integer scale of the zero snap, as in move_delta
+    long long Tz = 0;
+    if (snap) {
+      for (int j = gl; j < nent; j += G) {
+        const int slot = T.list[j];
+        const int u = T.key_of(slot);
+        const unsigned wu = T.w[slot];
+        if (u == r || u == s) continue;
+        if (wu & kCountMask) Tz += 2LL * (bm.M[(size_t)r * ld + u] + bm.M[(size_t)s * ld + u]);
+        if ((wu >> kInShift) & kCountMask) Tz += 2LL * (bm.MT[(size_t)r * ld + u] + bm.MT[(size_t)s * ld + u]);
+      }
+      for (int q = gl; q < 8; q += G) {
+        const int a = q == 0 ? M_rr : q == 1 ? M_rs : q == 2 ? M_sr : q == 3 ? M_ss
+                    : q == 4 ? dout_r : q == 5 ? dout_s : q == 6 ? din_r : din_s;
+        const int d = q == 0 ? d_rr : q == 1 ? d_rs : q == 2 ? d_sr : q == 3 ? d_ss : 0;
+        Tz += q < 4 ? (d ? 2LL * a + d : 0LL) : 2LL * a;
+      }
+    }
+    Tz = group_sum_ll<G>(Tz);
+    if (snap && fabs(dS) <= 0x1p-40 * (double)Tz * g.log_E) dS = 0.0;
+  }
   if (active) {
-    if (fabs(dS) <= 0x1p-40 * (double)Tz * g.log_E) dS = 0.0;
     const double H = (k == 0) ? 1.0 : bwd / fwd;
     double ap = exp(-3.0 * dS) * H;
     ap = ap >= 1.0 ? 1.0 : ap;
