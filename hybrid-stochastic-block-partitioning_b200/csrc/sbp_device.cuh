@@ -155,7 +155,7 @@ constexpr int kChunk = 128;   // columns per chunk-sum entry
 
 struct BlockView {
   int B;
-  int sparse;             // 0: dense M/MT below; 1: row-hashed regions (large B)
+  int sparse;             // 0: dense pairs below; 1: row-hashed regions (large B)
   // row-hashed storage: row r of M lives in rslot[rbase[r] .. rbase[r] + rmask[r]], slots
   // (col, count), col = -1 for an empty slot; MT likewise in cslot.  Keys are never removed
   // (a count can drop to 0).  An insertion that finds its row full sets overflow[0] and the
@@ -167,37 +167,21 @@ struct BlockView {
   const int* cmask;
   int2* cslot;
   int* overflow;
-  int ld;                 // row stride of M and MT (multiple of kChunk ints)
+  int ld;                 // row stride of P (multiple of kChunk pairs)
   int nch;                // chunks per row = ceil(B / kChunk)
-  int* CS;                // [B*nch] CS[row*nch+c] = sum of M[row, c*kChunk .. c*kChunk+kChunk)
-  int* CST;               // [B*nch] the same over MT (column sums of M per chunk of rows)
+  int* CS;                // [B*nch] CS[row*nch+c] = sum of M[row, c*kChunk .. c*kChunk+kChunk); kept when nch > 1
+  int* CST;               // [B*nch] the same over the columns of M (chunks of rows)
   int* b;                 // [V] assignment
-  int* M;                 // [B*ld] row-major counts M[row*ld+col]
-  int* MT;                // [B*ld] transpose: MT[col*ld+row] = M[row*ld+col]
+  // [B*ld] counts of both directions side by side: P[row*ld+col] = (M[row, col], M[col, row]).
+  // A visit needs M[r,u] with M[u,r] and M[s,u] with M[u,s]: one 8-byte load and one 32-byte
+  // sector each, where M and a separate transpose took two (200,000 vertices, 11,770 blocks: see
+  // the evaluation kernels); the walk gets row t and column t from the same lines.
+  int2* P;
   int* d_out;             // [B]
   int* d_in;              // [B]
   int* d;                 // [B] block degrees as the reference maintains them
   const double2* xlogxt;  // [kXlogxTable] x log x = hi + lo for integer x
 };
-
-// Walk values row[0..n) ascending and return the first index whose running sum exceeds
-// `target` (skipping index `skip`). Warp-cooperative; returns -1 if the row is exhausted.
-// Plain (coherent) loads: the Metropolis-Hastings kernel updates M while it runs.
-__device__ __forceinline__ int warp_select_dense(const int* row, int n, long long target, int skip,
-                                                 int lane) {
-  for (int base = 0; base < n; base += kWarp) {
-    const int c = base + lane;
-    long long v = (c < n && c != skip) ? (long long)row[c] : 0;
-    const long long incl = warp_incl_scan(v, lane);
-    const long long tot = __shfl_sync(kFull, incl, 31);
-    if (target < tot) {
-      const unsigned hit = __ballot_sync(kFull, incl > target);
-      return base + __ffs(hit) - 1;
-    }
-    target -= tot;
-  }
-  return -1;
-}
 
 // ---- row-hashed storage ------------------------------------------------------------------
 __device__ __forceinline__ unsigned slot_hash(int key) { return (unsigned)key * 2654435761u; }
@@ -248,20 +232,38 @@ __device__ __forceinline__ int ldi(const int* p) {
   if constexpr (S == Store::kDenseFrozen) return __ldg(p);
   else return *p;
 }
+template <Store S, class T>
+__device__ __forceinline__ T ldv(const T* p) {
+  if constexpr (S == Store::kDenseFrozen) return __ldg(p);
+  else return *p;
+}
 
+// (M[row, col], M[col, row])
+template <Store S = Store::kAny>
+__device__ __forceinline__ int2 bm_pair(const BlockView& bm, int row, int col) {
+  const bool hashed = S == Store::kHashed || (S == Store::kAny && bm.sparse);
+  if constexpr (S != Store::kDense && S != Store::kDenseFrozen) {
+    if (hashed)
+      return make_int2(hashed_get(bm.rbase, bm.rmask, bm.rslot, row, col),
+                       hashed_get(bm.cbase, bm.cmask, bm.cslot, row, col));
+  }
+  if constexpr (S != Store::kHashed) return ldv<S>(bm.P + (size_t)row * bm.ld + col);
+  return make_int2(0, 0);
+}
+// M[row, col]
 template <Store S = Store::kAny>
 __device__ __forceinline__ int bm_get(const BlockView& bm, int row, int col) {
-  if constexpr (S == Store::kDense) return bm.M[(size_t)row * bm.ld + col];
-  else if constexpr (S == Store::kDenseFrozen) return __ldg(bm.M + (size_t)row * bm.ld + col);
+  if constexpr (S == Store::kDense || S == Store::kDenseFrozen) return ldi<S>(&bm.P[(size_t)row * bm.ld + col].x);
   else if constexpr (S == Store::kHashed) return hashed_get(bm.rbase, bm.rmask, bm.rslot, row, col);
-  else return bm.sparse ? hashed_get(bm.rbase, bm.rmask, bm.rslot, row, col) : bm.M[(size_t)row * bm.ld + col];
+  else return bm.sparse ? hashed_get(bm.rbase, bm.rmask, bm.rslot, row, col) : bm.P[(size_t)row * bm.ld + col].x;
 }
+
+// M[col, row]
 template <Store S = Store::kAny>
 __device__ __forceinline__ int bm_getT(const BlockView& bm, int row, int col) {
-  if constexpr (S == Store::kDense) return bm.MT[(size_t)row * bm.ld + col];
-  else if constexpr (S == Store::kDenseFrozen) return __ldg(bm.MT + (size_t)row * bm.ld + col);
+  if constexpr (S == Store::kDense || S == Store::kDenseFrozen) return ldi<S>(&bm.P[(size_t)row * bm.ld + col].y);
   else if constexpr (S == Store::kHashed) return hashed_get(bm.cbase, bm.cmask, bm.cslot, row, col);
-  else return bm.sparse ? hashed_get(bm.cbase, bm.cmask, bm.cslot, row, col) : bm.MT[(size_t)row * bm.ld + col];
+  else return bm.sparse ? hashed_get(bm.cbase, bm.cmask, bm.cslot, row, col) : bm.P[(size_t)row * bm.ld + col].y;
 }
 
 // Walk of a hashed row in ascending column order: the first column whose running count
@@ -299,74 +301,73 @@ __device__ __forceinline__ int warp_select_hashed(const long long* base, const i
 
 __device__ __forceinline__ int select_in_chunk(int4 q, int chunk, long long target, int lane);
 
-// Two-level walk: find the chunk through the chunk sums, then the column inside the chunk
-// with one 16-byte load per lane.  Same result as warp_select_dense on the full row.  Up to
-// kWideChunks chunks, lane i loads the sums of chunks [16 i, 16 i + 16) at once (one memory
-// round trip instead of one per 32 chunks), scans its lane total across the warp and walks its
-// sixteen sums; longer rows take 32 chunks per step.
-constexpr int kWideChunks = 16 * kWarp;
-// The wide walk over chunk sums already loaded: lane i holds the sums of chunks [16 i, 16 i + 16)
-// (0 beyond the row).
-__device__ __forceinline__ int walk_loaded_chunk_sums(const int* row, const int (&cs)[16], long long target,
-                                                      int lane) {
-  long long lsum = 0;
-#pragma unroll
-  for (int q = 0; q < 16; ++q) lsum += cs[q];
-  const long long incl = warp_incl_scan(lsum, lane);
-  const unsigned hit = __ballot_sync(kFull, incl > target);
-  if (!hit) return -1;
-  const int src = __ffs(hit) - 1;
-  int chunk = -1;
-  long long before = 0;
-  if (lane == src) {
-    long long run = incl - lsum;
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      if (chunk < 0) {
-        if (target < run + cs[q]) {
-          chunk = lane * 16 + q;
-          before = run;
-        } else {
-          run += cs[q];
-        }
-      }
-    }
-  }
-  chunk = __shfl_sync(kFull, chunk, src);
-  before = __shfl_sync(kFull, before, src);
-  const int4 q4 = *reinterpret_cast<const int4*>(row + chunk * kChunk + 4 * lane);
-  return select_in_chunk(q4, chunk, target - before, lane);
+// Four counts from column c0 (a multiple of 4) of a row of pairs: M[row, .], or M[., row] when `col`.
+template <Store S>
+__device__ __forceinline__ int4 load_four(const int2* row, int c0, bool col) {
+  const int4 a = ldv<S>(reinterpret_cast<const int4*>(row + c0));
+  const int4 b = ldv<S>(reinterpret_cast<const int4*>(row + c0 + 2));
+  return col ? make_int4(a.y, a.w, b.y, b.w) : make_int4(a.x, a.z, b.x, b.z);
 }
 
-__device__ __forceinline__ int warp_select_chunked(const int* row, const int* csum, int nch, long long target,
-                                                   int lane) {
+// Two-level walk over row t of M (or column t when `col`): the first index whose running count
+// exceeds `target`, -1 if the row is exhausted.  The chunk is found through the chunk sums, then
+// the column inside the chunk, four counts per lane.  Up to kWideChunks chunks, lane i loads the
+// sums of chunks [16 i, 16 i + 16) at once (one memory round trip instead of one per 32
+// chunks), scans its lane total across the warp and walks its sixteen sums; longer rows take 32
+// chunks per step.
+constexpr int kWideChunks = 16 * kWarp;
+template <Store S>
+__device__ __forceinline__ int warp_select_chunked(const int2* row, bool col, const int* csum, int nch,
+                                                   long long target, int lane) {
+  int chunk = -1;
   if (nch <= kWideChunks) {
     int cs[16];
+    long long lsum = 0;
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
       const int c = lane * 16 + q;
-      cs[q] = c < nch ? csum[c] : 0;
+      cs[q] = c < nch ? ldi<S>(csum + c) : 0;
+      lsum += cs[q];
     }
-    return walk_loaded_chunk_sums(row, cs, target, lane);
-  }
-  int chunk = -1;
-  for (int base = 0; base < nch; base += kWarp) {
-    const int c = base + lane;
-    const long long v = c < nch ? (long long)csum[c] : 0;
-    const long long incl = warp_incl_scan(v, lane);
-    const long long tot = __shfl_sync(kFull, incl, 31);
-    if (target < tot) {
-      const unsigned hit = __ballot_sync(kFull, incl > target);
-      const int src = __ffs(hit) - 1;
-      target -= __shfl_sync(kFull, incl - v, src);
-      chunk = base + src;
-      break;
+    const long long incl = warp_incl_scan(lsum, lane);
+    const unsigned hit = __ballot_sync(kFull, incl > target);
+    if (!hit) return -1;
+    const int src = __ffs(hit) - 1;
+    long long before = 0;
+    if (lane == src) {
+      long long run = incl - lsum;
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        if (chunk < 0) {
+          if (target < run + cs[q]) {
+            chunk = lane * 16 + q;
+            before = run;
+          } else {
+            run += cs[q];
+          }
+        }
+      }
     }
-    target -= tot;
+    chunk = __shfl_sync(kFull, chunk, src);
+    target -= __shfl_sync(kFull, before, src);
+  } else {
+    for (int base = 0; base < nch; base += kWarp) {
+      const int c = base + lane;
+      const long long v = c < nch ? (long long)ldi<S>(csum + c) : 0;
+      const long long incl = warp_incl_scan(v, lane);
+      const long long tot = __shfl_sync(kFull, incl, 31);
+      if (target < tot) {
+        const unsigned hit = __ballot_sync(kFull, incl > target);
+        const int src = __ffs(hit) - 1;
+        target -= __shfl_sync(kFull, incl - v, src);
+        chunk = base + src;
+        break;
+      }
+      target -= tot;
+    }
+    if (chunk < 0) return -1;
   }
-  if (chunk < 0) return -1;
-  const int4 q = *reinterpret_cast<const int4*>(row + chunk * kChunk + 4 * lane);
-  return select_in_chunk(q, chunk, target, lane);
+  return select_in_chunk(load_four<S>(row, chunk * kChunk + 4 * lane, col), chunk, target, lane);
 }
 
 // The column inside one chunk of kChunk counts (four per lane, q) at which the running sum
@@ -388,7 +389,9 @@ __device__ __forceinline__ int select_in_chunk(int4 q, int chunk, long long targ
 
 // The walk of warp_select_chunked for a row of at most 32 chunks whose chunk sums are already
 // loaded (lane c holds chunk c's sum, 0 beyond the row).
-__device__ __forceinline__ int select_chunk_then_column(const int* row, int csum_lane, long long target, int lane) {
+template <Store S>
+__device__ __forceinline__ int select_chunk_then_column(const int2* row, bool col, int csum_lane, long long target,
+                                                        int lane) {
   const long long v = csum_lane;
   const long long incl = warp_incl_scan(v, lane);
   const long long tot = __shfl_sync(kFull, incl, 31);
@@ -396,12 +399,15 @@ __device__ __forceinline__ int select_chunk_then_column(const int* row, int csum
   const unsigned hit = __ballot_sync(kFull, incl > target);
   const int src = __ffs(hit) - 1;
   target -= __shfl_sync(kFull, incl - v, src);
-  const int4 q = *reinterpret_cast<const int4*>(row + src * kChunk + 4 * lane);
-  return select_in_chunk(q, src, target, lane);
+  return select_in_chunk(load_four<S>(row, src * kChunk + 4 * lane, col), src, target, lane);
 }
 
-__device__ __forceinline__ void chunk_add(int* cs, int nch, int row, int col, int delta) {
-  atomicAdd(cs + (size_t)row * nch + col / kChunk, delta);
+// The chunk sums of cell (row, col): not kept with one chunk per row, where the walks read the
+// row itself.
+__device__ __forceinline__ void chunks_add(const BlockView& bm, int row, int col, int delta) {
+  if (bm.nch == 1) return;
+  atomicAdd(bm.CS + (size_t)row * bm.nch + col / kChunk, delta);
+  atomicAdd(bm.CST + (size_t)col * bm.nch + row / kChunk, delta);
 }
 
 // Same walk over a compressed list (idx[i], val[i]), i in [0, n).
@@ -628,8 +634,9 @@ __device__ __forceinline__ void prefetch_nb(const BlockView& bm, int r, const Wa
     p->u = u;
     p->co = t.cout[h];
     p->ci = t.cin[h];
-    p->M_ru = bm_get<ST>(bm, r, u);
-    p->M_ur = bm_getT<ST>(bm, r, u);
+    const int2 m = bm_pair<ST>(bm, r, u);
+    p->M_ru = m.x;
+    p->M_ur = m.y;
     p->du = ldi<ST>(bm.d + u);
   }
   p->M_rr = bm_get<ST>(bm, r, r);
@@ -666,8 +673,9 @@ __device__ __forceinline__ double move_delta(const GraphView& g, const BlockView
   const int d_rs = -mc.co_s + mc.ci_r;
   const int d_sr = mc.co_r - mc.ci_s;
   const int d_ss = mc.co_s + mc.ci_s + self;
-  const int M_rr = pre ? pre->M_rr : bm_get<ST>(bm, r, r), M_rs = bm_get<ST>(bm, r, s);
-  const int M_sr = bm_get<ST>(bm, s, r), M_ss = bm_get<ST>(bm, s, s);
+  const int2 m_rs = bm_pair<ST>(bm, r, s);
+  const int M_rr = pre ? pre->M_rr : bm_get<ST>(bm, r, r), M_rs = m_rs.x;
+  const int M_sr = m_rs.y, M_ss = bm_get<ST>(bm, s, s);
   const int dout_r = pre ? pre->dout_r : ldi<ST>(bm.d_out + r), dout_s = ldi<ST>(bm.d_out + s);
   const int din_r = pre ? pre->din_r : ldi<ST>(bm.d_in + r), din_s = ldi<ST>(bm.d_in + s);
   const int kin_self = k_in + self;
@@ -688,11 +696,13 @@ __device__ __forceinline__ double move_delta(const GraphView& g, const BlockView
       u = t.keys[h];
       co = t.cout[h];
       ci = t.cin[h];
-      M_ru = bm_get<ST>(bm, r, u);
-      M_ur = bm_getT<ST>(bm, r, u);
+      const int2 m = bm_pair<ST>(bm, r, u);
+      M_ru = m.x;
+      M_ur = m.y;
       du = ldi<ST>(bm.d + u);
     }
-    const int M_su = bm_get<ST>(bm, s, u), M_us = bm_getT<ST>(bm, s, u);
+    const int2 m_su = bm_pair<ST>(bm, s, u);
+    const int M_su = m_su.x, M_us = m_su.y;
     const bool is_r = (u == r), is_s = (u == s);
     const double c = (double)(co + ci + (is_r ? self : 0));
     double inv = 1.0 / ((double)du + (double)B);   // a non-corner block's degree is unchanged
@@ -742,8 +752,8 @@ __device__ __forceinline__ double move_delta(const GraphView& g, const BlockView
       const int h = t.list[i];
       const int u = t.keys[h];
       if (u == r || u == s) continue;
-      if (t.cout[h]) T += 2LL * (bm_get<ST>(bm, r, u) + bm_get<ST>(bm, s, u));
-      if (t.cin[h]) T += 2LL * (bm_getT<ST>(bm, r, u) + bm_getT<ST>(bm, s, u));
+      const int2 a = bm_pair<ST>(bm, r, u), b = bm_pair<ST>(bm, s, u);
+      T += (t.cout[h] ? 2LL * (a.x + b.x) : 0LL) + (t.cin[h] ? 2LL * (a.y + b.y) : 0LL);
     }
     if (lane < 8) {
       const int a = lane == 0 ? M_rr : lane == 1 ? M_rs : lane == 2 ? M_sr : lane == 3 ? M_ss
@@ -809,33 +819,30 @@ __device__ __forceinline__ EvalResult evaluate_vertex(const GraphView& g, const 
       if (target < dot) s = warp_select_hashed(bm.rbase, bm.rmask, bm.rslot, tblk, bm.B, target, lane, bins);
       else s = warp_select_hashed(bm.cbase, bm.cmask, bm.cslot, tblk, bm.B, target - dot, lane, bins);
     } else if (ST != Store::kHashed) {
-      // the degrees of t and, in the same round trip, row t of M and of MT (B <= kChunk: the
-      // whole rows, four counts per lane) or their chunk sums (up to 32 chunks); the walk then
-      // picks the row (target < d_out[t]) or the column.  (Loading the chunk sums of
-      // both rows with the degrees for up to 512 chunks as well was measured 13 % slower at
-      // 11,770 blocks and no faster above.)
+      // the degrees of t and, in the same round trip, its row and column (B <= kChunk: the whole
+      // row of pairs, four per lane) or their chunk sums (up to 32 chunks); the walk then picks
+      // the row (target < d_out[t]) or the column.  (Loading the chunk sums of both with the
+      // degrees for up to 512 chunks as well was measured 13 % slower at 11,770 blocks and no
+      // faster above.)
       const int dot = ldi<ST>(bm.d_out + tblk), dit = ldi<ST>(bm.d_in + tblk);
-      const size_t ro = (size_t)tblk * bm.ld, co = (size_t)tblk * bm.nch;
+      const int2* row = bm.P + (size_t)tblk * bm.ld;
+      const size_t co = (size_t)tblk * bm.nch;
       int4 qa = make_int4(0, 0, 0, 0), qb = make_int4(0, 0, 0, 0);
       int ca = 0, cb = 0;
       if (bm.nch == 1) {
-        if constexpr (ST == Store::kDenseFrozen) {
-          qa = __ldg(reinterpret_cast<const int4*>(bm.M + ro) + lane);
-          qb = __ldg(reinterpret_cast<const int4*>(bm.MT + ro) + lane);
-        } else {
-          qa = *reinterpret_cast<const int4*>(bm.M + ro + 4 * lane);
-          qb = *reinterpret_cast<const int4*>(bm.MT + ro + 4 * lane);
-        }
+        qa = ldv<ST>(reinterpret_cast<const int4*>(row + 4 * lane));
+        qb = ldv<ST>(reinterpret_cast<const int4*>(row + 4 * lane + 2));
       } else if (lane < bm.nch) {
         ca = ldi<ST>(bm.CS + co + lane);
         cb = ldi<ST>(bm.CST + co + lane);
       }
       const long long target = scale32(x.y, (long long)dot + (long long)dit);
-      const bool in_row = target < dot;
-      const long long tg = in_row ? target : target - dot;
-      if (bm.nch == 1) s = select_in_chunk(in_row ? qa : qb, 0, tg, lane);
-      else if (bm.nch <= kWarp) s = select_chunk_then_column(in_row ? bm.M + ro : bm.MT + ro, in_row ? ca : cb, tg, lane);
-      else s = warp_select_chunked(in_row ? bm.M + ro : bm.MT + ro, in_row ? bm.CS + co : bm.CST + co, bm.nch, tg, lane);
+      const bool in_col = target >= dot;
+      const long long tg = in_col ? target - dot : target;
+      if (bm.nch == 1)
+        s = select_in_chunk(in_col ? make_int4(qa.y, qa.w, qb.y, qb.w) : make_int4(qa.x, qa.z, qb.x, qb.z), 0, tg, lane);
+      else if (bm.nch <= kWarp) s = select_chunk_then_column<ST>(row, in_col, in_col ? cb : ca, tg, lane);
+      else s = warp_select_chunked<ST>(row, in_col, in_col ? bm.CST + co : bm.CS + co, bm.nch, tg, lane);
     } else {
       s = -1;
     }

@@ -205,10 +205,11 @@ void rebuild(SbpBlockmodel& bm, const SbpGraph& g, bool recompute_d) {
   }
   Context& c = Context::get();
   const size_t cells = (size_t)bm.B * (size_t)bm.ld;
-  SBP_CUDA(cudaMemsetAsync(bm.M.p, 0, cells * sizeof(int), c.stream));
-  SBP_CUDA(cudaMemsetAsync(bm.MT.p, 0, cells * sizeof(int), c.stream));
-  SBP_CUDA(cudaMemsetAsync(bm.CS.p, 0, (size_t)bm.B * bm.nch * sizeof(int), c.stream));
-  SBP_CUDA(cudaMemsetAsync(bm.CST.p, 0, (size_t)bm.B * bm.nch * sizeof(int), c.stream));
+  SBP_CUDA(cudaMemsetAsync(bm.P.p, 0, cells * sizeof(int2), c.stream));
+  if (bm.nch > 1) {
+    SBP_CUDA(cudaMemsetAsync(bm.CS.p, 0, (size_t)bm.B * bm.nch * sizeof(int), c.stream));
+    SBP_CUDA(cudaMemsetAsync(bm.CST.p, 0, (size_t)bm.B * bm.nch * sizeof(int), c.stream));
+  }
   SBP_CUDA(cudaMemsetAsync(bm.d_out.p, 0, bm.B * sizeof(int), c.stream));
   SBP_CUDA(cudaMemsetAsync(bm.d_in.p, 0, bm.B * sizeof(int), c.stream));
   if (g.V > 0) {
@@ -790,14 +791,14 @@ void merge_blocks(SbpBlockmodel& bm, SbpGraph& g, const SbpMergeOptions& opt, co
     rows = Csr{ms.rptr.p, ms.ridx.p, ms.rval.p};
     cols = Csr{ms.cptr.p, ms.cidx.p, ms.cval.p};
   } else {
-  // compressed rows of M and of MT (outgoing_edges / incoming_edges views)
+  // compressed rows and columns of M (outgoing_edges / incoming_edges views)
   ms.rcnt.reserve(B);
   ms.ccnt.reserve(B);
   ms.rptr.reserve(B + 1);
   ms.cptr.reserve(B + 1);
   const int gw = grid_for((long long)B * 32, 256, 64 * c.num_sms);
-  k_row_nnz<<<gw, 256, 0, c.stream>>>(bm.M.p, B, bm.ld, ms.rcnt.p);
-  k_row_nnz<<<gw, 256, 0, c.stream>>>(bm.MT.p, B, bm.ld, ms.ccnt.p);
+  k_row_nnz<<<gw, 256, 0, c.stream>>>(bm.P.p, 0, B, bm.ld, ms.rcnt.p);
+  k_row_nnz<<<gw, 256, 0, c.stream>>>(bm.P.p, 1, B, bm.ld, ms.ccnt.p);
   k_excl_scan<<<1, 1024, 0, c.stream>>>(ms.rcnt.p, ms.rptr.p, B);
   k_excl_scan<<<1, 1024, 0, c.stream>>>(ms.ccnt.p, ms.cptr.p, B);
   SBP_CHECK_LAUNCH();
@@ -808,8 +809,8 @@ void merge_blocks(SbpBlockmodel& bm, SbpGraph& g, const SbpMergeOptions& opt, co
   ms.rval.reserve(nnz[0]);
   ms.cidx.reserve(nnz[1]);
   ms.cval.reserve(nnz[1]);
-  k_row_fill<<<gw, 256, 0, c.stream>>>(bm.M.p, B, bm.ld, ms.rptr.p, ms.ridx.p, ms.rval.p);
-  k_row_fill<<<gw, 256, 0, c.stream>>>(bm.MT.p, B, bm.ld, ms.cptr.p, ms.cidx.p, ms.cval.p);
+  k_row_fill<<<gw, 256, 0, c.stream>>>(bm.P.p, 0, B, bm.ld, ms.rptr.p, ms.ridx.p, ms.rval.p);
+  k_row_fill<<<gw, 256, 0, c.stream>>>(bm.P.p, 1, B, bm.ld, ms.cptr.p, ms.cidx.p, ms.cval.p);
   SBP_CHECK_LAUNCH();
   rows = Csr{ms.rptr.p, ms.ridx.p, ms.rval.p};
   cols = Csr{ms.cptr.p, ms.cidx.p, ms.cval.p};
@@ -1421,12 +1422,13 @@ SbpStatus sbp_blockmodel_copy(const SbpBlockmodel* src, SbpBlockmodel** out) {
   }
   const size_t cells = (size_t)src->B * src->ld;
   SBP_CUDA(SBP_COPY_ASYNC(bm->b.p, src->b.p, src->V * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
-  SBP_CUDA(SBP_COPY_ASYNC(bm->M.p, src->M.p, cells * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
-  SBP_CUDA(SBP_COPY_ASYNC(bm->MT.p, src->MT.p, cells * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
-  SBP_CUDA(SBP_COPY_ASYNC(bm->CS.p, src->CS.p, (size_t)src->B * src->nch * sizeof(int), cudaMemcpyDeviceToDevice,
-                          c.stream));
-  SBP_CUDA(SBP_COPY_ASYNC(bm->CST.p, src->CST.p, (size_t)src->B * src->nch * sizeof(int), cudaMemcpyDeviceToDevice,
-                          c.stream));
+  SBP_CUDA(SBP_COPY_ASYNC(bm->P.p, src->P.p, cells * sizeof(int2), cudaMemcpyDeviceToDevice, c.stream));
+  if (src->nch > 1) {
+    SBP_CUDA(SBP_COPY_ASYNC(bm->CS.p, src->CS.p, (size_t)src->B * src->nch * sizeof(int), cudaMemcpyDeviceToDevice,
+                            c.stream));
+    SBP_CUDA(SBP_COPY_ASYNC(bm->CST.p, src->CST.p, (size_t)src->B * src->nch * sizeof(int), cudaMemcpyDeviceToDevice,
+                            c.stream));
+  }
   SBP_CUDA(SBP_COPY_ASYNC(bm->d_out.p, src->d_out.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->d_in.p, src->d_in.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->d.p, src->d.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
@@ -1477,26 +1479,26 @@ SbpStatus sbp_get_block_matrix(const SbpBlockmodel* bm, int32_t* out) {
   SBP_API_BEGIN
   SBP_REQUIRE(bm && out, "NULL argument");
   Context& c = Context::get();
-  if (bm->sparse) {   // scatter the hashed rows into a dense device band, band by band
-    const int B = bm->B;
-    const int band = (int)std::max<long long>(1, std::min<long long>(B, (64LL << 20) / B));
-    DevBuf<int> dense;
-    dense.reserve((size_t)band * B);
-    for (int r0 = 0; r0 < B; r0 += band) {
-      const int rows = std::min(band, B - r0);
+  // the rows go to the host through a dense device band, band by band
+  const int B = bm->B;
+  const int band = (int)std::max<long long>(1, std::min<long long>(B, (64LL << 20) / B));
+  DevBuf<int> dense;
+  dense.reserve((size_t)band * B);
+  for (int r0 = 0; r0 < B; r0 += band) {
+    const int rows = std::min(band, B - r0);
+    if (bm->sparse) {
       SBP_CUDA(cudaMemsetAsync(dense.p, 0, (size_t)rows * B * sizeof(int), c.stream));
       k_hashed_to_dense<<<std::min(rows, 4096), 128, 0, c.stream>>>(bm->rbase.p, bm->rmask.p, bm->rslot.p, B, r0,
                                                                    rows, dense.p);
-      SBP_CHECK_LAUNCH();
-      SBP_CUDA(SBP_COPY_ASYNC(out + (size_t)r0 * B, dense.p, (size_t)rows * B * sizeof(int), cudaMemcpyDeviceToHost,
-                              c.stream));
-      c.sync();
+    } else {
+      k_pairs_to_dense<<<grid_for((long long)rows * B, 256, 16 * c.num_sms), 256, 0, c.stream>>>(bm->P.p, B, bm->ld,
+                                                                                                r0, rows, dense.p);
     }
-    return SBP_OK;
+    SBP_CHECK_LAUNCH();
+    SBP_CUDA(SBP_COPY_ASYNC(out + (size_t)r0 * B, dense.p, (size_t)rows * B * sizeof(int), cudaMemcpyDeviceToHost,
+                            c.stream));
+    c.sync();
   }
-  SBP_CUDA(cudaMemcpy2DAsync(out, bm->B * sizeof(int), bm->M.p, bm->ld * sizeof(int), bm->B * sizeof(int), bm->B,
-                             cudaMemcpyDeviceToHost, c.stream));
-  c.sync();
   SBP_API_END
 }
 

@@ -530,7 +530,8 @@ struct SbpGraph {
 struct SbpBlockmodel {
   int V = 0, B = 0, ld = 0;
   const SbpGraph* graph = nullptr;   // the graph the blockmodel was created on (must outlive it)
-  DevBuf<int> b, M, MT, CS, CST, d_out, d_in, d;
+  DevBuf<int> b, CS, CST, d_out, d_in, d;
+  DevBuf<int2> P;                            // dense counts of both directions (BlockView::P)
   DevBuf<int> prop, qr, qs, moved, n_moved;   // n_moved: two slots, alternating per batch
   DevBuf<unsigned long long> last;           // (batch generation << 32 | last mover) per block
   unsigned gen = 0;                          // batch generation
@@ -562,8 +563,7 @@ struct SbpBlockmodel {
     v.CS = CS.p;
     v.CST = CST.p;
     v.b = b.p;
-    v.M = M.p;
-    v.MT = MT.p;
+    v.P = P.p;
     v.d_out = d_out.p;
     v.d_in = d_in.p;
     v.d = d.p;
@@ -600,7 +600,7 @@ struct SbpBlockmodel {
       if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
         // buffers this blockmodel already holds, and those the device cache keeps for reuse,
         // count as free
-        const size_t have = M.n * sizeof(int) * 2 + DeviceCache::get().cached_bytes();
+        const size_t have = P.n * sizeof(int2) + DeviceCache::get().cached_bytes();
         if (dense_bytes > 0.01 * g_dense_max_memory_pct * (double)(free_b + have)) sparse = true;
       } else {
         cudaGetLastError();
@@ -616,10 +616,11 @@ struct SbpBlockmodel {
       overflow.reserve(1 + 2 * (size_t)B);   // any-row flag, then one flag per row of M and of MT
     } else {
       const size_t cells = (size_t)B * (size_t)ld;
-      M.reserve(cells);
-      MT.reserve(cells);
-      CS.reserve((size_t)B * nch);
-      CST.reserve((size_t)B * nch);
+      P.reserve(cells);
+      if (nch > 1) {
+        CS.reserve((size_t)B * nch);
+        CST.reserve((size_t)B * nch);
+      }
     }
     d_out.reserve(B);
     d_in.reserve(B);

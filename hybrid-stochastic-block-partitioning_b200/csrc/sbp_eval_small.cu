@@ -19,6 +19,7 @@
 // Summation orders differ from evaluate_vertex, so delta-MDL and the Hastings factor agree with
 // it to rounding; the integer zero-snap scale T and every integer input are the same.
 #include "sbp_engine.cuh"
+#include "sbp_steps.cuh"
 
 namespace sbpb {
 namespace {
@@ -116,13 +117,8 @@ struct GroupTable {
 // Loads of the blockmodel: through the read-only data cache when no thread of the launch writes it
 // (the evaluation half of a Gibbs batch), plain when commits of the same launch change it
 // (Metropolis-Hastings rounds; the writers share the SM, so its L1 stays coherent).
-template <bool kFrozen>
-__device__ __forceinline__ int ldb(const int* p) {
-  if constexpr (kFrozen) return __ldg(p);
-  else return *p;
-}
-template <bool kFrozen>
-__device__ __forceinline__ int4 ldb4(const int4* p) {
+template <bool kFrozen, class T>
+__device__ __forceinline__ T ldb(const T* p) {
   if constexpr (kFrozen) return __ldg(p);
   else return *p;
 }
@@ -135,7 +131,7 @@ __device__ __forceinline__ int4 ldb4(const int4* p) {
 constexpr int kSumsPerLane = 16;
 
 template <int G, bool kFrozen>
-__device__ __forceinline__ int group_walk(const int* row, const int* csum, int nch, long long tg, bool walk, int gl,
+__device__ __forceinline__ int group_walk(const int2* row, bool in_col, const int* csum, int nch, int B, long long tg, bool walk, int gl,
                                           int gbase) {
   const unsigned gmask = (G == 32 ? kFull : ((1u << G) - 1u) << gbase);
   int chunk = 0;
@@ -190,17 +186,17 @@ __device__ __forceinline__ int group_walk(const int* row, const int* csum, int n
     if (walk && chunk < 0) walk = false;
   }
   constexpr int kPer = kChunk / G;   // counts per lane
-  const int* base = row + (size_t)(chunk < 0 ? 0 : chunk) * kChunk + gl * kPer;
+  const int2* base = row + (size_t)(chunk < 0 ? 0 : chunk) * kChunk + gl * kPer;
   int vals[kPer];
   long long lsum = 0;
 #pragma unroll
-  for (int q = 0; q < kPer / 4; ++q) {
-    const int4 c4 = ldb4<kFrozen>(reinterpret_cast<const int4*>(base) + q);
-    vals[4 * q] = c4.x;
-    vals[4 * q + 1] = c4.y;
-    vals[4 * q + 2] = c4.z;
-    vals[4 * q + 3] = c4.w;
-    lsum += (long long)c4.x + c4.y + c4.z + c4.w;
+  for (int q = 0; q < kPer / 2; ++q) {
+    // a row of one chunk ends at column B: the pairs beyond it are not read
+    const int4 c4 = (nch > 1 || gl * kPer + 2 * q < B) ? ldb<kFrozen>(reinterpret_cast<const int4*>(base) + q)
+                                                       : make_int4(0, 0, 0, 0);
+    vals[2 * q] = in_col ? c4.y : c4.x;
+    vals[2 * q + 1] = in_col ? c4.w : c4.z;
+    lsum += (long long)vals[2 * q] + vals[2 * q + 1];
   }
   long long incl = lsum;
 #pragma unroll
@@ -295,9 +291,8 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       in_row = target < dot;
       tg = in_row ? target : target - dot;
     }
-    const int* row = (in_row ? bm.M : bm.MT) + (size_t)t * ld;
     const int* csum = (in_row ? bm.CS : bm.CST) + (size_t)t * bm.nch;
-    const int found = group_walk<G, kFrozen>(row, csum, bm.nch, tg, walk, gl, gbase);
+    const int found = group_walk<G, kFrozen>(bm.P + (size_t)t * ld, !in_row, csum, bm.nch, B, tg, walk, gl, gbase);
     if (walk) {
       s = found;
       if (s < 0 || s >= B) {
@@ -326,10 +321,11 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
     ci_r = (wr >> kInShift) & kCountMask;
     co_s = ws & kCountMask;
     ci_s = (ws >> kInShift) & kCountMask;
-    M_rr = ldb<kFrozen>(bm.M + (size_t)r * ld + r);
-    M_rs = ldb<kFrozen>(bm.M + (size_t)r * ld + s);
-    M_sr = ldb<kFrozen>(bm.M + (size_t)s * ld + r);
-    M_ss = ldb<kFrozen>(bm.M + (size_t)s * ld + s);
+    const int2 m_rs = ldb<kFrozen>(bm.P + (size_t)r * ld + s);
+    M_rr = ldb<kFrozen>(&bm.P[(size_t)r * ld + r].x);
+    M_rs = m_rs.x;
+    M_sr = m_rs.y;
+    M_ss = ldb<kFrozen>(&bm.P[(size_t)s * ld + s].x);
     dout_r = ldb<kFrozen>(bm.d_out + r);
     dout_s = ldb<kFrozen>(bm.d_out + s);
     din_r = ldb<kFrozen>(bm.d_in + r);
@@ -349,10 +345,8 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       const int u = T.key_of(slot);
       const unsigned wu = T.w[slot];
       const int co = wu & kCountMask, ci = (wu >> kInShift) & kCountMask;
-      const int M_ru = ldb<kFrozen>(bm.M + (size_t)r * ld + u);
-      const int M_ur = ldb<kFrozen>(bm.MT + (size_t)r * ld + u);
-      const int M_su = ldb<kFrozen>(bm.M + (size_t)s * ld + u);
-      const int M_us = ldb<kFrozen>(bm.MT + (size_t)s * ld + u);
+      const int2 m_ru = ldb<kFrozen>(bm.P + (size_t)r * ld + u), m_su = ldb<kFrozen>(bm.P + (size_t)s * ld + u);
+      const int M_ru = m_ru.x, M_ur = m_ru.y, M_su = m_su.x, M_us = m_su.y;
       const int du = ldb<kFrozen>(bm.d + u);
       const bool is_r = u == r, is_s = u == s, corner = is_r || is_s;
       const double c = (double)(co + ci + (is_r ? self : 0));
@@ -401,8 +395,8 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
         const int u = T.key_of(slot);
         const unsigned wu = T.w[slot];
         if (u == r || u == s) continue;
-        if (wu & kCountMask) Tz += 2LL * (bm.M[(size_t)r * ld + u] + bm.M[(size_t)s * ld + u]);
-        if ((wu >> kInShift) & kCountMask) Tz += 2LL * (bm.MT[(size_t)r * ld + u] + bm.MT[(size_t)s * ld + u]);
+        const int2 a = bm.P[(size_t)r * ld + u], b = bm.P[(size_t)s * ld + u];
+        Tz += ((wu & kCountMask) ? 2LL * (a.x + b.x) : 0LL) + (((wu >> kInShift) & kCountMask) ? 2LL * (a.y + b.y) : 0LL);
       }
       for (int q = gl; q < 8; q += G) {
         const int a = q == 0 ? M_rr : q == 1 ? M_rs : q == 2 ? M_sr : q == 3 ? M_ss
@@ -624,26 +618,10 @@ __global__ void __launch_bounds__(kMhGroupThreads)
         if (u == r || u == s) continue;
         const unsigned wu = T.w[slot];
         const int co = wu & kCountMask, ci = (wu >> kInShift) & kCountMask;
-        if (co) {
-          bm.M[(size_t)r * bm.ld + u] -= co;
-          bm.MT[(size_t)u * bm.ld + r] -= co;
-          bm.M[(size_t)s * bm.ld + u] += co;
-          bm.MT[(size_t)u * bm.ld + s] += co;
-          chunk_add(bm.CS, bm.nch, r, u, -co);
-          chunk_add(bm.CST, bm.nch, u, r, -co);
-          chunk_add(bm.CS, bm.nch, s, u, co);
-          chunk_add(bm.CST, bm.nch, u, s, co);
-        }
-        if (ci) {
-          bm.M[(size_t)u * bm.ld + r] -= ci;
-          bm.MT[(size_t)r * bm.ld + u] -= ci;
-          bm.M[(size_t)u * bm.ld + s] += ci;
-          bm.MT[(size_t)s * bm.ld + u] += ci;
-          chunk_add(bm.CS, bm.nch, u, r, -ci);
-          chunk_add(bm.CST, bm.nch, r, u, -ci);
-          chunk_add(bm.CS, bm.nch, u, s, ci);
-          chunk_add(bm.CST, bm.nch, s, u, ci);
-        }
+        cell_add_owned(bm, r, u, -co);
+        cell_add_owned(bm, s, u, co);
+        cell_add_owned(bm, u, r, -ci);
+        cell_add_owned(bm, u, s, ci);
       }
       // only this group's lanes are here (the other groups of the warp may not commit): a
       // full-warp barrier would wait for lanes that never arrive
@@ -652,23 +630,18 @@ __global__ void __launch_bounds__(kMhGroupThreads)
         const int self = e.self;
         const int d_rr = -co_r - ci_r - self, d_rs = -co_s + ci_r;
         const int d_sr = co_r - ci_s, d_ss = co_s + ci_s + self;
-        const int cells[4][3] = {{r, r, d_rr}, {r, s, d_rs}, {s, r, d_sr}, {s, s, d_ss}};
-        for (int q = 0; q < 4; ++q) {
-          const int a = cells[q][0], b = cells[q][1], d = cells[q][2];
-          if (!d) continue;
-          bm.M[(size_t)a * bm.ld + b] += d;
-          bm.MT[(size_t)b * bm.ld + a] += d;
-          chunk_add(bm.CS, bm.nch, a, b, d);
-          chunk_add(bm.CST, bm.nch, b, a, d);
-        }
+        cell_add_owned(bm, r, r, d_rr);
+        cell_add_owned(bm, r, s, d_rs);
+        cell_add_owned(bm, s, r, d_sr);
+        cell_add_owned(bm, s, s, d_ss);
         bm.b[e.v] = s;
         bm.d_out[r] -= e.k_out;
         bm.d_out[s] += e.k_out;
         bm.d_in[r] -= e.k_in + self;
         bm.d_in[s] += e.k_in + self;
         // Blockmodel::move_vertex reads the already-updated diagonal and adds the delta again
-        bm.d[r] = bm.d_out[r] + bm.d_in[r] - (bm.M[(size_t)r * bm.ld + r] + d_rr);
-        bm.d[s] = bm.d_out[s] + bm.d_in[s] - (bm.M[(size_t)s * bm.ld + s] + d_ss);
+        bm.d[r] = bm.d_out[r] + bm.d_in[r] - (bm.P[(size_t)r * bm.ld + r].x + d_rr);
+        bm.d[s] = bm.d_out[s] + bm.d_in[s] - (bm.P[(size_t)s * bm.ld + s].x + d_ss);
       }
     }
     pos += s_upto;

@@ -84,7 +84,7 @@ double2* make_xlogx_table(cudaStream_t stream) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Rebuild: M, MT, d_out, d_in from the assignment; d = d_out + d_in - M[x,x].
+// Rebuild: the counts, d_out, d_in from the assignment; d = d_out + d_in - M[x,x].
 // ------------------------------------------------------------------------------------------
 __global__ void k_rebuild_global(GraphView g, BlockView bm) {
   const int stride = gridDim.x * blockDim.x;
@@ -93,10 +93,9 @@ __global__ void k_rebuild_global(GraphView g, BlockView bm) {
     const int o0 = g.out_ptr[v], o1 = g.out_ptr[v + 1];
     for (int e = o0; e < o1; ++e) {
       const int bu = bm.b[__ldg(g.out_idx + e)];
-      atomicAdd(bm.M + (size_t)bv * bm.ld + bu, 1);
-      atomicAdd(bm.MT + (size_t)bu * bm.ld + bv, 1);
-      chunk_add(bm.CS, bm.nch, bv, bu, 1);
-      chunk_add(bm.CST, bm.nch, bu, bv, 1);
+      atomicAdd(&bm.P[(size_t)bv * bm.ld + bu].x, 1);
+      atomicAdd(&bm.P[(size_t)bu * bm.ld + bv].y, 1);
+      chunks_add(bm, bv, bu, 1);
     }
     atomicAdd(bm.d_out + bv, o1 - o0);
     atomicAdd(bm.d_in + bv, (g.in_ptr[v + 1] - g.in_ptr[v]) + g.self[v]);
@@ -122,10 +121,9 @@ __global__ void k_rebuild_smem(GraphView g, BlockView bm) {
     const int c = hist[i];
     if (c) {
       const int row = i / bm.B, col = i - row * bm.B;
-      atomicAdd(bm.M + (size_t)row * bm.ld + col, c);
-      atomicAdd(bm.MT + (size_t)col * bm.ld + row, c);
-      chunk_add(bm.CS, bm.nch, row, col, c);
-      chunk_add(bm.CST, bm.nch, col, row, c);
+      atomicAdd(&bm.P[(size_t)row * bm.ld + col].x, c);
+      atomicAdd(&bm.P[(size_t)col * bm.ld + row].y, c);
+      chunks_add(bm, row, col, c);
     }
   }
 }
@@ -462,16 +460,16 @@ __global__ void k_eval_list(GraphView g, BlockView bm, const int* verts, int n, 
 }
 
 // ------------------------------------------------------------------------------------------
-// Merge phase: compressed rows of M (out_blocks) and of MT (in_blocks), ascending.
+// Merge phase: compressed rows of M (out_blocks) and, with `col`, its columns (in_blocks), ascending.
 // ------------------------------------------------------------------------------------------
-__global__ void k_row_nnz(const int* A, int B, int ld, int* cnt) {
+__global__ void k_row_nnz(const int2* P, int col_side, int B, int ld, int* cnt) {
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int row = wid; row < B; row += nw) {
     int c = 0;
-    const int* p = A + (size_t)row * ld;
-    for (int col = lane; col < B; col += kWarp) c += (p[col] != 0);
+    const int2* p = P + (size_t)row * ld;
+    for (int col = lane; col < B; col += kWarp) c += (col_side ? p[col].y : p[col].x) != 0;
     c = warp_sum_int(c);
     if (lane == 0) cnt[row] = c;
   }
@@ -512,16 +510,16 @@ __global__ void k_excl_scan(const int* in, int* out, int n) {
   if (threadIdx.x == 0) out[n] = carry;
 }
 
-__global__ void k_row_fill(const int* A, int B, int ld, const int* ptr, int* idx, int* val) {
+__global__ void k_row_fill(const int2* P, int col_side, int B, int ld, const int* ptr, int* idx, int* val) {
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int row = wid; row < B; row += nw) {
     int pos = ptr[row];
-    const int* p = A + (size_t)row * ld;
+    const int2* p = P + (size_t)row * ld;
     for (int base = 0; base < B; base += kWarp) {
       const int col = base + lane;
-      const int x = col < B ? p[col] : 0;
+      const int x = col < B ? (col_side ? p[col].y : p[col].x) : 0;
       const unsigned m = __ballot_sync(kFull, x != 0);
       if (x != 0) {
         const int o = pos + __popc(m & ((1u << lane) - 1));
@@ -657,6 +655,15 @@ __global__ void k_block_stats(BlockView bm, unsigned long long* out) {
   atomicAdd(out + 0, tr);
   atomicAdd(out + 1, din);
   atomicAdd(out + 2, prod);
+}
+
+// Counts M[row, .] of rows row0 .. row0 + rows - 1 into a dense rows x B array.
+__global__ void k_pairs_to_dense(const int2* __restrict__ P, int B, int ld, int row0, int rows, int* dense) {
+  const long long n = (long long)rows * B, stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const int r = (int)(i / B), c = (int)(i - (long long)r * B);
+    dense[i] = P[(size_t)(row0 + r) * ld + c].x;
+  }
 }
 
 __global__ void k_relabel(int* b, int V, const int* map) {

@@ -88,9 +88,10 @@ __global__ void k_mh(GraphView g, BlockView bm, const int* __restrict__ verts, i
 __global__ void k_move_vertex(GraphView g, BlockView bm, int v, int s, int cap, int* status);
 __global__ void k_eval_list(GraphView g, BlockView bm, const int* verts, int n, const uint4* records, int cap,
                             int* out_s, double* out_dS, double* out_H, int* out_acc, int* status);
-__global__ void k_row_nnz(const int* A, int B, int ld, int* cnt);
+__global__ void k_row_nnz(const int2* P, int col_side, int B, int ld, int* cnt);
 __global__ void k_excl_scan(const int* in, int* out, int n);
-__global__ void k_row_fill(const int* A, int B, int ld, const int* ptr, int* idx, int* val);
+__global__ void k_row_fill(const int2* P, int col_side, int B, int ld, const int* ptr, int* idx, int* val);
+__global__ void k_pairs_to_dense(const int2* __restrict__ P, int B, int ld, int row0, int rows, int* dense);
 __global__ void k_merge_propose(BlockView bm, Csr rows, Csr cols, RngParams rng, int* best_s, double* best_dS,
                                 unsigned long long* counters, int* status);
 __global__ void k_block_sizes(const int* b, int V, int* size);

@@ -20,7 +20,7 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return t;
 }
 
-// M[row,col] += delta with the transpose kept in step: dense cells and both chunk sums, or the
+// M[row,col] += delta in both pairs that hold it and both chunk sums (dense), or in the
 // two hashed rows (atomic).
 __device__ __forceinline__ void cell_add(const BlockView& bm, int row, int col, int delta) {
   if (bm.sparse) {
@@ -28,13 +28,12 @@ __device__ __forceinline__ void cell_add(const BlockView& bm, int row, int col, 
     hashed_add(bm.cbase, bm.cmask, bm.cslot, col, row, delta, bm.overflow, bm.overflow + 1 + bm.B);
     return;
   }
-  atomicAdd(bm.M + (size_t)row * bm.ld + col, delta);
-  atomicAdd(bm.MT + (size_t)col * bm.ld + row, delta);
-  chunk_add(bm.CS, bm.nch, row, col, delta);
-  chunk_add(bm.CST, bm.nch, col, row, delta);
+  atomicAdd(&bm.P[(size_t)row * bm.ld + col].x, delta);
+  atomicAdd(&bm.P[(size_t)col * bm.ld + row].y, delta);
+  chunks_add(bm, row, col, delta);
 }
 
-// Same for a dense cell owned by one thread (plain update of M/MT, atomic chunk sums, which
+// Same for a dense cell owned by one thread (plain update of the pair, atomic chunk sums, which
 // lanes share); hashed rows are always updated atomically (lanes share their slots).
 __device__ __forceinline__ void cell_add_owned(const BlockView& bm, int row, int col, int delta) {
   if (!delta) return;
@@ -42,10 +41,9 @@ __device__ __forceinline__ void cell_add_owned(const BlockView& bm, int row, int
     cell_add(bm, row, col, delta);
     return;
   }
-  bm.M[(size_t)row * bm.ld + col] += delta;
-  bm.MT[(size_t)col * bm.ld + row] += delta;
-  chunk_add(bm.CS, bm.nch, row, col, delta);
-  chunk_add(bm.CST, bm.nch, col, row, delta);
+  bm.P[(size_t)row * bm.ld + col].x += delta;
+  bm.P[(size_t)col * bm.ld + row].y += delta;
+  chunks_add(bm, row, col, delta);
 }
 
 // Commit rule of a sequential Metropolis-Hastings round (finetune::metropolis_hastings,
@@ -154,7 +152,7 @@ __device__ __forceinline__ void mh_apply_move(const GraphView& g, const BlockVie
 }
 
 // Apply of one accepted move v: r -> prop[v] (Blockmodel::move_vertex, src/blockmodel/
-// blockmodel.cpp:344-360, for a batch of simultaneous moves): M, MT and the chunk sums by edge,
+// blockmodel.cpp:344-360, for a batch of simultaneous moves): the counts and chunk sums by edge,
 // d_out / d_in, the quirk terms qr/qs of d[r], d[s] (the neighbours that are counted in the
 // reference's sequential apply) and the batch's last mover of r and s.  One warp per vertex;
 // lanes whose edges change the same cell add their count with one atomic.
@@ -251,7 +249,7 @@ __device__ __forceinline__ double mdl_cells_part(const BlockView& bm, int cta, i
   const long long stride = (long long)ncta * blockDim.x;
   for (long long i = (long long)cta * blockDim.x + threadIdx.x; i < BB; i += stride) {
     const int row = (int)(i / bm.B), col = (int)(i - (long long)row * bm.B);
-    const int m = bm.M[(size_t)row * bm.ld + col];
+    const int m = bm.P[(size_t)row * bm.ld + col].x;
     if (m > 0) acc += xlogx((double)m);
   }
   for (long long x = (long long)cta * blockDim.x + threadIdx.x; x < bm.B; x += stride)
