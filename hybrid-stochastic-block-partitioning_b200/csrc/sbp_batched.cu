@@ -65,6 +65,7 @@ struct BGraph {   // one graph of the batch (device side)
   int nstages;
   int chunk;                 // light vertices per evaluation item
   int mdl_cells;             // 1: cell form of the MDL, 0: edge form
+  int mdl_ctas;              // its virtual grid
 };
 
 struct Queue {                 // per graph, reset before every launch
@@ -75,7 +76,6 @@ struct Queue {                 // per graph, reset before every launch
 
 struct SweepParams {
   int ngraphs;                 // graphs in this launch (indices in glist)
-  int mdl_ctas;
   int heavy_cap;
   unsigned wait_limit;         // idle claim attempts of a CTA before the launch gives up
 };
@@ -243,16 +243,16 @@ __global__ void __launch_bounds__(kBThreads, 2)
         break;
       }
       case kMdlPart: {
-        const int c0 = idx * kMdlCtasPerItem, c1 = min(c0 + kMdlCtasPerItem, P.mdl_ctas);
+        const int c0 = idx * kMdlCtasPerItem, c1 = min(c0 + kMdlCtasPerItem, gr.mdl_ctas);
         for (int cc = c0; cc < c1; ++cc) {
-          const double v = gr.mdl_cells ? mdl_cells_part(gr.bm, cc, P.mdl_ctas, red)
-                                        : mdl_edges_part(gr.g, gr.bm, gr.out_src, cc, P.mdl_ctas, red);
+          const double v = gr.mdl_cells ? mdl_cells_part(gr.bm, cc, gr.mdl_ctas, red)
+                                        : mdl_edges_part(gr.g, gr.bm, gr.out_src, cc, gr.mdl_ctas, red);
           if (tid == 0) gr.partial[cc] = v;
         }
         break;
       }
       case kMdlFinal: {
-        const double v = mdl_final_value(gr.partial, P.mdl_ctas, gr.g.V, gr.g.E, gr.bm.B, red);
+        const double v = mdl_final_value(gr.partial, gr.mdl_ctas, gr.g.V, gr.g.E, gr.bm.B, red);
         if (tid == 0) *gr.mdl_out = v;
         break;
       }
@@ -332,7 +332,7 @@ struct Slot {
   double initial = 0.0;
   std::vector<double> deltas;
   int sweep = 0;
-  int stage_chunk = -1;
+  int stage_chunk = -1, stage_mdl = -1;   // what the uploaded stages were made for
   std::chrono::steady_clock::time_point t0;
   DevBuf<int4> batches, stages;
   DevBuf<unsigned long long> counters;
@@ -593,10 +593,12 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
     // one sweep of every finetuning graph
     const Shape shape = current_shape();
     for (Slot* s : act) {
-      if (s->stage_chunk != shape.chunk) {
-        const std::vector<int4> st = sweep_stages(*s->plan, shape.chunk, c.npartial);
+      const int mdl_ctas = mdl_grid(s->ps->bm, *s->g);
+      if (s->stage_chunk != shape.chunk || s->stage_mdl != mdl_ctas) {
+        const std::vector<int4> st = sweep_stages(*s->plan, shape.chunk, mdl_ctas);
         SBP_CUDA(SBP_COPY_ASYNC(s->stages.p, st.data(), st.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream));
         s->stage_chunk = shape.chunk;
+        s->stage_mdl = mdl_ctas;
       }
       BGraph& b = hG[s->index];
       SbpBlockmodel& bm = s->ps->bm;
@@ -623,11 +625,11 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
       b.gen0 = bm.gen;
       b.nstages = (int)(3 * s->plan->light_n.size() + 2);
       b.chunk = shape.chunk;
-      b.mdl_cells = (!bm.sparse && (long long)bm.B * bm.B <= 4LL * s->g->E) ? 1 : 0;
+      b.mdl_cells = mdl_cell_form(bm, *s->g) ? 1 : 0;
+      b.mdl_ctas = mdl_grid(bm, *s->g);
     }
     for (size_t k = 0; k < act.size(); ++k) hList[k] = act[k]->index;
     hP->ngraphs = (int)act.size();
-    hP->mdl_ctas = c.npartial;
     hP->heavy_cap = heavy_cap;
     hP->wait_limit = (unsigned)g_batched_wait_limit;
     // fault injection for the failure-detection test: the stalled graph's first stage starts

@@ -27,6 +27,7 @@ enum : int {
   kErrScan = 2,           // multinomial walk ran off the row (inconsistent counts)
   kErrReplay = 4,         // replay record index out of range
   kErrBounds = 8,         // block or vertex id out of range
+  kErrGridWait = 32,      // a barrier of a persistent kernel gave up waiting
 };
 
 // ------------------------------------------------------------------------------------------
@@ -148,6 +149,7 @@ struct GraphView {
   const int* out_idx;     // out-neighbours incl. self loop, first-occurrence order
   const int* in_ptr;      // [V+1]
   const int* in_idx;      // in-neighbours, self loop removed
+  const int* adj;         // both lists of a vertex joined, its out-list first, from out_ptr[v] + in_ptr[v]
   const unsigned char* self;
 };
 
@@ -169,8 +171,9 @@ struct BlockView {
   int* overflow;
   int ld;                 // row stride of P (multiple of kChunk pairs)
   int nch;                // chunks per row = ceil(B / kChunk)
-  int* CS;                // [B*nch] CS[row*nch+c] = sum of M[row, c*kChunk .. c*kChunk+kChunk); kept when nch > 1
-  int* CST;               // [B*nch] the same over the columns of M (chunks of rows)
+  int ncs;                // row stride of CS and CST: nch rounded up to four, the rest zero
+  int* CS;                // [B*ncs] CS[row*ncs+c] = sum of M[row, c*kChunk .. c*kChunk+kChunk); kept when nch > 1
+  int* CST;               // [B*ncs] the same over the columns of M (chunks of rows)
   int* b;                 // [V] assignment
   // [B*ld] counts of both directions side by side: P[row*ld+col] = (M[row, col], M[col, row]).
   // A visit needs M[r,u] with M[u,r] and M[s,u] with M[u,s]: one 8-byte load and one 32-byte
@@ -406,8 +409,8 @@ __device__ __forceinline__ int select_chunk_then_column(const int2* row, bool co
 // row itself.
 __device__ __forceinline__ void chunks_add(const BlockView& bm, int row, int col, int delta) {
   if (bm.nch == 1) return;
-  atomicAdd(bm.CS + (size_t)row * bm.nch + col / kChunk, delta);
-  atomicAdd(bm.CST + (size_t)col * bm.nch + row / kChunk, delta);
+  atomicAdd(bm.CS + (size_t)row * bm.ncs + col / kChunk, delta);
+  atomicAdd(bm.CST + (size_t)col * bm.ncs + row / kChunk, delta);
 }
 
 // Same walk over a compressed list (idx[i], val[i]), i in [0, n).
@@ -826,7 +829,7 @@ __device__ __forceinline__ EvalResult evaluate_vertex(const GraphView& g, const 
       // faster above.)
       const int dot = ldi<ST>(bm.d_out + tblk), dit = ldi<ST>(bm.d_in + tblk);
       const int2* row = bm.P + (size_t)tblk * bm.ld;
-      const size_t co = (size_t)tblk * bm.nch;
+      const size_t co = (size_t)tblk * bm.ncs;
       int4 qa = make_int4(0, 0, 0, 0), qb = make_int4(0, 0, 0, 0);
       int ca = 0, cb = 0;
       if (bm.nch == 1) {

@@ -207,8 +207,8 @@ void rebuild(SbpBlockmodel& bm, const SbpGraph& g, bool recompute_d) {
   const size_t cells = (size_t)bm.B * (size_t)bm.ld;
   SBP_CUDA(cudaMemsetAsync(bm.P.p, 0, cells * sizeof(int2), c.stream));
   if (bm.nch > 1) {
-    SBP_CUDA(cudaMemsetAsync(bm.CS.p, 0, (size_t)bm.B * bm.nch * sizeof(int), c.stream));
-    SBP_CUDA(cudaMemsetAsync(bm.CST.p, 0, (size_t)bm.B * bm.nch * sizeof(int), c.stream));
+    SBP_CUDA(cudaMemsetAsync(bm.CS.p, 0, (size_t)bm.B * bm.ncs * sizeof(int), c.stream));
+    SBP_CUDA(cudaMemsetAsync(bm.CST.p, 0, (size_t)bm.B * bm.ncs * sizeof(int), c.stream));
   }
   SBP_CUDA(cudaMemsetAsync(bm.d_out.p, 0, bm.B * sizeof(int), c.stream));
   SBP_CUDA(cudaMemsetAsync(bm.d_in.p, 0, bm.B * sizeof(int), c.stream));
@@ -278,9 +278,8 @@ void tidy_hashed(SbpBlockmodel& bm, const SbpGraph& g, long long overflows_befor
 // entropy::mdl (src/entropy.cpp:584-589).
 double mdl(SbpBlockmodel& bm, const SbpGraph& g) {
   Context& c = Context::get();
-  const int cells = !bm.sparse && (long long)bm.B * bm.B <= 4LL * g.E;
-  k_mdl<<<c.npartial, 256, 0, c.stream>>>(g.view(), bm.view(), g.out_src.p, cells, c.partial, c.done, c.scalar,
-                                         nullptr, 0);
+  k_mdl<<<mdl_grid(bm, g), 256, 0, c.stream>>>(g.view(), bm.view(), g.out_src.p, mdl_cell_form(bm, g) ? 1 : 0,
+                                              c.partial, c.done, c.scalar);
   SBP_CHECK_LAUNCH();
   double out = 0.0;
   SBP_CUDA(SBP_COPY_ASYNC(&out, c.scalar, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
@@ -372,53 +371,47 @@ MhResult mh_pass(SbpBlockmodel& bm, const SbpGraph& g, const int* verts, int n, 
   return res;
 }
 
-// One asynchronous-Gibbs batch: evaluate every vertex of the batch, then apply the moves.
-void gibbs_batch(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, int bt, RngParams rng,
-                        int sweep) {
+// The evaluation half of an asynchronous-Gibbs batch: accepted moves to bm.moved.
+void gibbs_eval_batch(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, int bt, const RngParams& rng,
+                      int sweep) {
   Context& c = Context::get();
   const int nl = plan.light_n[bt], nh = plan.heavy_n[bt];
   int* n_cur = bm.n_moved.p + (bm.gen & 1);
-  const GibbsEvalKernel k_eval = gibbs_eval_kernel(bm.sparse, bm.B);
-  if (nl > 0) {
-    const bool small = use_group_kernel(bm);
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  if (nl > 0 && g_prof.on) {
+    e0 = g_prof.get();
+    e1 = g_prof.get();
+    SBP_CUDA(cudaEventRecord(e0, c.stream));
+  }
+  if (!bm.sparse) {
+    launch_gibbs_eval(g, bm, plan, bt, rng, sweep, n_cur);
+    SBP_CHECK_LAUNCH();
+  } else if (nl > 0) {
     const size_t smem = (size_t)table_ints(g.light_cap) * sizeof(int) * kLightWarps;
-    set_smem_limit((const void*)k_eval, smem);
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (g_prof.on) {
-      e0 = g_prof.get();
-      e1 = g_prof.get();
-      SBP_CUDA(cudaEventRecord(e0, c.stream));
-    }
-    if (small) {
-      // direct-indexed tables take every light vertex; hashed ones those of k <= kGroupMaxK, the
-      // warp kernel the rest
-      const int ng = bm.B <= kSmallB ? nl : plan.group_n[bt];
-      if (ng > 0)
-        launch_group_eval(g, bm, plan.order.p + plan.light_begin[bt], ng, rng, sweep, n_cur, nullptr, 0, c.stream);
-      if (nl > ng)
-        k_eval<<<grid_for(nl - ng, kLightWarps, 64 * c.num_sms), kLightWarps * 32, smem, c.stream>>>(
-            g.view(), bm.view(), plan.order.p + plan.light_begin[bt] + ng, nl - ng, rng, sweep, bm.prop.p,
-            bm.moved.p, n_cur, c.counters, g.light_cap, c.status, nullptr, 0);
-    } else {
-      k_eval<<<grid_for(nl, kLightWarps, 64 * c.num_sms), kLightWarps * 32, smem, c.stream>>>(
-          g.view(), bm.view(), plan.order.p + plan.light_begin[bt], nl, rng, sweep, bm.prop.p, bm.moved.p, n_cur,
-          c.counters, g.light_cap, c.status, nullptr, 0);
-    }
+    set_smem_limit((const void*)k_gibbs_eval_hashed, smem);
+    k_gibbs_eval_hashed<<<grid_for(nl, kLightWarps, 64 * c.num_sms), kLightWarps * 32, smem, c.stream>>>(
+        g.view(), bm.view(), plan.order.p + plan.light_begin[bt], nl, rng, sweep, bm.prop.p, bm.moved.p, n_cur,
+        c.counters, g.light_cap, c.status);
     SBP_CHECK_LAUNCH();
-    if (g_prof.on) {
-      SBP_CUDA(cudaEventRecord(e1, c.stream));
-      g_prof.add(e0, e1, nl, plan.light_bytes[bt]);
-    }
   }
-  if (nh > 0) {
+  if (e0) {
+    SBP_CUDA(cudaEventRecord(e1, c.stream));
+    g_prof.add(e0, e1, nl, plan.light_bytes[bt]);
+  }
+  if (bm.sparse && nh > 0) {
     const size_t smem = (size_t)table_ints(g.heavy_cap) * sizeof(int);
-    set_smem_limit((const void*)k_eval, std::max(smem, (size_t)table_ints(g.light_cap) * sizeof(int) * kLightWarps));
-    k_eval<<<grid_for(nh, 1, 64 * c.num_sms), 32, smem, c.stream>>>(
+    set_smem_limit((const void*)k_gibbs_eval_hashed, smem);
+    k_gibbs_eval_hashed<<<grid_for(nh, 1, 64 * c.num_sms), 32, smem, c.stream>>>(
         g.view(), bm.view(), plan.order.p + plan.heavy_begin[bt], nh, rng, sweep, bm.prop.p, bm.moved.p, n_cur,
-        c.counters, g.heavy_cap, c.status, nullptr, 0);
+        c.counters, g.heavy_cap, c.status);
     SBP_CHECK_LAUNCH();
   }
-  gibbs_apply(bm, g, nl + nh);
+}
+
+// One asynchronous-Gibbs batch: evaluate every vertex of the batch, then apply the moves.
+void gibbs_batch(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, int bt, const RngParams& rng, int sweep) {
+  gibbs_eval_batch(bm, g, plan, bt, rng, sweep);
+  gibbs_apply(bm, g, plan.light_n[bt] + plan.heavy_n[bt]);
 }
 
 void gibbs_apply(SbpBlockmodel& bm, const SbpGraph& g, int batch) {
@@ -429,7 +422,7 @@ void gibbs_apply(SbpBlockmodel& bm, const SbpGraph& g, int batch) {
   const unsigned gen = ++bm.gen;
   const int gw = grid_for((long long)batch * 32, 256, 64 * c.num_sms);
   k_apply_edges<<<gw, 256, 0, c.stream>>>(g.view(), bm.view(), bm.moved.p, n_cur, bm.prop.p, bm.qr.p, bm.qs.p,
-                                          bm.last.p, gen, nullptr, 0);
+                                          bm.last.p, gen);
   SBP_CHECK_LAUNCH();
   if (bm.sparse) {
     int ovf = 0;
@@ -450,107 +443,10 @@ void gibbs_apply(SbpBlockmodel& bm, const SbpGraph& g, int batch) {
     }
   }
   k_apply_finish<<<grid_for(batch, 256, 64 * c.num_sms), 256, 0, c.stream>>>(
-      bm.view(), bm.moved.p, n_cur, n_next, bm.prop.p, bm.qr.p, bm.qs.p, bm.last.p, gen, nullptr, 0);
+      bm.view(), bm.moved.p, n_cur, n_next, bm.prop.p, bm.qr.p, bm.qs.p, bm.last.p, gen);
   SBP_CHECK_LAUNCH();
 }
 
-
-// Asynchronous-Gibbs sweeps of one finetune call as ONE CUDA graph launch: a conditional while
-// node whose body is a sweep (every batch's evaluation, apply and degree step, then the MDL,
-// whose last CTA applies the early stop on the GPU and sets the loop condition).
-// Same kernels, same order and the same early-stop arithmetic as the host loop, so the chain
-// and the sweep count are the host loop's.  Returns the sweeps run.
-static thread_local DevBuf<SweepCtl> g_ctl;
-
-static int gibbs_sweeps_graph(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, RngParams rng,
-                              int max_sweeps, bool bracket, double initial_entropy) {
-  Context& c = Context::get();
-  const int nb = (int)plan.light_n.size();
-  g_ctl.reserve(1);
-  SweepCtl h;
-  std::memset(&h, 0, sizeof h);
-  h.sweep = 0;
-  h.gen0 = bm.gen;
-  h.nbatches = nb;
-  h.count = 0;
-  h.max_sweeps = max_sweeps;
-  h.bracket = bracket ? 1 : 0;
-  h.n_moved = bm.n_moved.p;
-  h.initial = initial_entropy;
-  SBP_CUDA(SBP_COPY_ASYNC(g_ctl.p, &h, sizeof h, cudaMemcpyHostToDevice, c.stream));
-  const size_t smem_light = (size_t)table_ints(g.light_cap) * sizeof(int) * kLightWarps;
-  const size_t smem_heavy = (size_t)table_ints(g.heavy_cap) * sizeof(int);
-  const GibbsEvalKernel k_eval = gibbs_eval_kernel(false, bm.B);   // the graph runs dense storage only
-  set_smem_limit((const void*)k_eval, std::max(smem_light, smem_heavy));
-  const bool cells = (long long)bm.B * bm.B <= 4LL * g.E;
-  const int mdl_grid = c.npartial;
-
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  struct Guard {
-    cudaGraph_t* g;
-    cudaGraphExec_t* e;
-    ~Guard() {
-      if (*e) cudaGraphExecDestroy(*e);
-      if (*g) cudaGraphDestroy(*g);
-    }
-  } guard{&graph, &exec};
-  SBP_CUDA(cudaGraphCreate(&graph, 0));
-  cudaGraphConditionalHandle loop;
-  SBP_CUDA(cudaGraphConditionalHandleCreate(&loop, graph, 1, cudaGraphCondAssignDefault));
-  // cudaGraphNodeParams holds a union of non-trivial members: build it in zeroed storage
-  alignas(cudaGraphNodeParams) unsigned char cp_storage[sizeof(cudaGraphNodeParams)] = {};
-  cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(cp_storage);
-  cp.type = cudaGraphNodeTypeConditional;
-  cp.conditional.handle = loop;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  cudaGraphNode_t node;
-  SBP_CUDA(cudaGraphAddNode(&node, graph, nullptr, 0, &cp));
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  SBP_CUDA(cudaStreamBeginCaptureToGraph(c.stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  int launches = 0;
-  for (int bt = 0; bt < nb; ++bt) {
-    const int nl = plan.light_n[bt], nh = plan.heavy_n[bt];
-    if (nl > 0) {
-      const int ng = !use_group_kernel(bm) ? 0 : bm.B <= kSmallB ? nl : plan.group_n[bt];
-      if (ng > 0) {
-        launch_group_eval(g, bm, plan.order.p + plan.light_begin[bt], ng, rng, 0, nullptr, g_ctl.p, bt, c.stream);
-        ++launches;
-      }
-      if (nl > ng) {
-        k_eval<<<grid_for(nl - ng, kLightWarps, 64 * c.num_sms), kLightWarps * 32, smem_light, c.stream>>>(
-            g.view(), bm.view(), plan.order.p + plan.light_begin[bt] + ng, nl - ng, rng, 0, bm.prop.p, bm.moved.p,
-            nullptr, c.counters, g.light_cap, c.status, g_ctl.p, bt);
-        ++launches;
-      }
-    }
-    if (nh > 0) {
-      k_eval<<<grid_for(nh, 1, 64 * c.num_sms), 32, smem_heavy, c.stream>>>(
-          g.view(), bm.view(), plan.order.p + plan.heavy_begin[bt], nh, rng, 0, bm.prop.p, bm.moved.p, nullptr,
-          c.counters, g.heavy_cap, c.status, g_ctl.p, bt);
-      ++launches;
-    }
-    const int batch = nl + nh;
-    k_apply_edges<<<grid_for((long long)batch * 32, 256, 64 * c.num_sms), 256, 0, c.stream>>>(
-        g.view(), bm.view(), bm.moved.p, nullptr, bm.prop.p, bm.qr.p, bm.qs.p, bm.last.p, 0u, g_ctl.p, bt);
-    k_apply_finish<<<grid_for(batch, 256, 64 * c.num_sms), 256, 0, c.stream>>>(
-        bm.view(), bm.moved.p, nullptr, nullptr, bm.prop.p, bm.qr.p, bm.qs.p, bm.last.p, 0u, g_ctl.p, bt);
-    launches += 2;
-  }
-  k_mdl<<<mdl_grid, 256, 0, c.stream>>>(g.view(), bm.view(), g.out_src.p, cells ? 1 : 0, c.partial, c.done,
-                                       c.scalar, g_ctl.p, loop);
-  launches += 1;
-  const cudaError_t ce = cudaStreamEndCapture(c.stream, &body);
-  SBP_CUDA(ce);
-  SBP_CUDA(cudaGraphInstantiate(&exec, graph, 0));
-  SBP_CUDA(cudaGraphLaunch(exec, c.stream));
-  SBP_CUDA(SBP_COPY_ASYNC(&h, g_ctl.p, sizeof h, cudaMemcpyDeviceToHost, c.stream));
-  c.sync();
-  g_launches += (long long)launches * h.count;
-  bm.gen += (unsigned)(nb * h.count);
-  return h.count;
-}
 
 // finetune::{metropolis_hastings, asynchronous_gibbs, hybrid_mcmc}.
 void finetune(SbpBlockmodel& bm, SbpGraph& g, int algo, const SbpFinetuneOptions& opt, const SbpReplay* replay,
@@ -578,16 +474,19 @@ void finetune(SbpBlockmodel& bm, SbpGraph& g, int algo, const SbpFinetuneOptions
   const bool bracket = opt.bracket_established != 0;
   SBP_CUDA(cudaMemsetAsync(c.counters, 0, 8 * sizeof(unsigned long long), c.stream));
   const long long ovf0 = g_overflow_rebuilds;
-  bm.overall_entropy = (float)mdl(bm, g);
-  const double initial_entropy = bm.overall_entropy;
   std::vector<double> deltas;
   long long mh_visits = 0, mh_moved = 0, mh_acc = 0;
   const BatchPlan* plan = nullptr;
   if (algo != SBP_METROPOLIS_HASTINGS) plan = &g.plan(algo, opt.batches);
-  if (algo == SBP_ASYNC_GIBBS && g_graph_sweeps && !bm.sparse && !g_prof.on && !plan->light_n.empty()) {
-    st.sweeps = gibbs_sweeps_graph(bm, g, *plan, rng, max_sweeps, bracket, initial_entropy);
-    c.check_status();
-  } else
+  const bool persistent = algo == SBP_ASYNC_GIBBS && g_graph_sweeps && !bm.sparse && !g_prof.on &&
+                          !plan->desc.empty() && &c == &Context::primary();
+  if (persistent) {
+    const SweepsResult r = gibbs_sweeps(bm, g, *plan, rng, max_sweeps, bracket);
+    st.sweeps = r.sweeps;
+    bm.overall_entropy = (float)r.mdl;
+  } else {
+  bm.overall_entropy = (float)mdl(bm, g);
+  const double initial_entropy = bm.overall_entropy;
   for (int it = 0; it < max_sweeps; ++it) {
     if (algo == SBP_METROPOLIS_HASTINGS) {
       const MhResult r = mh_pass(bm, g, g.identity.p, g.V, g.max_k, rng, it);
@@ -616,6 +515,7 @@ void finetune(SbpBlockmodel& bm, SbpGraph& g, int algo, const SbpFinetuneOptions
     }
   }
   bm.overall_entropy = (float)mdl(bm, g);
+  }
   unsigned long long cnt[8];
   SBP_CUDA(SBP_COPY_ASYNC(cnt, c.counters, sizeof cnt, cudaMemcpyDeviceToHost, c.stream));
   SBP_CUDA(cudaEventRecord(c.ev1, c.stream));
@@ -1298,6 +1198,10 @@ SbpStatus sbp_graph_create(int32_t V, int64_t n, const int32_t* src, const int32
   k_ingest_ptr<<<grid_for((long long)V + 1, 256, 8 * c.num_sms), 256, 0, c.stream>>>(iptr.p, g->in_ptr.p,
                                                                                     (long long)V + 1);
   SBP_CHECK_LAUNCH();
+  g->adj.reserve((size_t)m + (size_t)mi);
+  k_join_lists<<<grid_for(8LL * V, 256, 16 * c.num_sms), 256, 0, c.stream>>>(V, g->out_ptr.p, g->out_idx.p,
+                                                                            g->in_ptr.p, g->in_idx.p, g->adj.p);
+  SBP_CHECK_LAUNCH();
   std::vector<int> op((size_t)V + 1), ip((size_t)V + 1);
   SBP_CUDA(SBP_COPY_ASYNC(op.data(), g->out_ptr.p, ((size_t)V + 1) * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(ip.data(), g->in_ptr.p, ((size_t)V + 1) * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
@@ -1424,9 +1328,9 @@ SbpStatus sbp_blockmodel_copy(const SbpBlockmodel* src, SbpBlockmodel** out) {
   SBP_CUDA(SBP_COPY_ASYNC(bm->b.p, src->b.p, src->V * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->P.p, src->P.p, cells * sizeof(int2), cudaMemcpyDeviceToDevice, c.stream));
   if (src->nch > 1) {
-    SBP_CUDA(SBP_COPY_ASYNC(bm->CS.p, src->CS.p, (size_t)src->B * src->nch * sizeof(int), cudaMemcpyDeviceToDevice,
+    SBP_CUDA(SBP_COPY_ASYNC(bm->CS.p, src->CS.p, (size_t)src->B * src->ncs * sizeof(int), cudaMemcpyDeviceToDevice,
                             c.stream));
-    SBP_CUDA(SBP_COPY_ASYNC(bm->CST.p, src->CST.p, (size_t)src->B * src->nch * sizeof(int), cudaMemcpyDeviceToDevice,
+    SBP_CUDA(SBP_COPY_ASYNC(bm->CST.p, src->CST.p, (size_t)src->B * src->ncs * sizeof(int), cudaMemcpyDeviceToDevice,
                             c.stream));
   }
   SBP_CUDA(SBP_COPY_ASYNC(bm->d_out.p, src->d_out.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));

@@ -254,6 +254,8 @@ struct Context {
   double* partial = nullptr;             // MDL partial sums
   double* scalar = nullptr;              // MDL result
   double* mh_out = nullptr;              // MH sweep outputs [4]
+  int* sweep_words = nullptr;            // [8] moved counts and barrier words of the persistent finetune kernel
+  SweepsResult* sweep_result = nullptr;
   unsigned* done = nullptr;              // CTAs finished in the current k_mdl launch (0 between launches)
   double2* xlogxt = nullptr;             // [kXlogxTable] x log x as hi + lo doubles
   int npartial = 0;
@@ -273,6 +275,8 @@ struct Context {
     SBP_CUDA(cudaMalloc(&c->scalar, sizeof(double)));
     SBP_CUDA(cudaMalloc(&c->mh_out, 16 * sizeof(double)));
     SBP_CUDA(cudaMalloc(&c->done, sizeof(unsigned)));
+    SBP_CUDA(cudaMalloc(&c->sweep_words, 8 * sizeof(int)));
+    SBP_CUDA(cudaMalloc(&c->sweep_result, sizeof(SweepsResult)));
     SBP_CUDA(cudaMemset(c->status, 0, 8 * sizeof(int)));
     SBP_CUDA(cudaMemset(c->done, 0, sizeof(unsigned)));
     SBP_CUDA(cudaEventCreate(&c->ev0));
@@ -322,7 +326,7 @@ struct Context {
       char msg[200];
       snprintf(msg, sizeof msg,
                "device status 0x%x (table overflow=1, multinomial walk=2, bounds=8, batched sweep found no "
-               "claimable work within its wait limit=16)", st);
+               "claimable work within its wait limit=16, grid barrier wait=32)", st);
       throw Error(SBP_ERR_DEVICE, msg);
     }
   }
@@ -409,15 +413,14 @@ inline int g_dense_max_blocks = 131072;
 inline int g_dense_max_memory_pct = 60;
 // Hashed row capacity = power of two >= factor * (cells after a rebuild) + 4 * factor.
 inline int g_hashed_row_factor = 4;
-// 1: an asynchronous-Gibbs finetune on dense storage runs as one CUDA graph launch with the
-// sweep loop decided on the GPU; 0: one host-driven launch sequence per sweep (sbp_set_option).
+// 1: an asynchronous-Gibbs finetune on dense storage runs as one persistent kernel, its sweep loop
+// and early stop on the GPU; 0: one host-driven launch sequence per sweep (sbp_set_option).
 inline int g_graph_sweeps = 1;
 inline thread_local long long g_overflow_rebuilds = 0;   // rebuilds forced by a full hashed row (calling thread)
-// Light vertices of dense blockmodels (sbp_set_option "group_kernel"): 1 (default) evaluated by the
-// group kernels (sbp_eval_small.cu) when B <= kSmallB (direct-indexed group tables), by the warp-
-// per-vertex kernels above; 2 by the group kernels at every B (hashed group tables above kSmallB:
-// half the occupancy of the warp kernel at the light-table size of the 200,000-vertex graph,
-// measured slower there); 0 by the warp-per-vertex kernels always.
+// Lanes per vertex of the evaluation on dense blockmodels (sbp_set_option "group_kernel"): 1
+// (default) chosen from the batch and the vertex's degree, 2 as few as its degree allows, 0 a whole
+// warp.  Metropolis-Hastings: 1 groups of eight up to kSmallB blocks, a warp above; 2 groups at every
+// block count where they fit; 0 a warp.
 inline int g_group_kernel = 1;
 // Batched partitioner: idle claim attempts of a persistent CTA before the launch gives up with an
 // error (each attempt sleeps ~0.25 us), and the fault injection of the failure-detection test
@@ -439,9 +442,11 @@ using namespace sbpb;
 // Graph
 // ------------------------------------------------------------------------------------------
 struct BatchPlan {
-  DevBuf<int> order;                       // per batch: light vertices then heavy vertices
+  DevBuf<int> order;                       // per batch: light vertices then heavy vertices, each by degree descending
+  DevBuf<int4> recs;                       // their records (vertex_record), in the same order
+  DevBuf<BatchDesc> desc_dev;
+  std::vector<BatchDesc> desc;
   std::vector<int> light_begin, light_n, heavy_begin, heavy_n;
-  std::vector<int> group_n;                // light vertices of k <= kGroupMaxK, at the front of each light list
   std::vector<double> light_bytes;         // algorithmic bytes of each light evaluation launch
   int max_batch = 0;
 };
@@ -449,7 +454,7 @@ struct BatchPlan {
 struct SbpGraph {
   int V = 0;
   long long E = 0;
-  DevBuf<int> out_ptr, out_idx, out_src, in_ptr, in_idx, identity, high_dev;
+  DevBuf<int> out_ptr, out_idx, out_src, in_ptr, in_idx, adj, identity, high_dev;
   DevBuf<unsigned char> self;
   std::vector<int> h_k;        // k_out + k_in per vertex (self loop counted once, on the out side)
   std::vector<int> high, low;  // hybrid split
@@ -467,6 +472,7 @@ struct SbpGraph {
     g.out_idx = out_idx.p;
     g.in_ptr = in_ptr.p;
     g.in_idx = in_idx.p;
+    g.adj = adj.p;
     g.self = self.p;
     return g;
   }
@@ -496,28 +502,58 @@ struct SbpGraph {
     std::vector<int> order;
     order.reserve(n);
     if (batch_size > 0) {
-      for (int bt = 0; bt < n / batch_size; ++bt) {
-        const int start = bt * batch_size, end = std::min(n, (bt + 1) * batch_size);
-        p->light_begin.push_back((int)order.size());
-        for (int i = start; i < end; ++i)   // vertices that fit the group tables first
-          if (h_k[list[i]] <= std::min(kGroupMaxK, light_cap / 2)) order.push_back(list[i]);
-        p->group_n.push_back((int)order.size() - p->light_begin.back());
-        for (int i = start; i < end; ++i)
-          if (h_k[list[i]] > kGroupMaxK && h_k[list[i]] <= light_cap / 2) order.push_back(list[i]);
-        p->light_n.push_back((int)order.size() - p->light_begin.back());
+      // Inside a batch the evaluation order is free (every vertex sees the frozen state): by
+      // degree, largest first, so that the groups of a warp finish together and the last tasks
+      // are the short ones.  A counting sort of the whole list by degree (equal degrees in list
+      // order), then each vertex to its batch.
+      const int nb = n / batch_size;
+      std::vector<int> start((size_t)max_k + 2, 0), by_degree(n), sorted((size_t)nb * batch_size), fill(nb, 0);
+      for (int i = 0; i < n; ++i) start[(size_t)(max_k - h_k[list[i]]) + 1]++;
+      for (int k = 0; k <= max_k; ++k) start[k + 1] += start[k];
+      for (int i = 0; i < n; ++i) by_degree[start[max_k - h_k[list[i]]]++] = i;
+      for (int i : by_degree) {
+        const int bt = i / batch_size;
+        if (bt < nb) sorted[(size_t)bt * batch_size + fill[bt]++] = list[i];
+      }
+      for (int bt = 0; bt < nb; ++bt) {
+        const int first = bt * batch_size, end = first + batch_size;
+        const int* part = sorted.data() + (size_t)first;
+        BatchDesc d = {};
+        while (d.heavy_n < end - first && h_k[part[d.heavy_n]] > light_cap / 2) d.heavy_n++;
+        d.light_begin = (int)order.size();
+        d.light_n = end - first - d.heavy_n;
+        d.heavy_begin = d.light_begin + d.light_n;
         double lb = 0.0;   // 12 B (CSR offsets + b[v]) + 8 B per neighbour (id + block gather)
-        for (int i = p->light_begin.back(); i < (int)order.size(); ++i) lb += 12.0 + 8.0 * h_k[order[i]];
+        for (int i = d.heavy_n; i < end - first; ++i) {
+          const int k = h_k[part[i]];
+          order.push_back(part[i]);
+          lb += 12.0 + 8.0 * k;
+          if (k > group_max_k(16)) d.n32++;
+          else if (k > group_max_k(8)) d.n16++;
+        }
+        order.insert(order.end(), part, part + d.heavy_n);
+        p->light_begin.push_back(d.light_begin);
+        p->light_n.push_back(d.light_n);
         p->light_bytes.push_back(lb);
-        p->heavy_begin.push_back((int)order.size());
-        for (int i = start; i < end; ++i)
-          if (h_k[list[i]] > light_cap / 2) order.push_back(list[i]);
-        p->heavy_n.push_back((int)order.size() - p->heavy_begin.back());
-        p->max_batch = std::max(p->max_batch, end - start);
+        p->heavy_begin.push_back(d.heavy_begin);
+        p->heavy_n.push_back(d.heavy_n);
+        p->desc.push_back(d);
+        p->max_batch = std::max(p->max_batch, end - first);
       }
     }
     p->order.reserve(order.size());
-    if (!order.empty())
-      SBP_CUDA(SBP_COPY(p->order.p, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice));
+    p->recs.reserve(order.size());
+    p->desc_dev.reserve(p->desc.size());
+    if (!order.empty()) {
+      Context& c = Context::get();
+      SBP_CUDA(SBP_COPY_ASYNC(p->order.p, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, c.stream));
+      SBP_CUDA(SBP_COPY_ASYNC(p->desc_dev.p, p->desc.data(), p->desc.size() * sizeof(BatchDesc), cudaMemcpyHostToDevice,
+                              c.stream));
+      k_vertex_records<<<grid_for((long long)order.size(), 256, 8 * c.num_sms), 256, 0, c.stream>>>(
+          view(), p->order.p, (int)order.size(), p->recs.p);
+      SBP_CHECK_LAUNCH();
+      c.sync();
+    }
     auto& ref = *p;
     plans[key] = std::move(p);
     return ref;
@@ -535,7 +571,7 @@ struct SbpBlockmodel {
   DevBuf<int> prop, qr, qs, moved, n_moved;   // n_moved: two slots, alternating per batch
   DevBuf<unsigned long long> last;           // (batch generation << 32 | last mover) per block
   unsigned gen = 0;                          // batch generation
-  int nch = 0;
+  int nch = 0, ncs = 0;
   // row-hashed representation (B > dense_max_blocks)
   bool sparse = false;
   DevBuf<long long> rbase, cbase;
@@ -560,6 +596,7 @@ struct SbpBlockmodel {
     v.overflow = overflow.p;
     v.ld = ld;
     v.nch = nch;
+    v.ncs = ncs;
     v.CS = CS.p;
     v.CST = CST.p;
     v.b = b.p;
@@ -608,6 +645,7 @@ struct SbpBlockmodel {
     }
     ld = ((B + kChunk - 1) / kChunk) * kChunk;
     nch = (B + kChunk - 1) / kChunk;
+    ncs = (nch + 3) & ~3;
     if (sparse) {
       rbase.reserve(B);
       cbase.reserve(B);
@@ -618,8 +656,8 @@ struct SbpBlockmodel {
       const size_t cells = (size_t)B * (size_t)ld;
       P.reserve(cells);
       if (nch > 1) {
-        CS.reserve((size_t)B * nch);
-        CST.reserve((size_t)B * nch);
+        CS.reserve((size_t)B * ncs);
+        CST.reserve((size_t)B * ncs);
       }
     }
     d_out.reserve(B);
@@ -638,19 +676,22 @@ inline bool use_group_kernel(const SbpBlockmodel& bm) {
 
 void set_smem_limit(const void* fn, size_t bytes);
 
-// Launch of the group kernel over n light vertices (dense storage); with hashed group tables
-// (B > kSmallB) every vertex must have k <= kGroupMaxK.
-inline void launch_group_eval(const SbpGraph& g, SbpBlockmodel& bm, const int* verts, int n, const RngParams& rng,
-                              int sweep, int* n_moved, const SweepCtl* ctl, int batch, cudaStream_t stream) {
-  Context& c = Context::get();
-  const bool hashed_table = bm.B > kSmallB;
-  const int cap = std::min(g.light_cap, 2 * kGroupMaxK);
-  const size_t smem = gibbs_eval_group_smem(hashed_table, cap);
-  const GibbsEvalGroupKernel k = gibbs_eval_group_kernel(hashed_table);
-  set_smem_limit((const void*)k, smem);
-  k<<<grid_for(n, kSmallThreads / kSmallGroup, 64 * c.num_sms), kSmallThreads, smem, stream>>>(
-      g.view(), bm.view(), verts, n, rng, sweep, bm.prop.p, bm.moved.p, n_moved, c.counters, cap, c.status, ctl,
-      batch);
+// Evaluation of one asynchronous-Gibbs batch on dense storage (sbp_gibbs.cu).
+void launch_gibbs_eval(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& plan, int bt, const RngParams& rng,
+                       int sweep, int* n_moved);
+// A whole asynchronous-Gibbs finetune call on dense storage as one persistent kernel.  Only on the
+// process's primary context: two such kernels at once could each hold SMs the other waits for.
+SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, const RngParams& rng,
+                          int max_sweeps, bool bracket);
+// entropy::mdl sums over the cells when there are few of them, else over the edges, on a virtual
+// grid of this many CTAs on every path, so that every path gets the same bits: one CTA per four
+// elements a thread, at most npartial.
+inline bool mdl_cell_form(const SbpBlockmodel& bm, const SbpGraph& g) {
+  return !bm.sparse && (long long)bm.B * bm.B <= 4LL * g.E;
+}
+inline int mdl_grid(const SbpBlockmodel& bm, const SbpGraph& g) {
+  const long long n = std::max<long long>(mdl_cell_form(bm, g) ? (long long)bm.B * bm.B : g.E, bm.B);
+  return grid_for(n, 4 * 256, Context::get().npartial);
 }
 
 struct MhResult {
@@ -778,7 +819,10 @@ void set_smem_limit(const void* fn, size_t bytes);
 void tidy_hashed(SbpBlockmodel& bm, const SbpGraph& g, long long overflows_before);
 void gibbs_apply(SbpBlockmodel& bm, const SbpGraph& g, int batch);
 // One asynchronous-Gibbs batch with the plain proposal (evaluation + apply).
-void gibbs_batch(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, int bt, RngParams rng, int sweep);
+void gibbs_batch(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, int bt, const RngParams& rng, int sweep);
+// Its evaluation half alone.
+void gibbs_eval_batch(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, int bt, const RngParams& rng,
+                      int sweep);
 // finetune::{metropolis_hastings, asynchronous_gibbs, hybrid_mcmc} on the device.
 // `moves` (optional) replays proposals instead of random words.
 void finetune(SbpBlockmodel& bm, SbpGraph& g, int algo, const SbpFinetuneOptions& opt, const SbpReplay* replay,

@@ -24,10 +24,6 @@
 namespace sbpb {
 namespace {
 
-constexpr unsigned kInShift = 15;
-constexpr unsigned kCountMask = (1u << 15) - 1;
-constexpr unsigned kPresent = 1u << 30;
-
 template <int G>
 __device__ __forceinline__ double group_sum(double v) {
 #pragma unroll
@@ -38,11 +34,6 @@ template <int G>
 __device__ __forceinline__ long long group_sum_ll(long long v) {
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o, G);
-  return v;
-}
-__device__ __forceinline__ unsigned long long warp_sum_ull(unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
   return v;
 }
 __device__ __forceinline__ int warp_max_int(int v) {
@@ -291,7 +282,7 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       in_row = target < dot;
       tg = in_row ? target : target - dot;
     }
-    const int* csum = (in_row ? bm.CS : bm.CST) + (size_t)t * bm.nch;
+    const int* csum = (in_row ? bm.CS : bm.CST) + (size_t)t * bm.ncs;
     const int found = group_walk<G, kFrozen>(bm.P + (size_t)t * ld, !in_row, csum, bm.nch, B, tg, walk, gl, gbase);
     if (walk) {
       s = found;
@@ -453,64 +444,6 @@ __device__ __forceinline__ void group_table_clear(const GroupTable<kHash>& T, in
   __syncwarp();
 }
 
-// Direct-indexed tables (33 KB of shared memory per CTA): registers capped for three CTAs per SM
-// (measured 17 % shorter launches than at two CTAs per SM on 71 blocks).  Hashed tables of 256
-// slots take 98 KB per CTA, two CTAs per SM whatever the registers.  (Issuing the loads of four
-// gather steps, or of four delta-MDL entries, together was measured 3-8 % slower.)
-template <int G, bool kHash>
-__global__ void __launch_bounds__(kSmallThreads, kHash ? 2 : 3)
-    k_gibbs_eval_group(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
-                       int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status,
-                       const SweepCtl* ctl, int batch) {
-  constexpr int kGroups = kSmallThreads / G;
-  extern __shared__ int group_smem[];
-  const int slots = kHash ? cap : kSmallB;
-  if (ctl) {
-    sweep = ctl->sweep;
-    n_moved = ctl->n_moved + ((ctl->gen0 + (unsigned)batch) & 1u);
-  }
-  const int lane = threadIdx.x & 31;
-  const int gl = lane & (G - 1);
-  const int gid = threadIdx.x / G;
-  const int gbase = lane & ~(G - 1);   // first lane of this group in the warp
-  const GroupTable<kHash> T = group_table<kHash>(group_smem, kGroups, gid, slots, status);
-  group_table_init<kHash, G>(T, slots, gl);
-  unsigned long long c_visit = 0, c_moved = 0, c_acc = 0;
-  const bool given = rng.moves != 0;
-  const int groups_total = gridDim.x * kGroups;
-  // warp-uniform outer loop: the warp's groups take consecutive list entries
-  const int warp_first = (blockIdx.x * kSmallThreads + (threadIdx.x & ~31)) / G;
-  for (int base = warp_first; base < n; base += groups_total) {
-    const int item = base + (lane / G);
-    const bool valid = item < n;
-    int v = 0;
-    uint4 x = make_uint4(0, 0, 0, 0);
-    if (valid) {
-      v = __ldg(verts + item);
-      x = draw_record(rng, (uint32_t)v, (uint32_t)sweep, 0u, (long long)sweep * g.V + v, status);
-    }
-    const GroupEval e = group_evaluate<G, kHash, true>(g, bm, T, valid, v, given, x, gl, gbase, status);
-    if (e.accepted && gl == 0) {
-      c_acc++;
-      prop[v] = e.s;
-      moved_list[atomicAdd(n_moved, 1)] = v;
-    }
-    if (valid && gl == 0) {
-      c_visit++;
-      if (e.s != e.r) c_moved++;
-    }
-    group_table_clear<kHash, G>(T, gl);
-  }
-  c_visit = warp_sum_ull(c_visit);
-  c_moved = warp_sum_ull(c_moved);
-  c_acc = warp_sum_ull(c_acc);
-  if (lane == 0 && c_visit) {
-    atomicAdd(counters + 0, c_visit);
-    atomicAdd(counters + 1, c_moved);
-    atomicAdd(counters + 2, c_acc);
-  }
-}
-
 // Metropolis-Hastings over a vertex list with exact sequential semantics (finetune::
 // metropolis_hastings, src/finetune.cpp:412-444), dense storage, one CTA of kMhGroupThreads:
 // each round the groups evaluate the next kMhGroupThreads / G vertices of the list against the
@@ -659,16 +592,6 @@ __global__ void __launch_bounds__(kMhGroupThreads)
 }
 
 }  // namespace
-
-GibbsEvalGroupKernel gibbs_eval_group_kernel(bool hashed_table) {
-  return hashed_table ? k_gibbs_eval_group<kSmallGroup, true> : k_gibbs_eval_group<kSmallGroup, false>;
-}
-
-size_t gibbs_eval_group_smem(bool hashed_table, int cap) {
-  const int groups = kSmallThreads / kSmallGroup;
-  const int slots = hashed_table ? cap : kSmallB;
-  return sizeof(int) * ((size_t)groups + (size_t)groups * (hashed_table ? 3 : 2) * slots);
-}
 
 MhGroupKernel mh_group_kernel(bool hashed_table) {
   return hashed_table ? k_mh_group<kSmallGroup, true> : k_mh_group<kSmallGroup, false>;

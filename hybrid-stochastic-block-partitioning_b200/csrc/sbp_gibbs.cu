@@ -1,0 +1,355 @@
+// Asynchronous Gibbs on a dense block matrix (finetune::asynchronous_gibbs, src/finetune.cpp:31-89):
+// the evaluation of one batch as a kernel of its own, and a whole finetune call -- every sweep's
+// batches, the MDL and the early stop -- as one persistent kernel.
+#include <cooperative_groups.h>
+
+#include "sbp_engine.cuh"
+#include "sbp_group.cuh"
+#include "sbp_steps.cuh"
+
+namespace sbpb {
+namespace {
+
+struct EvalCounts {
+  unsigned visit = 0, moved = 0, acc = 0;
+};
+
+// Everything one batch's evaluation needs; `store_index`: the moved list gets plan indices
+// (records are looked up again by the apply), else vertex ids.
+struct EvalArgs {
+  GraphView g;
+  BlockView bm;
+  const int4* recs;      // vertex records in plan order
+  RngParams rng;
+  int* prop;
+  int* moved;
+  int* status;
+  int gmin;              // smallest group
+  int slots;             // table slots of the CTA (kGroupWarps regions, or more for a heavy vertex)
+  int store_index;
+};
+
+template <bool kDirect, Store ST>
+__device__ __forceinline__ void eval_task(const EvalArgs& a, const GroupTab<kDirect>& T, int index, bool valid, int sweep,
+                                          int* n_moved, const Lanes& L, EvalCounts& cnt) {
+  const int4 rec = valid ? __ldg(a.recs + index) : make_int4(0, 0, 0, 0);
+  uint4 x = make_uint4(0, 0, 0, 0);
+  if (valid)
+    x = draw_record(a.rng, (uint32_t)rec.x, (uint32_t)sweep, 0u, (long long)sweep * a.g.V + rec.x, a.status);
+  const GroupEval e = group_evaluate<kDirect, ST>(a.g, a.bm, T, valid, rec, a.rng.moves != 0, x, L, a.status);
+  if (valid && L.gl == 0) {
+    cnt.visit++;
+    if (e.s != e.r) cnt.moved++;
+    if (e.accepted) {
+      cnt.acc++;
+      a.prop[e.v] = e.s;
+      a.moved[atomicAdd(n_moved, 1)] = a.store_index ? index : e.v;
+    }
+  }
+  T.clear(e.n, L);
+}
+
+// One batch: tasks of 32 / G vertices, a warp each, the largest degrees first.  Strided over the
+// grid, so with the batch ordered by degree every warp gets a similar share.
+template <bool kDirect, Store ST>
+__device__ __forceinline__ void eval_batch(const EvalArgs& a, BatchDesc b, int sweep, int* n_moved, int* smem,
+                                           EvalCounts& cnt) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wid = blockIdx.x * kGroupWarps + warp, nw = gridDim.x * kGroupWarps;
+  if (kDirect) {   // any degree fits a direct-indexed histogram
+    const Lanes L(32, lane);
+    const GroupTab<kDirect> T = group_tab<kDirect>(smem, a.slots, warp * kRegionSlots, kRegionSlots);
+    for (int h = wid; h < b.heavy_n; h += nw) eval_task<kDirect, ST>(a, T, b.heavy_begin + h, true, sweep, n_moved, L, cnt);
+  } else if (b.heavy_n > 0) {   // one warp with the whole CTA's table
+    const Lanes L(32, lane);
+    const GroupTab<kDirect> T = group_tab<kDirect>(smem, a.slots, 0, a.slots);
+    for (int h = blockIdx.x; h < b.heavy_n; h += gridDim.x)
+      if (warp == 0) eval_task<kDirect, ST>(a, T, b.heavy_begin + h, true, sweep, n_moved, L, cnt);
+    __syncthreads();
+  }
+  const int n = b.light_n;
+  const int c32 = a.gmin >= 32 ? n : b.n32;
+  const int c16 = a.gmin >= 32 ? 0 : a.gmin >= 16 ? n - c32 : b.n16;
+  const int t16 = (c16 + 1) >> 1, t8 = (n - c32 - c16 + 3) >> 2;
+  for (int task = wid; task < c32 + t16 + t8; task += nw) {
+    const int G = task < c32 ? 32 : task < c32 + t16 ? 16 : 8;
+    const int first = G == 32 ? task : G == 16 ? c32 + 2 * (task - c32) : c32 + c16 + 4 * (task - c32 - t16);
+    const int end = G == 32 ? c32 : G == 16 ? c32 + c16 : n;
+    const Lanes L(G, lane);
+    const int item = first + lane / G;
+    const GroupTab<kDirect> T =
+        group_tab<kDirect>(smem, a.slots, warp * kRegionSlots + (lane / G) * (kRegionSlots / 32) * G, kRegionSlots / 32 * G);
+    eval_task<kDirect, ST>(a, T, b.light_begin + item, item < end, sweep, n_moved, L, cnt);
+  }
+}
+
+__device__ __forceinline__ void add_counts(EvalCounts c, unsigned long long* counters) {
+  const unsigned v = __reduce_add_sync(kFull, c.visit), m = __reduce_add_sync(kFull, c.moved),
+                 x = __reduce_add_sync(kFull, c.acc);
+  if ((threadIdx.x & 31) == 0 && v) {
+    atomicAdd(counters + 0, (unsigned long long)v);
+    atomicAdd(counters + 1, (unsigned long long)m);
+    atomicAdd(counters + 2, (unsigned long long)x);
+  }
+}
+
+template <bool kDirect>
+__global__ void __launch_bounds__(kGroupThreads, 3)
+    k_gibbs_eval(const __grid_constant__ EvalArgs a, BatchDesc b, int sweep, int* n_moved, unsigned long long* counters) {
+  extern __shared__ int smem[];
+  group_tabs_init<kDirect>(smem, a.slots);
+  __syncthreads();
+  EvalCounts cnt;
+  eval_batch<kDirect, Store::kDenseFrozen>(a, b, sweep, n_moved, smem, cnt);
+  add_counts(cnt, counters);
+}
+
+// ------------------------------------------------------------------------------------------
+// A whole finetune call in one kernel.  Per batch: evaluation, apply, degree step, each over the
+// whole grid and separated by a barrier over the grid; per sweep: the MDL's partial sums, then
+// every CTA forms the same total and takes the same early-stop decision
+// (src/finetune.cpp:144-162), so no CTA waits for another's.  As launches (three per batch, replayed
+// by a CUDA graph) the same work paid a launch gap and a ramp-up and tail per step.
+//
+// The barrier is the cluster's where the grid is one cluster (small batches), else a counter in
+// global memory, for which the kernel is launched cooperatively: every CTA is resident.  A wait
+// gives up after an iteration limit: the CTA that gives up sets the status word and the abort flag
+// and every CTA leaves at its next barrier.
+// Loads of state that another phase writes are plain loads: the barrier's acquire makes them
+// coherent.  Only what no phase writes goes through the read-only cache.
+// ------------------------------------------------------------------------------------------
+struct SweepsArgs {
+  EvalArgs e;
+  const BatchDesc* batches;
+  int nbatches;
+  int max_sweeps;
+  int bracket;
+  int mdl_cells;
+  int mdl_ctas;
+  int cluster;              // 1: the grid is one cluster
+  unsigned gen0;            // batch generation before the call
+  unsigned wait_limit;      // polls of a barrier before it gives up
+  int* qr;
+  int* qs;
+  unsigned long long* last;
+  const int* out_src;
+  double* partial;
+  unsigned long long* counters;
+  int* n_moved;             // three slots taken in turn, zero at launch
+  unsigned* bar;            // [0] arrivals (0 at launch), [1] abort flag (0 at launch)
+  SweepsResult* result;
+};
+
+// Barrier over the grid; false when a wait gave up (the same for every thread of the CTA).
+__device__ __forceinline__ bool sync_grid(const SweepsArgs& a, unsigned* target, int* s_abort) {
+  if (a.cluster) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return true;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    *target += gridDim.x;
+    atomicAdd(a.bar, 1u);
+    unsigned polls = 0, seen;
+    for (;;) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.bar) : "memory");
+      if ((int)(seen - *target) >= 0) break;
+      ++polls;
+      if ((polls & 1023u) == 0 && *(volatile unsigned*)(a.bar + 1)) {
+        *s_abort = 1;
+        break;
+      }
+      if (polls > a.wait_limit) {
+        atomicOr(a.e.status, kErrGridWait);
+        atomicExch(a.bar + 1, 1u);
+        *s_abort = 1;
+        break;
+      }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  return *(volatile int*)s_abort == 0;
+}
+
+template <bool kDirect>
+__global__ void __launch_bounds__(kGroupThreads, 3) k_gibbs_sweeps(const __grid_constant__ SweepsArgs a) {
+  extern __shared__ int smem[];
+  __shared__ double red[32];
+  __shared__ int s_abort, s_stop;
+  const GraphView& g = a.e.g;
+  const BlockView& bm = a.e.bm;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wid = blockIdx.x * kGroupWarps + warp, nw = gridDim.x * kGroupWarps;
+  group_tabs_init<kDirect>(smem, a.e.slots);
+  if (tid == 0) s_abort = 0;
+  unsigned target = 0;
+  EvalCounts cnt;
+  double constant = 0.0, initial = 0.0, mdl = 0.0, d1 = 0.0, d2 = 0.0;   // thread 0: MDL terms, the last two deltas
+  if (tid == 0) constant = mdl_constant(g.V, g.E, bm.B);
+  unsigned gen = a.gen0;
+  int slot = 0;
+  int count = 0;
+  for (int it = -1;; ++it) {
+    if (it >= 0) {
+      for (int bt = 0; bt < a.nbatches; ++bt) {
+        const BatchDesc b = a.batches[bt];
+        int* n_cur = a.n_moved + slot;
+        slot = slot == 2 ? 0 : slot + 1;
+        if (blockIdx.x == 0 && tid == 0) a.n_moved[slot] = 0;   // the next batch's; last read two barriers ago
+        eval_batch<kDirect, Store::kDense>(a.e, b, it, n_cur, smem, cnt);
+        if (!sync_grid(a, &target, &s_abort)) return;
+        const int n = *(volatile int*)n_cur;
+        ++gen;
+        if (n == 0) continue;   // the same for the whole grid
+        for (int i = wid; i < n; i += nw)
+          apply_moved_record(g, bm, __ldg(a.e.recs + a.e.moved[i]), a.e.prop, a.qr, a.qs, a.last, gen, lane);
+        if (!sync_grid(a, &target, &s_abort)) return;
+        for (int i = blockIdx.x * kGroupThreads + tid; i < n; i += gridDim.x * kGroupThreads)
+          finish_moved_vertex(bm, __ldg(&a.e.recs[a.e.moved[i]].x), a.e.prop, a.qr, a.qs, a.last, gen);
+        if (!sync_grid(a, &target, &s_abort)) return;
+      }
+    }
+    // entropy::mdl over the virtual grid of every other path
+    for (int vc = blockIdx.x; vc < a.mdl_ctas; vc += gridDim.x) {
+      const double t = a.mdl_cells ? mdl_cells_part(bm, vc, a.mdl_ctas, red)
+                                   : mdl_edges_part(g, bm, a.out_src, vc, a.mdl_ctas, red);
+      if (tid == 0) a.partial[vc] = t;
+    }
+    if (!sync_grid(a, &target, &s_abort)) return;
+    const double L = mdl_total(a.partial, a.mdl_ctas, red);
+    if (tid == 0) {
+      mdl = constant - L;
+      bool stop = false;
+      if (it < 0) {
+        initial = (double)(float)mdl;   // the reference stores the entropy as float
+        if (blockIdx.x == 0) a.result->initial = mdl;
+      } else {
+        const double d0 = mdl - initial;   // last_iteration_entropy is never updated
+        if (d0 == 0.0) {
+          stop = true;
+        } else if (it >= 3) {
+          double average = d0 + d1 + d2;
+          average /= -3.0;
+          stop = average < (a.bracket ? 1e-4 * initial : 5e-4 * initial);
+        }
+        d2 = d1;
+        d1 = d0;
+        if (it + 1 >= a.max_sweeps) stop = true;
+      }
+      s_stop = stop ? 1 : 0;
+    }
+    __syncthreads();
+    count = it + 1;
+    if (s_stop) break;
+    __syncthreads();
+  }
+  add_counts(cnt, a.counters);
+  if (blockIdx.x == 0 && tid == 0) {
+    a.result->mdl = mdl;
+    a.result->sweeps = count;
+  }
+}
+
+EvalArgs eval_args(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& plan, const RngParams& rng) {
+  EvalArgs a;
+  a.g = g.view();
+  a.bm = bm.view();
+  a.recs = plan.recs.p;
+  a.rng = rng;
+  a.prop = bm.prop.p;
+  a.moved = bm.moved.p;
+  a.status = Context::get().status;
+  // a heavy vertex needs a slot for each of its distinct neighbour blocks, of which there are at
+  // most B; twice that many while they fit
+  const int distinct = std::min(g.max_k, bm.B);
+  a.slots = std::max(kGroupWarps * kRegionSlots, std::min(kMaxCap, pow2_at_least(2 * distinct)));
+  a.store_index = 0;
+  a.gmin = 8;
+  return a;
+}
+
+// Smallest group for a batch: eight lanes a vertex once that still gives every resident warp a
+// task, else as many lanes as the idle warps allow -- a visit's chain gets shorter with more lanes.
+int group_min(int batch, int warps) {
+  if (g_group_kernel == 0) return 32;
+  if (g_group_kernel == 2) return 8;
+  return batch >= 4 * warps / 2 ? 8 : batch >= warps ? 16 : 32;
+}
+
+}  // namespace
+
+void launch_gibbs_eval(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& plan, int bt, const RngParams& rng,
+                       int sweep, int* n_moved) {
+  Context& c = Context::get();
+  EvalArgs a = eval_args(g, bm, plan, rng);
+  const BatchDesc& d = plan.desc[bt];
+  const int n = d.light_n + d.heavy_n;
+  const bool direct = bm.B <= kSmallB;
+  a.gmin = group_min(n, 3 * kGroupWarps * c.num_sms);
+  const size_t smem = group_smem_bytes(direct, a.slots);
+  const auto k = direct ? k_gibbs_eval<true> : k_gibbs_eval<false>;
+  set_smem_limit((const void*)k, smem);
+  k<<<grid_for((long long)n * a.gmin, 32 * kGroupWarps, 64 * c.num_sms), kGroupThreads, smem, c.stream>>>(
+      a, d, sweep, n_moved, c.counters);
+}
+
+SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, const RngParams& rng,
+                          int max_sweeps, bool bracket) {
+  Context& c = Context::get();
+  SweepsArgs a;
+  a.e = eval_args(g, bm, plan, rng);
+  a.e.store_index = 1;
+  a.batches = plan.desc_dev.p;
+  a.nbatches = (int)plan.desc.size();
+  a.max_sweeps = max_sweeps;
+  a.bracket = bracket ? 1 : 0;
+  a.mdl_cells = mdl_cell_form(bm, g) ? 1 : 0;
+  a.mdl_ctas = mdl_grid(bm, g);
+  a.gen0 = bm.gen;
+  a.wait_limit = kGridWaitLimit;
+  a.qr = bm.qr.p;
+  a.qs = bm.qs.p;
+  a.last = bm.last.p;
+  a.out_src = g.out_src.p;
+  a.partial = c.partial;
+  a.counters = c.counters;
+  a.n_moved = c.sweep_words;
+  a.bar = reinterpret_cast<unsigned*>(c.sweep_words + 4);
+  a.result = c.sweep_result;
+  const bool direct = bm.B <= kSmallB;
+  const size_t smem = group_smem_bytes(direct, a.e.slots);
+  const auto k = direct ? k_gibbs_sweeps<true> : k_gibbs_sweeps<false>;
+  set_smem_limit((const void*)k, smem);
+  int per_sm = 0;
+  SBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kGroupThreads, smem));
+  if (per_sm < 1) throw Error(SBP_ERR_UNSUPPORTED, "vertex degree too large for the finetune kernel");
+  const int resident = per_sm * c.num_sms;
+  a.e.gmin = group_min(plan.max_batch, resident * kGroupWarps);
+  const int wanted = (int)std::max<long long>(((long long)plan.max_batch * a.e.gmin / 32 + kGroupWarps - 1) / kGroupWarps,
+                                              a.mdl_ctas);
+  const int grid = std::max(1, std::min(resident, wanted));
+  a.cluster = 0;
+  SBP_CUDA(cudaMemsetAsync(c.sweep_words, 0, 8 * sizeof(int), c.stream));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kGroupThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c.stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  SBP_CUDA(cudaLaunchKernelEx(&cfg, k, a));
+  SBP_CHECK_LAUNCH();
+  SweepsResult r;
+  SBP_CUDA(SBP_COPY_ASYNC(&r, c.sweep_result, sizeof r, cudaMemcpyDeviceToHost, c.stream));
+  c.sync();
+  c.check_status();   // before the result is used: an aborted kernel leaves none
+  bm.gen += (unsigned)(a.nbatches * r.sweeps);
+  return r;
+}
+
+}  // namespace sbpb

@@ -3,7 +3,7 @@
 // Kernel map (reference function each one stands in for):
 //   k_rebuild_*        Blockmodel::initialize_edge_counts     src/blockmodel/blockmodel.cpp:187-255
 //   k_mdl              entropy::mdl / log_posterior_probability src/entropy.cpp:584-589, blockmodel.cpp:267-285
-//   k_gibbs_eval_*     asynchronous_gibbs evaluation half     src/finetune.cpp:49-57, 531-545
+//   k_gibbs_eval_hashed asynchronous_gibbs evaluation half    src/finetune.cpp:49-57, 531-545
 //   k_apply_*          asynchronous_gibbs apply half          src/finetune.cpp:58-71 + Blockmodel::move_vertex
 //   k_mh               metropolis_hastings sweep              src/finetune.cpp:412-444, 446-501
 //   k_row_nnz/fill     ISparseMatrix row/column views for the merge phase
@@ -133,19 +133,14 @@ __global__ void k_rebuild_degrees(BlockView bm) {
   if (x < bm.B) bm.d[x] = bm.d_out[x] + bm.d_in[x] - bm_get(bm, x, x);
 }
 // ------------------------------------------------------------------------------------------
-// Asynchronous Gibbs: evaluate a list of vertices against the frozen state.  Accepted moves
+// Asynchronous Gibbs on row-hashed storage: evaluate a list of vertices against the frozen state,
+// one warp per vertex (dense storage: sbp_gibbs.cu).  Accepted moves
 // go to prop[v] and the moved list; counters: [0] visits [1] proposals_moved [2] accepted.
 // ------------------------------------------------------------------------------------------
-template <Store ST>
-__device__ __forceinline__ void gibbs_eval_body(GraphView g, BlockView bm, const int* __restrict__ verts, int n,
-                                                RngParams rng, int sweep, int* prop, int* moved_list, int* n_moved,
-                                                unsigned long long* counters, int cap, int* status,
-                                                const SweepCtl* ctl, int batch) {
+__global__ void __launch_bounds__(256, 2)
+    k_gibbs_eval_hashed(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
+                        int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status) {
   extern __shared__ int smem[];
-  if (ctl) {
-    sweep = ctl->sweep;
-    n_moved = ctl->n_moved + ((ctl->gen0 + (unsigned)batch) & 1u);
-  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wpb = blockDim.x >> 5;
   WarpTable t = carve_table(smem, cap, warp);
@@ -155,7 +150,8 @@ __device__ __forceinline__ void gibbs_eval_body(GraphView g, BlockView bm, const
     const int v = verts[i];
     const uint4 x = draw_record(rng, (uint32_t)v, (uint32_t)sweep, 0u, (long long)sweep * g.V + v, status);
     int r, k_out, k_in;
-    const EvalResult res = evaluate_vertex<ST>(g, bm, v, x, t, lane, status, &r, &k_out, &k_in, rng.moves != 0);
+    const EvalResult res =
+        evaluate_vertex<Store::kHashed>(g, bm, v, x, t, lane, status, &r, &k_out, &k_in, rng.moves != 0);
     c_visit++;
     if (res.s != r) c_moved++;
     if (res.accepted) {
@@ -174,45 +170,13 @@ __device__ __forceinline__ void gibbs_eval_body(GraphView g, BlockView bm, const
   }
 }
 
-__global__ void __launch_bounds__(256, 2)
-    k_gibbs_eval_dense(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
-                       int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status,
-                       const SweepCtl* ctl, int batch) {
-  gibbs_eval_body<Store::kDenseFrozen>(g, bm, verts, n, rng, sweep, prop, moved_list, n_moved, counters, cap, status,
-                                       ctl, batch);
-}
-// The same with registers capped for three CTAs per SM (a few spilled values): more vertices in
-// flight, which pays while the block matrix is small enough for its cells to hit in L2.
-__global__ void __launch_bounds__(256, 3)
-    k_gibbs_eval_dense_occ3(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
-                            int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap,
-                            int* status, const SweepCtl* ctl, int batch) {
-  gibbs_eval_body<Store::kDenseFrozen>(g, bm, verts, n, rng, sweep, prop, moved_list, n_moved, counters, cap, status,
-                                       ctl, batch);
-}
-__global__ void __launch_bounds__(256, 2)
-    k_gibbs_eval_hashed(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
-                        int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status,
-                        const SweepCtl* ctl, int batch) {
-  gibbs_eval_body<Store::kHashed>(g, bm, verts, n, rng, sweep, prop, moved_list, n_moved, counters, cap, status, ctl,
-                                  batch);
-}
-
-
-// Apply accepted moves of one batch.  Every edge incident to a moved vertex moves once from
-// its old cell to its new cell; the result equals the reference's one-by-one application.
-// qr/qs keep the reference's diagonal delta of each move as seen at its turn in vertex order,
-// which Blockmodel::move_vertex folds into d[r], d[s] (blockmodel.cpp:348-359).
+// Apply accepted moves of one batch.
 // Every edge incident to a moved vertex moves once from its old cell to its new cell; the
 // result equals the reference's one-by-one application.  qr/qs keep the reference's diagonal
 // delta of each move as seen at its turn in vertex order, which Blockmodel::move_vertex folds
 // into d[r], d[s] (blockmodel.cpp:348-359); last[x] keeps (batch generation, last mover of x).
 __global__ void k_apply_edges(GraphView g, BlockView bm, const int* moved_list, const int* n_moved, const int* prop,
-                              int* qr, int* qs, unsigned long long* last, unsigned gen, const SweepCtl* ctl, int batch) {
-  if (ctl) {
-    gen = ctl->gen0 + (unsigned)batch + 1u;
-    n_moved = ctl->n_moved + ((gen - 1u) & 1u);
-  }
+                              int* qr, int* qs, unsigned long long* last, unsigned gen) {
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -223,49 +187,19 @@ __global__ void k_apply_edges(GraphView g, BlockView bm, const int* moved_list, 
 // d[r], d[s] from the last mover of each block, then the new assignment; clears the other
 // moved-count slot for the next batch.
 __global__ void k_apply_finish(BlockView bm, const int* moved_list, const int* n_moved, int* next_n_moved, int* prop,
-                               const int* qr, const int* qs, const unsigned long long* last, unsigned gen,
-                               const SweepCtl* ctl, int batch) {
-  if (ctl) {
-    gen = ctl->gen0 + (unsigned)batch + 1u;
-    n_moved = ctl->n_moved + ((gen - 1u) & 1u);
-    next_n_moved = ctl->n_moved + (gen & 1u);
-  }
+                               const int* qr, const int* qs, const unsigned long long* last, unsigned gen) {
   const int n = *n_moved;
   if (blockIdx.x == 0 && threadIdx.x == 0) *next_n_moved = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     finish_moved_vertex(bm, moved_list[i], prop, qr, qs, last, gen);
 }
 
-// End of one sweep of a graph-run finetune: record delta = MDL - first MDL (the asynchronous-
-// Gibbs rule, src/finetune.cpp:40,74) and apply finetune::early_stop (src/finetune.cpp:144-162)
-// in the host's arithmetic; the loop continues while it does not stop.
-__device__ __forceinline__ void sweep_control(SweepCtl* ctl, double mdl, cudaGraphConditionalHandle loop) {
-  const int it = ctl->count;
-  ctl->deltas[it] = mdl - ctl->initial;
-  ctl->count = it + 1;
-  bool stop;
-  if (ctl->deltas[it] == 0.0) {
-    stop = true;
-  } else if (it < 3) {
-    stop = false;
-  } else {
-    double average = ctl->deltas[it] + ctl->deltas[it - 1] + ctl->deltas[it - 2];
-    average /= -3.0;
-    const double threshold = ctl->bracket ? 1e-4 * ctl->initial : 5e-4 * ctl->initial;
-    stop = average < threshold;
-  }
-  if (ctl->count >= ctl->max_sweeps) stop = true;
-  ctl->sweep = it + 1;
-  ctl->gen0 += (unsigned)ctl->nbatches;
-  cudaGraphSetConditional(loop, stop ? 0u : 1u);
-}
-
 // entropy::mdl (src/entropy.cpp:584-589) in one launch.  Every CTA writes its partial sum (cell
 // form when B*B <= 4E on dense storage, else the edge form); the CTA that finishes last (a
 // counter taken after a memory fence) sums the partials in a fixed order and applies the
-// formula.  With a graph-run sweep (ctl) it then records the sweep and sets the loop condition.
+// formula.
 __global__ void k_mdl(GraphView g, BlockView bm, const int* __restrict__ out_src, int cells, double* partial,
-                      unsigned* done, double* out, SweepCtl* ctl, cudaGraphConditionalHandle loop) {
+                      unsigned* done, double* out) {
   __shared__ double red[32];
   __shared__ int s_last;
   const double t = cells ? mdl_cells_part(bm, blockIdx.x, gridDim.x, red)
@@ -282,7 +216,6 @@ __global__ void k_mdl(GraphView g, BlockView bm, const int* __restrict__ out_src
   if (threadIdx.x == 0) {
     *out = v;
     *done = 0u;
-    if (ctl) sweep_control(ctl, v, loop);
   }
 }
 
@@ -664,6 +597,24 @@ __global__ void k_pairs_to_dense(const int2* __restrict__ P, int B, int ld, int 
     const int r = (int)(i / B), c = (int)(i - (long long)r * B);
     dense[i] = P[(size_t)(row0 + r) * ld + c].x;
   }
+}
+
+// The joint neighbour list: each vertex's out-list, then its in-list.  Eight lanes per vertex.
+__global__ void k_join_lists(int V, const int* __restrict__ out_ptr, const int* __restrict__ out_idx,
+                             const int* __restrict__ in_ptr, const int* __restrict__ in_idx, int* adj) {
+  const int gl = threadIdx.x & 7;
+  const int step = (gridDim.x * blockDim.x) >> 3;
+  for (int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; v < V; v += step) {
+    const int o0 = out_ptr[v], ko = out_ptr[v + 1] - o0, i0 = in_ptr[v], ki = in_ptr[v + 1] - i0;
+    int* to = adj + ((unsigned)o0 + (unsigned)i0);
+    for (int j = gl; j < ko; j += 8) to[j] = __ldg(out_idx + o0 + j);
+    for (int j = gl; j < ki; j += 8) to[ko + j] = __ldg(in_idx + i0 + j);
+  }
+}
+
+__global__ void k_vertex_records(GraphView g, const int* __restrict__ verts, int n, int4* recs) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    recs[i] = vertex_record(g, verts[i]);
 }
 
 __global__ void k_relabel(int* b, int V, const int* map) {

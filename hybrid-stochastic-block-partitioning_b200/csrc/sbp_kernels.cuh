@@ -1,25 +1,25 @@
 // Kernel prototypes shared by the kernel and host translation units.
 #pragma once
-#include "sbp_device.cuh"
+#include "sbp_group.cuh"
 
 namespace sbpb {
 
 constexpr int kProposalsPerBlock = 10;   // block_merge::NUM_AGG_PROPOSALS_PER_BLOCK (include/block_merge.hpp:24)
 constexpr int kMaxIterations = 100;      // finetune::MAX_NUM_ITERATIONS (include/finetune.hpp:56)
 
-// Device-side state of an asynchronous-Gibbs finetune run as one CUDA graph: the loop over
-// sweeps and its early stop are decided on the GPU (k_mdl).  Kernels given a
-// control block read the sweep index and the batch generation from it.
-struct SweepCtl {
-  int sweep;               // index of the sweep being run
-  unsigned gen0;           // batch generation before the sweep
-  int nbatches;
-  int count;               // sweeps finished
-  int max_sweeps;
-  int bracket;
-  int* n_moved;            // the blockmodel's two moved-count slots
-  double initial;          // the call's first MDL, as stored (float) by the reference
-  double deltas[kMaxIterations];
+// One batch of an asynchronous-Gibbs plan: its light vertices, by degree descending, and its
+// heavy ones; n32 / n16 of the light ones are too large for a group of 16 / 8 lanes.
+struct BatchDesc {
+  int light_begin, light_n, heavy_begin, heavy_n;
+  int n32, n16;
+};
+// Polls of a persistent kernel's grid barrier before it gives up (about 0.7 us each).
+constexpr unsigned kGridWaitLimit = 1u << 23;
+// What a whole finetune call in one kernel reports.
+struct SweepsResult {
+  double initial, mdl;   // MDL before the first sweep and after the last
+  int sweeps;
+  int pad;
 };
 
 struct Csr {
@@ -38,51 +38,21 @@ __global__ void k_mdl_cells_list(const int* __restrict__ rows, const int* __rest
                                  const int* __restrict__ d_in, double* partial);
 __global__ void k_mdl_cells_list_final(const double* partial, int n, int V, long long E, int B, double* out);
 __global__ void k_mdl(GraphView g, BlockView bm, const int* __restrict__ out_src, int cells, double* partial,
-                      unsigned* done, double* out, SweepCtl* ctl, cudaGraphConditionalHandle loop);
-// Asynchronous-Gibbs evaluation compiled for one storage of the block matrix.
-__global__ void __launch_bounds__(256, 2)
-    k_gibbs_eval_dense(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
-                       int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status,
-                       const SweepCtl* ctl, int batch);
+                      unsigned* done, double* out);
+// Asynchronous-Gibbs evaluation on row-hashed storage.
 __global__ void __launch_bounds__(256, 2)
     k_gibbs_eval_hashed(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
-                        int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status,
-                        const SweepCtl* ctl, int batch);
-__global__ void __launch_bounds__(256, 3)
-    k_gibbs_eval_dense_occ3(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
-                            int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap,
-                            int* status, const SweepCtl* ctl, int batch);
-using GibbsEvalKernel = void (*)(GraphView, BlockView, const int* __restrict__, int, RngParams, int, int*, int*, int*,
-                                 unsigned long long*, int, int*, const SweepCtl*, int);
-// Dense blockmodels up to this many blocks take the three-CTAs-per-SM build of the evaluation
-// (measured on the 200,000-vertex graph: 10-17 % shorter launches up to 11,771 blocks, 5 % longer
-// at 39,366, where the cells come from DRAM and more warps in flight only add misses).
-constexpr int kEvalOcc3MaxB = 16384;
-inline GibbsEvalKernel gibbs_eval_kernel(bool hashed, int B) {
-  return hashed ? k_gibbs_eval_hashed : B <= kEvalOcc3MaxB ? k_gibbs_eval_dense_occ3 : k_gibbs_eval_dense;
-}
-// Asynchronous-Gibbs evaluation of light vertices on dense storage (sbp_eval_small.cu): groups of
-// kSmallGroup lanes per vertex; neighbour-block histograms direct-indexed (B <= kSmallB) or in
-// per-group hash tables of `cap` slots (hashed_table), in dynamic shared memory of
-// gibbs_eval_group_smem bytes.
-constexpr int kSmallB = 128;
-constexpr int kSmallThreads = 256;
+                        int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status);
 constexpr int kSmallGroup = 8;
-constexpr int kGroupMaxK = 128;   // largest degree of a vertex on hashed group tables (256 slots)
-using GibbsEvalGroupKernel = void (*)(GraphView, BlockView, const int* __restrict__, int, RngParams, int, int*, int*,
-                                      int*, unsigned long long*, int, int*, const SweepCtl*, int);
-GibbsEvalGroupKernel gibbs_eval_group_kernel(bool hashed_table);
-size_t gibbs_eval_group_smem(bool hashed_table, int cap);
 // Metropolis-Hastings rounds of kMhGroupThreads / kSmallGroup vertices (one CTA, dense storage).
 constexpr int kMhGroupThreads = 512;
 using MhGroupKernel = void (*)(GraphView, BlockView, const int* __restrict__, int, RngParams, int, int, double*, int*);
 MhGroupKernel mh_group_kernel(bool hashed_table);
 size_t mh_group_smem(bool hashed_table, int cap);
 __global__ void k_apply_edges(GraphView g, BlockView bm, const int* moved_list, const int* n_moved, const int* prop,
-                              int* qr, int* qs, unsigned long long* last, unsigned gen, const SweepCtl* ctl, int batch);
+                              int* qr, int* qs, unsigned long long* last, unsigned gen);
 __global__ void k_apply_finish(BlockView bm, const int* moved_list, const int* n_moved, int* next_n_moved, int* prop,
-                               const int* qr, const int* qs, const unsigned long long* last, unsigned gen,
-                               const SweepCtl* ctl, int batch);
+                               const int* qr, const int* qs, const unsigned long long* last, unsigned gen);
 __global__ void k_mh(GraphView g, BlockView bm, const int* __restrict__ verts, int n, int start, RngParams rng,
                      int sweep, int cap, double* out, int* status);
 __global__ void k_move_vertex(GraphView g, BlockView bm, int v, int s, int cap, int* status);
@@ -99,6 +69,9 @@ __global__ void k_block_sizes(const int* b, int V, int* size);
 // d_out[b] * d_in[b] (the interblock-edge fraction and the modularity of a partition).
 __global__ void k_block_stats(BlockView bm, unsigned long long* out);
 __global__ void k_relabel(int* b, int V, const int* map);
+__global__ void k_join_lists(int V, const int* __restrict__ out_ptr, const int* __restrict__ out_idx,
+                             const int* __restrict__ in_ptr, const int* __restrict__ in_idx, int* adj);
+__global__ void k_vertex_records(GraphView g, const int* __restrict__ verts, int n, int4* recs);
 
 // row-hashed block matrix (sbp_sparse.cu)
 __global__ void k_edge_keys(GraphView g, const int* __restrict__ b, const int* __restrict__ out_src, int B,

@@ -1252,27 +1252,9 @@ SbpStatus sbp_collect_moves(SbpBlockmodel* bm, const SbpGraph* cg, SbpDataset* d
     const long long ovf_sweep = g_overflow_rebuilds;
     for (size_t bt = 0; bt < plan.light_n.size(); ++bt) {
       // plain evaluation (gibbs_batch without its apply), record, then apply
-      const int nl = plan.light_n[bt], nh = plan.heavy_n[bt];
       int* n_cur = bm->n_moved.p + (bm->gen & 1);
-      const GibbsEvalKernel k_eval = gibbs_eval_kernel(bm->sparse, bm->B);
-      if (nl > 0) {
-        const size_t smem = (size_t)table_ints(g.light_cap) * sizeof(int) * kLightWarps;
-        set_smem_limit((const void*)k_eval, smem);
-        k_eval<<<grid_for(nl, kLightWarps, 64 * c.num_sms), kLightWarps * 32, smem, c.stream>>>(
-            g.view(), bm->view(), plan.order.p + plan.light_begin[bt], nl, rng, it, bm->prop.p, bm->moved.p, n_cur,
-            c.counters, g.light_cap, c.status, nullptr, 0);
-        SBP_CHECK_LAUNCH();
-      }
-      if (nh > 0) {
-        const size_t smem = (size_t)table_ints(g.heavy_cap) * sizeof(int);
-        set_smem_limit((const void*)k_eval,
-                       std::max(smem, (size_t)table_ints(g.light_cap) * sizeof(int) * kLightWarps));
-        k_eval<<<grid_for(nh, 1, 64 * c.num_sms), 32, smem, c.stream>>>(
-            g.view(), bm->view(), plan.order.p + plan.heavy_begin[bt], nh, rng, it, bm->prop.p, bm->moved.p, n_cur,
-            c.counters, g.heavy_cap, c.status, nullptr, 0);
-        SBP_CHECK_LAUNCH();
-      }
-      const int batch = nl + nh;
+      gibbs_eval_batch(*bm, g, plan, (int)bt, rng, it);
+      const int batch = plan.light_n[bt] + plan.heavy_n[bt];
       launch_warps(k_learn_collect, batch, cap, 1, g.view(), bm->view(), bm->moved.p, n_cur, bm->prop.p, lp,
                    d->X.p, d->target.p, d->nvalid.p, d->count.p, d->capacity, cap, c.status);
       gibbs_apply(*bm, g, batch);

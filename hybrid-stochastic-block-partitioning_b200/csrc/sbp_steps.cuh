@@ -2,7 +2,7 @@
 // kernels (sbp_kernels.cu) and the batched persistent kernel (sbp_batched.cu) so both run the
 // same arithmetic in the same order.
 #pragma once
-#include "sbp_device.cuh"
+#include "sbp_group.cuh"
 
 namespace sbpb {
 
@@ -156,16 +156,14 @@ __device__ __forceinline__ void mh_apply_move(const GraphView& g, const BlockVie
 // d_out / d_in, the quirk terms qr/qs of d[r], d[s] (the neighbours that are counted in the
 // reference's sequential apply) and the batch's last mover of r and s.  One warp per vertex;
 // lanes whose edges change the same cell add their count with one atomic.
-__device__ __forceinline__ void apply_moved_vertex(const GraphView& g, const BlockView& bm, int v, const int* prop,
+__device__ __forceinline__ void apply_moved_record(const GraphView& g, const BlockView& bm, int4 rec, const int* prop,
                                                    int* qr, int* qs, unsigned long long* last, unsigned gen,
                                                    int lane) {
+  const int v = rec.x, k_out = rec.z, k_in = rec.w >> 1, self = rec.w & 1, k = k_out + k_in;
+  const int* nbr = g.adj + (unsigned)rec.y;
   const int r = bm.b[v], s = prop[v];
-  const int self = g.self[v];
   int cr = 0, cs = 0;
-  const int o0 = g.out_ptr[v], o1 = g.out_ptr[v + 1];
-  const int i0 = g.in_ptr[v], i1 = g.in_ptr[v + 1];
-  const int k_out = o1 - o0, k = k_out + (i1 - i0);
-  // One pass over the virtual neighbour list (out-edges, then in-edges), two elements per lane
+  // One pass over the joint neighbour list (out-edges, then in-edges), two elements per lane
   // in flight.  Out-edge v -> u (not the self loop): (r, b_u) -= 1 and (s, b'_u) += 1, b'_u the
   // block u moves to in this batch.  In-edge u -> v of a u that stays: (b_u, r) -= 1 and
   // (b_u, s) += 1 (a moving u's own out-edge covers the cell otherwise).
@@ -174,7 +172,7 @@ __device__ __forceinline__ void apply_moved_vertex(const GraphView& g, const Blo
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int j = base + h * kWarp + lane;
-      u[h] = j < k ? (j < k_out ? __ldg(g.out_idx + o0 + j) : __ldg(g.in_idx + i0 + (j - k_out))) : -1;
+      u[h] = j < k ? __ldg(nbr + j) : -1;
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -183,6 +181,7 @@ __device__ __forceinline__ void apply_moved_vertex(const GraphView& g, const Blo
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
+      if (base + h * kWarp >= k) break;   // warp-uniform
       const int j = base + h * kWarp + lane;
       const bool out_edge = j < k_out;
       int ko = -1, kn = -1, ks = -1;
@@ -216,7 +215,7 @@ __device__ __forceinline__ void apply_moved_vertex(const GraphView& g, const Blo
       cell_add(bm, r, r, -1);
       cell_add(bm, s, s, 1);
     }
-    const int k_in_self = (i1 - i0) + self;
+    const int k_in_self = k_in + self;
     atomicAdd(bm.d_out + r, -k_out);
     atomicAdd(bm.d_out + s, k_out);
     atomicAdd(bm.d_in + r, -k_in_self);
@@ -227,6 +226,11 @@ __device__ __forceinline__ void apply_moved_vertex(const GraphView& g, const Blo
     atomicMax(last + r, key);
     atomicMax(last + s, key);
   }
+}
+__device__ __forceinline__ void apply_moved_vertex(const GraphView& g, const BlockView& bm, int v, const int* prop,
+                                                   int* qr, int* qs, unsigned long long* last, unsigned gen,
+                                                   int lane) {
+  apply_moved_record(g, bm, vertex_record(g, v), prop, qr, qs, last, gen, lane);
 }
 
 // d[r], d[s] from the last mover of each block, then the new assignment of v.
@@ -262,7 +266,25 @@ __device__ __forceinline__ double mdl_edges_part(const GraphView& g, const Block
                                                  int ncta, double* red) {
   double acc = 0.0;
   const long long stride = (long long)ncta * blockDim.x;
-  for (long long e = (long long)cta * blockDim.x + threadIdx.x; e < g.E; e += stride) {
+  long long e = (long long)cta * blockDim.x + threadIdx.x;
+  for (; e + 3 * stride < g.E; e += 4 * stride) {   // four chains of dependent loads in flight, added in order
+    int bv[4], bu[4], m[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      bv[j] = __ldg(out_src + e + j * stride);
+      bu[j] = __ldg(g.out_idx + e + j * stride);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      bv[j] = bm.b[bv[j]];
+      bu[j] = bm.b[bu[j]];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) m[j] = bm_get(bm, bv[j], bu[j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc += log((double)m[j]);
+  }
+  for (; e < g.E; e += stride) {
     const int bv = bm.b[__ldg(out_src + e)], bu = bm.b[__ldg(g.out_idx + e)];
     acc += log((double)bm_get(bm, bv, bu));
   }
@@ -271,14 +293,22 @@ __device__ __forceinline__ double mdl_edges_part(const GraphView& g, const Block
   return block_sum(acc, red);
 }
 
-__device__ __forceinline__ double mdl_final_value(const double* partial, int n, int V, long long E, int B,
-                                                  double* red) {
+// The sum of the partials in a fixed order (thread 0).
+__device__ __forceinline__ double mdl_total(const double* partial, int n, double* red) {
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) acc += __ldcg(partial + i);
-  const double L = block_sum(acc, red);
+  return block_sum(acc, red);
+}
+// E h(B^2 / E) + V log B
+__device__ __forceinline__ double mdl_constant(int V, long long E, int B) {
   const double x = pow((double)B, 2) / (double)E;
   const double h = ((1 + x) * log(1 + x)) - (x * log(x));
-  return ((double)E * h) + ((double)V * log((double)B)) - L;
+  return ((double)E * h) + ((double)V * log((double)B));
+}
+__device__ __forceinline__ double mdl_final_value(const double* partial, int n, int V, long long E, int B,
+                                                  double* red) {
+  const double L = mdl_total(partial, n, red);
+  return mdl_constant(V, E, B) - L;
 }
 
 }  // namespace sbpb
