@@ -153,7 +153,14 @@ struct GraphView {
   const unsigned char* self;
 };
 
-constexpr int kChunk = 128;   // columns per chunk-sum entry
+constexpr int kRowPad = 128;   // rows of P are padded to a multiple of this many pairs
+// Sums kept per row and column of M for the multinomial walk when B > kSmallB: of chunks of kChunk
+// cells and, beyond kFan chunks, of spans of kFan chunks.  Every level of the walk is then one
+// load of at most 256 bytes (with chunks of 128 cells and one level of sums a walk at 50,000
+// blocks read 2.5 KB in six dependent steps and took a third of a visit).
+constexpr int kChunk = 64;
+constexpr int kFan = 64;
+constexpr int kSmallB = 128;   // up to this many blocks: no sums, and direct-indexed histograms
 
 struct BlockView {
   int B;
@@ -169,11 +176,14 @@ struct BlockView {
   const int* cmask;
   int2* cslot;
   int* overflow;
-  int ld;                 // row stride of P (multiple of kChunk pairs)
+  int ld;                 // row stride of P (multiple of kRowPad pairs)
   int nch;                // chunks per row = ceil(B / kChunk)
-  int ncs;                // row stride of CS and CST: nch rounded up to four, the rest zero
-  int* CS;                // [B*ncs] CS[row*ncs+c] = sum of M[row, c*kChunk .. c*kChunk+kChunk); kept when nch > 1
-  int* CST;               // [B*ncs] the same over the columns of M (chunks of rows)
+  int ncs;                // row stride of CS and CST: nch rounded up to kFan, the rest zero
+  int nss;                // row stride of SS and SST: spans rounded up to kFan; 0 up to kFan chunks
+  int* CS;                // [B*ncs] CS[row*ncs+c] = sum of M[row, c*kChunk .. c*kChunk+kChunk)
+  int* CST;               // [B*ncs] the same over the columns of M
+  int* SS;                // [B*nss] sums of kFan chunk sums of CS
+  int* SST;               // [B*nss] of CST
   int* b;                 // [V] assignment
   // [B*ld] counts of both directions side by side: P[row*ld+col] = (M[row, col], M[col, row]).
   // A visit needs M[r,u] with M[u,r] and M[s,u] with M[u,s]: one 8-byte load and one 32-byte
@@ -183,8 +193,15 @@ struct BlockView {
   int* d_out;             // [B]
   int* d_in;              // [B]
   int* d;                 // [B] block degrees as the reference maintains them
+  double* inv_d;          // [B] 1 / (d + B), the Hastings weight of a block: kept with d, so that a
+                          // visit loads it where it took a conversion and a division per entry
   const double2* xlogxt;  // [kXlogxTable] x log x = hi + lo for integer x
 };
+
+__device__ __forceinline__ void set_degree(const BlockView& bm, int x, int value) {
+  bm.d[x] = value;
+  bm.inv_d[x] = 1.0 / ((double)value + (double)bm.B);
+}
 
 // ---- row-hashed storage ------------------------------------------------------------------
 __device__ __forceinline__ unsigned slot_hash(int key) { return (unsigned)key * 2654435761u; }
@@ -302,115 +319,153 @@ __device__ __forceinline__ int warp_select_hashed(const long long* base, const i
   return lo;
 }
 
-__device__ __forceinline__ int select_in_chunk(int4 q, int chunk, long long target, int lane);
-
-// Four counts from column c0 (a multiple of 4) of a row of pairs: M[row, .], or M[., row] when `col`.
-template <Store S>
-__device__ __forceinline__ int4 load_four(const int2* row, int c0, bool col) {
-  const int4 a = ldv<S>(reinterpret_cast<const int4*>(row + c0));
-  const int4 b = ldv<S>(reinterpret_cast<const int4*>(row + c0 + 2));
-  return col ? make_int4(a.y, a.w, b.y, b.w) : make_int4(a.x, a.z, b.x, b.z);
-}
-
-// Two-level walk over row t of M (or column t when `col`): the first index whose running count
-// exceeds `target`, -1 if the row is exhausted.  The chunk is found through the chunk sums, then
-// the column inside the chunk, four counts per lane.  Up to kWideChunks chunks, lane i loads the
-// sums of chunks [16 i, 16 i + 16) at once (one memory round trip instead of one per 32
-// chunks), scans its lane total across the warp and walks its sixteen sums; longer rows take 32
-// chunks per step.
-constexpr int kWideChunks = 16 * kWarp;
-template <Store S>
-__device__ __forceinline__ int warp_select_chunked(const int2* row, bool col, const int* csum, int nch,
-                                                   long long target, int lane) {
-  int chunk = -1;
-  if (nch <= kWideChunks) {
-    int cs[16];
-    long long lsum = 0;
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const int c = lane * 16 + q;
-      cs[q] = c < nch ? ldi<S>(csum + c) : 0;
-      lsum += cs[q];
-    }
-    const long long incl = warp_incl_scan(lsum, lane);
-    const unsigned hit = __ballot_sync(kFull, incl > target);
-    if (!hit) return -1;
-    const int src = __ffs(hit) - 1;
-    long long before = 0;
-    if (lane == src) {
-      long long run = incl - lsum;
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        if (chunk < 0) {
-          if (target < run + cs[q]) {
-            chunk = lane * 16 + q;
-            before = run;
-          } else {
-            run += cs[q];
-          }
-        }
-      }
-    }
-    chunk = __shfl_sync(kFull, chunk, src);
-    target -= __shfl_sync(kFull, before, src);
-  } else {
-    for (int base = 0; base < nch; base += kWarp) {
-      const int c = base + lane;
-      const long long v = c < nch ? (long long)ldi<S>(csum + c) : 0;
-      const long long incl = warp_incl_scan(v, lane);
-      const long long tot = __shfl_sync(kFull, incl, 31);
-      if (target < tot) {
-        const unsigned hit = __ballot_sync(kFull, incl > target);
-        const int src = __ffs(hit) - 1;
-        target -= __shfl_sync(kFull, incl - v, src);
-        chunk = base + src;
-        break;
-      }
-      target -= tot;
-    }
-    if (chunk < 0) return -1;
-  }
-  return select_in_chunk(load_four<S>(row, chunk * kChunk + 4 * lane, col), chunk, target, lane);
-}
-
-// The column inside one chunk of kChunk counts (four per lane, q) at which the running sum
-// first exceeds target; -1 if the chunk is exhausted.
-__device__ __forceinline__ int select_in_chunk(int4 q, int chunk, long long target, int lane) {
-  const long long lsum = (long long)q.x + q.y + q.z + q.w;
-  const long long incl = warp_incl_scan(lsum, lane);
-  const unsigned hit = __ballot_sync(kFull, incl > target);
-  if (!hit) return -1;
-  const int src = __ffs(hit) - 1;
-  long long t = target - __shfl_sync(kFull, incl - lsum, src);
-  const int qx = __shfl_sync(kFull, q.x, src), qy = __shfl_sync(kFull, q.y, src), qz = __shfl_sync(kFull, q.z, src);
-  int k = 3;
-  if (t < qx) k = 0;
-  else if (t < (long long)qx + qy) k = 1;
-  else if (t < (long long)qx + qy + qz) k = 2;
-  return chunk * kChunk + 4 * src + k;
-}
-
-// The walk of warp_select_chunked for a row of at most 32 chunks whose chunk sums are already
-// loaded (lane c holds chunk c's sum, 0 beyond the row).
-template <Store S>
-__device__ __forceinline__ int select_chunk_then_column(const int2* row, bool col, int csum_lane, long long target,
-                                                        int lane) {
-  const long long v = csum_lane;
-  const long long incl = warp_incl_scan(v, lane);
-  const long long tot = __shfl_sync(kFull, incl, 31);
-  if (target >= tot) return -1;
-  const unsigned hit = __ballot_sync(kFull, incl > target);
-  const int src = __ffs(hit) - 1;
-  target -= __shfl_sync(kFull, incl - v, src);
-  return select_in_chunk(load_four<S>(row, src * kChunk + 4 * lane, col), src, target, lane);
-}
-
-// The chunk sums of cell (row, col): not kept with one chunk per row, where the walks read the
-// row itself.
+// The sums that cell (row, col) belongs to.
 __device__ __forceinline__ void chunks_add(const BlockView& bm, int row, int col, int delta) {
-  if (bm.nch == 1) return;
+  if (bm.B <= kSmallB) return;
   atomicAdd(bm.CS + (size_t)row * bm.ncs + col / kChunk, delta);
   atomicAdd(bm.CST + (size_t)col * bm.ncs + row / kChunk, delta);
+  if (bm.nss) {
+    atomicAdd(bm.SS + (size_t)row * bm.nss + col / (kChunk * kFan), delta);
+    atomicAdd(bm.SST + (size_t)col * bm.nss + row / (kChunk * kFan), delta);
+  }
+}
+
+// The calling lane's place in a group of G = 8, 16 or 32 lanes of its warp.
+struct Lanes {
+  int G, gl, lane, gbase;
+  unsigned gmask;
+  __device__ __forceinline__ Lanes(int group, int lane_) : G(group), lane(lane_) {
+    gl = lane & (G - 1);
+    gbase = lane & ~(G - 1);
+    gmask = G == 32 ? kFull : ((1u << G) - 1u) << gbase;
+  }
+};
+
+// ------------------------------------------------------------------------------------------
+// The multinomial walk over row t of M (column t when `col`), ascending: the first index whose
+// running count exceeds tg.  One group per walk, of which the first eight lanes read; every lane of
+// the warp calls it; groups with !on get -1.
+// ------------------------------------------------------------------------------------------
+// One level: lane g8 holds the N sums v[] of entries [N g8, N g8 + N).  Finds the entry of the
+// running count tg, leaves the count before it taken off tg; *ok cleared when there is none.
+template <int N>
+__device__ __forceinline__ int walk_level(const int (&v)[N], int* tg, bool* ok, const Lanes& L) {
+  const int g8 = L.lane & 7;
+  int sum = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) sum += v[j];
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, incl, o);
+    if (g8 >= o) incl += y;
+  }
+  const unsigned hit = __ballot_sync(kFull, *ok && L.gl < 8 && incl > *tg) & L.gmask;
+  const int src = hit ? __ffs(hit) - 1 : L.gbase;
+  int rest = *tg - (incl - sum), at = N * g8, run = 0, base = 0;   // meaningful on lane src
+#pragma unroll
+  for (int j = 0; j < N - 1; ++j) {
+    run += v[j];
+    if (rest >= run) {
+      at = N * g8 + j + 1;
+      base = run;
+    }
+  }
+  *ok = *ok && hit;
+  *tg = __shfl_sync(kFull, rest - base, src);
+  return __shfl_sync(kFull, at, src);
+}
+
+template <Store ST>
+__device__ __forceinline__ int walk_sums(const int* sums, int* tg, bool* ok, const Lanes& L) {   // kFan sums
+  const bool rd = *ok && L.gl < 8;
+  const int4* p = reinterpret_cast<const int4*>(sums + 8 * (L.lane & 7));
+  const int4 a = rd ? ldv<ST>(p) : make_int4(0, 0, 0, 0), b = rd ? ldv<ST>(p + 1) : make_int4(0, 0, 0, 0);
+  const int v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  return walk_level<8>(v, tg, ok, L);
+}
+
+// B > kSmallB: through the spans (if any), the chunks of one span, the cells of one chunk.
+template <Store ST>
+__device__ __forceinline__ int walk_tree(const BlockView& bm, int t, bool col, int tg, bool on, const Lanes& L) {
+  bool ok = on;
+  int span = 0;
+  if (bm.nss) {
+    const int* ss = (col ? bm.SST : bm.SS) + (size_t)t * bm.nss;
+    if (bm.nss == kFan) {
+      span = walk_sums<ST>(ss, &tg, &ok, L);
+    } else {   // more than kFan spans: window by window
+      bool found = false;
+      for (int w = 0; w < bm.nss; w += kFan) {
+        int rest = tg, tot = 0;
+        bool here = on && !found;
+        const int at = walk_sums<ST>(ss + w, &rest, &here, L);
+        if (!found && on && !here)
+          for (int j = 0; j < kFan; ++j) tot += ldi<ST>(ss + w + j);
+        if (here) {
+          found = true;
+          span = w + at;
+          tg = rest;
+        }
+        if (!found) tg -= tot;
+      }
+      ok = on && found;
+    }
+  }
+  const int chunk = span * kFan + walk_sums<ST>((col ? bm.CST : bm.CS) + (size_t)t * bm.ncs + (ok ? span : 0) * kFan,
+                                                &tg, &ok, L);
+  ok = ok && chunk < bm.nch;
+  const bool rd = ok && L.gl < 8;
+  constexpr int kPer = kChunk / 8;   // cells a lane
+  const int4* p =
+      reinterpret_cast<const int4*>(bm.P + (size_t)t * bm.ld + (size_t)(ok ? chunk : 0) * kChunk + kPer * (L.lane & 7));
+  int v[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer / 2; ++j) {
+    const int4 a = rd ? ldv<ST>(p + j) : make_int4(0, 0, 0, 0);
+    v[2 * j] = col ? a.y : a.x;
+    v[2 * j + 1] = col ? a.w : a.z;
+  }
+  const int at = walk_level<kPer>(v, &tg, &ok, L);
+  return ok ? chunk * kChunk + at : -1;
+}
+
+// B <= kSmallB: the whole row in up to eight coalesced steps of 16 cells; a transposing reduction
+// leaves step q's total on lane q, and the step picked is read again (from L1) two cells a lane.
+template <Store ST>
+__device__ __forceinline__ int walk_row(const BlockView& bm, int t, bool col, int tg, bool on, const Lanes& L) {
+  bool ok = on;
+  const int g8 = L.lane & 7;
+  const bool rd = ok && L.gl < 8;
+  const int2* row = bm.P + (size_t)t * bm.ld;
+  int v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int c = 16 * q + 2 * g8;
+    const int4 x = (rd && c < bm.B) ? ldv<ST>(reinterpret_cast<const int4*>(row + c)) : make_int4(0, 0, 0, 0);
+    v[q] = col ? x.y + x.w : x.x + x.z;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const bool up = g8 & 4;
+    const int give = up ? v[q] : v[q + 4], keep = up ? v[q + 4] : v[q];
+    v[q] = keep + __shfl_xor_sync(kFull, give, 4);
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const bool up = g8 & 2;
+    const int give = up ? v[q] : v[q + 2], keep = up ? v[q + 2] : v[q];
+    v[q] = keep + __shfl_xor_sync(kFull, give, 2);
+  }
+  const bool up = g8 & 1;
+  const int give = up ? v[0] : v[1], keep = up ? v[1] : v[0];
+  const int total[1] = {keep + __shfl_xor_sync(kFull, give, 1)};
+  const int step = walk_level<1>(total, &tg, &ok, L);
+  int4 x = make_int4(0, 0, 0, 0);
+  if (ok && L.gl < 8) x = ldv<ST>(reinterpret_cast<const int4*>(row + 16 * step + 2 * g8));
+  const int two[2] = {col ? x.y : x.x, col ? x.w : x.z};
+  const int at = walk_level<2>(two, &tg, &ok, L);
+  return ok ? 16 * step + at : -1;
 }
 
 // Same walk over a compressed list (idx[i], val[i]), i in [0, n).
@@ -621,7 +676,8 @@ __device__ __forceinline__ int gather_neighbour_blocks(const GraphView& g, const
 // Loads of move_delta that do not depend on the proposed block s: issued right after the
 // neighbour table is built, so that they overlap the multinomial walk that picks s.
 struct NbPrefetch {
-  int u, co, ci, M_ru, M_ur, du;   // this lane's first table entry (u = -1: none)
+  int u, co, ci, M_ru, M_ur;   // this lane's first table entry (u = -1: none)
+  double inv;
   int M_rr, dout_r, din_r;
 };
 
@@ -630,7 +686,8 @@ __device__ __forceinline__ void prefetch_nb(const BlockView& bm, int r, const Wa
   __syncwarp();
   const int n = *t.nlist;
   p->u = -1;
-  p->co = p->ci = p->M_ru = p->M_ur = p->du = 0;
+  p->co = p->ci = p->M_ru = p->M_ur = 0;
+  p->inv = 0.0;
   if (lane < n) {
     const int h = t.list[lane];
     const int u = t.keys[h];
@@ -640,20 +697,20 @@ __device__ __forceinline__ void prefetch_nb(const BlockView& bm, int r, const Wa
     const int2 m = bm_pair<ST>(bm, r, u);
     p->M_ru = m.x;
     p->M_ur = m.y;
-    p->du = ldi<ST>(bm.d + u);
+    p->inv = ldv<ST>(bm.inv_d + u);
   }
   p->M_rr = bm_get<ST>(bm, r, r);
   p->dout_r = ldi<ST>(bm.d_out + r);
   p->din_r = ldi<ST>(bm.d_in + r);
 }
 
-// Above this |delta-MDL| the zero snap (below) cannot apply, whatever the integer scale T of the
-// changed cells and degrees is: every changed cell lies in a row or column of r or s, so T is at
-// most six times the block degrees of r and s plus four times the vertex's.
+// Whether the zero snap (below) can apply: the integer scale T of the changed cells and degrees is
+// at most six times the block degrees of r and s plus four times the vertex's, as every changed
+// cell lies in a row or column of r or s.  In single precision, with room for its rounding.
 __device__ __forceinline__ bool maybe_zero_delta(double dS, int dout_r, int dout_s, int din_r, int din_s, int k,
                                                  double log_E) {
-  const double bound = 6.0 * ((double)dout_r + (double)dout_s + (double)din_r + (double)din_s) + 4.0 * (double)k + 4.0;
-  return fabs(dS) <= 0x1p-40 * bound * log_E;
+  const float bound = 6.0f * ((float)dout_r + (float)dout_s + (float)din_r + (float)din_s) + 4.0f * (float)k + 4.0f;
+  return fabsf((float)dS) <= 0x1.1p-40f * bound * (float)log_E;
 }
 
 // Delta-MDL of moving v from r to s (s != r) against the current state, with the gathered
@@ -686,14 +743,15 @@ __device__ __forceinline__ double move_delta(const GraphView& g, const BlockView
   double fwd = 0.0, bwd = 0.0, dS = 0.0;
   const int n = *t.nlist;
   for (int i = lane; i < n; i += kWarp) {
-    int u, co, ci, du, M_ru, M_ur;
+    int u, co, ci, M_ru, M_ur;
+    double inv;   // 1 / (d[u] + B): a non-corner block's degree is unchanged
     if (pre && i < kWarp) {
       u = pre->u;
       co = pre->co;
       ci = pre->ci;
       M_ru = pre->M_ru;
       M_ur = pre->M_ur;
-      du = pre->du;
+      inv = pre->inv;
     } else {
       const int h = t.list[i];
       u = t.keys[h];
@@ -702,13 +760,12 @@ __device__ __forceinline__ double move_delta(const GraphView& g, const BlockView
       const int2 m = bm_pair<ST>(bm, r, u);
       M_ru = m.x;
       M_ur = m.y;
-      du = ldi<ST>(bm.d + u);
+      inv = ldv<ST>(bm.inv_d + u);
     }
     const int2 m_su = bm_pair<ST>(bm, s, u);
     const int M_su = m_su.x, M_us = m_su.y;
     const bool is_r = (u == r), is_s = (u == s);
     const double c = (double)(co + ci + (is_r ? self : 0));
-    double inv = 1.0 / ((double)du + (double)B);   // a non-corner block's degree is unchanged
     fwd += c * (M_su + M_us + 1.0) * inv;
     if (is_r || is_s) {
       const int nd = is_r ? (dout_r - k_out) + (din_r - k_in) - (M_rr + d_rr)
@@ -822,30 +879,13 @@ __device__ __forceinline__ EvalResult evaluate_vertex(const GraphView& g, const 
       if (target < dot) s = warp_select_hashed(bm.rbase, bm.rmask, bm.rslot, tblk, bm.B, target, lane, bins);
       else s = warp_select_hashed(bm.cbase, bm.cmask, bm.cslot, tblk, bm.B, target - dot, lane, bins);
     } else if (ST != Store::kHashed) {
-      // the degrees of t and, in the same round trip, its row and column (B <= kChunk: the whole
-      // row of pairs, four per lane) or their chunk sums (up to 32 chunks); the walk then picks
-      // the row (target < d_out[t]) or the column.  (Loading the chunk sums of both with the
-      // degrees for up to 512 chunks as well was measured 13 % slower at 11,770 blocks and no
-      // faster above.)
       const int dot = ldi<ST>(bm.d_out + tblk), dit = ldi<ST>(bm.d_in + tblk);
-      const int2* row = bm.P + (size_t)tblk * bm.ld;
-      const size_t co = (size_t)tblk * bm.ncs;
-      int4 qa = make_int4(0, 0, 0, 0), qb = make_int4(0, 0, 0, 0);
-      int ca = 0, cb = 0;
-      if (bm.nch == 1) {
-        qa = ldv<ST>(reinterpret_cast<const int4*>(row + 4 * lane));
-        qb = ldv<ST>(reinterpret_cast<const int4*>(row + 4 * lane + 2));
-      } else if (lane < bm.nch) {
-        ca = ldi<ST>(bm.CS + co + lane);
-        cb = ldi<ST>(bm.CST + co + lane);
-      }
       const long long target = scale32(x.y, (long long)dot + (long long)dit);
       const bool in_col = target >= dot;
-      const long long tg = in_col ? target - dot : target;
-      if (bm.nch == 1)
-        s = select_in_chunk(in_col ? make_int4(qa.y, qa.w, qb.y, qb.w) : make_int4(qa.x, qa.z, qb.x, qb.z), 0, tg, lane);
-      else if (bm.nch <= kWarp) s = select_chunk_then_column<ST>(row, in_col, in_col ? cb : ca, tg, lane);
-      else s = warp_select_chunked<ST>(row, in_col, in_col ? bm.CST + co : bm.CS + co, bm.nch, tg, lane);
+      const int tg = (int)(in_col ? target - dot : target);
+      const Lanes L(32, lane);
+      if (bm.B <= kSmallB) s = walk_row<ST>(bm, tblk, in_col, tg, true, L);
+      else s = walk_tree<ST>(bm, tblk, in_col, tg, true, L);
     } else {
       s = -1;
     }

@@ -16,6 +16,86 @@ void set_last_error(const char* msg) {
 }
 const char* last_error() { return g_last_error; }
 
+// ------------------------------------------------------------------------------------------
+// Table of x log x for dxlogx_int, once per process, in double-double arithmetic (error-free sums
+// and products of Knuth and Dekker, the product by FMA).  log x = log(x - 1) + 2 atanh(1 / (2x - 1));
+// each thread's first logarithm, and those of small x, come from the whole power series (x = m 2^e
+// with m in [sqrt(1/2), sqrt(2)), log m = 2 atanh((m - 1) / (m + 1)), log 2 = 2 atanh(1/3)).
+// ------------------------------------------------------------------------------------------
+namespace {
+struct DD {
+  double hi, lo;
+};
+DD dd_renorm(double hi, double lo) {
+  const double s = hi + lo;
+  return {s, lo - (s - hi)};
+}
+DD dd_add(DD a, DD b) {
+  const double s = a.hi + b.hi, t = s - a.hi;
+  const double e = (a.hi - (s - t)) + (b.hi - t);
+  return dd_renorm(s, e + (a.lo + b.lo));
+}
+DD dd_mul(DD a, DD b) {
+  const double p = a.hi * b.hi;
+  return dd_renorm(p, std::fma(a.hi, b.hi, -p) + (a.hi * b.lo + a.lo * b.hi));
+}
+DD dd_ratio(double n, double d) {   // n / d of exact doubles
+  const double q = n / d;
+  return dd_renorm(q, std::fma(-q, d, n) / d);
+}
+DD dd_2atanh(double n, double d) {   // for |n / d| <= 1/3: 36 terms, 9^-36 < 2^-114
+  const DD z = dd_ratio(n, d), w = dd_mul(z, z);
+  DD s = dd_ratio(1.0, 73.0);
+  for (int k = 35; k >= 0; --k) s = dd_add(dd_mul(s, w), dd_ratio(1.0, 2.0 * k + 1.0));
+  const DD r = dd_mul(z, s);
+  return {2.0 * r.hi, 2.0 * r.lo};
+}
+DD dd_log(int x) {
+  int e = 0;
+  double m = std::frexp((double)x, &e);   // [1/2, 1)
+  if (m * m < 0.5) {
+    m *= 2.0;
+    --e;
+  }
+  return dd_add(dd_mul(dd_2atanh(1.0, 3.0), {(double)e, 0.0}), dd_2atanh(m - 1.0, m + 1.0));
+}
+}  // namespace
+
+double2* make_xlogx_table() {
+  std::vector<double2> h(kXlogxTable);
+  const int nt = 8, whole = 2048;   // whole series below this
+  std::vector<std::thread> th;
+  for (int t = 0; t < nt; ++t)
+    th.emplace_back([&h, t, nt, whole] {
+      const int a = (int)((long long)kXlogxTable * t / nt), b = (int)((long long)kXlogxTable * (t + 1) / nt);
+      const DD third = dd_ratio(1.0, 3.0);
+      DD l = {0.0, 0.0};
+      for (int x = a; x < b; ++x) {
+        if (x < 2) {
+          h[x] = make_double2(0.0, 0.0);
+          continue;
+        }
+        if (x < whole || x == a) {
+          l = dd_log(x);
+        } else {
+          // 2 atanh(z) = 2 z (1 + w / 3 + w^2 / 5 + ...), w = z^2 < 2^-23: past w / 3 doubles do
+          const DD z = dd_ratio(2.0, 2.0 * x - 1.0), w = dd_mul(z, z);   // z is 2 / (2x - 1)
+          const double w1 = 0.25 * w.hi;
+          DD s = dd_mul({0.25 * w.hi, 0.25 * w.lo}, third);
+          s = dd_add(s, {w1 * w1 * (0.2 + w1 * (1.0 / 7.0)), 0.0});
+          l = dd_add(l, dd_add(z, dd_mul(z, s)));
+        }
+        const DD g = dd_mul(l, {(double)x, 0.0});
+        h[x] = make_double2(g.hi, g.lo);
+      }
+    });
+  for (auto& t : th) t.join();
+  double2* d = nullptr;
+  SBP_CUDA(cudaMalloc(&d, sizeof(double2) * kXlogxTable));
+  SBP_CUDA(cudaMemcpy(d, h.data(), sizeof(double2) * kXlogxTable, cudaMemcpyHostToDevice));
+  return d;
+}
+
 // Scratch of the sparse rebuild (grow-only, shared by all blockmodels).
 struct SortScratch {
   DevBuf<unsigned long long> keys, keysT, tmp, ukeys, partial;
@@ -206,9 +286,13 @@ void rebuild(SbpBlockmodel& bm, const SbpGraph& g, bool recompute_d) {
   Context& c = Context::get();
   const size_t cells = (size_t)bm.B * (size_t)bm.ld;
   SBP_CUDA(cudaMemsetAsync(bm.P.p, 0, cells * sizeof(int2), c.stream));
-  if (bm.nch > 1) {
+  if (bm.B > kSmallB) {
     SBP_CUDA(cudaMemsetAsync(bm.CS.p, 0, (size_t)bm.B * bm.ncs * sizeof(int), c.stream));
     SBP_CUDA(cudaMemsetAsync(bm.CST.p, 0, (size_t)bm.B * bm.ncs * sizeof(int), c.stream));
+    if (bm.nss) {
+      SBP_CUDA(cudaMemsetAsync(bm.SS.p, 0, (size_t)bm.B * bm.nss * sizeof(int), c.stream));
+      SBP_CUDA(cudaMemsetAsync(bm.SST.p, 0, (size_t)bm.B * bm.nss * sizeof(int), c.stream));
+    }
   }
   SBP_CUDA(cudaMemsetAsync(bm.d_out.p, 0, bm.B * sizeof(int), c.stream));
   SBP_CUDA(cudaMemsetAsync(bm.d_in.p, 0, bm.B * sizeof(int), c.stream));
@@ -1318,6 +1402,8 @@ SbpStatus sbp_blockmodel_copy(const SbpBlockmodel* src, SbpBlockmodel** out) {
     bm->graph = src->graph;
     rebuild(*bm, *src->graph, false);
     SBP_CUDA(SBP_COPY_ASYNC(bm->d.p, src->d.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
+    k_inverse_degrees<<<grid_for(bm->B, 256, 1 << 20), 256, 0, c.stream>>>(bm->view());
+    SBP_CHECK_LAUNCH();
     bm->overall_entropy = src->overall_entropy;
     bm->num_blocks_to_merge = 0;
     c.sync();
@@ -1327,15 +1413,22 @@ SbpStatus sbp_blockmodel_copy(const SbpBlockmodel* src, SbpBlockmodel** out) {
   const size_t cells = (size_t)src->B * src->ld;
   SBP_CUDA(SBP_COPY_ASYNC(bm->b.p, src->b.p, src->V * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->P.p, src->P.p, cells * sizeof(int2), cudaMemcpyDeviceToDevice, c.stream));
-  if (src->nch > 1) {
-    SBP_CUDA(SBP_COPY_ASYNC(bm->CS.p, src->CS.p, (size_t)src->B * src->ncs * sizeof(int), cudaMemcpyDeviceToDevice,
-                            c.stream));
-    SBP_CUDA(SBP_COPY_ASYNC(bm->CST.p, src->CST.p, (size_t)src->B * src->ncs * sizeof(int), cudaMemcpyDeviceToDevice,
-                            c.stream));
+  if (src->B > kSmallB) {
+    auto sums = [&](DevBuf<int>& to, const DevBuf<int>& from, int stride) {
+      SBP_CUDA(SBP_COPY_ASYNC(to.p, from.p, (size_t)src->B * stride * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
+    };
+    sums(bm->CS, src->CS, src->ncs);
+    sums(bm->CST, src->CST, src->ncs);
+    if (src->nss) {
+      sums(bm->SS, src->SS, src->nss);
+      sums(bm->SST, src->SST, src->nss);
+    }
   }
   SBP_CUDA(SBP_COPY_ASYNC(bm->d_out.p, src->d_out.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->d_in.p, src->d_in.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->d.p, src->d.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
+  k_inverse_degrees<<<grid_for(bm->B, 256, 1 << 20), 256, 0, c.stream>>>(bm->view());
+  SBP_CHECK_LAUNCH();
   bm->overall_entropy = src->overall_entropy;
   bm->num_blocks_to_merge = 0;
   c.sync();
@@ -1422,6 +1515,8 @@ SbpStatus sbp_set_degrees(SbpBlockmodel* bm, const int32_t* d) {
   SBP_REQUIRE(bm && d, "NULL argument");
   Context& c = Context::get();
   SBP_CUDA(SBP_COPY_ASYNC(bm->d.p, d, bm->B * sizeof(int), cudaMemcpyHostToDevice, c.stream));
+  k_inverse_degrees<<<grid_for(bm->B, 256, 1 << 20), 256, 0, c.stream>>>(bm->view());
+  SBP_CHECK_LAUNCH();
   c.sync();
   SBP_API_END
 }

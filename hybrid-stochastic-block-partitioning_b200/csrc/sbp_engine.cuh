@@ -242,9 +242,8 @@ struct DevBuf {
 // ------------------------------------------------------------------------------------------
 // Process-wide context: one stream, the device status word, counters and readback buffers.
 // ------------------------------------------------------------------------------------------
-// x log x of the integers 0 <= x < kXlogxTable as a pair of doubles (dxlogx_int), computed on the
-// device in double-double arithmetic (k_xlogx_table).
-double2* make_xlogx_table(cudaStream_t stream);
+// x log x of the integers 0 <= x < kXlogxTable as a pair of doubles (dxlogx_int) on the device.
+double2* make_xlogx_table();
 
 struct Context {
   cudaStream_t stream = nullptr;
@@ -281,7 +280,7 @@ struct Context {
     SBP_CUDA(cudaMemset(c->done, 0, sizeof(unsigned)));
     SBP_CUDA(cudaEventCreate(&c->ev0));
     SBP_CUDA(cudaEventCreate(&c->ev1));
-    c->xlogxt = xlogxt ? xlogxt : make_xlogx_table(c->stream);
+    c->xlogxt = xlogxt ? xlogxt : make_xlogx_table();
     return c;
   }
   // The process's context: every entry point runs on it.
@@ -566,12 +565,13 @@ struct SbpGraph {
 struct SbpBlockmodel {
   int V = 0, B = 0, ld = 0;
   const SbpGraph* graph = nullptr;   // the graph the blockmodel was created on (must outlive it)
-  DevBuf<int> b, CS, CST, d_out, d_in, d;
+  DevBuf<int> b, CS, CST, SS, SST, d_out, d_in, d;
+  DevBuf<double> inv_d;
   DevBuf<int2> P;                            // dense counts of both directions (BlockView::P)
   DevBuf<int> prop, qr, qs, moved, n_moved;   // n_moved: two slots, alternating per batch
   DevBuf<unsigned long long> last;           // (batch generation << 32 | last mover) per block
   unsigned gen = 0;                          // batch generation
-  int nch = 0, ncs = 0;
+  int nch = 0, ncs = 0, nss = 0;
   // row-hashed representation (B > dense_max_blocks)
   bool sparse = false;
   DevBuf<long long> rbase, cbase;
@@ -597,6 +597,9 @@ struct SbpBlockmodel {
     v.ld = ld;
     v.nch = nch;
     v.ncs = ncs;
+    v.nss = nss;
+    v.SS = SS.p;
+    v.SST = SST.p;
     v.CS = CS.p;
     v.CST = CST.p;
     v.b = b.p;
@@ -604,6 +607,7 @@ struct SbpBlockmodel {
     v.d_out = d_out.p;
     v.d_in = d_in.p;
     v.d = d.p;
+    v.inv_d = inv_d.p;
     v.xlogxt = Context::get().xlogxt;
     return v;
   }
@@ -628,7 +632,7 @@ struct SbpBlockmodel {
     Context& c = Context::get();
     B = nb;
     sparse = B > g_dense_max_blocks;
-    const double dense_bytes = 2.0 * (double)B * (double)(((B + kChunk - 1) / kChunk) * kChunk) * sizeof(int);
+    const double dense_bytes = 2.0 * (double)B * (double)(((B + kRowPad - 1) / kRowPad) * kRowPad) * sizeof(int);
     // dense only while it takes at most 60 % of the free device memory; cudaMemGetInfo can
     // stall the host for tens of milliseconds, so it is asked only for a matrix above 5 % of
     // the device's memory
@@ -643,9 +647,10 @@ struct SbpBlockmodel {
         cudaGetLastError();
       }
     }
-    ld = ((B + kChunk - 1) / kChunk) * kChunk;
+    ld = ((B + kRowPad - 1) / kRowPad) * kRowPad;
     nch = (B + kChunk - 1) / kChunk;
-    ncs = (nch + 3) & ~3;
+    ncs = (nch + kFan - 1) / kFan * kFan;
+    nss = nch > kFan ? (ncs / kFan + kFan - 1) / kFan * kFan : 0;
     if (sparse) {
       rbase.reserve(B);
       cbase.reserve(B);
@@ -655,14 +660,19 @@ struct SbpBlockmodel {
     } else {
       const size_t cells = (size_t)B * (size_t)ld;
       P.reserve(cells);
-      if (nch > 1) {
+      if (B > kSmallB) {
         CS.reserve((size_t)B * ncs);
         CST.reserve((size_t)B * ncs);
+        if (nss) {
+          SS.reserve((size_t)B * nss);
+          SST.reserve((size_t)B * nss);
+        }
       }
     }
     d_out.reserve(B);
     d_in.reserve(B);
     d.reserve(B);
+    inv_d.reserve(B);
     last.reserve(B);
     SBP_CUDA(cudaMemsetAsync(last.p, 0, sizeof(unsigned long long) * B, c.stream));
   }

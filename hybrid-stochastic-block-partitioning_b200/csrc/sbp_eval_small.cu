@@ -114,104 +114,6 @@ __device__ __forceinline__ T ldb(const T* p) {
   else return *p;
 }
 
-// The multinomial walk of evaluate_vertex over a dense row (or column) of M: the first column
-// whose running count exceeds tg.  Chunk sums (kChunk columns each) locate the chunk, sixteen per
-// lane per step (one memory round trip per 16 G chunks); the chunk's counts are then scanned
-// sixteen per lane.  Every lane of the warp
-// takes part (loop bounds are warp-uniform); groups with walk == false get -1.
-constexpr int kSumsPerLane = 16;
-
-template <int G, bool kFrozen>
-__device__ __forceinline__ int group_walk(const int2* row, bool in_col, const int* csum, int nch, int B, long long tg, bool walk, int gl,
-                                          int gbase) {
-  const unsigned gmask = (G == 32 ? kFull : ((1u << G) - 1u) << gbase);
-  int chunk = 0;
-  long long before = 0;   // counts of the row before the chosen chunk
-  if (nch > 1) {
-    bool found = !walk;
-    chunk = -1;
-    long long acc = 0;
-    for (int c0 = 0; c0 < nch; c0 += kSumsPerLane * G) {
-      int cs[kSumsPerLane];
-      long long lsum = 0;
-#pragma unroll
-      for (int q = 0; q < kSumsPerLane; ++q) {
-        const int c = c0 + gl * kSumsPerLane + q;
-        cs[q] = (walk && c < nch) ? ldb<kFrozen>(csum + c) : 0;
-        lsum += cs[q];
-      }
-      long long incl = lsum;
-#pragma unroll
-      for (int o = 1; o < G; o <<= 1) {
-        const long long y = __shfl_up_sync(kFull, incl, o, G);
-        if (gl >= o) incl += y;
-      }
-      const long long tot = __shfl_sync(kFull, incl, G - 1, G);
-      const unsigned hit = __ballot_sync(kFull, !found && acc + incl > tg) & gmask;
-      int pick = -1;
-      long long pb = 0;
-      if (hit && gl == __ffs(hit) - 1 - gbase) {
-        long long run = acc + incl - lsum;
-#pragma unroll
-        for (int q = 0; q < kSumsPerLane; ++q) {
-          if (pick < 0) {
-            if (tg < run + cs[q]) {
-              pick = c0 + gl * kSumsPerLane + q;
-              pb = run;
-            } else {
-              run += cs[q];
-            }
-          }
-        }
-      }
-      const int src = hit ? __ffs(hit) - 1 - gbase : 0;
-      const int pk = __shfl_sync(kFull, pick, src, G);
-      const long long pbb = __shfl_sync(kFull, pb, src, G);
-      if (hit && !found) {
-        chunk = pk;
-        before = pbb;
-        found = true;
-      }
-      acc += tot;
-    }
-    if (walk && chunk < 0) walk = false;
-  }
-  constexpr int kPer = kChunk / G;   // counts per lane
-  const int2* base = row + (size_t)(chunk < 0 ? 0 : chunk) * kChunk + gl * kPer;
-  int vals[kPer];
-  long long lsum = 0;
-#pragma unroll
-  for (int q = 0; q < kPer / 2; ++q) {
-    // a row of one chunk ends at column B: the pairs beyond it are not read
-    const int4 c4 = (nch > 1 || gl * kPer + 2 * q < B) ? ldb<kFrozen>(reinterpret_cast<const int4*>(base) + q)
-                                                       : make_int4(0, 0, 0, 0);
-    vals[2 * q] = in_col ? c4.y : c4.x;
-    vals[2 * q + 1] = in_col ? c4.w : c4.z;
-    lsum += (long long)vals[2 * q] + vals[2 * q + 1];
-  }
-  long long incl = lsum;
-#pragma unroll
-  for (int o = 1; o < G; o <<= 1) {
-    const long long y = __shfl_up_sync(kFull, incl, o, G);
-    if (gl >= o) incl += y;
-  }
-  const long long t2 = tg - before;
-  const unsigned hit = __ballot_sync(kFull, walk && incl > t2) & gmask;
-  int col = -1;
-  if (walk && hit && gl == __ffs(hit) - 1 - gbase) {
-    long long rem = t2 - (incl - lsum);
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      if (col < 0) {
-        if (rem < vals[q]) col = (chunk < 0 ? 0 : chunk) * kChunk + gl * kPer + q;
-        else rem -= vals[q];
-      }
-    }
-  }
-  const int found = __shfl_sync(kFull, col, hit ? __ffs(hit) - 1 - gbase : 0, G);
-  return walk ? found : -1;
-}
-
 // Result of one group's evaluation of a vertex; every lane of the group holds it.
 struct GroupEval {
   int v, r, s, t;        // vertex, its block, proposed block, the proposal's neighbour block (-1: none)
@@ -282,8 +184,9 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       in_row = target < dot;
       tg = in_row ? target : target - dot;
     }
-    const int* csum = (in_row ? bm.CS : bm.CST) + (size_t)t * bm.ncs;
-    const int found = group_walk<G, kFrozen>(bm.P + (size_t)t * ld, !in_row, csum, bm.nch, B, tg, walk, gl, gbase);
+    const Lanes L(G, threadIdx.x & 31);
+    const int found = kHash ? walk_tree<Store::kDense>(bm, t, !in_row, (int)tg, walk, L)
+                            : walk_row<Store::kDense>(bm, t, !in_row, (int)tg, walk, L);
     if (walk) {
       s = found;
       if (s < 0 || s >= B) {
@@ -338,16 +241,15 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       const int co = wu & kCountMask, ci = (wu >> kInShift) & kCountMask;
       const int2 m_ru = ldb<kFrozen>(bm.P + (size_t)r * ld + u), m_su = ldb<kFrozen>(bm.P + (size_t)s * ld + u);
       const int M_ru = m_ru.x, M_ur = m_ru.y, M_su = m_su.x, M_us = m_su.y;
-      const int du = ldb<kFrozen>(bm.d + u);
+      const double inv_u = ldb<kFrozen>(bm.inv_d + u);   // a non-corner block's degree is unchanged
       const bool is_r = u == r, is_s = u == s, corner = is_r || is_s;
       const double c = (double)(co + ci + (is_r ? self : 0));
-      const double inv_u = 1.0 / ((double)du + (double)B);   // a non-corner block's degree is unchanged
       fwd += c * (M_su + M_us + 1.0) * inv_u;
       const double bw = is_r ? (double)(M_rr + d_rr) + (double)(M_rr + d_rr) + 1.0
                       : is_s ? (double)(M_rs + d_rs) + (double)(M_sr + d_sr) + 1.0
                              : (double)(M_ru - co) + (double)(M_ur - ci) + 1.0;
       const int nd = is_r ? (dout_r - k_out) + (din_r - k_in) - (M_rr + d_rr)
-                   : is_s ? (dout_s + k_out) + (din_s + k_in) - (M_ss + d_ss) : du;
+                   : (dout_s + k_out) + (din_s + k_in) - (M_ss + d_ss);   // corner blocks only
       bwd += c * bw * (corner ? 1.0 / ((double)nd + (double)B) : inv_u);
       if (!corner) {   // cells (r,u) (s,u) for out-edges to u, (u,r) (u,s) for in-edges
         if (co) {
@@ -573,8 +475,8 @@ __global__ void __launch_bounds__(kMhGroupThreads)
         bm.d_in[r] -= e.k_in + self;
         bm.d_in[s] += e.k_in + self;
         // Blockmodel::move_vertex reads the already-updated diagonal and adds the delta again
-        bm.d[r] = bm.d_out[r] + bm.d_in[r] - (bm.P[(size_t)r * bm.ld + r].x + d_rr);
-        bm.d[s] = bm.d_out[s] + bm.d_in[s] - (bm.P[(size_t)s * bm.ld + s].x + d_ss);
+        set_degree(bm, r, bm.d_out[r] + bm.d_in[r] - (bm.P[(size_t)r * bm.ld + r].x + d_rr));
+        set_degree(bm, s, bm.d_out[s] + bm.d_in[s] - (bm.P[(size_t)s * bm.ld + s].x + d_ss));
       }
     }
     pos += s_upto;

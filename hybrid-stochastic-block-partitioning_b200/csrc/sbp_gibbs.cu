@@ -94,7 +94,7 @@ __device__ __forceinline__ void add_counts(EvalCounts c, unsigned long long* cou
 }
 
 template <bool kDirect>
-__global__ void __launch_bounds__(kGroupThreads, 3)
+__global__ void __launch_bounds__(kGroupThreads, 2)
     k_gibbs_eval(const __grid_constant__ EvalArgs a, BatchDesc b, int sweep, int* n_moved, unsigned long long* counters) {
   extern __shared__ int smem[];
   group_tabs_init<kDirect>(smem, a.slots);
@@ -174,7 +174,7 @@ __device__ __forceinline__ bool sync_grid(const SweepsArgs& a, unsigned* target,
 }
 
 template <bool kDirect>
-__global__ void __launch_bounds__(kGroupThreads, 3) k_gibbs_sweeps(const __grid_constant__ SweepsArgs a) {
+__global__ void __launch_bounds__(kGroupThreads, 2) k_gibbs_sweeps(const __grid_constant__ SweepsArgs a) {
   extern __shared__ int smem[];
   __shared__ double red[32];
   __shared__ int s_abort, s_stop;
@@ -287,7 +287,7 @@ void launch_gibbs_eval(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& pl
   const BatchDesc& d = plan.desc[bt];
   const int n = d.light_n + d.heavy_n;
   const bool direct = bm.B <= kSmallB;
-  a.gmin = group_min(n, 3 * kGroupWarps * c.num_sms);
+  a.gmin = group_min(n, 2 * kGroupWarps * c.num_sms);
   const size_t smem = group_smem_bytes(direct, a.slots);
   const auto k = direct ? k_gibbs_eval<true> : k_gibbs_eval<false>;
   set_smem_limit((const void*)k, smem);

@@ -7,12 +7,12 @@
 // them, so what counts is how many visits are in flight and how few instructions each costs:
 //   * a group of G = 8, 16 or 32 lanes evaluates one vertex, so a warp carries 32 / G of them and
 //     pays the scalar part of a visit (random record, walk, reductions, accept) once for all;
-//   * G is chosen per task from the vertex's degree: with G lanes a group owns 16 G slots of its
-//     warp's table region, at least twice the degree.  Every loop runs to the largest trip count
-//     of the warp's groups, so the vertices of a batch are ordered by degree;
+//   * G is chosen per task from the vertex's degree, at most four neighbours a lane; a group owns 16 G
+//     slots of its warp's table region.  Every loop runs to the largest trip count of the warp's
+//     groups, so the vertices of a batch are ordered by degree;
 //   * a vertex's CSR ranges come as one 16-byte record and its out- and in-neighbours as one list;
-//   * the block of the proposal's neighbour and that block's degrees are fetched while the
-//     neighbour-block histogram is being built.
+//   * the loads of a step are issued together, and what does not depend on the proposal before
+//     the walk that picks it.
 // Summation orders differ from evaluate_vertex, so delta-MDL and the Hastings factor agree with it
 // to rounding; every integer input is the same.
 #pragma once
@@ -23,34 +23,12 @@ namespace sbpb {
 constexpr int kRegionSlots = 512;   // table slots of one warp, shared by its groups
 constexpr int kGroupWarps = 8;      // warps per CTA
 constexpr int kGroupThreads = 32 * kGroupWarps;
-constexpr int kSmallB = 128;        // direct-indexed histograms up to this many blocks
-
-struct Lanes {   // the calling lane's place in its group
-  int G, gl, lane, gbase;
-  unsigned gmask;
-  __device__ __forceinline__ Lanes(int group, int lane_) : G(group), lane(lane_) {
-    gl = lane & (G - 1);
-    gbase = lane & ~(G - 1);
-    gmask = G == 32 ? kFull : ((1u << G) - 1u) << gbase;
-  }
-};
-
 __device__ __forceinline__ double group_sum(double v, const Lanes& L) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
     if (o < L.G) v += __shfl_xor_sync(kFull, v, o);
   return v;
 }
-__device__ __forceinline__ int group_incl_scan(int v, const Lanes& L) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1)
-    if (o < L.G) {
-      const int y = __shfl_up_sync(kFull, v, o);
-      if (L.gl >= o) v += y;
-    }
-  return v;
-}
-
 // Neighbour-block histogram of one group.  Slot words hold out count | in count << 15 | presence <<
 // 30; the list holds the slots in use.  kDirect (B <= kSmallB): the slot is the block; otherwise an
 // open-addressing table of mask + 1 slots.
@@ -65,7 +43,7 @@ struct GroupTab {
   unsigned short* list;
   int mask;
   __device__ __forceinline__ unsigned home(int key) const { return ((unsigned)key * 2654435761u) >> 16 & (unsigned)mask; }
-  // Add `delta` to the word of `key`, whose home slot was tried with the result `k` (the slot's key
+  // Add `delta` to the word of `key`, whose home slot h was tried with the result `k` (the slot's key
   // before the try); returns the slot when this lane made it, else -1.
   __device__ __forceinline__ int finish_add(int key, unsigned h, int k, unsigned delta, int* status) const {
     for (int probe = 0; k != -1 && k != key; ++probe) {
@@ -137,115 +115,13 @@ __device__ __forceinline__ void group_tabs_init(int* smem, int slots) {
   }
 }
 
-// The multinomial walk over row t of M (column t when `col`): the first index whose running count
-// exceeds tg.  The chunk sums locate the chunk: each lane sums a piece of the range, a scan picks
-// the piece, until four sums are left; pieces after the first level hit in L1.  Then the first
-// eight lanes of the group read the chunk's 128 pairs in eight coalesced steps, a transposing
-// reduction leaves sub-chunk q's total on lane q, and the sub-chunk picked is scanned two columns
-// a lane.  Every lane of the warp calls it; groups with !on get -1.
-template <Store ST>
-__device__ __forceinline__ int group_walk(const BlockView& bm, const int2* row, bool col, const int* csum, int tg,
-                                          bool on, const Lanes& L) {
-  int chunk = 0;
-  bool ok = on;
-  if (bm.nch > 1) {
-    int lo = 0, len = bm.ncs;
-    while (len > 4) {
-      const int piece = ((len + L.G - 1) / L.G + 3) & ~3;
-      const int a = lo + L.gl * piece, e = min(lo + min(len, (L.gl + 1) * piece), bm.ncs);
-      int v = 0;
-      if (ok) {
-#pragma unroll 4
-        for (int c = a; c < e; c += 4) {
-          const int4 q = ldv<ST>(reinterpret_cast<const int4*>(csum + c));
-          v += (q.x + q.y) + (q.z + q.w);
-        }
-      }
-      const int incl = group_incl_scan(v, L);
-      const unsigned hit = __ballot_sync(kFull, ok && incl > tg) & L.gmask;
-      ok = ok && hit;
-      const int src = hit ? __ffs(hit) - 1 : L.gbase;
-      tg -= __shfl_sync(kFull, incl - v, src);
-      lo += (src - L.gbase) * piece;
-      len = piece;
-    }
-    if (ok) {
-      const int4 q = ldv<ST>(reinterpret_cast<const int4*>(csum + lo));
-      int j = 0;
-      if (tg >= q.x) { tg -= q.x; j = 1;
-        if (tg >= q.y) { tg -= q.y; j = 2;
-          if (tg >= q.z) { tg -= q.z; j = 3; } } }
-      chunk = lo + j;
-      ok = chunk < bm.nch;
-    }
-  }
-  const int g8 = L.lane & 7;
-  const bool rd = ok && L.gl < 8;
-  const int2* base = row + (size_t)(ok ? chunk : 0) * kChunk;
-  const int ncol = bm.nch > 1 ? kChunk : bm.B;   // a single chunk ends at column B
-  int v[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int c = 16 * q + 2 * g8;
-    const int4 x = (rd && c < ncol) ? ldv<ST>(reinterpret_cast<const int4*>(base + c)) : make_int4(0, 0, 0, 0);
-    v[q] = col ? x.y + x.w : x.x + x.z;
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const bool up = g8 & 4;
-    const int give = up ? v[q] : v[q + 4], keep = up ? v[q + 4] : v[q];
-    v[q] = keep + __shfl_xor_sync(kFull, give, 4);
-  }
-#pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const bool up = g8 & 2;
-    const int give = up ? v[q] : v[q + 2], keep = up ? v[q + 2] : v[q];
-    v[q] = keep + __shfl_xor_sync(kFull, give, 2);
-  }
-  int total;
-  {
-    const bool up = g8 & 1;
-    const int give = up ? v[0] : v[1], keep = up ? v[1] : v[0];
-    total = keep + __shfl_xor_sync(kFull, give, 1);
-  }
-  int incl = total;   // scan over eight lanes
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) {
-    const int y = __shfl_up_sync(kFull, incl, o);
-    if (g8 >= o) incl += y;
-  }
-  unsigned hit = __ballot_sync(kFull, rd && incl > tg) & L.gmask;
-  ok = ok && hit;
-  int src = hit ? __ffs(hit) - 1 : L.gbase;
-  tg -= __shfl_sync(kFull, incl - total, src);
-  const int sub = 16 * (src - L.gbase);
-  int c0 = 0, c1 = 0;
-  if (ok && L.gl < 8) {
-    const int4 x = ldv<ST>(reinterpret_cast<const int4*>(base + sub + 2 * g8));
-    c0 = col ? x.y : x.x;
-    c1 = col ? x.w : x.z;
-  }
-  incl = c0 + c1;
-#pragma unroll
-  for (int o = 1; o < 8; o <<= 1) {
-    const int y = __shfl_up_sync(kFull, incl, o);
-    if (g8 >= o) incl += y;
-  }
-  hit = __ballot_sync(kFull, ok && L.gl < 8 && incl > tg) & L.gmask;
-  src = hit ? __ffs(hit) - 1 : L.gbase;
-  const int second = tg >= incl - c1 ? 1 : 0;   // on the lane picked: its first or second column
-  const int at = chunk * kChunk + sub + 2 * g8 + second;
-  const int found = __shfl_sync(kFull, at, src);
-  return ok && hit ? found : -1;
-}
-
 // Result of one group's evaluation; every lane of the group holds it.
 struct GroupEval {
   int v, r, s, t;        // vertex, its block, proposed block, the proposal's neighbour block (-1: none)
   int k_out, k_in, self;
   int n;                 // table slots in use
   bool valid, accepted;
-  double dS, H;
+  double dS;
 };
 
 // A vertex of a batch: (vertex, first neighbour in the joint list, out-degree incl. the self loop,
@@ -270,9 +146,38 @@ static __device__ __noinline__ double net_zero_term(int m, int a, int b, int c, 
   return (double)m * (log1p((double)a / (double)b) + log1p((double)c / (double)d));
 }
 
+// Accept test u <= min(1, exp(-3 dS) H), H = bwd / fwd (1 for a vertex without neighbours).  A
+// single-precision estimate decides wherever it is further from u than its error (under 1e-4
+// relative) can reach; only the rest, about one visit in a thousand, takes the FP64 exponential
+// and division, a chain of some 800 cycles.  The decision is the FP64 test's in every case.
+__device__ __forceinline__ bool accept_move(double dS, double fwd, double bwd, bool alone, double u) {
+  const double x = -3.0 * dS;
+  const float xf = (float)x, hf = alone ? 1.0f : __fdividef((float)bwd, (float)fwd);
+  if (hf > 1e-6f && hf < 1e6f) {
+    if (xf < -80.0f) {
+      if (u > 1e-20) return false;
+    } else if (xf > 80.0f) {
+      if (u <= 1.0) return true;
+    } else {
+      const float af = __expf(xf) * hf, uf = (float)u;
+      if (uf > af * 1.001f) return false;
+      if (uf < af * 0.999f && u <= 1.0) return true;
+    }
+  }
+  const double H = alone ? 1.0 : bwd / fwd;
+  double ap = exp(x) * H;
+  ap = ap >= 1.0 ? 1.0 : ap;
+  return u <= ap;
+}
+
 // Evaluate the vertex of `rec` (groups with `valid`) against the blockmodel with random record x:
 // gather its neighbour blocks into the group's table (left filled: res.n slots; the caller clears
 // it), propose, delta-MDL, Hastings, accept.  Every lane of the warp calls it.
+//
+// A lane holds up to four neighbours, and up to four table entries, at a time, so the loads of a
+// step are all in flight together: the classes of group_max_k give a group four neighbours a lane
+// at most (a vertex beyond the largest class takes several rounds).  Row r of the entries is
+// fetched before the walk, which does not depend on it.
 template <bool kDirect, Store ST>
 __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const BlockView& bm, const GroupTab<kDirect>& T,
                                                     bool valid, int4 rec, bool given, uint4 x, const Lanes& L,
@@ -282,25 +187,28 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
   res.valid = valid;
   res.accepted = false;
   res.dS = 0.0;
-  res.H = 1.0;
   const int v = res.v = rec.x;
   const int k_out = res.k_out = valid ? rec.z : 0, k_in = res.k_in = valid ? rec.w >> 1 : 0;
   const int self = res.self = valid ? rec.w & 1 : 0;
   const int k = k_out + k_in;
-  const int r = res.r = valid ? ldv<ST>(bm.b + v) : 0;
   const int* nbr = g.adj + (unsigned)rec.y;
   const bool walk = valid && !given && k > 0;
-  // 1. the proposal's neighbour and its block's degrees, and the neighbour-block histogram
-  int t = 0, dot = 0, dit = 0;
-  if (walk) t = ldv<ST>(bm.b + __ldg(nbr + scale32(x.x, k)));
-  int n = 0;
+  // 1. the neighbour-block histogram, and the block of the proposal's neighbour with its degrees
+  int r = 0, t = 0, dot = 0, dit = 0, n = 0;
+  const int pick = walk ? (int)scale32(x.x, k) : -1;
   const int kmax = (int)__reduce_max_sync(kFull, (unsigned)k);
-  for (int e0 = 0; e0 < kmax; e0 += 4 * L.G) {
+  for (int e0 = 0; e0 == 0 || e0 < kmax; e0 += 4 * L.G) {
     int u[4], bu[4];
+    int ut = -1;
+    if (e0 == 0 && walk) ut = __ldg(nbr + pick);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int e = e0 + j * L.G + L.gl;
       u[j] = e < k ? __ldg(nbr + e) : -1;
+    }
+    if (e0 == 0) {
+      if (valid) r = ldv<ST>(bm.b + v);
+      if (walk) t = ldv<ST>(bm.b + ut);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) bu[j] = u[j] >= 0 ? ldv<ST>(bm.b + u[j]) : -1;
@@ -336,7 +244,8 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       n += __popc(fresh);
     }
   }
-  {   // the self loop only marks r present
+  res.r = r;
+  if (__any_sync(kFull, self)) {   // the self loop only marks r present
     int made = -1;
     if (self && L.gl == 0) made = T.add(r, kPresent, status);
     const unsigned fresh = __ballot_sync(kFull, made >= 0) & L.gmask;
@@ -346,14 +255,38 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
   __syncwarp();
   res.n = n;
   res.t = walk ? t : -1;
+  // this lane's first entries and what of them depends on r alone
+  const int2* Pr = bm.P + (size_t)r * bm.ld;
+  int u[4];
+  unsigned wu[4];
+  int2 m_ru[4];
+  double inv[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    const int j = L.gl + h * L.G;
+    const int slot = j < n ? T.list[j] : -1;
+    u[h] = slot >= 0 ? T.key_of(slot) : r;
+    wu[h] = slot >= 0 ? T.w[slot] : 0u;
+  }
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    m_ru[h] = wu[h] ? ldv<ST>(Pr + u[h]) : make_int2(0, 0);
+    inv[h] = wu[h] ? ldv<ST>(bm.inv_d + u[h]) : 0.0;
+  }
+  int M_rr = 0, dout_r = 0, din_r = 0;
+  if (valid) {
+    M_rr = ldi<ST>(&Pr[r].x);
+    dout_r = ldv<ST>(bm.d_out + r);
+    din_r = ldv<ST>(bm.d_in + r);
+  }
+  const unsigned wr = T.counts_of(r);
   // 2. the proposal: the multinomial over row t of M, then column t (ascending)
   int s = r;
   {
     const long long target = scale32(x.y, (long long)dot + (long long)dit);
     const bool in_col = target >= dot;
     const int tg = (int)(in_col ? target - dot : target);
-    const int found = group_walk<ST>(bm, bm.P + (size_t)t * bm.ld, in_col,
-                                     (in_col ? bm.CST : bm.CS) + (size_t)t * bm.ncs, tg, walk, L);
+    const int found = kDirect ? walk_row<ST>(bm, t, in_col, tg, walk, L) : walk_tree<ST>(bm, t, in_col, tg, walk, L);
     if (walk) {
       s = found;
       if (s < 0 || s >= B) {
@@ -374,79 +307,31 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
   const bool active = valid && s != r;
   if (!__any_sync(kFull, active)) return res;
   // 3. delta-MDL and the Hastings correction of the move r -> s
-  const int2* Pr = bm.P + (size_t)r * bm.ld;
   const int2* Ps = bm.P + (size_t)s * bm.ld;
-  double fwd = 0.0, bwd = 0.0, dS = 0.0;
-  int co_r = 0, ci_r = 0, co_s = 0, ci_s = 0;
-  int M_rr = 0, M_rs = 0, M_sr = 0, M_ss = 0, dout_r = 0, dout_s = 0, din_r = 0, din_s = 0;
+  int2 m_su[4], m_rs = make_int2(0, 0);
+  int M_ss = 0, dout_s = 0, din_s = 0;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) m_su[h] = active && wu[h] ? ldv<ST>(Ps + u[h]) : make_int2(0, 0);
   if (active) {
-    const int2 m_rs = ldv<ST>(Pr + s);
-    M_rr = ldi<ST>(&Pr[r].x);
-    M_rs = m_rs.x;
-    M_sr = m_rs.y;
+    m_rs = ldv<ST>(Pr + s);
     M_ss = ldi<ST>(&Ps[s].x);
-    dout_r = ldv<ST>(bm.d_out + r);
     dout_s = ldv<ST>(bm.d_out + s);
-    din_r = ldv<ST>(bm.d_in + r);
     din_s = ldv<ST>(bm.d_in + s);
-    const unsigned wr = T.counts_of(r), ws = T.counts_of(s);
-    co_r = wr & kCountMask;
-    ci_r = (wr >> kInShift) & kCountMask;
-    co_s = ws & kCountMask;
-    ci_s = (ws >> kInShift) & kCountMask;
   }
+  const unsigned ws = T.counts_of(s);
+  const int co_r = wr & kCountMask, ci_r = (wr >> kInShift) & kCountMask;
+  const int co_s = ws & kCountMask, ci_s = (ws >> kInShift) & kCountMask;
+  const int M_rs = m_rs.x, M_sr = m_rs.y;
   const int d_rr = -co_r - ci_r - self;
   const int d_rs = -co_s + ci_r;
   const int d_sr = co_r - ci_s;
   const int d_ss = co_s + ci_s + self;
   const int kin_self = k_in + self;
-  const int nent = active ? n : 0;
   // every count that changes lies in a row or column of r or s: at most their degrees after the move
   const bool small = dout_r + k < kXlogxTable && dout_s + k < kXlogxTable && din_r + k < kXlogxTable &&
                      din_s + k < kXlogxTable;
   const double2* __restrict__ gt = bm.xlogxt;
-  for (int j0 = L.gl; j0 < nent; j0 += 2 * L.G) {   // two entries in flight
-    int2 m_ru[2], m_su[2];
-    int u[2], du[2];
-    unsigned wu[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int j = j0 + h * L.G;
-      const bool on = j < nent;
-      const int slot = on ? T.list[j] : 0;
-      u[h] = on ? T.key_of(slot) : r;
-      wu[h] = on ? T.w[slot] : 0u;
-      m_ru[h] = on ? ldv<ST>(Pr + u[h]) : make_int2(0, 0);
-      m_su[h] = on ? ldv<ST>(Ps + u[h]) : make_int2(0, 0);
-      du[h] = on ? ldv<ST>(bm.d + u[h]) : 0;
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int co = wu[h] & kCountMask, ci = (wu[h] >> kInShift) & kCountMask;
-      const bool is_r = u[h] == r, corner = is_r || u[h] == s;
-      const int c = co + ci;
-      const double inv = 1.0 / ((double)du[h] + (double)B);   // a non-corner block's degree is unchanged
-      const double cf = (double)(c + (is_r && wu[h] ? self : 0)), cb = corner ? 0.0 : (double)c;
-      fwd += cf * ((double)m_su[h].x + (double)m_su[h].y + 1.0) * inv;
-      bwd += cb * ((double)(m_ru[h].x - co) + (double)(m_ru[h].y - ci) + 1.0) * inv;
-      // cells (r,u) (s,u) for out-edges to u, (u,r) (u,s) for in-edges; the corners are added below
-      if (small) {
-        const bool out = co != 0;
-        const int d = corner ? 0 : out ? co : ci;
-        const int ar = out ? m_ru[h].x : m_ru[h].y, as = out ? m_su[h].x : m_su[h].y;
-        const double2 g0 = __ldg(gt + ar), g1 = __ldg(gt + ar - d), g2 = __ldg(gt + as), g3 = __ldg(gt + as + d);
-        dS += ((g0.x - g1.x) + (g0.y - g1.y)) + ((g2.x - g3.x) + (g2.y - g3.y));
-        if (co && ci && !corner) {
-          const double2 h0 = __ldg(gt + m_ru[h].y), h1 = __ldg(gt + m_ru[h].y - ci);
-          const double2 h2 = __ldg(gt + m_su[h].y), h3 = __ldg(gt + m_su[h].y + ci);
-          dS += ((h0.x - h1.x) + (h0.y - h1.y)) + ((h2.x - h3.x) + (h2.y - h3.y));
-        }
-      } else if (!corner) {
-        if (co) dS += dxlogx_wide(gt, m_ru[h].x, m_ru[h].x - co) + dxlogx_wide(gt, m_su[h].x, m_su[h].x + co);
-        if (ci) dS += dxlogx_wide(gt, m_ru[h].y, m_ru[h].y - ci) + dxlogx_wide(gt, m_su[h].y, m_su[h].y + ci);
-      }
-    }
-  }
+  double fwd = 0.0, bwd = 0.0, dS = 0.0;
   // corner cells (r,r) (r,s) (s,r) (s,s), then the out- and in-degrees of r and s
   const int q = L.gl;
   const int qa = q == 0 ? M_rr : q == 1 ? M_rs : q == 2 ? M_sr : q == 3 ? M_ss
@@ -472,6 +357,48 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       dS += q == 0 ? net_zero_term(M_rs, kin_self, din_s, -k_out, dout_r)
                    : net_zero_term(M_sr, -kin_self, din_r, k_out, dout_s);
   }
+  const int nent = active ? n : 0;
+  const int nmax = (int)__reduce_max_sync(kFull, (unsigned)nent);
+  for (int j0 = 0;;) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      if (j0 + h * L.G >= nmax) break;   // warp-uniform
+      const int co = active ? wu[h] & kCountMask : 0, ci = active ? (wu[h] >> kInShift) & kCountMask : 0;
+      const bool is_r = u[h] == r, corner = is_r || u[h] == s;
+      const int c = co + ci;
+      const double cf = (double)(c + (is_r && wu[h] ? self : 0)), cb = corner ? 0.0 : (double)c;
+      fwd += cf * ((double)m_su[h].x + (double)m_su[h].y + 1.0) * inv[h];
+      bwd += cb * ((double)(m_ru[h].x - co) + (double)(m_ru[h].y - ci) + 1.0) * inv[h];
+      // cells (r,u) (s,u) for out-edges to u, (u,r) (u,s) for in-edges; the corners were added above
+      if (small) {
+        const bool out = co != 0;
+        const int d = corner ? 0 : out ? co : ci;
+        const int ar = out ? m_ru[h].x : m_ru[h].y, as = out ? m_su[h].x : m_su[h].y;
+        const double2 g0 = __ldg(gt + ar), g1 = __ldg(gt + ar - d), g2 = __ldg(gt + as), g3 = __ldg(gt + as + d);
+        dS += ((g0.x - g1.x) + (g0.y - g1.y)) + ((g2.x - g3.x) + (g2.y - g3.y));
+        if (co && ci && !corner) {
+          const double2 h0 = __ldg(gt + m_ru[h].y), h1 = __ldg(gt + m_ru[h].y - ci);
+          const double2 h2 = __ldg(gt + m_su[h].y), h3 = __ldg(gt + m_su[h].y + ci);
+          dS += ((h0.x - h1.x) + (h0.y - h1.y)) + ((h2.x - h3.x) + (h2.y - h3.y));
+        }
+      } else if (!corner) {
+        if (co) dS += dxlogx_wide(gt, m_ru[h].x, m_ru[h].x - co) + dxlogx_wide(gt, m_su[h].x, m_su[h].x + co);
+        if (ci) dS += dxlogx_wide(gt, m_ru[h].y, m_ru[h].y - ci) + dxlogx_wide(gt, m_su[h].y, m_su[h].y + ci);
+      }
+    }
+    j0 += 4 * L.G;
+    if (j0 >= nmax) break;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {   // the next entries of a vertex of more than 4 G distinct blocks
+      const int j = j0 + L.gl + h * L.G;
+      const int slot = j < nent ? T.list[j] : -1;
+      u[h] = slot >= 0 ? T.key_of(slot) : r;
+      wu[h] = slot >= 0 ? T.w[slot] : 0u;
+      m_ru[h] = wu[h] ? ldv<ST>(Pr + u[h]) : make_int2(0, 0);
+      m_su[h] = wu[h] ? ldv<ST>(Ps + u[h]) : make_int2(0, 0);
+      inv[h] = wu[h] ? ldv<ST>(bm.inv_d + u[h]) : 0.0;
+    }
+  }
   fwd = group_sum(fwd, L);
   bwd = group_sum(bwd, L);
   dS = group_sum(dS, L);
@@ -481,12 +408,12 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
     if (snap) {
       for (int j = L.gl; j < nent; j += L.G) {
         const int slot = T.list[j];
-        const int u = T.key_of(slot);
-        const unsigned wu = T.w[slot];
-        if (u == r || u == s) continue;
-        const int2 a = Pr[u], b = Ps[u];
-        if (wu & kCountMask) Tz += 2.0 * ((double)a.x + (double)b.x);
-        if ((wu >> kInShift) & kCountMask) Tz += 2.0 * ((double)a.y + (double)b.y);
+        const int uu = T.key_of(slot);
+        const unsigned w = T.w[slot];
+        if (uu == r || uu == s) continue;
+        const int2 a = Pr[uu], b = Ps[uu];
+        if (w & kCountMask) Tz += 2.0 * ((double)a.x + (double)b.x);
+        if ((w >> kInShift) & kCountMask) Tz += 2.0 * ((double)a.y + (double)b.y);
       }
       if (q < 4 && qd) Tz += 2.0 * (double)qa + (double)qd;
       if (q >= 4 && q < 8) Tz += 2.0 * (double)qa;
@@ -495,17 +422,13 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
     if (snap && fabs(dS) <= 0x1p-40 * Tz * g.log_E) dS = 0.0;
   }
   if (active) {
-    const double H = (k == 0) ? 1.0 : bwd / fwd;
-    double ap = exp(-3.0 * dS) * H;
-    ap = ap >= 1.0 ? 1.0 : ap;
-    res.accepted = (given ? record_uniform(x) : u53(x.z, x.w)) <= ap;
+    res.accepted = accept_move(dS, fwd, bwd, k == 0, given ? record_uniform(x) : u53(x.z, x.w));
     res.dS = dS;
-    res.H = H;
   }
   return res;
 }
 
-// Largest degree a group of G lanes takes: its share of the region is at least twice that many slots.
-__host__ __device__ constexpr int group_max_k(int G) { return kRegionSlots * G / 32 / 2; }
+// Largest degree of the class of G lanes: four neighbours a lane, a quarter of its slots.
+__host__ __device__ constexpr int group_max_k(int G) { return 4 * G; }
 
 }  // namespace sbpb

@@ -9,79 +9,10 @@
 //   k_row_nnz/fill     ISparseMatrix row/column views for the merge phase
 //   k_merge_propose    merge_blocks proposal scoring          src/block_merge.cpp:278-301, 335-368
 //   k_relabel          carry-out relabel                      src/blockmodel/blockmodel.cpp:71-76
-#include "sbp_engine.cuh"
+#include "sbp_kernels.cuh"
 #include "sbp_steps.cuh"
 
 namespace sbpb {
-
-// ------------------------------------------------------------------------------------------
-// Table of x log x for dxlogx_int, in double-double arithmetic (error-free sums and products of
-// Knuth and Dekker, the product by FMA): x = m 2^e with m in [sqrt(1/2), sqrt(2)), log m =
-// 2 atanh(z), z = (m - 1) / (m + 1), by its power series; log 2 = 2 atanh(1/3) by the same
-// series.  Once per process: 2^20 entries, some 40 double-double steps each.
-// ------------------------------------------------------------------------------------------
-struct DD {
-  double hi, lo;
-};
-__device__ __forceinline__ DD two_sum(double a, double b) {
-  const double s = __dadd_rn(a, b), t = __dsub_rn(s, a);
-  return {s, __dadd_rn(__dsub_rn(a, __dsub_rn(s, t)), __dsub_rn(b, t))};
-}
-__device__ __forceinline__ DD dd_renorm(double hi, double lo) {
-  const double s = __dadd_rn(hi, lo);
-  return {s, __dsub_rn(lo, __dsub_rn(s, hi))};
-}
-__device__ __forceinline__ DD dd_add(DD a, DD b) {
-  const DD s = two_sum(a.hi, b.hi), t = two_sum(a.lo, b.lo);
-  const DD r = dd_renorm(s.hi, __dadd_rn(s.lo, t.hi));
-  return dd_renorm(r.hi, __dadd_rn(r.lo, t.lo));
-}
-__device__ __forceinline__ DD dd_mul(DD a, DD b) {
-  const double p = __dmul_rn(a.hi, b.hi);
-  const double e = __fma_rn(a.hi, b.hi, -p);
-  return dd_renorm(p, __dadd_rn(e, __fma_rn(a.hi, b.lo, __dmul_rn(a.lo, b.hi))));
-}
-// n / d of exact doubles
-__device__ __forceinline__ DD dd_ratio(double n, double d) {
-  const double q = __ddiv_rn(n, d), r = __fma_rn(-q, d, n);
-  return dd_renorm(q, __ddiv_rn(r, d));
-}
-// 2 atanh(n / d) for |n / d| <= 1/3 (36 terms: 9^-36 < 2^-114)
-__device__ DD dd_2atanh(double n, double d) {
-  const DD z = dd_ratio(n, d), w = dd_mul(z, z);
-  DD s = dd_ratio(1.0, 73.0);
-  for (int k = 35; k >= 0; --k) s = dd_add(dd_mul(s, w), dd_ratio(1.0, 2.0 * k + 1.0));
-  const DD r = dd_mul(z, s);
-  return {2.0 * r.hi, 2.0 * r.lo};
-}
-
-__global__ void k_xlogx_table(double2* table, int n) {
-  const DD ln2 = dd_2atanh(1.0, 3.0);
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
-    if (x < 2) {
-      table[x] = make_double2(0.0, 0.0);
-      continue;
-    }
-    int e = 31 - __clz(x);
-    double m = ldexp((double)x, -e);   // [1, 2)
-    if (m * m > 2.0) {
-      m *= 0.5;
-      ++e;
-    }
-    const DD l = dd_add(dd_mul(ln2, {(double)e, 0.0}), dd_2atanh(m - 1.0, m + 1.0));
-    const DD g = dd_mul(l, {(double)x, 0.0});
-    table[x] = make_double2(g.hi, g.lo);
-  }
-}
-
-double2* make_xlogx_table(cudaStream_t stream) {
-  double2* t = nullptr;
-  SBP_CUDA(cudaMalloc(&t, sizeof(double2) * kXlogxTable));
-  k_xlogx_table<<<1024, 256, 0, stream>>>(t, kXlogxTable);
-  SBP_CHECK_LAUNCH();
-  SBP_CUDA(cudaStreamSynchronize(stream));
-  return t;
-}
 
 // ------------------------------------------------------------------------------------------
 // Rebuild: the counts, d_out, d_in from the assignment; d = d_out + d_in - M[x,x].
@@ -128,9 +59,14 @@ __global__ void k_rebuild_smem(GraphView g, BlockView bm) {
   }
 }
 
+__global__ void k_inverse_degrees(BlockView bm) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x < bm.B) set_degree(bm, x, bm.d[x]);
+}
+
 __global__ void k_rebuild_degrees(BlockView bm) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x < bm.B) bm.d[x] = bm.d_out[x] + bm.d_in[x] - bm_get(bm, x, x);
+  if (x < bm.B) set_degree(bm, x, bm.d_out[x] + bm.d_in[x] - bm_get(bm, x, x));
 }
 // ------------------------------------------------------------------------------------------
 // Asynchronous Gibbs on row-hashed storage: evaluate a list of vertices against the frozen state,
@@ -362,8 +298,8 @@ __global__ void k_move_vertex(GraphView g, BlockView bm, int v, int s, int cap, 
     bm.d_in[s] += k_in + self;
     __threadfence_block();
     if (!*bm.overflow) {
-      bm.d[r] = bm.d_out[r] + bm.d_in[r] - (bm_get(bm, r, r) + d_rr);
-      bm.d[s] = bm.d_out[s] + bm.d_in[s] - (bm_get(bm, s, s) + d_ss);
+      set_degree(bm, r, bm.d_out[r] + bm.d_in[r] - (bm_get(bm, r, r) + d_rr));
+      set_degree(bm, s, bm.d_out[s] + bm.d_in[s] - (bm_get(bm, s, s) + d_ss));
     }
     status[1] = d_rr;   // kept for the d fix-up after a row-capacity rebuild
     status[2] = d_ss;

@@ -31,6 +31,7 @@ struct Csr {
 __global__ void k_rebuild_global(GraphView g, BlockView bm);
 __global__ void k_rebuild_smem(GraphView g, BlockView bm);
 __global__ void k_rebuild_degrees(BlockView bm);
+__global__ void k_inverse_degrees(BlockView bm);   // inv_d from d
 // entropy::mdl of host-supplied nonzero cells (row, col, count) and block degrees: the per-cell
 // form count * log(count / (d_out[row] * d_in[col])) of Blockmodel::log_posterior_probability.
 __global__ void k_mdl_cells_list(const int* __restrict__ rows, const int* __restrict__ cols,

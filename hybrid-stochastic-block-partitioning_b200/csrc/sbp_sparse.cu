@@ -158,8 +158,8 @@ __global__ void k_recover_finish(BlockView bm, const int* moved_list, const int*
     const int v = moved_list[i];
     const int r = old_block[v], s = prop[v];
     const unsigned long long key = ((unsigned long long)gen << 32) | (unsigned)v;
-    if (last[r] == key) bm.d[r] = bm.d_out[r] + bm.d_in[r] - bm_get(bm, r, r) - qr[v];
-    if (last[s] == key) bm.d[s] = bm.d_out[s] + bm.d_in[s] - bm_get(bm, s, s) - qs[v];
+    if (last[r] == key) set_degree(bm, r, bm.d_out[r] + bm.d_in[r] - bm_get(bm, r, r) - qr[v]);
+    if (last[s] == key) set_degree(bm, s, bm.d_out[s] + bm.d_in[s] - bm_get(bm, s, s) - qs[v]);
     prop[v] = -1;
   }
 }
@@ -167,8 +167,8 @@ __global__ void k_recover_finish(BlockView bm, const int* moved_list, const int*
 // d[r], d[s] of one move (Blockmodel::move_vertex) after its rows were rebuilt.
 __global__ void k_fix_move_degrees(BlockView bm, int r, int s, int d_rr, int d_ss) {
   if (threadIdx.x || blockIdx.x) return;
-  bm.d[r] = bm.d_out[r] + bm.d_in[r] - (bm_get(bm, r, r) + d_rr);
-  bm.d[s] = bm.d_out[s] + bm.d_in[s] - (bm_get(bm, s, s) + d_ss);
+  set_degree(bm, r, bm.d_out[r] + bm.d_in[r] - (bm_get(bm, r, r) + d_rr));
+  set_degree(bm, s, bm.d_out[s] + bm.d_in[s] - (bm_get(bm, s, s) + d_ss));
 }
 
 // Dense dump of the hashed rows of M (for sbp_get_block_matrix): one thread per slot.

@@ -145,8 +145,8 @@ __device__ __forceinline__ void mh_apply_move(const GraphView& g, const BlockVie
       out[9] = (double)d_ss;
     } else {
       // Blockmodel::move_vertex reads the already-updated diagonal and adds the delta again
-      bm.d[r] = bm.d_out[r] + bm.d_in[r] - (bm_get(bm, r, r) + d_rr);
-      bm.d[s] = bm.d_out[s] + bm.d_in[s] - (bm_get(bm, s, s) + d_ss);
+      set_degree(bm, r, bm.d_out[r] + bm.d_in[r] - (bm_get(bm, r, r) + d_rr));
+      set_degree(bm, s, bm.d_out[s] + bm.d_in[s] - (bm_get(bm, s, s) + d_ss));
     }
   }
 }
@@ -238,8 +238,8 @@ __device__ __forceinline__ void finish_moved_vertex(const BlockView& bm, int v, 
                                                     const int* qs, const unsigned long long* last, unsigned gen) {
   const int r = bm.b[v], s = prop[v];
   const unsigned long long key = ((unsigned long long)gen << 32) | (unsigned)v;
-  if (last[r] == key) bm.d[r] = bm.d_out[r] + bm.d_in[r] - bm_get(bm, r, r) - qr[v];
-  if (last[s] == key) bm.d[s] = bm.d_out[s] + bm.d_in[s] - bm_get(bm, s, s) - qs[v];
+  if (last[r] == key) set_degree(bm, r, bm.d_out[r] + bm.d_in[r] - bm_get(bm, r, r) - qr[v]);
+  if (last[s] == key) set_degree(bm, s, bm.d_out[s] + bm.d_in[s] - bm_get(bm, s, s) - qs[v]);
   bm.b[v] = s;
   prop[v] = -1;
 }
