@@ -401,40 +401,20 @@ void set_smem_limit(const void* fn, size_t bytes) {
 }
 
 // One sequential Metropolis-Hastings pass over verts (device list of n vertices).
-MhResult mh_pass(SbpBlockmodel& bm, const SbpGraph& g, const int* verts, int n, int max_k, RngParams rng,
-                        int sweep) {
+MhResult mh_pass(SbpBlockmodel& bm, const SbpGraph& g, const VertexList& list, const RngParams& rng, int sweep) {
   Context& c = Context::get();
   MhResult res;
-  if (n == 0) return res;
-  if (use_group_kernel(bm) && (bm.B <= kSmallB || 2 * max_k <= g.light_cap)) {
-    // rounds of one vertex per lane group (every vertex of the list fits the group tables)
-    const bool hashed_table = bm.B > kSmallB;
-    const int cap = g.light_cap;
-    const size_t smem = mh_group_smem(hashed_table, cap);
-    if (smem <= kSmemBudget) {
-      const MhGroupKernel k = mh_group_kernel(hashed_table);
-      set_smem_limit((const void*)k, smem);
-      k<<<1, kMhGroupThreads, smem, c.stream>>>(g.view(), bm.view(), verts, n, rng, sweep, cap, c.mh_out, c.status);
-      SBP_CHECK_LAUNCH();
-      double out[4];
-      SBP_CUDA(SBP_COPY_ASYNC(out, c.mh_out, sizeof(out), cudaMemcpyDeviceToHost, c.stream));
-      c.sync();
-      res.visits = (long long)out[0];
-      res.moved = (long long)out[1];
-      res.accepted = (long long)out[2];
-      res.sum_dS = out[3];
-      return res;
-    }
-  }
-  const int cap = mh_cap(max_k);
+  if (list.n == 0) return res;
+  if (!bm.sparse) return mh_pass_dense(bm, g, list, rng, sweep);
+  const int cap = mh_cap(list.max_k);
   const size_t per_warp = (size_t)table_ints(cap) * sizeof(int);
   int W = (int)std::min<size_t>(16, kSmemBudget / per_warp);
   if (W < 1) throw Error(SBP_ERR_UNSUPPORTED, "vertex degree too large for the Metropolis-Hastings kernel");
   const size_t smem = per_warp * W;
   set_smem_limit((const void*)k_mh, smem);
   int start = 0;
-  while (start < n) {
-    k_mh<<<1, W * 32, smem, c.stream>>>(g.view(), bm.view(), verts, n, start, rng, sweep, cap, c.mh_out, c.status);
+  while (start < list.n) {
+    k_mh<<<1, W * 32, smem, c.stream>>>(g.view(), bm.view(), list.verts, list.n, start, rng, sweep, cap, c.mh_out, c.status);
     SBP_CHECK_LAUNCH();
     double out[10];
     SBP_CUDA(SBP_COPY_ASYNC(out, c.mh_out, sizeof(out), cudaMemcpyDeviceToHost, c.stream));
@@ -573,7 +553,7 @@ void finetune(SbpBlockmodel& bm, SbpGraph& g, int algo, const SbpFinetuneOptions
   const double initial_entropy = bm.overall_entropy;
   for (int it = 0; it < max_sweeps; ++it) {
     if (algo == SBP_METROPOLIS_HASTINGS) {
-      const MhResult r = mh_pass(bm, g, g.identity.p, g.V, g.max_k, rng, it);
+      const MhResult r = mh_pass(bm, g, g.all(), rng, it);
       mh_visits += r.visits;
       mh_moved += r.moved;
       mh_acc += r.accepted;
@@ -583,7 +563,7 @@ void finetune(SbpBlockmodel& bm, SbpGraph& g, int algo, const SbpFinetuneOptions
       if (early_stop(it, bracket, (double)bm.overall_entropy, deltas)) break;
     } else {
       if (algo == SBP_HYBRID_MCMC && !g.high.empty()) {
-        const MhResult r = mh_pass(bm, g, g.high_dev.p, (int)g.high.size(), g.max_k_of(g.high), rng, it);
+        const MhResult r = mh_pass(bm, g, g.high_list(), rng, it);
         mh_visits += r.visits;
         mh_moved += r.moved;
         mh_acc += r.accepted;
@@ -1315,12 +1295,12 @@ SbpStatus sbp_graph_create(int32_t V, int64_t n, const int32_t* src, const int32
     }
   }
   g->identity.reserve(V);
-  g->high_dev.reserve(g->high.size());
+  g->all_recs.reserve(V);
+  g->mean_k = (double)(m + mi) / V;
   k_iota<<<grid_for(V, 256, 8 * c.num_sms), 256, 0, c.stream>>>(g->identity.p, V);
+  k_vertex_records<<<grid_for(V, 256, 8 * c.num_sms), 256, 0, c.stream>>>(g->view(), g->identity.p, V, g->all_recs.p);
   SBP_CHECK_LAUNCH();
-  if (!g->high.empty())
-    SBP_CUDA(SBP_COPY_ASYNC(g->high_dev.p, g->high.data(), g->high.size() * sizeof(int), cudaMemcpyHostToDevice,
-                            c.stream));
+  g->upload_high();
   c.sync();
   *out = g.release();
   SBP_API_END
@@ -1364,8 +1344,8 @@ SbpStatus sbp_graph_set_split(SbpGraph* g, int32_t nh, const int32_t* high, int3
   g->high.assign(high, high + nh);
   g->low.assign(low, low + nl);
   g->plans.clear();
-  g->high_dev.reserve(std::max(nh, 1));
-  if (nh) SBP_CUDA(SBP_COPY(g->high_dev.p, high, nh * sizeof(int), cudaMemcpyHostToDevice));
+  g->upload_high();
+  Context::get().sync();
   SBP_API_END
 }
 

@@ -417,9 +417,8 @@ inline int g_hashed_row_factor = 4;
 inline int g_graph_sweeps = 1;
 inline thread_local long long g_overflow_rebuilds = 0;   // rebuilds forced by a full hashed row (calling thread)
 // Lanes per vertex of the evaluation on dense blockmodels (sbp_set_option "group_kernel"): 1
-// (default) chosen from the batch and the vertex's degree, 2 as few as its degree allows, 0 a whole
-// warp.  Metropolis-Hastings: 1 groups of eight up to kSmallB blocks, a warp above; 2 groups at every
-// block count where they fit; 0 a warp.
+// (default) chosen from the batch or round and the vertex's degree, 2 as few as its degree allows
+// (asynchronous Gibbs), 0 a whole warp.  The results are the same.
 inline int g_group_kernel = 1;
 // Batched partitioner: idle claim attempts of a persistent CTA before the launch gives up with an
 // error (each attempt sleeps ~0.25 us), and the fault injection of the failure-detection test
@@ -450,6 +449,14 @@ struct BatchPlan {
   int max_batch = 0;
 };
 
+// A Metropolis-Hastings pass's vertices, in list order.
+struct VertexList {
+  const int* verts;
+  const int4* recs;
+  int n, max_k;
+  double mean_k;
+};
+
 struct SbpGraph {
   int V = 0;
   long long E = 0;
@@ -458,6 +465,9 @@ struct SbpGraph {
   std::vector<int> h_k;        // k_out + k_in per vertex (self loop counted once, on the out side)
   std::vector<int> high, low;  // hybrid split
   int max_k = 0;
+  int high_max_k = 0;
+  double mean_k = 0.0, high_mean_k = 0.0;
+  DevBuf<int4> all_recs, high_recs;   // vertex_record of 0..V-1 and of the high-degree list
   int heavy_cap = 512;         // table slots for heavy vertices
   int light_cap = 256;         // table slots per warp for light vertices (k <= light_cap / 2)
   std::unordered_map<long long, std::unique_ptr<BatchPlan>> plans;
@@ -480,6 +490,24 @@ struct SbpGraph {
     int m = 0;
     for (int v : verts) m = std::max(m, h_k[v]);
     return m;
+  }
+
+  VertexList all() const { return {identity.p, all_recs.p, V, max_k, mean_k}; }
+  VertexList high_list() const { return {high_dev.p, high_recs.p, (int)high.size(), high_max_k, high_mean_k}; }
+  // Upload the high-degree list (set from `high`) and what the passes over it need.
+  void upload_high() {
+    Context& c = Context::get();
+    const int n = (int)high.size();
+    high_dev.reserve(n);
+    high_recs.reserve(n);
+    high_max_k = max_k_of(high);
+    double sum = 0.0;
+    for (int v : high) sum += h_k[v];
+    high_mean_k = n ? sum / n : 0.0;
+    if (!n) return;
+    SBP_CUDA(SBP_COPY_ASYNC(high_dev.p, high.data(), n * sizeof(int), cudaMemcpyHostToDevice, c.stream));
+    k_vertex_records<<<grid_for(n, 256, 8 * c.num_sms), 256, 0, c.stream>>>(view(), high_dev.p, n, high_recs.p);
+    SBP_CHECK_LAUNCH();
   }
 
   // Batches of asynchronous Gibbs over `list` (src/finetune.cpp:43-47, 352-366): batch_size =
@@ -680,10 +708,6 @@ struct SbpBlockmodel {
 
 namespace sbpb {
 
-inline bool use_group_kernel(const SbpBlockmodel& bm) {
-  return !bm.sparse && (g_group_kernel == 2 || (g_group_kernel == 1 && bm.B <= kSmallB));
-}
-
 void set_smem_limit(const void* fn, size_t bytes);
 
 // Evaluation of one asynchronous-Gibbs batch on dense storage (sbp_gibbs.cu).
@@ -865,7 +889,9 @@ Snapshot snapshot(SbpBlockmodel& bm);
 void restore(SbpBlockmodel& bm, SbpGraph& g, const Snapshot& x);
 // Per-warp table slots of the Metropolis-Hastings kernels for vertices of degree up to max_k.
 int mh_cap(int max_k);
-// One sequential Metropolis-Hastings pass over a device list of n vertices.
-MhResult mh_pass(SbpBlockmodel& bm, const SbpGraph& g, const int* verts, int n, int max_k, RngParams rng, int sweep);
+// One sequential Metropolis-Hastings pass over a vertex list.
+MhResult mh_pass(SbpBlockmodel& bm, const SbpGraph& g, const VertexList& list, const RngParams& rng, int sweep);
+// The same on dense storage (sbp_mh.cu).
+MhResult mh_pass_dense(SbpBlockmodel& bm, const SbpGraph& g, const VertexList& list, const RngParams& rng, int sweep);
 
 }  // namespace sbpb

@@ -122,6 +122,9 @@ struct GroupEval {
   int n;                 // table slots in use
   bool valid, accepted;
   double dS;
+  // what a commit needs of the state the move was evaluated against (set when s != r)
+  unsigned wr, ws;       // histogram words of r and s
+  int M_rr, M_ss, dout_r, dout_s, din_r, din_s;
 };
 
 // A vertex of a batch: (vertex, first neighbour in the joint list, out-degree incl. the self loop,
@@ -424,6 +427,14 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
   if (active) {
     res.accepted = accept_move(dS, fwd, bwd, k == 0, given ? record_uniform(x) : u53(x.z, x.w));
     res.dS = dS;
+    res.wr = wr;
+    res.ws = ws;
+    res.M_rr = M_rr;
+    res.M_ss = M_ss;
+    res.dout_r = dout_r;
+    res.dout_s = dout_s;
+    res.din_r = din_r;
+    res.din_s = din_s;
   }
   return res;
 }

@@ -214,7 +214,7 @@ __global__ void k_mh(GraphView g, BlockView bm, const int* __restrict__ verts, i
     if (i < n) {
       v = verts[i];
       const uint4 x = draw_record(rng, (uint32_t)v, (uint32_t)sweep, 0u, (long long)sweep * g.V + v, status);
-      res = evaluate_vertex(g, bm, v, x, t, lane, status, &r, &k_out, &k_in, rng.moves != 0);
+      res = evaluate_vertex<Store::kHashed>(g, bm, v, x, t, lane, status, &r, &k_out, &k_in, rng.moves != 0);
     }
     if (lane == 0) {
       s_acc[warp] = (i < n) ? res.accepted : 0;

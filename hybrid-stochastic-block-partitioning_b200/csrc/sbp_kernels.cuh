@@ -44,12 +44,6 @@ __global__ void k_mdl(GraphView g, BlockView bm, const int* __restrict__ out_src
 __global__ void __launch_bounds__(256, 2)
     k_gibbs_eval_hashed(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
                         int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status);
-constexpr int kSmallGroup = 8;
-// Metropolis-Hastings rounds of kMhGroupThreads / kSmallGroup vertices (one CTA, dense storage).
-constexpr int kMhGroupThreads = 512;
-using MhGroupKernel = void (*)(GraphView, BlockView, const int* __restrict__, int, RngParams, int, int, double*, int*);
-MhGroupKernel mh_group_kernel(bool hashed_table);
-size_t mh_group_smem(bool hashed_table, int cap);
 __global__ void k_apply_edges(GraphView g, BlockView bm, const int* moved_list, const int* n_moved, const int* prop,
                               int* qr, int* qs, unsigned long long* last, unsigned gen);
 __global__ void k_apply_finish(BlockView bm, const int* moved_list, const int* n_moved, int* next_n_moved, int* prop,

@@ -728,11 +728,9 @@ static void finetune_learned(SbpBlockmodel& bm, SbpGraph& g, int algorithm, cons
     long long pass_visits = 0, pass_acc = 0;   // this sweep's Metropolis-Hastings pass
     double pass_dS = 0.0;
     if (mh || (algorithm == SBP_HYBRID_MCMC && !g.high.empty())) {
-      const int* list = mh ? g.identity.p : g.high_dev.p;
-      const int nl = mh ? g.V : (int)g.high.size();
-      const int mk = mh ? g.max_k : g.max_k_of(g.high);
-      const MhResult r = learned ? learned_mh_pass(bm, g, list, nl, mk, *m, lp, rng, it)
-                                 : mh_pass(bm, g, list, nl, mk, rng, it);
+      const VertexList list = mh ? g.all() : g.high_list();
+      const MhResult r = learned ? learned_mh_pass(bm, g, list.verts, list.n, list.max_k, *m, lp, rng, it)
+                                 : mh_pass(bm, g, list, rng, it);
       mh_visits += r.visits;
       mh_moved += r.moved;
       mh_acc += r.accepted;
