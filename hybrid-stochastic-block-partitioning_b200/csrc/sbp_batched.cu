@@ -232,21 +232,21 @@ __global__ void __launch_bounds__(kBThreads, 2)
       case kApply: {
         const int n = *(volatile int*)n_cur;
         for (int i = idx * kBWarps + warp; i < n; i += stg.z * kBWarps)
-          apply_moved_vertex(gr.g, gr.bm, gr.moved[i], gr.prop, gr.qr, gr.qs, gr.last, gen, lane);
+          apply_moved_vertex<Store::kDense>(gr.g, gr.bm, gr.moved[i], gr.prop, gr.qr, gr.qs, gr.last, gen, lane);
         break;
       }
       case kFinish: {
         const int n = *(volatile int*)n_cur;
         if (idx == 0 && tid == 0) gr.n_moved[gen & 1u] = 0;   // the next batch's slot
         for (int i = idx * kBThreads + tid; i < n; i += stg.z * kBThreads)
-          finish_moved_vertex(gr.bm, gr.moved[i], gr.prop, gr.qr, gr.qs, gr.last, gen);
+          finish_moved_vertex<Store::kDense>(gr.bm, gr.moved[i], gr.prop, gr.qr, gr.qs, gr.last, gen);
         break;
       }
       case kMdlPart: {
         const int c0 = idx * kMdlCtasPerItem, c1 = min(c0 + kMdlCtasPerItem, gr.mdl_ctas);
         for (int cc = c0; cc < c1; ++cc) {
           const double v = gr.mdl_cells ? mdl_cells_part(gr.bm, cc, gr.mdl_ctas, red)
-                                        : mdl_edges_part(gr.g, gr.bm, gr.out_src, cc, gr.mdl_ctas, red);
+                                        : mdl_edges_part<Store::kDense>(gr.g, gr.bm, gr.out_src, cc, gr.mdl_ctas, red);
           if (tid == 0) gr.partial[cc] = v;
         }
         break;

@@ -1,8 +1,6 @@
 // Asynchronous Gibbs on a dense block matrix (finetune::asynchronous_gibbs, src/finetune.cpp:31-89):
 // the evaluation of one batch as a kernel of its own, and a whole finetune call -- every sweep's
 // batches, the MDL and the early stop -- as one persistent kernel.
-#include <cooperative_groups.h>
-
 #include "sbp_engine.cuh"
 #include "sbp_group.cuh"
 #include "sbp_steps.cuh"
@@ -56,30 +54,30 @@ __device__ __forceinline__ void eval_batch(const EvalArgs& a, BatchDesc b, int s
                                            EvalCounts& cnt) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wid = blockIdx.x * kGroupWarps + warp, nw = gridDim.x * kGroupWarps;
-  if (kDirect) {   // any degree fits a direct-indexed histogram
-    const Lanes L(32, lane);
-    const GroupTab<kDirect> T = group_tab<kDirect>(smem, a.slots, warp * kRegionSlots, kRegionSlots);
-    for (int h = wid; h < b.heavy_n; h += nw) eval_task<kDirect, ST>(a, T, b.heavy_begin + h, true, sweep, n_moved, L, cnt);
-  } else if (b.heavy_n > 0) {   // one warp with the whole CTA's table
-    const Lanes L(32, lane);
-    const GroupTab<kDirect> T = group_tab<kDirect>(smem, a.slots, 0, a.slots);
-    for (int h = blockIdx.x; h < b.heavy_n; h += gridDim.x)
-      if (warp == 0) eval_task<kDirect, ST>(a, T, b.heavy_begin + h, true, sweep, n_moved, L, cnt);
-    __syncthreads();
-  }
   const int n = b.light_n;
   const int c32 = a.gmin >= 32 ? n : b.n32;
   const int c16 = a.gmin >= 32 ? 0 : a.gmin >= 16 ? n - c32 : b.n16;
   const int t16 = (c16 + 1) >> 1, t8 = (n - c32 - c16 + 3) >> 2;
-  for (int task = wid; task < c32 + t16 + t8; task += nw) {
-    const int G = task < c32 ? 32 : task < c32 + t16 ? 16 : 8;
-    const int first = G == 32 ? task : G == 16 ? c32 + 2 * (task - c32) : c32 + c16 + 4 * (task - c32 - t16);
-    const int end = G == 32 ? c32 : G == 16 ? c32 + c16 : n;
-    const Lanes L(G, lane);
-    const int item = first + lane / G;
-    const GroupTab<kDirect> T =
-        group_tab<kDirect>(smem, a.slots, warp * kRegionSlots + (lane / G) * (kRegionSlots / 32) * G, kRegionSlots / 32 * G);
-    eval_task<kDirect, ST>(a, T, b.light_begin + item, item < end, sweep, n_moved, L, cnt);
+  // Two passes over one body: the heavy vertices, each by one warp with the whole CTA's table (any
+  // degree fits a direct-indexed histogram, so there by any warp), then the light ones.
+#pragma unroll 1
+  for (int light = b.heavy_n > 0 ? 0 : 1; light < 2; ++light) {
+    const bool whole = !kDirect && !light;
+    const int first_task = whole ? (warp == 0 ? (int)blockIdx.x : b.heavy_n) : wid, step = whole ? (int)gridDim.x : nw;
+    const int tasks = light ? c32 + t16 + t8 : b.heavy_n;
+#pragma unroll 1
+    for (int task = first_task; task < tasks; task += step) {
+      const int lg = !light || task < c32 ? 0 : task < c32 + t16 ? 1 : 2;   // log2 of the vertices of the task
+      const int first = lg == 0 ? task : lg == 1 ? c32 + 2 * (task - c32) : c32 + c16 + 4 * (task - c32 - t16);
+      const int end = !light ? tasks : lg == 0 ? c32 : lg == 1 ? c32 + c16 : n;
+      const Lanes L(32 >> lg, lane);
+      const int sub = lane >> (5 - lg), share = kRegionSlots >> lg;
+      const GroupTab<kDirect> T = group_tab<kDirect>(smem, a.slots, whole ? 0 : warp * kRegionSlots + sub * share,
+                                                     whole ? a.slots : share);
+      eval_task<kDirect, ST>(a, T, (light ? b.light_begin : b.heavy_begin) + first + sub, first + sub < end, sweep,
+                             n_moved, L, cnt);
+    }
+    if (whole) __syncthreads();
   }
 }
 
@@ -204,17 +202,17 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_gibbs_sweeps(const __grid_
         ++gen;
         if (n == 0) continue;   // the same for the whole grid
         for (int i = wid; i < n; i += nw)
-          apply_moved_record(g, bm, __ldg(a.e.recs + a.e.moved[i]), a.e.prop, a.qr, a.qs, a.last, gen, lane);
+          apply_moved_record<Store::kDense>(g, bm, __ldg(a.e.recs + a.e.moved[i]), a.e.prop, a.qr, a.qs, a.last, gen, lane);
         if (!sync_grid(a, &target, &s_abort)) return;
         for (int i = blockIdx.x * kGroupThreads + tid; i < n; i += gridDim.x * kGroupThreads)
-          finish_moved_vertex(bm, __ldg(&a.e.recs[a.e.moved[i]].x), a.e.prop, a.qr, a.qs, a.last, gen);
+          finish_moved_vertex<Store::kDense>(bm, __ldg(&a.e.recs[a.e.moved[i]].x), a.e.prop, a.qr, a.qs, a.last, gen);
         if (!sync_grid(a, &target, &s_abort)) return;
       }
     }
     // entropy::mdl over the virtual grid of every other path
     for (int vc = blockIdx.x; vc < a.mdl_ctas; vc += gridDim.x) {
       const double t = a.mdl_cells ? mdl_cells_part(bm, vc, a.mdl_ctas, red)
-                                   : mdl_edges_part(g, bm, a.out_src, vc, a.mdl_ctas, red);
+                                   : mdl_edges_part<Store::kDense>(g, bm, a.out_src, vc, a.mdl_ctas, red);
       if (tid == 0) a.partial[vc] = t;
     }
     if (!sync_grid(a, &target, &s_abort)) return;
@@ -251,6 +249,9 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_gibbs_sweeps(const __grid_
     a.result->sweeps = count;
   }
 }
+
+constexpr int kMaxCluster = 16;
+constexpr int kClusterBatch = 128;   // largest batch run on one cluster: a warp for every vertex
 
 EvalArgs eval_args(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& plan, const RngParams& rng) {
   EvalArgs a;
@@ -325,23 +326,49 @@ SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan&
   int per_sm = 0;
   SBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kGroupThreads, smem));
   if (per_sm < 1) throw Error(SBP_ERR_UNSUPPORTED, "vertex degree too large for the finetune kernel");
-  const int resident = per_sm * c.num_sms;
-  a.e.gmin = group_min(plan.max_batch, resident * kGroupWarps);
-  const int wanted = (int)std::max<long long>(((long long)plan.max_batch * a.e.gmin / 32 + kGroupWarps - 1) / kGroupWarps,
-                                              a.mdl_ctas);
-  const int grid = std::max(1, std::min(resident, wanted));
-  a.cluster = 0;
-  SBP_CUDA(cudaMemsetAsync(c.sweep_words, 0, 8 * sizeof(int), c.stream));
+  // Small batches: one cluster of up to 16 CTAs, whose hardware barrier takes 0.3 us against 1 us
+  // through global memory (three of them in a batch of some 12 us).  Only while every vertex gets a
+  // warp: at 250 vertices a batch the second round of evaluations costs more than the barriers
+  // (1,000 vertices in ten batches: 69 ms a partition against 80; 2,500: 127 against 110).
+  int cluster = 0;
+  if (plan.max_batch <= kClusterBatch) {
+    a.e.gmin = group_min(plan.max_batch, kMaxCluster * kGroupWarps);
+    cluster = std::min(kMaxCluster, grid_for((long long)plan.max_batch * a.e.gmin, 32 * kGroupWarps, kMaxCluster));
+    cluster = pow2_at_least(cluster);
+    if (cluster > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();
+      cluster = 8;
+    }
+  }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kGroupThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = c.stream;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeCooperative;
-  at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  if (cluster > 0) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(cluster);
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) != cudaSuccess || fit < 1) {
+      cudaGetLastError();
+      cluster = 0;
+    }
+  }
+  a.cluster = cluster > 0 ? 1 : 0;
+  if (!cluster) {
+    const int resident = per_sm * c.num_sms;
+    a.e.gmin = group_min(plan.max_batch, resident * kGroupWarps);
+    const int wanted = (int)std::max<long long>(
+        ((long long)plan.max_batch * a.e.gmin / 32 + kGroupWarps - 1) / kGroupWarps, a.mdl_ctas);
+    cfg.gridDim = dim3(std::max(1, std::min(resident, wanted)));
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  }
+  SBP_CUDA(cudaMemsetAsync(c.sweep_words, 0, 8 * sizeof(int), c.stream));
   SBP_CUDA(cudaLaunchKernelEx(&cfg, k, a));
   SBP_CHECK_LAUNCH();
   SweepsResult r;

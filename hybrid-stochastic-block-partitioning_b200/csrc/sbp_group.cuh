@@ -80,6 +80,13 @@ struct GroupTab {
       return 0u;
     }
   }
+  // What the home slot of `key` holds, and from it whether the table holds the key (a slot in use has
+  // a nonzero word): apart, so that several look-ups go out together.
+  __device__ __forceinline__ int peek(int key) const { return kDirect ? (int)w[key] : keys[home(key)]; }
+  __device__ __forceinline__ bool holds(int key, int peeked) const {
+    if constexpr (kDirect) return peeked != 0;
+    else return peeked == key || (peeked != -1 && counts_of(key) != 0u);
+  }
   __device__ __forceinline__ int key_of(int slot) const { return kDirect ? slot : keys[slot]; }
   // Empty the n slots in use.
   __device__ __forceinline__ void clear(int n, const Lanes& L) const {
@@ -138,7 +145,7 @@ __device__ __forceinline__ int4 vertex_record(const GraphView& g, int v) {
 // Rare terms, out of line to keep the evaluation's code small: a count beyond the table, and the
 // double count of a net-zero Delta cell, m (log1p(a / b) + log1p(c / d)).
 static __device__ __noinline__ double dxlogx_far(int a, int b) { return dxlogx((double)a, (double)b); }
-__device__ __forceinline__ double dxlogx_wide(const double2* __restrict__ gt, int a, int b) {
+static __device__ __noinline__ double dxlogx_wide(const double2* __restrict__ gt, int a, int b) {
   if ((unsigned)a < (unsigned)kXlogxTable && (unsigned)b < (unsigned)kXlogxTable) {
     const double2 ga = __ldg(gt + a), gb = __ldg(gt + b);
     return (ga.x - gb.x) + (ga.y - gb.y);
@@ -153,6 +160,11 @@ static __device__ __noinline__ double net_zero_term(int m, int a, int b, int c, 
 // single-precision estimate decides wherever it is further from u than its error (under 1e-4
 // relative) can reach; only the rest, about one visit in a thousand, takes the FP64 exponential
 // and division, a chain of some 800 cycles.  The decision is the FP64 test's in every case.
+static __device__ __noinline__ bool accept_exact(double x, double H, double u) {
+  double ap = exp(x) * H;
+  ap = ap >= 1.0 ? 1.0 : ap;
+  return u <= ap;
+}
 __device__ __forceinline__ bool accept_move(double dS, double fwd, double bwd, bool alone, double u) {
   const double x = -3.0 * dS;
   const float xf = (float)x, hf = alone ? 1.0f : __fdividef((float)bwd, (float)fwd);
@@ -167,10 +179,7 @@ __device__ __forceinline__ bool accept_move(double dS, double fwd, double bwd, b
       if (uf < af * 0.999f && u <= 1.0) return true;
     }
   }
-  const double H = alone ? 1.0 : bwd / fwd;
-  double ap = exp(x) * H;
-  ap = ap >= 1.0 ? 1.0 : ap;
-  return u <= ap;
+  return accept_exact(x, alone ? 1.0 : bwd / fwd, u);
 }
 
 // Evaluate the vertex of `rec` (groups with `valid`) against the blockmodel with random record x:
@@ -341,10 +350,10 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
                : q == 4 ? dout_r : q == 5 ? dout_s : q == 6 ? din_r : din_s;
   const int qd = q == 0 ? d_rr : q == 1 ? d_rs : q == 2 ? d_sr : q == 3 ? d_ss
                : q == 4 ? -k_out : q == 5 ? k_out : q == 6 ? -kin_self : kin_self;
-  if (active && q < 8 && qd) {
-    const double y = dxlogx_wide(gt, qa, qa + qd);
-    dS += q < 4 ? y : -y;
-  }
+  const bool corner_term = active && q < 8 && qd;
+  const bool in_table = (unsigned)qa < (unsigned)kXlogxTable && (unsigned)(qa + qd) < (unsigned)kXlogxTable;
+  const double2 c0 = __ldg(gt + (corner_term && in_table ? qa : 0));   // consumed after the entries
+  const double2 c1 = __ldg(gt + (corner_term && in_table ? qa + qd : 0));
   if (active && q < 2) {
     // the backward terms of neighbours in r (lane 0) and s (lane 1), whose degrees change
     const int c = q == 0 ? co_r + ci_r + self : co_s + ci_s;
@@ -372,21 +381,16 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       const double cf = (double)(c + (is_r && wu[h] ? self : 0)), cb = corner ? 0.0 : (double)c;
       fwd += cf * ((double)m_su[h].x + (double)m_su[h].y + 1.0) * inv[h];
       bwd += cb * ((double)(m_ru[h].x - co) + (double)(m_ru[h].y - ci) + 1.0) * inv[h];
-      // cells (r,u) (s,u) for out-edges to u, (u,r) (u,s) for in-edges; the corners were added above
-      if (small) {
-        const bool out = co != 0;
-        const int d = corner ? 0 : out ? co : ci;
-        const int ar = out ? m_ru[h].x : m_ru[h].y, as = out ? m_su[h].x : m_su[h].y;
-        const double2 g0 = __ldg(gt + ar), g1 = __ldg(gt + ar - d), g2 = __ldg(gt + as), g3 = __ldg(gt + as + d);
-        dS += ((g0.x - g1.x) + (g0.y - g1.y)) + ((g2.x - g3.x) + (g2.y - g3.y));
-        if (co && ci && !corner) {
-          const double2 h0 = __ldg(gt + m_ru[h].y), h1 = __ldg(gt + m_ru[h].y - ci);
-          const double2 h2 = __ldg(gt + m_su[h].y), h3 = __ldg(gt + m_su[h].y + ci);
-          dS += ((h0.x - h1.x) + (h0.y - h1.y)) + ((h2.x - h3.x) + (h2.y - h3.y));
-        }
-      } else if (!corner) {
-        if (co) dS += dxlogx_wide(gt, m_ru[h].x, m_ru[h].x - co) + dxlogx_wide(gt, m_su[h].x, m_su[h].x + co);
-        if (ci) dS += dxlogx_wide(gt, m_ru[h].y, m_ru[h].y - ci) + dxlogx_wide(gt, m_su[h].y, m_su[h].y + ci);
+      // cells (r,u) (s,u) for out-edges to u, (u,r) (u,s) for in-edges; the corners are terms of their own
+      const bool out = co != 0;
+      const int d = corner || !small ? 0 : out ? co : ci;
+      const int ar = small ? (out ? m_ru[h].x : m_ru[h].y) : 0, as = small ? (out ? m_su[h].x : m_su[h].y) : 0;
+      const double2 g0 = __ldg(gt + ar), g1 = __ldg(gt + ar - d), g2 = __ldg(gt + as), g3 = __ldg(gt + as + d);
+      dS += ((g0.x - g1.x) + (g0.y - g1.y)) + ((g2.x - g3.x) + (g2.y - g3.y));
+      if (d && co && ci) {
+        const double2 h0 = __ldg(gt + m_ru[h].y), h1 = __ldg(gt + m_ru[h].y - ci);
+        const double2 h2 = __ldg(gt + m_su[h].y), h3 = __ldg(gt + m_su[h].y + ci);
+        dS += ((h0.x - h1.x) + (h0.y - h1.y)) + ((h2.x - h3.x) + (h2.y - h3.y));
       }
     }
     j0 += 4 * L.G;
@@ -401,6 +405,21 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       m_su[h] = wu[h] ? ldv<ST>(Ps + u[h]) : make_int2(0, 0);
       inv[h] = wu[h] ? ldv<ST>(bm.inv_d + u[h]) : 0.0;
     }
+  }
+  if (!small) {   // counts beyond the table: the same terms once more, one entry at a time
+#pragma unroll 1
+    for (int j = L.gl; j < nent; j += L.G) {
+      const int slot = T.list[j], uu = T.key_of(slot);
+      const int co = T.w[slot] & kCountMask, ci = (T.w[slot] >> kInShift) & kCountMask;
+      if (uu == r || uu == s) continue;
+      const int2 a = ldv<ST>(Pr + uu), b = ldv<ST>(Ps + uu);
+      if (co) dS += dxlogx_wide(gt, a.x, a.x - co) + dxlogx_wide(gt, b.x, b.x + co);
+      if (ci) dS += dxlogx_wide(gt, a.y, a.y - ci) + dxlogx_wide(gt, b.y, b.y + ci);
+    }
+  }
+  if (corner_term) {
+    const double y = in_table ? (c0.x - c1.x) + (c0.y - c1.y) : dxlogx_far(qa, qa + qd);
+    dS += q < 4 ? y : -y;
   }
   fwd = group_sum(fwd, L);
   bwd = group_sum(bwd, L);

@@ -66,27 +66,25 @@ __global__ void __launch_bounds__(kMhWarps * 32, 1) k_mh_dense(const __grid_cons
   extern __shared__ int smem[];
   __shared__ int s_r[kMhMaxWidth], s_s[kMhMaxWidth], s_t[kMhMaxWidth];
   __shared__ double s_dS[kMhMaxWidth];
-  __shared__ unsigned s_acc[2], s_moved[2];
-  __shared__ int s_stop;
+  __shared__ unsigned s_acc[kMhWarps], s_moved[kMhWarps];   // a bit per group of the warp
+  __shared__ int s_first[kMhWarps];                         // the warp's first invalid or dependent position
   const GraphView& g = a.g;
   const BlockView& bm = a.bm;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int slots = warps * a.region;
   group_tabs_init<kDirect>(smem, slots);
-  if (threadIdx.x < 2) s_acc[threadIdx.x] = s_moved[threadIdx.x] = 0u;
-  if (threadIdx.x == 0) s_stop = kMhMaxWidth;
   __syncthreads();
-  long long visits = 0, moved = 0, accepted = 0;   // thread 0
+  long long visits = 0, moved = 0, accepted = 0;   // warp 0; sum_dS its first lane
   double sum_dS = 0.0;
   float expect = 16.f;
   bool whole_warp = false;   // the next vertex does not fit a smaller group's table
   for (int pos = 0; pos < a.n;) {
     const int G = whole_warp ? 32 : max(a.min_lanes, mh_group_lanes(expect, warps, a.kref));
     const Lanes L(G, lane);
-    const int per = 32 / G, W = warps * per;
-    const int w = warp * per + lane / G;
-    const int share = a.region / per;
-    auto tab = [&](int x) { return group_tab<kDirect>(smem, slots, (x / per) * a.region + (x % per) * share, share); };
+    const int lg = G == 32 ? 0 : G == 16 ? 1 : 2, per = 1 << lg, W = warps * per;   // groups of a warp, of the CTA
+    const int w = warp * per + (lane >> (5 - lg));
+    const int share = a.region >> lg;
+    auto tab = [&](int x) { return group_tab<kDirect>(smem, slots, x * share, share); };   // group x's
     const GroupTab<kDirect> T = tab(w);
     int4 rec = make_int4(0, 0, 0, 0);
     bool valid = pos + w < a.n;
@@ -101,32 +99,49 @@ __global__ void __launch_bounds__(kMhWarps * 32, 1) k_mh_dense(const __grid_cons
       s_s[w] = e.s;
       s_t[w] = e.t;
       s_dS[w] = e.dS;
-      if (e.accepted) atomicOr(&s_acc[w >> 5], 1u << (w & 31));
-      if (valid && e.s != e.r) atomicOr(&s_moved[w >> 5], 1u << (w & 31));
-      if (!valid) atomicMin(&s_stop, w);
+    }
+    const unsigned firsts = G == 32 ? 1u : G == 16 ? 0x10001u : 0x1010101u;   // the groups' first lanes
+    auto squeeze = [&](unsigned m) {   // one bit per group, from the bits of their first lanes
+      m &= firsts;
+      return (m | m >> (G - 1) | (G == 8 ? m >> (2 * (G - 1)) | m >> (3 * (G - 1)) : 0u)) & (unsigned)((1 << per) - 1);
+    };
+    const unsigned acc_w = squeeze(__ballot_sync(kFull, e.accepted));
+    const unsigned moved_w = squeeze(__ballot_sync(kFull, valid && e.s != e.r));
+    if (lane == 0) {
+      s_acc[warp] = acc_w;
+      s_moved[warp] = moved_w;
     }
     __syncthreads();
-    const unsigned long long acc = (unsigned long long)s_acc[1] << 32 | s_acc[0];
+    auto gather = [&](const unsigned* bits) {   // the warps' bits as one mask over the round's positions
+      const unsigned m = lane < warps ? bits[lane] : 0u;
+      const unsigned long long x = (unsigned long long)m << (lane < warps ? lane * per : 0);
+      return (unsigned long long)__reduce_or_sync(kFull, (unsigned)(x >> 32)) << 32 | __reduce_or_sync(kFull, (unsigned)x);
+    };
+    const unsigned long long acc = gather(s_acc);
+    bool halt = !valid;
     if (valid) {
-      bool dep = false;
       for (int c = L.gl; c < w; c += G) {
         if (!(acc >> c & 1ull)) continue;
         const GroupTab<kDirect> Tc = tab(c);
-        const int rc = s_r[c], sc = s_s[c];
-        dep = dep || rc == e.r || rc == e.s || rc == e.t || sc == e.r || sc == e.s || sc == e.t || T.counts_of(rc) ||
-              T.counts_of(sc) || (e.t >= 0 && Tc.counts_of(e.t)) || Tc.counts_of(e.r) || Tc.counts_of(e.s);
+        const int rc = s_r[c], sc = s_s[c], tw = e.t >= 0 ? e.t : e.r;
+        const int p0 = Tc.peek(e.r), p1 = Tc.peek(e.s), p2 = Tc.peek(tw), p3 = T.peek(rc), p4 = T.peek(sc);
+        halt |= (rc == e.r) | (rc == e.s) | (rc == e.t) | (sc == e.r) | (sc == e.s) | (sc == e.t) | Tc.holds(e.r, p0) |
+                Tc.holds(e.s, p1) | Tc.holds(tw, p2) | T.holds(rc, p3) | T.holds(sc, p4);
       }
-      if (dep) atomicMin(&s_stop, w);
     }
+    const unsigned halted = __ballot_sync(kFull, halt);
+    if (lane == 0) s_first[warp] = halted ? warp * per + ((__ffs(halted) - 1) >> (5 - lg)) : kMhMaxWidth;
     __syncthreads();
-    const int stop = min(s_stop, W);
-    if (threadIdx.x == 0) {
+    const int stop = min(W, (int)__reduce_min_sync(kFull, (unsigned)(lane < warps ? s_first[lane] : kMhMaxWidth)));
+    if (warp == 0) {
       const unsigned long long below = stop >= 64 ? ~0ull : (1ull << stop) - 1ull;
-      visits += stop;
-      moved += __popcll(((unsigned long long)s_moved[1] << 32 | s_moved[0]) & below);
+      const unsigned long long mv = gather(s_moved);
       unsigned long long done = acc & below;
+      visits += stop;
+      moved += __popcll(mv & below);
       accepted += __popcll(done);
-      for (; done; done &= done - 1ull) sum_dS += s_dS[__ffsll((long long)done) - 1];   // in list order
+      if (lane == 0)
+        for (; done; done &= done - 1ull) sum_dS += s_dS[__ffsll((long long)done) - 1];   // in list order
     }
     if (e.accepted && w < stop) {
       // Blockmodel::move_vertex (src/blockmodel/blockmodel.cpp:344-360): lanes take the non-corner
@@ -141,21 +156,21 @@ __global__ void __launch_bounds__(kMhWarps * 32, 1) k_mh_dense(const __grid_cons
         const unsigned wu = T.w[slot];
         const int co = wu & kCountMask, ci = (wu >> kInShift) & kCountMask;
         if (co) {
-          cell_add(bm, r, u, -co);
-          cell_add(bm, s, u, co);
+          cell_add<Store::kDense>(bm, r, u, -co);
+          cell_add<Store::kDense>(bm, s, u, co);
         }
         if (ci) {
-          cell_add(bm, u, r, -ci);
-          cell_add(bm, u, s, ci);
+          cell_add<Store::kDense>(bm, u, r, -ci);
+          cell_add<Store::kDense>(bm, u, s, ci);
         }
       }
       if (L.gl == 0) {
         const int d_rr = -co_r - ci_r - e.self, d_rs = -co_s + ci_r;
         const int d_sr = co_r - ci_s, d_ss = co_s + ci_s + e.self;
-        if (d_rr) cell_add(bm, r, r, d_rr);
-        if (d_rs) cell_add(bm, r, s, d_rs);
-        if (d_sr) cell_add(bm, s, r, d_sr);
-        if (d_ss) cell_add(bm, s, s, d_ss);
+        if (d_rr) cell_add<Store::kDense>(bm, r, r, d_rr);
+        if (d_rs) cell_add<Store::kDense>(bm, r, s, d_rs);
+        if (d_sr) cell_add<Store::kDense>(bm, s, r, d_sr);
+        if (d_ss) cell_add<Store::kDense>(bm, s, s, d_ss);
         bm.b[e.v] = s;
         const int kin_self = e.k_in + e.self;
         const int out_r = e.dout_r - e.k_out, out_s = e.dout_s + e.k_out;
@@ -170,10 +185,6 @@ __global__ void __launch_bounds__(kMhWarps * 32, 1) k_mh_dense(const __grid_cons
       }
     }
     T.clear(e.n, L);
-    __threadfence_block();
-    __syncthreads();
-    if (threadIdx.x < 2) s_acc[threadIdx.x] = s_moved[threadIdx.x] = 0u;
-    if (threadIdx.x == 0) s_stop = kMhMaxWidth;
     __syncthreads();
     whole_warp = stop == 0;   // only a vertex that did not fit stops a round at its start
     if (stop > 0) expect = 0.75f * expect + 0.25f * (stop >= W ? 2.f * (float)W : (float)stop);

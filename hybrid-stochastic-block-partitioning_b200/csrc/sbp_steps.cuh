@@ -22,8 +22,9 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 
 // M[row,col] += delta in both pairs that hold it and both chunk sums (dense), or in the
 // two hashed rows (atomic).
+template <Store ST = Store::kAny>
 __device__ __forceinline__ void cell_add(const BlockView& bm, int row, int col, int delta) {
-  if (bm.sparse) {
+  if (ST != Store::kDense && (ST == Store::kHashed || bm.sparse)) {
     hashed_add(bm.rbase, bm.rmask, bm.rslot, row, col, delta, bm.overflow, bm.overflow + 1);
     hashed_add(bm.cbase, bm.cmask, bm.cslot, col, row, delta, bm.overflow, bm.overflow + 1 + bm.B);
     return;
@@ -156,6 +157,7 @@ __device__ __forceinline__ void mh_apply_move(const GraphView& g, const BlockVie
 // d_out / d_in, the quirk terms qr/qs of d[r], d[s] (the neighbours that are counted in the
 // reference's sequential apply) and the batch's last mover of r and s.  One warp per vertex;
 // lanes whose edges change the same cell add their count with one atomic.
+template <Store ST = Store::kAny>
 __device__ __forceinline__ void apply_moved_record(const GraphView& g, const BlockView& bm, int4 rec, const int* prop,
                                                    int* qr, int* qs, unsigned long long* last, unsigned gen,
                                                    int lane) {
@@ -197,14 +199,14 @@ __device__ __forceinline__ void apply_moved_record(const GraphView& g, const Blo
         cs += (ba == s);
       }
       const unsigned po = __match_any_sync(kFull, ko);
-      if (ko >= 0 && (__ffs(po) - 1) == lane) cell_add(bm, r, ko, -__popc(po));
+      if (ko >= 0 && (__ffs(po) - 1) == lane) cell_add<ST>(bm, r, ko, -__popc(po));
       const unsigned pn = __match_any_sync(kFull, kn);
-      if (kn >= 0 && (__ffs(pn) - 1) == lane) cell_add(bm, s, kn, __popc(pn));
+      if (kn >= 0 && (__ffs(pn) - 1) == lane) cell_add<ST>(bm, s, kn, __popc(pn));
       const unsigned pb = __match_any_sync(kFull, ks);
       if (ks >= 0 && (__ffs(pb) - 1) == lane) {
         const int c = __popc(pb);
-        cell_add(bm, ks, r, -c);
-        cell_add(bm, ks, s, c);
+        cell_add<ST>(bm, ks, r, -c);
+        cell_add<ST>(bm, ks, s, c);
       }
     }
   }
@@ -212,8 +214,8 @@ __device__ __forceinline__ void apply_moved_record(const GraphView& g, const Blo
   cs = warp_sum_int(cs);
   if (lane == 0) {
     if (self) {
-      cell_add(bm, r, r, -1);
-      cell_add(bm, s, s, 1);
+      cell_add<ST>(bm, r, r, -1);
+      cell_add<ST>(bm, s, s, 1);
     }
     const int k_in_self = k_in + self;
     atomicAdd(bm.d_out + r, -k_out);
@@ -227,70 +229,84 @@ __device__ __forceinline__ void apply_moved_record(const GraphView& g, const Blo
     atomicMax(last + s, key);
   }
 }
+template <Store ST = Store::kAny>
 __device__ __forceinline__ void apply_moved_vertex(const GraphView& g, const BlockView& bm, int v, const int* prop,
                                                    int* qr, int* qs, unsigned long long* last, unsigned gen,
                                                    int lane) {
-  apply_moved_record(g, bm, vertex_record(g, v), prop, qr, qs, last, gen, lane);
+  apply_moved_record<ST>(g, bm, vertex_record(g, v), prop, qr, qs, last, gen, lane);
 }
 
 // d[r], d[s] from the last mover of each block, then the new assignment of v.
+template <Store ST = Store::kAny>
 __device__ __forceinline__ void finish_moved_vertex(const BlockView& bm, int v, int* prop, const int* qr,
                                                     const int* qs, const unsigned long long* last, unsigned gen) {
   const int r = bm.b[v], s = prop[v];
   const unsigned long long key = ((unsigned long long)gen << 32) | (unsigned)v;
-  if (last[r] == key) set_degree(bm, r, bm.d_out[r] + bm.d_in[r] - bm_get(bm, r, r) - qr[v]);
-  if (last[s] == key) set_degree(bm, s, bm.d_out[s] + bm.d_in[s] - bm_get(bm, s, s) - qs[v]);
+  if (last[r] == key) set_degree(bm, r, bm.d_out[r] + bm.d_in[r] - bm_get<ST>(bm, r, r) - qr[v]);
+  if (last[s] == key) set_degree(bm, s, bm.d_out[s] + bm.d_in[s] - bm_get<ST>(bm, s, s) - qs[v]);
   bm.b[v] = s;
   prop[v] = -1;
 }
 
 // MDL: L = sum_cells g(M) - sum g(d_out) - sum g(d_in); mdl = E h(B^2/E) + V log B - L.
 // Deterministic two-pass reduction: partial cta of ncta CTAs of 256 threads (elements in
-// grid-stride order), then the partials summed in a fixed order.
+// grid-stride order), then the partials summed in a fixed order.  x log x comes from the table; four
+// of a thread's elements are in flight.
+static __device__ __noinline__ double xlogx_far(int m) { return xlogx((double)m); }
+__device__ __forceinline__ double xlogx_int(const BlockView& bm, int m) {
+  if ((unsigned)m < (unsigned)kXlogxTable) return __ldg(&bm.xlogxt[m].x);
+  return m > 0 ? xlogx_far(m) : 0.0;
+}
+__device__ __forceinline__ double mdl_degrees(const BlockView& bm, int cta, int ncta) {
+  double acc = 0.0;
+  for (long long x = (long long)cta * blockDim.x + threadIdx.x; x < bm.B; x += (long long)ncta * blockDim.x)
+    acc += xlogx_int(bm, bm.d_out[x]) + xlogx_int(bm, bm.d_in[x]);
+  return acc;
+}
 __device__ __forceinline__ double mdl_cells_part(const BlockView& bm, int cta, int ncta, double* red) {
   double acc = 0.0;
   const long long BB = (long long)bm.B * bm.B;
   const long long stride = (long long)ncta * blockDim.x;
-  for (long long i = (long long)cta * blockDim.x + threadIdx.x; i < BB; i += stride) {
-    const int row = (int)(i / bm.B), col = (int)(i - (long long)row * bm.B);
-    const int m = bm.P[(size_t)row * bm.ld + col].x;
-    if (m > 0) acc += xlogx((double)m);
+  for (long long i = (long long)cta * blockDim.x + threadIdx.x; i < BB; i += 4 * stride) {
+    int m[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const long long c = i + j * stride;
+      const int row = (int)(c / bm.B), col = (int)(c - (long long)row * bm.B);
+      m[j] = c < BB ? bm.P[(size_t)row * bm.ld + col].x : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc += xlogx_int(bm, m[j]);
   }
-  for (long long x = (long long)cta * blockDim.x + threadIdx.x; x < bm.B; x += stride)
-    acc -= xlogx((double)bm.d_out[x]) + xlogx((double)bm.d_in[x]);
-  return block_sum(acc, red);
+  return block_sum(acc - mdl_degrees(bm, cta, ncta), red);
 }
 
 // Edge form: sum_cells M log M = sum over edges of log M[b_src, b_dst].
+template <Store ST = Store::kAny>
 __device__ __forceinline__ double mdl_edges_part(const GraphView& g, const BlockView& bm, const int* out_src, int cta,
                                                  int ncta, double* red) {
   double acc = 0.0;
   const long long stride = (long long)ncta * blockDim.x;
-  long long e = (long long)cta * blockDim.x + threadIdx.x;
-  for (; e + 3 * stride < g.E; e += 4 * stride) {   // four chains of dependent loads in flight, added in order
+  for (long long e = (long long)cta * blockDim.x + threadIdx.x; e < g.E; e += 4 * stride) {
     int bv[4], bu[4], m[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      bv[j] = __ldg(out_src + e + j * stride);
-      bu[j] = __ldg(g.out_idx + e + j * stride);
+      const bool on = e + j * stride < g.E;
+      bv[j] = on ? __ldg(out_src + e + j * stride) : -1;
+      bu[j] = on ? __ldg(g.out_idx + e + j * stride) : -1;
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      bv[j] = bm.b[bv[j]];
-      bu[j] = bm.b[bu[j]];
-    }
+    for (int j = 0; j < 4; ++j)
+      if (bv[j] >= 0) {
+        bv[j] = bm.b[bv[j]];
+        bu[j] = bm.b[bu[j]];
+      }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) m[j] = bm_get(bm, bv[j], bu[j]);
+    for (int j = 0; j < 4; ++j) m[j] = bv[j] >= 0 ? bm_get<ST>(bm, bv[j], bu[j]) : 1;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc += log((double)m[j]);
+    for (int j = 0; j < 4; ++j) acc += log((double)m[j]);   // (from a table: 8 % slower at 11,770 blocks)
   }
-  for (; e < g.E; e += stride) {
-    const int bv = bm.b[__ldg(out_src + e)], bu = bm.b[__ldg(g.out_idx + e)];
-    acc += log((double)bm_get(bm, bv, bu));
-  }
-  for (long long x = (long long)cta * blockDim.x + threadIdx.x; x < bm.B; x += stride)
-    acc -= xlogx((double)bm.d_out[x]) + xlogx((double)bm.d_in[x]);
-  return block_sum(acc, red);
+  return block_sum(acc - mdl_degrees(bm, cta, ncta), red);
 }
 
 // The sum of the partials in a fixed order (thread 0).
@@ -300,7 +316,7 @@ __device__ __forceinline__ double mdl_total(const double* partial, int n, double
   return block_sum(acc, red);
 }
 // E h(B^2 / E) + V log B
-__device__ __forceinline__ double mdl_constant(int V, long long E, int B) {
+static __device__ __noinline__ double mdl_constant(int V, long long E, int B) {
   const double x = pow((double)B, 2) / (double)E;
   const double h = ((1 + x) * log(1 + x)) - (x * log(x));
   return ((double)E * h) + ((double)V * log((double)B));
