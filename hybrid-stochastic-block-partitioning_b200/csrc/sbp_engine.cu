@@ -99,7 +99,7 @@ double2* make_xlogx_table() {
 // Scratch of the sparse rebuild (grow-only, shared by all blockmodels).
 struct SortScratch {
   DevBuf<unsigned long long> keys, keysT, tmp, ukeys, partial;
-  DevBuf<unsigned> hist, flags, rowcnt, caps;
+  DevBuf<unsigned> hist, flags, caps;
   DevBuf<long long> pos, heads, rowptr;
 };
 static thread_local SortScratch g_sort;   // per host thread (the batched partitioner merges on several)
@@ -146,23 +146,22 @@ static std::vector<int> stable_order_by(const std::vector<double>& key) {
   return order;
 }
 
-static int key_bits(int B) {
-  const unsigned long long maxkey = (unsigned long long)B * (unsigned long long)B;
+// Bits of a block id in a sort key (row << bits | column).
+static int block_bits(int B) {
   int bits = 1;
-  while (bits < 64 && (1ull << bits) < maxkey) ++bits;
+  while ((1LL << bits) < B) ++bits;
   return bits;
 }
 
-// One orientation of the sparse rebuild: sort keys, unique them, size the rows, fill them.
-static void rebuild_hashed_side(SbpBlockmodel& bm, long long E, unsigned long long* keys, DevBuf<long long>& base,
-                                DevBuf<int>& mask, DevBuf<int2>& slot, DevBuf<int>& cptr, DevBuf<int>& cidx,
-                                DevBuf<int>& cval, long long* top, long long* limit) {
+// Unique (row, column) keys of one orientation, sorted, with the first edge of each in g_sort.heads
+// and the row offsets in g_sort.rowptr; returns their number.
+static long long unique_cells(long long E, int B, unsigned long long* keys) {
   Context& c = Context::get();
-  const int B = bm.B;
+  const int bits = block_bits(B);
   long long nu = 0;
-  unsigned long long* sorted = keys;
   if (E > 0) {
-    radix_sort_u64(keys, g_sort.tmp.p, E, key_bits(B), g_sort.hist.p, g_sort.partial.p, c.num_sms, c.stream, &sorted);
+    unsigned long long* sorted = keys;
+    radix_sort_u64(keys, g_sort.tmp.p, E, 0, 2 * bits, g_sort.hist.p, g_sort.partial.p, c.num_sms, c.stream, &sorted);
     rle(sorted, E, g_sort.flags.p, g_sort.pos.p, g_sort.ukeys.p, g_sort.heads.p, g_sort.partial.p, c.num_sms, c.stream);
     long long lastpos = 0;
     unsigned lastflag = 0;
@@ -172,13 +171,20 @@ static void rebuild_hashed_side(SbpBlockmodel& bm, long long E, unsigned long lo
     c.sync();
     nu = lastpos + lastflag;
   }
-  SBP_CUDA(cudaMemsetAsync(g_sort.rowcnt.p, 0, B * sizeof(unsigned), c.stream));
-  if (nu > 0) {
-    k_unique_rows<<<grid_for(nu, 256, 8 * c.num_sms), 256, 0, c.stream>>>(g_sort.ukeys.p, nu, B, g_sort.rowcnt.p);
-    SBP_CHECK_LAUNCH();
-  }
-  exclusive_scan_u32(g_sort.rowcnt.p, g_sort.rowptr.p, B, g_sort.partial.p, c.num_sms, c.stream);
-  k_row_caps<<<grid_for(B, 256, 8 * c.num_sms), 256, 0, c.stream>>>(g_sort.rowcnt.p, B, (unsigned)g_hashed_row_factor,
+  k_unique_rows<<<grid_for(nu + 1, 256, 16 * c.num_sms), 256, 0, c.stream>>>(g_sort.ukeys.p, nu, B, bits,
+                                                                            g_sort.rowptr.p);
+  SBP_CHECK_LAUNCH();
+  return nu;
+}
+
+// One orientation of the sparse rebuild: sort keys, unique them, size the rows, fill them.
+static void rebuild_hashed_side(SbpBlockmodel& bm, long long E, unsigned long long* keys, DevBuf<long long>& base,
+                                DevBuf<int>& mask, DevBuf<int2>& slot, DevBuf<int>& cptr, DevBuf<int>& cidx,
+                                DevBuf<int>& cval, long long* top, long long* limit) {
+  Context& c = Context::get();
+  const int B = bm.B;
+  const long long nu = unique_cells(E, B, keys);
+  k_row_caps<<<grid_for(B, 256, 8 * c.num_sms), 256, 0, c.stream>>>(g_sort.rowptr.p, B, (unsigned)g_hashed_row_factor,
                                                                    g_sort.caps.p, mask.p);
   exclusive_scan_u32(g_sort.caps.p, base.p, B, g_sort.partial.p, c.num_sms, c.stream);
   SBP_CHECK_LAUNCH();
@@ -196,43 +202,26 @@ static void rebuild_hashed_side(SbpBlockmodel& bm, long long E, unsigned long lo
   cidx.reserve(std::max(nu, 1LL));
   cval.reserve(std::max(nu, 1LL));
   k_fill_empty<<<grid_for(total, 256, 16 * c.num_sms), 256, 0, c.stream>>>(slot.p, total);
-  k_fill_rows<<<grid_for(B, 128, 16 * c.num_sms), 128, 0, c.stream>>>(g_sort.rowptr.p, g_sort.ukeys.p, g_sort.heads.p,
-                                                                     nu, E, B, base.p, mask.p, slot.p, cptr.p,
-                                                                     cidx.p, cval.p);
+  k_fill_rows<<<grid_for(std::max<long long>(nu, B + 1), 256, 16 * c.num_sms), 256, 0, c.stream>>>(
+      g_sort.rowptr.p, g_sort.ukeys.p, g_sort.heads.p, nu, E, B, block_bits(B), base.p, mask.p, slot.p, cptr.p, cidx.p,
+      cval.p);
   SBP_CHECK_LAUNCH();
 }
 
-// Compressed rows of M (or of MT, keys of the transposed edges) from the sorted (b_src, b_dst)
-// keys of the edges, ascending by column: the merge step's outgoing / incoming edge views of a
+// Compressed rows of M (or of MT, keys of the transposed edges) from the (b_src, b_dst) keys of
+// the edges, ascending by column: the merge step's outgoing / incoming edge views of a
 // dense blockmodel too large to scan cell by cell.
 static void sorted_rows(const SbpBlockmodel& bm, long long E, unsigned long long* keys, DevBuf<int>& cptr,
                         DevBuf<int>& cidx, DevBuf<int>& cval) {
   Context& c = Context::get();
   const int B = bm.B;
-  long long nu = 0;
-  if (E > 0) {
-    unsigned long long* sorted = keys;
-    radix_sort_u64(keys, g_sort.tmp.p, E, key_bits(B), g_sort.hist.p, g_sort.partial.p, c.num_sms, c.stream, &sorted);
-    rle(sorted, E, g_sort.flags.p, g_sort.pos.p, g_sort.ukeys.p, g_sort.heads.p, g_sort.partial.p, c.num_sms, c.stream);
-    long long lastpos = 0;
-    unsigned lastflag = 0;
-    SBP_CUDA(SBP_COPY_ASYNC(&lastpos, g_sort.pos.p + E - 1, sizeof(long long), cudaMemcpyDeviceToHost, c.stream));
-    SBP_CUDA(SBP_COPY_ASYNC(&lastflag, g_sort.flags.p + E - 1, sizeof(unsigned), cudaMemcpyDeviceToHost, c.stream));
-    SBP_CHECK_LAUNCH();
-    c.sync();
-    nu = lastpos + lastflag;
-  }
-  SBP_CUDA(cudaMemsetAsync(g_sort.rowcnt.p, 0, B * sizeof(unsigned), c.stream));
-  if (nu > 0) {
-    k_unique_rows<<<grid_for(nu, 256, 8 * c.num_sms), 256, 0, c.stream>>>(g_sort.ukeys.p, nu, B, g_sort.rowcnt.p);
-    SBP_CHECK_LAUNCH();
-  }
-  exclusive_scan_u32(g_sort.rowcnt.p, g_sort.rowptr.p, B, g_sort.partial.p, c.num_sms, c.stream);
+  const long long nu = unique_cells(E, B, keys);
   cptr.reserve(B + 1);
   cidx.reserve(std::max(nu, 1LL));
   cval.reserve(std::max(nu, 1LL));
-  k_fill_csr<<<grid_for(B, 128, 16 * c.num_sms), 128, 0, c.stream>>>(g_sort.rowptr.p, g_sort.ukeys.p, g_sort.heads.p,
-                                                                    nu, E, B, cptr.p, cidx.p, cval.p);
+  k_fill_rows<<<grid_for(std::max<long long>(nu, B + 1), 256, 16 * c.num_sms), 256, 0, c.stream>>>(
+      g_sort.rowptr.p, g_sort.ukeys.p, g_sort.heads.p, nu, E, B, block_bits(B), nullptr, nullptr, nullptr, cptr.p,
+      cidx.p, cval.p);
   SBP_CHECK_LAUNCH();
 }
 
@@ -247,9 +236,8 @@ static void reserve_sort_scratch(long long E, int B) {
   g_sort.heads.reserve(std::max(E, 1LL));
   g_sort.hist.reserve(radix_hist_capacity(std::max(E, 1LL), c.num_sms));
   g_sort.partial.reserve(scan_partial_capacity(c.num_sms));
-  g_sort.rowcnt.reserve(B);
   g_sort.caps.reserve(B);
-  g_sort.rowptr.reserve(B);
+  g_sort.rowptr.reserve((size_t)B + 1);
 }
 
 // Sparse Blockmodel::initialize_edge_counts: rows of M and MT from sorted (b_src, b_dst) keys.
@@ -263,7 +251,7 @@ static void rebuild_sparse(SbpBlockmodel& bm, const SbpGraph& g, bool recompute_
   SBP_CUDA(cudaMemsetAsync(bm.overflow.p, 0, (1 + 2 * (size_t)B) * sizeof(int), c.stream));
   k_block_degrees<<<grid_for(g.V, 256, 8 * c.num_sms), 256, 0, c.stream>>>(g.view(), bm.b.p, bm.d_out.p, bm.d_in.p);
   if (E > 0)
-    k_edge_keys<<<grid_for(E, 256, 16 * c.num_sms), 256, 0, c.stream>>>(g.view(), bm.b.p, g.out_src.p, B,
+    k_edge_keys<<<grid_for(E, 256, 16 * c.num_sms), 256, 0, c.stream>>>(g.view(), bm.b.p, g.out_src.p, block_bits(B),
                                                                        g_sort.keys.p, g_sort.keysT.p);
   SBP_CHECK_LAUNCH();
   rebuild_hashed_side(bm, E, g_sort.keys.p, bm.rbase, bm.rmask, bm.rslot, bm.csr_rptr, bm.csr_ridx, bm.csr_rval,
@@ -439,7 +427,7 @@ MhResult mh_pass(SbpBlockmodel& bm, const SbpGraph& g, const VertexList& list, c
 void gibbs_eval_batch(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& plan, int bt, const RngParams& rng,
                       int sweep) {
   Context& c = Context::get();
-  const int nl = plan.light_n[bt], nh = plan.heavy_n[bt];
+  const int nl = plan.light_n[bt];
   int* n_cur = bm.n_moved.p + (bm.gen & 1);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (nl > 0 && g_prof.on) {
@@ -447,28 +435,11 @@ void gibbs_eval_batch(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan& pla
     e1 = g_prof.get();
     SBP_CUDA(cudaEventRecord(e0, c.stream));
   }
-  if (!bm.sparse) {
-    launch_gibbs_eval(g, bm, plan, bt, rng, sweep, n_cur);
-    SBP_CHECK_LAUNCH();
-  } else if (nl > 0) {
-    const size_t smem = (size_t)table_ints(g.light_cap) * sizeof(int) * kLightWarps;
-    set_smem_limit((const void*)k_gibbs_eval_hashed, smem);
-    k_gibbs_eval_hashed<<<grid_for(nl, kLightWarps, 64 * c.num_sms), kLightWarps * 32, smem, c.stream>>>(
-        g.view(), bm.view(), plan.order.p + plan.light_begin[bt], nl, rng, sweep, bm.prop.p, bm.moved.p, n_cur,
-        c.counters, g.light_cap, c.status);
-    SBP_CHECK_LAUNCH();
-  }
+  launch_gibbs_eval(g, bm, plan, bt, rng, sweep, n_cur);
+  SBP_CHECK_LAUNCH();
   if (e0) {
     SBP_CUDA(cudaEventRecord(e1, c.stream));
     g_prof.add(e0, e1, nl, plan.light_bytes[bt]);
-  }
-  if (bm.sparse && nh > 0) {
-    const size_t smem = (size_t)table_ints(g.heavy_cap) * sizeof(int);
-    set_smem_limit((const void*)k_gibbs_eval_hashed, smem);
-    k_gibbs_eval_hashed<<<grid_for(nh, 1, 64 * c.num_sms), 32, smem, c.stream>>>(
-        g.view(), bm.view(), plan.order.p + plan.heavy_begin[bt], nh, rng, sweep, bm.prop.p, bm.moved.p, n_cur,
-        c.counters, g.heavy_cap, c.status);
-    SBP_CHECK_LAUNCH();
   }
 }
 
@@ -747,7 +718,7 @@ void merge_blocks(SbpBlockmodel& bm, SbpGraph& g, const SbpMergeOptions& opt, co
     // compressed rows from the sorted edge keys: fewer bytes than scanning B x ld cells twice
     reserve_sort_scratch(g.E, B);
     if (g.E > 0)
-      k_edge_keys<<<grid_for(g.E, 256, 16 * c.num_sms), 256, 0, c.stream>>>(g.view(), bm.b.p, g.out_src.p, B,
+      k_edge_keys<<<grid_for(g.E, 256, 16 * c.num_sms), 256, 0, c.stream>>>(g.view(), bm.b.p, g.out_src.p, block_bits(B),
                                                                             g_sort.keys.p, g_sort.keysT.p);
     SBP_CHECK_LAUNCH();
     sorted_rows(bm, g.E, g_sort.keys.p, ms.rptr, ms.ridx, ms.rval);
@@ -1184,7 +1155,7 @@ SbpStatus sbp_graph_create(int32_t V, int64_t n, const int32_t* src, const int32
   // Device ingest (sbp_ingest.cu): first occurrence of each (src, dst) pair, adjacency lists in
   // input order, self loops on the out side only.
   DevBuf<int> d_src, d_dst, first, bad;
-  DevBuf<unsigned long long> table, okeys, ikeys, tmp, partial, ctr;
+  DevBuf<unsigned long long> table, okeys, ikeys, tmp, partial;
   DevBuf<unsigned> ocnt, icnt, hist;
   DevBuf<long long> optr, iptr;
   g->self.reserve(V);
@@ -1196,8 +1167,14 @@ SbpStatus sbp_graph_create(int32_t V, int64_t n, const int32_t* src, const int32
   int ib = 1;
   while ((1LL << ib) < n) ++ib;
   int vb = 1;
-  while ((1LL << vb) < V) ++vb;
-  long long m = 0, mi = 0;
+  while ((1LL << vb) < V + 1LL) ++vb;   // V marks a key that is not in the list
+  partial.reserve(scan_partial_capacity(c.num_sms));
+  optr.reserve((size_t)V + 1);
+  iptr.reserve((size_t)V + 1);
+  g->out_ptr.reserve((size_t)V + 1);
+  g->in_ptr.reserve((size_t)V + 1);
+  bad.reserve(1);
+  SBP_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), c.stream));
   if (n > 0) {
     d_src.reserve(n);
     d_dst.reserve(n);
@@ -1208,53 +1185,16 @@ SbpStatus sbp_graph_create(int32_t V, int64_t n, const int32_t* src, const int32
     const long long cap = 1LL << tbits;
     table.reserve(cap);
     first.reserve(cap);
-    bad.reserve(1);
-    ctr.reserve(2);
     okeys.reserve(n);
     ikeys.reserve(n);
     SBP_CUDA(cudaMemsetAsync(table.p, 0xff, cap * sizeof(unsigned long long), c.stream));
     SBP_CUDA(cudaMemsetAsync(first.p, 0x7f, cap * sizeof(int), c.stream));
-    SBP_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), c.stream));
-    SBP_CUDA(cudaMemsetAsync(ctr.p, 0, 2 * sizeof(unsigned long long), c.stream));
     const int grid = grid_for(n, 256, 16 * c.num_sms);
     k_ingest_first<<<grid, 256, 0, c.stream>>>(d_src.p, d_dst.p, n, V, table.p, first.p, tbits, bad.p);
     k_ingest_keep<<<grid, 256, 0, c.stream>>>(d_src.p, d_dst.p, n, V, table.p, first.p, tbits, ib, okeys.p, ikeys.p,
-                                              ctr.p, ocnt.p, icnt.p, g->self.p);
-    SBP_CHECK_LAUNCH();
-    unsigned long long cnt[2] = {0, 0};
-    int any_bad = 0;
-    SBP_CUDA(SBP_COPY_ASYNC(cnt, ctr.p, sizeof cnt, cudaMemcpyDeviceToHost, c.stream));
-    SBP_CUDA(SBP_COPY_ASYNC(&any_bad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.sync();
-    if (any_bad) throw Error(SBP_ERR_INVALID_ARGUMENT, "edge endpoint out of range");
-    m = (long long)cnt[0];
-    mi = (long long)cnt[1];
-  }
-  g->E = m;
-  partial.reserve(scan_partial_capacity(c.num_sms));
-  g->out_idx.reserve(m);
-  g->out_src.reserve(m);
-  g->in_idx.reserve(mi);
-  if (m > 0) {
-    tmp.reserve(m);
-    hist.reserve(radix_hist_capacity(m, c.num_sms));
-    unsigned long long* sorted = nullptr;
-    radix_sort_u64(okeys.p, tmp.p, m, vb + ib, hist.p, partial.p, c.num_sms, c.stream, &sorted);
-    k_ingest_fill<<<grid_for(m, 256, 16 * c.num_sms), 256, 0, c.stream>>>(sorted, m, ib, d_dst.p, g->out_idx.p,
-                                                                        g->out_src.p);
+                                              ocnt.p, icnt.p, g->self.p);
     SBP_CHECK_LAUNCH();
   }
-  if (mi > 0) {
-    unsigned long long* sorted = nullptr;
-    radix_sort_u64(ikeys.p, tmp.p, mi, vb + ib, hist.p, partial.p, c.num_sms, c.stream, &sorted);
-    k_ingest_fill<<<grid_for(mi, 256, 16 * c.num_sms), 256, 0, c.stream>>>(sorted, mi, ib, d_src.p, g->in_idx.p,
-                                                                         nullptr);
-    SBP_CHECK_LAUNCH();
-  }
-  optr.reserve((size_t)V + 1);
-  iptr.reserve((size_t)V + 1);
-  g->out_ptr.reserve((size_t)V + 1);
-  g->in_ptr.reserve((size_t)V + 1);
   exclusive_scan_u32(ocnt.p, optr.p, (long long)V + 1, partial.p, c.num_sms, c.stream);
   k_ingest_ptr<<<grid_for((long long)V + 1, 256, 8 * c.num_sms), 256, 0, c.stream>>>(optr.p, g->out_ptr.p,
                                                                                     (long long)V + 1);
@@ -1262,14 +1202,35 @@ SbpStatus sbp_graph_create(int32_t V, int64_t n, const int32_t* src, const int32
   k_ingest_ptr<<<grid_for((long long)V + 1, 256, 8 * c.num_sms), 256, 0, c.stream>>>(iptr.p, g->in_ptr.p,
                                                                                     (long long)V + 1);
   SBP_CHECK_LAUNCH();
+  std::vector<int> op((size_t)V + 1), ip((size_t)V + 1);
+  int any_bad = 0;
+  SBP_CUDA(SBP_COPY_ASYNC(op.data(), g->out_ptr.p, ((size_t)V + 1) * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  SBP_CUDA(SBP_COPY_ASYNC(ip.data(), g->in_ptr.p, ((size_t)V + 1) * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  SBP_CUDA(SBP_COPY_ASYNC(&any_bad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  c.sync();
+  if (any_bad) throw Error(SBP_ERR_INVALID_ARGUMENT, "edge endpoint out of range");
+  const long long m = op[V], mi = ip[V];
+  g->E = m;
+  g->out_idx.reserve(m);
+  g->out_src.reserve(m);
+  g->in_idx.reserve(mi);
+  if (n > 0) {
+    // the keys are in input order, so a stable sort by vertex leaves every list in that order
+    tmp.reserve(n);
+    hist.reserve(radix_hist_capacity(n, c.num_sms));
+    unsigned long long* sorted = nullptr;
+    radix_sort_u64(okeys.p, tmp.p, n, ib, vb, hist.p, partial.p, c.num_sms, c.stream, &sorted);
+    k_ingest_fill<<<grid_for(m, 256, 16 * c.num_sms), 256, 0, c.stream>>>(sorted, m, ib, d_dst.p, g->out_idx.p,
+                                                                        g->out_src.p);
+    radix_sort_u64(ikeys.p, tmp.p, n, ib, vb, hist.p, partial.p, c.num_sms, c.stream, &sorted);
+    k_ingest_fill<<<grid_for(mi, 256, 16 * c.num_sms), 256, 0, c.stream>>>(sorted, mi, ib, d_src.p, g->in_idx.p,
+                                                                         nullptr);
+    SBP_CHECK_LAUNCH();
+  }
   g->adj.reserve((size_t)m + (size_t)mi);
   k_join_lists<<<grid_for(8LL * V, 256, 16 * c.num_sms), 256, 0, c.stream>>>(V, g->out_ptr.p, g->out_idx.p,
                                                                             g->in_ptr.p, g->in_idx.p, g->adj.p);
   SBP_CHECK_LAUNCH();
-  std::vector<int> op((size_t)V + 1), ip((size_t)V + 1);
-  SBP_CUDA(SBP_COPY_ASYNC(op.data(), g->out_ptr.p, ((size_t)V + 1) * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-  SBP_CUDA(SBP_COPY_ASYNC(ip.data(), g->in_ptr.p, ((size_t)V + 1) * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-  c.sync();
   g->h_k.resize(V);
   for (int v = 0; v < V; ++v) {
     g->h_k[v] = (op[v + 1] - op[v]) + (ip[v + 1] - ip[v]);

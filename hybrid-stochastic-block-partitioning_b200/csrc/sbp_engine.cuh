@@ -710,7 +710,7 @@ namespace sbpb {
 
 void set_smem_limit(const void* fn, size_t bytes);
 
-// Evaluation of one asynchronous-Gibbs batch on dense storage (sbp_gibbs.cu).
+// Evaluation of one asynchronous-Gibbs batch (sbp_gibbs.cu).
 void launch_gibbs_eval(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& plan, int bt, const RngParams& rng,
                        int sweep, int* n_moved);
 // A whole asynchronous-Gibbs finetune call on dense storage as one persistent kernel.  Only on the

@@ -1,6 +1,6 @@
-// Asynchronous Gibbs on a dense block matrix (finetune::asynchronous_gibbs, src/finetune.cpp:31-89):
-// the evaluation of one batch as a kernel of its own, and a whole finetune call -- every sweep's
-// batches, the MDL and the early stop -- as one persistent kernel.
+// Asynchronous Gibbs (finetune::asynchronous_gibbs, src/finetune.cpp:31-89): the evaluation of one
+// batch as a kernel of its own, on either storage, and a whole finetune call on a dense block matrix
+// -- every sweep's batches, the MDL and the early stop -- as one persistent kernel.
 #include "sbp_engine.cuh"
 #include "sbp_group.cuh"
 #include "sbp_steps.cuh"
@@ -29,12 +29,12 @@ struct EvalArgs {
 
 template <bool kDirect, Store ST>
 __device__ __forceinline__ void eval_task(const EvalArgs& a, const GroupTab<kDirect>& T, int index, bool valid, int sweep,
-                                          int* n_moved, const Lanes& L, EvalCounts& cnt) {
+                                          int* n_moved, const Lanes& L, EvalCounts& cnt, int* bins) {
   const int4 rec = valid ? __ldg(a.recs + index) : make_int4(0, 0, 0, 0);
   uint4 x = make_uint4(0, 0, 0, 0);
   if (valid)
     x = draw_record(a.rng, (uint32_t)rec.x, (uint32_t)sweep, 0u, (long long)sweep * a.g.V + rec.x, a.status);
-  const GroupEval e = group_evaluate<kDirect, ST>(a.g, a.bm, T, valid, rec, a.rng.moves != 0, x, L, a.status);
+  const GroupEval e = group_evaluate<kDirect, ST>(a.g, a.bm, T, valid, rec, a.rng.moves != 0, x, L, a.status, bins);
   if (valid && L.gl == 0) {
     cnt.visit++;
     if (e.s != e.r) cnt.moved++;
@@ -75,7 +75,7 @@ __device__ __forceinline__ void eval_batch(const EvalArgs& a, BatchDesc b, int s
       const GroupTab<kDirect> T = group_tab<kDirect>(smem, a.slots, whole ? 0 : warp * kRegionSlots + sub * share,
                                                      whole ? a.slots : share);
       eval_task<kDirect, ST>(a, T, (light ? b.light_begin : b.heavy_begin) + first + sub, first + sub < end, sweep,
-                             n_moved, L, cnt);
+                             n_moved, L, cnt, smem + group_smem_bytes(kDirect, a.slots) / sizeof(int) + 32 * warp);
     }
     if (whole) __syncthreads();
   }
@@ -91,14 +91,14 @@ __device__ __forceinline__ void add_counts(EvalCounts c, unsigned long long* cou
   }
 }
 
-template <bool kDirect>
+template <bool kDirect, Store ST>
 __global__ void __launch_bounds__(kGroupThreads, 2)
     k_gibbs_eval(const __grid_constant__ EvalArgs a, BatchDesc b, int sweep, int* n_moved, unsigned long long* counters) {
   extern __shared__ int smem[];
   group_tabs_init<kDirect>(smem, a.slots);
   __syncthreads();
   EvalCounts cnt;
-  eval_batch<kDirect, Store::kDenseFrozen>(a, b, sweep, n_moved, smem, cnt);
+  eval_batch<kDirect, ST>(a, b, sweep, n_moved, smem, cnt);
   add_counts(cnt, counters);
 }
 
@@ -287,10 +287,12 @@ void launch_gibbs_eval(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& pl
   EvalArgs a = eval_args(g, bm, plan, rng);
   const BatchDesc& d = plan.desc[bt];
   const int n = d.light_n + d.heavy_n;
-  const bool direct = bm.B <= kSmallB;
+  const bool direct = !bm.sparse && bm.B <= kSmallB;
   a.gmin = group_min(n, 2 * kGroupWarps * c.num_sms);
-  const size_t smem = group_smem_bytes(direct, a.slots);
-  const auto k = direct ? k_gibbs_eval<true> : k_gibbs_eval<false>;
+  const size_t smem = group_smem_bytes(direct, a.slots) + (bm.sparse ? 32 * kGroupWarps * sizeof(int) : 0);   // walk bins
+  const auto k = bm.sparse ? k_gibbs_eval<false, Store::kHashed>
+                 : direct  ? k_gibbs_eval<true, Store::kDenseFrozen>
+                           : k_gibbs_eval<false, Store::kDenseFrozen>;
   set_smem_limit((const void*)k, smem);
   k<<<grid_for((long long)n * a.gmin, 32 * kGroupWarps, 64 * c.num_sms), kGroupThreads, smem, c.stream>>>(
       a, d, sweep, n_moved, c.counters);

@@ -1,7 +1,7 @@
 // Evaluation of a vertex move by a group of lanes of a warp (the same proposal, Hastings
 // correction, delta-MDL and accept test as evaluate_vertex in sbp_device.cuh; reference
-// src/common.cpp:131-192, src/entropy.cpp:296-401, 495-557, src/finetune.cpp:19-29) on a dense block
-// matrix.
+// src/common.cpp:131-192, src/entropy.cpp:296-401, 495-557, src/finetune.cpp:19-29), on either
+// storage of the block matrix.
 //
 // A visit is a chain of about a dozen dependent memory round trips with little work between
 // them, so what counts is how many visits are in flight and how few instructions each costs:
@@ -142,6 +142,61 @@ __device__ __forceinline__ int4 vertex_record(const GraphView& g, int v) {
                    (g.in_ptr[v + 1] - i0) << 1 | (int)g.self[v]);
 }
 
+// Row x of M and of its transpose, for look-ups of (M[x, u], M[u, x]): the row of pairs (dense), or
+// the two hashed rows with their places and masks read once.
+template <Store ST>
+struct RowRef {
+  const int2* p;
+  __device__ __forceinline__ RowRef(const BlockView& bm, int x) : p(bm.P + (size_t)x * bm.ld) {}
+  template <int N>   // on[] masks the look-ups; all N in flight together
+  __device__ __forceinline__ void get(const BlockView&, const int (&u)[N], const bool (&on)[N], int2 (&m)[N]) const {
+#pragma unroll
+    for (int h = 0; h < N; ++h) m[h] = on[h] ? ldv<ST>(p + u[h]) : make_int2(0, 0);
+  }
+};
+template <>
+struct RowRef<Store::kHashed> {
+  long long rb, cb;
+  int rm, cm;
+  __device__ __forceinline__ RowRef(const BlockView& bm, int x)
+      : rb(bm.rbase[x]), cb(bm.cbase[x]), rm(bm.rmask[x]), cm(bm.cmask[x]) {}
+  // The count of column u from the first slot probed, e, on.
+  static __device__ __forceinline__ int follow(const int2* slot, long long base, int mask, int u, int2 e) {
+    unsigned h = slot_hash(u) & (unsigned)mask;
+    for (int probe = 0; probe <= mask; ++probe) {
+      if (e.x == u) return e.y;
+      if (e.x == -1) return 0;
+      h = (h + 1) & (unsigned)mask;
+      e = slot[base + h];
+    }
+    return 0;
+  }
+  template <int N>
+  __device__ __forceinline__ void get(const BlockView& bm, const int (&u)[N], const bool (&on)[N], int2 (&m)[N]) const {
+    int2 a[N], b[N];
+#pragma unroll
+    for (int h = 0; h < N; ++h) {
+      a[h] = b[h] = make_int2(-1, 0);
+      if (on[h]) {
+        a[h] = bm.rslot[rb + (slot_hash(u[h]) & (unsigned)rm)];
+        b[h] = bm.cslot[cb + (slot_hash(u[h]) & (unsigned)cm)];
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < N; ++h)
+      m[h] = on[h] ? make_int2(follow(bm.rslot, rb, rm, u[h], a[h]), follow(bm.cslot, cb, cm, u[h], b[h]))
+                   : make_int2(0, 0);
+  }
+};
+template <Store ST>
+__device__ __forceinline__ int2 row_pair(const RowRef<ST>& row, const BlockView& bm, int u) {
+  const int uu[1] = {u};
+  const bool on[1] = {true};
+  int2 m[1];
+  row.get(bm, uu, on, m);
+  return m[0];
+}
+
 // Rare terms, out of line to keep the evaluation's code small: a count beyond the table, and the
 // double count of a net-zero Delta cell, m (log1p(a / b) + log1p(c / d)).
 static __device__ __noinline__ double dxlogx_far(int a, int b) { return dxlogx((double)a, (double)b); }
@@ -193,7 +248,7 @@ __device__ __forceinline__ bool accept_move(double dS, double fwd, double bwd, b
 template <bool kDirect, Store ST>
 __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const BlockView& bm, const GroupTab<kDirect>& T,
                                                     bool valid, int4 rec, bool given, uint4 x, const Lanes& L,
-                                                    int* status) {
+                                                    int* status, int* bins = nullptr) {
   const int B = bm.B;
   GroupEval res;
   res.valid = valid;
@@ -268,9 +323,10 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
   res.n = n;
   res.t = walk ? t : -1;
   // this lane's first entries and what of them depends on r alone
-  const int2* Pr = bm.P + (size_t)r * bm.ld;
+  const RowRef<ST> Pr(bm, r);
   int u[4];
   unsigned wu[4];
+  bool on[4];
   int2 m_ru[4];
   double inv[4];
 #pragma unroll
@@ -279,15 +335,14 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
     const int slot = j < n ? T.list[j] : -1;
     u[h] = slot >= 0 ? T.key_of(slot) : r;
     wu[h] = slot >= 0 ? T.w[slot] : 0u;
+    on[h] = wu[h] != 0u;
   }
 #pragma unroll
-  for (int h = 0; h < 4; ++h) {
-    m_ru[h] = wu[h] ? ldv<ST>(Pr + u[h]) : make_int2(0, 0);
-    inv[h] = wu[h] ? ldv<ST>(bm.inv_d + u[h]) : 0.0;
-  }
+  for (int h = 0; h < 4; ++h) inv[h] = on[h] ? ldv<ST>(bm.inv_d + u[h]) : 0.0;
+  Pr.get(bm, u, on, m_ru);
   int M_rr = 0, dout_r = 0, din_r = 0;
   if (valid) {
-    M_rr = ldi<ST>(&Pr[r].x);
+    M_rr = row_pair(Pr, bm, r).x;
     dout_r = ldv<ST>(bm.d_out + r);
     din_r = ldv<ST>(bm.d_in + r);
   }
@@ -298,7 +353,20 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
     const long long target = scale32(x.y, (long long)dot + (long long)dit);
     const bool in_col = target >= dot;
     const int tg = (int)(in_col ? target - dot : target);
-    const int found = kDirect ? walk_row<ST>(bm, t, in_col, tg, walk, L) : walk_tree<ST>(bm, t, in_col, tg, walk, L);
+    int found = -1;
+    if constexpr (ST == Store::kHashed) {   // the whole warp walks for its groups in turn
+      for (int first = 0; first < 32; first += L.G) {
+        if (!__shfl_sync(kFull, walk, first)) continue;
+        const int tt = __shfl_sync(kFull, t, first), goal = __shfl_sync(kFull, tg, first);
+        const bool cc = __shfl_sync(kFull, in_col, first);
+        const int at = warp_select_hashed(cc ? bm.cbase : bm.rbase, cc ? bm.cmask : bm.rmask, cc ? bm.cslot : bm.rslot,
+                                          tt, B, goal, L.lane, bins);
+        __syncwarp();
+        if (L.gbase == first) found = at;
+      }
+    } else {
+      found = kDirect ? walk_row<ST>(bm, t, in_col, tg, walk, L) : walk_tree<ST>(bm, t, in_col, tg, walk, L);
+    }
     if (walk) {
       s = found;
       if (s < 0 || s >= B) {
@@ -319,14 +387,15 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
   const bool active = valid && s != r;
   if (!__any_sync(kFull, active)) return res;
   // 3. delta-MDL and the Hastings correction of the move r -> s
-  const int2* Ps = bm.P + (size_t)s * bm.ld;
+  const RowRef<ST> Ps(bm, s);
   int2 m_su[4], m_rs = make_int2(0, 0);
   int M_ss = 0, dout_s = 0, din_s = 0;
 #pragma unroll
-  for (int h = 0; h < 4; ++h) m_su[h] = active && wu[h] ? ldv<ST>(Ps + u[h]) : make_int2(0, 0);
+  for (int h = 0; h < 4; ++h) on[h] = on[h] && active;
+  Ps.get(bm, u, on, m_su);
   if (active) {
-    m_rs = ldv<ST>(Pr + s);
-    M_ss = ldi<ST>(&Ps[s].x);
+    m_rs = row_pair(Pr, bm, s);
+    M_ss = row_pair(Ps, bm, s).x;
     dout_s = ldv<ST>(bm.d_out + s);
     din_s = ldv<ST>(bm.d_in + s);
   }
@@ -401,10 +470,11 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       const int slot = j < nent ? T.list[j] : -1;
       u[h] = slot >= 0 ? T.key_of(slot) : r;
       wu[h] = slot >= 0 ? T.w[slot] : 0u;
-      m_ru[h] = wu[h] ? ldv<ST>(Pr + u[h]) : make_int2(0, 0);
-      m_su[h] = wu[h] ? ldv<ST>(Ps + u[h]) : make_int2(0, 0);
-      inv[h] = wu[h] ? ldv<ST>(bm.inv_d + u[h]) : 0.0;
+      on[h] = wu[h] != 0u;
+      inv[h] = on[h] ? ldv<ST>(bm.inv_d + u[h]) : 0.0;
     }
+    Pr.get(bm, u, on, m_ru);
+    Ps.get(bm, u, on, m_su);
   }
   if (!small) {   // counts beyond the table: the same terms once more, one entry at a time
 #pragma unroll 1
@@ -412,7 +482,7 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
       const int slot = T.list[j], uu = T.key_of(slot);
       const int co = T.w[slot] & kCountMask, ci = (T.w[slot] >> kInShift) & kCountMask;
       if (uu == r || uu == s) continue;
-      const int2 a = ldv<ST>(Pr + uu), b = ldv<ST>(Ps + uu);
+      const int2 a = row_pair(Pr, bm, uu), b = row_pair(Ps, bm, uu);
       if (co) dS += dxlogx_wide(gt, a.x, a.x - co) + dxlogx_wide(gt, b.x, b.x + co);
       if (ci) dS += dxlogx_wide(gt, a.y, a.y - ci) + dxlogx_wide(gt, b.y, b.y + ci);
     }
@@ -433,7 +503,7 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
         const int uu = T.key_of(slot);
         const unsigned w = T.w[slot];
         if (uu == r || uu == s) continue;
-        const int2 a = Pr[uu], b = Ps[uu];
+        const int2 a = row_pair(Pr, bm, uu), b = row_pair(Ps, bm, uu);
         if (w & kCountMask) Tz += 2.0 * ((double)a.x + (double)b.x);
         if ((w >> kInShift) & kCountMask) Tz += 2.0 * ((double)a.y + (double)b.y);
       }

@@ -3,7 +3,6 @@
 // Kernel map (reference function each one stands in for):
 //   k_rebuild_*        Blockmodel::initialize_edge_counts     src/blockmodel/blockmodel.cpp:187-255
 //   k_mdl              entropy::mdl / log_posterior_probability src/entropy.cpp:584-589, blockmodel.cpp:267-285
-//   k_gibbs_eval_hashed asynchronous_gibbs evaluation half    src/finetune.cpp:49-57, 531-545
 //   k_apply_*          asynchronous_gibbs apply half          src/finetune.cpp:58-71 + Blockmodel::move_vertex
 //   k_mh               metropolis_hastings sweep              src/finetune.cpp:412-444, 446-501
 //   k_row_nnz/fill     ISparseMatrix row/column views for the merge phase
@@ -69,43 +68,6 @@ __global__ void k_rebuild_degrees(BlockView bm) {
   if (x < bm.B) set_degree(bm, x, bm.d_out[x] + bm.d_in[x] - bm_get(bm, x, x));
 }
 // ------------------------------------------------------------------------------------------
-// Asynchronous Gibbs on row-hashed storage: evaluate a list of vertices against the frozen state,
-// one warp per vertex (dense storage: sbp_gibbs.cu).  Accepted moves
-// go to prop[v] and the moved list; counters: [0] visits [1] proposals_moved [2] accepted.
-// ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256, 2)
-    k_gibbs_eval_hashed(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
-                        int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status) {
-  extern __shared__ int smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wpb = blockDim.x >> 5;
-  WarpTable t = carve_table(smem, cap, warp);
-  init_table(t, lane);
-  unsigned long long c_visit = 0, c_moved = 0, c_acc = 0;
-  for (int i = blockIdx.x * wpb + warp; i < n; i += gridDim.x * wpb) {
-    const int v = verts[i];
-    const uint4 x = draw_record(rng, (uint32_t)v, (uint32_t)sweep, 0u, (long long)sweep * g.V + v, status);
-    int r, k_out, k_in;
-    const EvalResult res =
-        evaluate_vertex<Store::kHashed>(g, bm, v, x, t, lane, status, &r, &k_out, &k_in, rng.moves != 0);
-    c_visit++;
-    if (res.s != r) c_moved++;
-    if (res.accepted) {
-      c_acc++;
-      if (lane == 0) {
-        prop[v] = res.s;
-        moved_list[atomicAdd(n_moved, 1)] = v;
-      }
-    }
-    table_reset(t, lane);
-  }
-  if (lane == 0 && c_visit) {
-    atomicAdd(counters + 0, c_visit);
-    atomicAdd(counters + 1, c_moved);
-    atomicAdd(counters + 2, c_acc);
-  }
-}
-
 // Apply accepted moves of one batch.
 // Every edge incident to a moved vertex moves once from its old cell to its new cell; the
 // result equals the reference's one-by-one application.  qr/qs keep the reference's diagonal

@@ -40,10 +40,6 @@ __global__ void k_mdl_cells_list(const int* __restrict__ rows, const int* __rest
 __global__ void k_mdl_cells_list_final(const double* partial, int n, int V, long long E, int B, double* out);
 __global__ void k_mdl(GraphView g, BlockView bm, const int* __restrict__ out_src, int cells, double* partial,
                       unsigned* done, double* out);
-// Asynchronous-Gibbs evaluation on row-hashed storage.
-__global__ void __launch_bounds__(256, 2)
-    k_gibbs_eval_hashed(GraphView g, BlockView bm, const int* __restrict__ verts, int n, RngParams rng, int sweep,
-                        int* prop, int* moved_list, int* n_moved, unsigned long long* counters, int cap, int* status);
 __global__ void k_apply_edges(GraphView g, BlockView bm, const int* moved_list, const int* n_moved, const int* prop,
                               int* qr, int* qs, unsigned long long* last, unsigned gen);
 __global__ void k_apply_finish(BlockView bm, const int* moved_list, const int* n_moved, int* next_n_moved, int* prop,
@@ -69,19 +65,17 @@ __global__ void k_join_lists(int V, const int* __restrict__ out_ptr, const int* 
 __global__ void k_vertex_records(GraphView g, const int* __restrict__ verts, int n, int4* recs);
 
 // row-hashed block matrix (sbp_sparse.cu)
-__global__ void k_edge_keys(GraphView g, const int* __restrict__ b, const int* __restrict__ out_src, int B,
+__global__ void k_edge_keys(GraphView g, const int* __restrict__ b, const int* __restrict__ out_src, int bits,
                             unsigned long long* keys, unsigned long long* keysT);
-__global__ void k_unique_rows(const unsigned long long* __restrict__ ukeys, long long n, int B, unsigned* rowcnt);
-__global__ void k_row_caps(const unsigned* __restrict__ rowcnt, int B, unsigned factor, unsigned* cap, int* mask);
+__global__ void k_unique_rows(const unsigned long long* __restrict__ ukeys, long long n, int B, int bits,
+                              long long* rowptr);
+__global__ void k_row_caps(const long long* __restrict__ rowptr, int B, unsigned factor, unsigned* cap, int* mask);
 __global__ void k_fill_empty(int2* slot, long long n);
 __global__ void k_fill_rows(const long long* __restrict__ rowptr, const unsigned long long* __restrict__ ukeys,
-                            const long long* __restrict__ heads, long long nu, long long nedges, int B,
+                            const long long* __restrict__ heads, long long nu, long long nedges, int B, int bits,
                             const long long* __restrict__ base, const int* __restrict__ mask, int2* slot,
                             int* csr_ptr, int* csr_idx, int* csr_val);
 __global__ void k_block_degrees(GraphView g, const int* __restrict__ b, int* d_out, int* d_in);
-__global__ void k_fill_csr(const long long* __restrict__ rowptr, const unsigned long long* __restrict__ ukeys,
-                           const long long* __restrict__ heads, long long nu, long long nedges, int B, int* csr_ptr,
-                           int* csr_idx, int* csr_val);
 __global__ void k_recover_assign(int* b, const int* moved, const int* n_moved, const int* prop, int* old_block);
 __global__ void k_regrow_alloc(const int* __restrict__ full, const int* __restrict__ deg, int B, long long top,
                                long long limit, unsigned long long* used, unsigned long long* nrows, long long* base,
@@ -94,8 +88,8 @@ __global__ void k_ingest_first(const int* __restrict__ src, const int* __restric
                                unsigned long long* keys, int* first, int tbits, int* bad);
 __global__ void k_ingest_keep(const int* __restrict__ src, const int* __restrict__ dst, long long n, int V,
                               const unsigned long long* __restrict__ keys, const int* __restrict__ first, int tbits,
-                              int ib, unsigned long long* out_keys, unsigned long long* in_keys,
-                              unsigned long long* ctr, unsigned* out_cnt, unsigned* in_cnt, unsigned char* self);
+                              int ib, unsigned long long* out_keys, unsigned long long* in_keys, unsigned* out_cnt,
+                              unsigned* in_cnt, unsigned char* self);
 __global__ void k_ingest_fill(const unsigned long long* __restrict__ sorted, long long m, int ib,
                               const int* __restrict__ other, int* idx, int* srcs);
 __global__ void k_ingest_ptr(const long long* __restrict__ in, int* out, long long n);

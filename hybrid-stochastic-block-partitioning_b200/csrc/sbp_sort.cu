@@ -21,43 +21,82 @@ __global__ void k_radix_hist(const unsigned long long* __restrict__ keys, long l
   for (int i = threadIdx.x; i < kRadix; i += blockDim.x) hist[(size_t)i * gridDim.x + blockIdx.x] = h[i];
 }
 
-// Stable scatter: elements of a tile keep their order inside each digit.  Each chunk of
-// blockDim elements ranks its elements per warp (match_any) and across warps (per-digit
-// exclusive prefix over warps in warp order).
-__global__ void k_radix_scatter(const unsigned long long* __restrict__ in, unsigned long long* __restrict__ out,
-                                long long n, long long tile, int shift, const unsigned* __restrict__ offsets) {
-  __shared__ unsigned base[kRadix];
-  __shared__ unsigned tot[kRadix];
+// Stable scatter: elements of a tile keep their order inside each digit.  A CTA takes 4,096 elements
+// at a time, 512 consecutive ones a warp, all loaded before the first is ranked; a warp ranks its
+// elements 32 at a time in order (match_any, running counts per warp), then the counts become
+// offsets per digit across the warps and across the digits, and the elements go through shared
+// memory into digit order, so that a digit's run (16 elements on average) is written as whole
+// lines.  Bound by the ranking and the scattered lines: 12 million keys 247 us at 256 elements and
+// five barriers a round before (78 us of reads and writes at the copy rate).
+constexpr int kSortItems = 16;
+constexpr int kSortChunk = kSortThreads * kSortItems;
+
+__global__ void __launch_bounds__(kSortThreads)
+    k_radix_scatter(const unsigned long long* __restrict__ in, unsigned long long* __restrict__ out, long long n,
+                    long long tile, int shift, const unsigned* __restrict__ offsets) {
+  __shared__ unsigned long long buf[kSortChunk];
   __shared__ unsigned wcount[kSortThreads / 32][kRadix];
+  __shared__ unsigned base[kRadix], start[kRadix];
+  __shared__ unsigned wtot[kSortThreads / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int nw = blockDim.x >> 5;
-  for (int i = threadIdx.x; i < kRadix; i += blockDim.x) base[i] = offsets[(size_t)i * gridDim.x + blockIdx.x];
+  const unsigned below = (1u << lane) - 1u;
+  base[threadIdx.x] = offsets[(size_t)threadIdx.x * gridDim.x + blockIdx.x];   // kRadix == kSortThreads
   const long long b0 = (long long)blockIdx.x * tile, b1 = min(n, b0 + tile);
-  for (long long c0 = b0; c0 < b1; c0 += blockDim.x) {
-    for (int i = threadIdx.x; i < nw * kRadix; i += blockDim.x) (&wcount[0][0])[i] = 0;
-    __syncthreads();
-    const long long i = c0 + threadIdx.x;
-    const bool valid = i < b1;
-    const unsigned long long k = valid ? in[i] : 0ull;
-    const int d = valid ? (int)((k >> shift) & (kRadix - 1)) : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const unsigned rank_in_warp = __popc(peers & ((1u << lane) - 1));
-    if (valid && (__ffs(peers) - 1) == lane) wcount[w][d] = __popc(peers);
-    __syncthreads();
-    for (int dd = threadIdx.x; dd < kRadix; dd += blockDim.x) {
-      unsigned run = 0;
-      for (int ww = 0; ww < nw; ++ww) {
-        const unsigned c = wcount[ww][dd];
-        wcount[ww][dd] = run;
-        run += c;
-      }
-      tot[dd] = run;
+  for (long long c0 = b0; c0 < b1; c0 += kSortChunk) {
+    for (int i = lane; i < kRadix; i += 32) wcount[w][i] = 0;
+    __syncwarp();
+    const long long seg = c0 + (long long)w * (32 * kSortItems) + lane;
+    unsigned long long key[kSortItems];
+    unsigned rank[kSortItems];
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j) key[j] = seg + 32 * j < b1 ? __ldcs(in + seg + 32 * j) : 0ull;
+#pragma unroll
+    for (int j = 0; j < kSortItems; ++j) {
+      const bool valid = seg + 32 * j < b1;
+      const int d = valid ? (int)((key[j] >> shift) & (kRadix - 1)) : kRadix;
+      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      const unsigned before = valid ? wcount[w][d] : 0u;
+      rank[j] = before + __popc(peers & below);
+      __syncwarp();
+      if (valid && (peers & below) == 0) wcount[w][d] = before + __popc(peers);
+      __syncwarp();
     }
     __syncthreads();
-    if (valid) out[base[d] + wcount[w][d] + rank_in_warp] = k;
-    __syncthreads();
-    for (int dd = threadIdx.x; dd < kRadix; dd += blockDim.x) base[dd] += tot[dd];
-    __syncthreads();
+    {   // thread = digit: exclusive counts over the warps, then over the digits
+      unsigned run = 0;
+#pragma unroll
+      for (int ww = 0; ww < kSortThreads / 32; ++ww) {
+        const unsigned c = wcount[ww][threadIdx.x];
+        wcount[ww][threadIdx.x] = run;
+        run += c;
+      }
+      unsigned incl = run;
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) wtot[w] = incl;
+      __syncthreads();
+      unsigned pre = 0;
+      for (int ww = 0; ww < w; ++ww) pre += wtot[ww];
+      start[threadIdx.x] = pre + incl - run;
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < kSortItems; ++j)
+        if (seg + 32 * j < b1) {
+          const int d = (int)((key[j] >> shift) & (kRadix - 1));
+          buf[start[d] + wcount[w][d] + rank[j]] = key[j];
+        }
+      __syncthreads();
+      const int count = (int)min((long long)kSortChunk, b1 - c0);
+      for (int i = threadIdx.x; i < count; i += kSortThreads) {
+        const unsigned long long k = buf[i];
+        const int d = (int)((k >> shift) & (kRadix - 1));
+        out[base[d] + (unsigned)i - start[d]] = k;
+      }
+      __syncthreads();
+      base[threadIdx.x] += run;
+    }
   }
 }
 
@@ -78,15 +117,30 @@ __global__ void k_scan_partials(const unsigned* __restrict__ in, long long n, lo
   }
 }
 
-__global__ void k_scan_top(unsigned long long* partial, int g) {   // single thread: g is small
-  if (threadIdx.x || blockIdx.x) return;
-  unsigned long long run = 0;
-  for (int i = 0; i < g; ++i) {
-    const unsigned long long c = partial[i];
-    partial[i] = run;
-    run += c;
+__global__ void __launch_bounds__(1024) k_scan_top(unsigned long long* partial, int g) {   // one CTA
+  __shared__ unsigned long long wsum[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long carry = 0;
+  for (int c0 = 0; c0 < g; c0 += 1024) {
+    const int i = c0 + threadIdx.x;
+    const unsigned long long v = i < g ? partial[i] : 0;
+    unsigned long long incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();
+    unsigned long long pre = carry, all = carry;
+    for (int ww = 0; ww < 32; ++ww) {
+      if (ww < w) pre += wsum[ww];
+      all += wsum[ww];
+    }
+    if (i < g) partial[i] = pre + incl - v;
+    carry = all;
+    __syncthreads();
   }
-  partial[g] = run;
+  if (threadIdx.x == 0) partial[g] = carry;
 }
 
 // out[i] = partial[cta] + exclusive prefix inside the tile (tile-serial chunks of blockDim).
@@ -156,25 +210,25 @@ void exclusive_scan_u32(const unsigned* in, long long* out, long long n, unsigne
   const int g = scan_grid(n, sms);
   const long long tile = (n + g - 1) / g;
   k_scan_partials<<<g, 256, 0, s>>>(in, n, tile, partial);
-  k_scan_top<<<1, 32, 0, s>>>(partial, g);
+  k_scan_top<<<1, 1024, 0, s>>>(partial, g);
   k_scan_down<long long><<<g, 256, 0, s>>>(in, out, n, tile, partial);
 }
 
 long long scan_partial_capacity(int sms) { return 4LL * sms + 1; }
 
-void radix_sort_u64(unsigned long long* keys, unsigned long long* tmp, long long n, int bits, unsigned* hist,
+void radix_sort_u64(unsigned long long* keys, unsigned long long* tmp, long long n, int low, int bits, unsigned* hist,
                     unsigned long long* partial, int sms, cudaStream_t s, unsigned long long** result) {
   unsigned long long* a = keys;
   unsigned long long* b = tmp;
   const int g = (int)std::min<long long>(std::max<long long>((n + 8191) / 8192, 1), 2LL * sms);
   const long long tile = (n + g - 1) / g;
-  for (int shift = 0; shift < bits; shift += kRadixBits) {
+  for (int shift = low; shift < low + bits; shift += kRadixBits) {
     k_radix_hist<<<g, kSortThreads, 0, s>>>(a, n, tile, shift, hist);
     const long long hn = (long long)kRadix * g;
     const int sg = scan_grid(hn, sms);
     const long long stile = (hn + sg - 1) / sg;
     k_scan_partials<<<sg, 256, 0, s>>>(hist, hn, stile, partial);
-    k_scan_top<<<1, 32, 0, s>>>(partial, sg);
+    k_scan_top<<<1, 1024, 0, s>>>(partial, sg);
     k_scan_down<unsigned><<<sg, 256, 0, s>>>(hist, hist, hn, stile, partial);
     k_radix_scatter<<<g, kSortThreads, 0, s>>>(a, b, n, tile, shift, hist);
     std::swap(a, b);

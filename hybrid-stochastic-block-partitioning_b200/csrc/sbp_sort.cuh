@@ -11,9 +11,10 @@ void exclusive_scan_u32(const unsigned* in, long long* out, long long n, unsigne
                         cudaStream_t s);
 long long scan_partial_capacity(int sms);
 
-// Stable LSD radix sort of the low `bits` bits of n 64-bit keys; `tmp` has n entries, `hist`
+// Stable LSD radix sort of n 64-bit keys by their bits [low, low + bits) (rounded up to whole bytes
+// above: higher bits must be zero or order as wanted); `tmp` has n entries, `hist`
 // radix_hist_capacity(n, sms) entries.  *result points at keys or tmp (the sorted copy).
-void radix_sort_u64(unsigned long long* keys, unsigned long long* tmp, long long n, int bits, unsigned* hist,
+void radix_sort_u64(unsigned long long* keys, unsigned long long* tmp, long long n, int low, int bits, unsigned* hist,
                     unsigned long long* partial, int sms, cudaStream_t s, unsigned long long** result);
 long long radix_hist_capacity(long long n, int sms);
 

@@ -5,31 +5,38 @@
 
 namespace sbpb {
 
-// (b[src], b[dst]) and (b[dst], b[src]) keys of every edge.
-__global__ void k_edge_keys(GraphView g, const int* __restrict__ b, const int* __restrict__ out_src, int B,
+// (b[src], b[dst]) and (b[dst], b[src]) keys of every edge: row << bits | column.
+__global__ void k_edge_keys(GraphView g, const int* __restrict__ b, const int* __restrict__ out_src, int bits,
                             unsigned long long* keys, unsigned long long* keysT) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < g.E; e += stride) {
     const unsigned long long bs = (unsigned)b[__ldg(out_src + e)], bd = (unsigned)b[__ldg(g.out_idx + e)];
-    keys[e] = bs * (unsigned long long)B + bd;
-    keysT[e] = bd * (unsigned long long)B + bs;
+    keys[e] = bs << bits | bd;
+    keysT[e] = bd << bits | bs;
   }
 }
 
-// Non-zero cells per row from the unique sorted keys.
-__global__ void k_unique_rows(const unsigned long long* __restrict__ ukeys, long long n, int B, unsigned* rowcnt) {
-  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x)
-    atomicAdd(rowcnt + (ukeys[j] / (unsigned long long)B), 1u);
+// First unique key of every row: the unique keys are sorted, so the thread that sees a row change
+// writes the offsets of the rows it opens (empty rows before it included).  rowptr has B + 1 entries.
+__global__ void k_unique_rows(const unsigned long long* __restrict__ ukeys, long long n, int B, int bits,
+                              long long* rowptr) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j <= n; j += stride) {
+    const int row = j < n ? (int)(ukeys[j] >> bits) : B;
+    const int before = j > 0 ? (int)(ukeys[j - 1] >> bits) : -1;
+    for (int r = before + 1; r <= row; ++r) rowptr[r] = j;
+  }
 }
 
 // Row capacity: a power of two of at least factor * cells + 4 factor slots (room to grow: at
 // large B most moves add cells, and a full row has to be regrown).  Rows of more than 128
 // cells get at most factor 2: the hashed walk reads a row's whole region, and for long rows
 // that costs more than the occasional regrowth.
-__global__ void k_row_caps(const unsigned* __restrict__ rowcnt, int B, unsigned factor, unsigned* cap, int* mask) {
+__global__ void k_row_caps(const long long* __restrict__ rowptr, int B, unsigned factor, unsigned* cap, int* mask) {
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < B; r += gridDim.x * blockDim.x) {
-    const unsigned f = rowcnt[r] > 128u && factor > 2u ? 2u : factor;
-    unsigned want = f * rowcnt[r] + 4u * f, c = 8u;
+    const unsigned cells = (unsigned)(rowptr[r + 1] - rowptr[r]);
+    const unsigned f = cells > 128u && factor > 2u ? 2u : factor;
+    unsigned want = f * cells + 4u * f, c = 8u;
     while (c < want) c <<= 1;
     cap[r] = c;
     mask[r] = (int)c - 1;
@@ -41,42 +48,33 @@ __global__ void k_fill_empty(int2* slot, long long n) {
     slot[i] = make_int2(-1, 0);
 }
 
-// One thread per row inserts its cells in ascending column order, so the slot layout of a
-// rebuilt row is the same on every run.  Also writes the compressed (sorted) row.
+// One thread per cell: its entry of the compressed (sorted) row and, with slots given, its hashed
+// slot (a cell's key is its own, so the thread whose compare-and-swap takes a free slot owns it; the
+// row's capacity is at least twice its cells and 8).  Where a cell sits in its row depends on the
+// order of arrival, which no result does.  (One thread per row, its insertions one after another,
+// took 1.2 ms for 10 million cells.)
 __global__ void k_fill_rows(const long long* __restrict__ rowptr, const unsigned long long* __restrict__ ukeys,
-                            const long long* __restrict__ heads, long long nu, long long nedges, int B,
+                            const long long* __restrict__ heads, long long nu, long long nedges, int B, int bits,
                             const long long* __restrict__ base, const int* __restrict__ mask, int2* slot,
                             int* csr_ptr, int* csr_idx, int* csr_val) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < B; r += gridDim.x * blockDim.x) {
-    const long long j0 = rowptr[r], j1 = (r + 1 < B) ? rowptr[r + 1] : nu;
-    csr_ptr[r] = (int)j0;
-    if (r == B - 1) csr_ptr[B] = (int)nu;
-    const long long b0 = base[r];
-    const int m = mask[r];
-    for (long long j = j0; j < j1; ++j) {
-      const int col = (int)(ukeys[j] % (unsigned long long)B);
-      const int cnt = (int)(((j + 1 < nu) ? heads[j + 1] : nedges) - heads[j]);
-      csr_idx[j] = col;
-      csr_val[j] = cnt;
-      unsigned h = slot_hash(col) & (unsigned)m;
-      while (slot[b0 + h].x != -1) h = (h + 1) & (unsigned)m;   // capacity >= 2 * count + 8
-      slot[b0 + h] = make_int2(col, cnt);
-    }
-  }
-}
-
-// Compressed rows only (no hashed slots): the merge step of a large dense blockmodel, whose B x B
-// matrix is too large to scan for its non-zero cells.
-__global__ void k_fill_csr(const long long* __restrict__ rowptr, const unsigned long long* __restrict__ ukeys,
-                           const long long* __restrict__ heads, long long nu, long long nedges, int B, int* csr_ptr,
-                           int* csr_idx, int* csr_val) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < B; r += gridDim.x * blockDim.x) {
-    const long long j0 = rowptr[r], j1 = (r + 1 < B) ? rowptr[r + 1] : nu;
-    csr_ptr[r] = (int)j0;
-    if (r == B - 1) csr_ptr[B] = (int)nu;
-    for (long long j = j0; j < j1; ++j) {
-      csr_idx[j] = (int)(ukeys[j] % (unsigned long long)B);
-      csr_val[j] = (int)(((j + 1 < nu) ? heads[j + 1] : nedges) - heads[j]);
+  const long long stride = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long r = first; r <= B; r += stride) csr_ptr[r] = (int)rowptr[r];
+  for (long long j = first; j < nu; j += stride) {
+    const unsigned long long key = ukeys[j];
+    const int row = (int)(key >> bits), col = (int)(key & ((1ull << bits) - 1ull));
+    const int cnt = (int)((j + 1 < nu ? heads[j + 1] : nedges) - heads[j]);
+    csr_idx[j] = col;
+    csr_val[j] = cnt;
+    if (!slot) continue;
+    const long long b0 = base[row];
+    const int m = mask[row];
+    unsigned h = slot_hash(col) & (unsigned)m;
+    for (int probe = 0; probe <= m; ++probe) {
+      if (atomicCAS(&slot[b0 + h].x, -1, col) == -1) {
+        slot[b0 + h].y = cnt;
+        break;
+      }
+      h = (h + 1) & (unsigned)m;
     }
   }
 }
