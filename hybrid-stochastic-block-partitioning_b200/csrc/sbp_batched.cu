@@ -6,13 +6,15 @@
 // launch per sweep:
 //
 //   * every graph has a work queue: its sweep is a fixed list of stages (per batch: evaluation
-//     items - a chunk of light vertices or one heavy vertex -, apply stripes, finish stripes;
-//     then the MDL's partial sums, one item per run of virtual CTAs, and its final sum);
+//     items - a task of the group evaluation for each warp, or one heavy vertex -, apply stripes,
+//     finish stripes; then the MDL's partial sums, one item per run of virtual CTAs, and its final
+//     sum).  The CTA that ends a short apply does the degree step itself, and the one that ends the
+//     MDL's partial sums the final sum: a stage's hand-over costs more than they do;
 //   * a CTA claims the next item of any graph whose current stage still has unclaimed items
 //     (one 64-bit atomic: stage << 32 | next item); the CTA finishing a stage's last item opens
 //     the graph's next stage.  No CTA ever waits while holding an item, so one graph's stages
 //     stay in order while the other graphs keep the GPU busy;
-//   * the per-element work is the single-graph kernels' own code (evaluate_vertex,
+//   * the per-element work is the single-graph kernels' own code (group_evaluate,
 //     apply_moved_vertex, finish_moved_vertex, the MDL parts with the same virtual grid), so
 //     every graph's chain and MDL are those of sbp_partition, bit for bit;
 //   * each sweep's launch (parameter upload, queue reset, kernel, result read-back) is a
@@ -38,7 +40,7 @@
 namespace sbpb {
 namespace {
 
-enum StageKind : int { kEval = 0, kApply = 1, kFinish = 2, kMdlPart = 3, kMdlFinal = 4 };
+enum StageKind : int { kEval = 0, kApply = 1, kFinish = 2, kMdlPart = 3 };
 
 // One stage of a graph's sweep: kind, batch, items, light-vertex chunks among the items.
 // (int4: x kind, y batch, z items, w light chunks)
@@ -46,8 +48,8 @@ enum StageKind : int { kEval = 0, kApply = 1, kFinish = 2, kMdlPart = 3, kMdlFin
 struct BGraph {   // one graph of the batch (device side)
   GraphView g;
   BlockView bm;
-  const int* order;          // the batch plan's vertex order
-  const int4* batches;       // per batch: light begin, light count, heavy begin, heavy count
+  const int4* recs;          // the batch plan's vertex records
+  const BatchDesc* batches;
   const int4* stages;        // the sweep's stages
   const int* out_src;
   int* prop;
@@ -63,7 +65,7 @@ struct BGraph {   // one graph of the batch (device side)
   int sweep;                 // the graph's sweep index within its finetune
   unsigned gen0;             // batch generation before the sweep
   int nstages;
-  int chunk;                 // light vertices per evaluation item
+  int gmin;                  // smallest group of an evaluation
   int mdl_cells;             // 1: cell form of the MDL, 0: edge form
   int mdl_ctas;              // its virtual grid
 };
@@ -76,7 +78,6 @@ struct Queue {                 // per graph, reset before every launch
 
 struct SweepParams {
   int ngraphs;                 // graphs in this launch (indices in glist)
-  int heavy_cap;
   unsigned wait_limit;         // idle claim attempts of a CTA before the launch gives up
 };
 
@@ -85,6 +86,7 @@ constexpr int kBThreads = kBWarps * 32;
 constexpr int kErrBatchWait = 16;        // no claimable work for too long
 constexpr int kMdlCtasPerItem = 16;
 constexpr int kApplyPerStripe = 256;     // moved vertices per apply / finish stripe (bound)
+constexpr int kFusedFinish = 2048;       // moved vertices up to which the CTA that ends an apply runs the degree step
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   unsigned long long v;
@@ -94,14 +96,13 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 
 __global__ void __launch_bounds__(kBThreads, 2)
     k_batched_sweep(const BGraph* __restrict__ G, const int* __restrict__ glist, Queue* queue, int* nfinished,
-                    int* abort_flag, const SweepParams* __restrict__ sp, int cap, int* status) {
+                    int* abort_flag, const SweepParams* __restrict__ sp, int slots, int* status) {
   extern __shared__ int smem[];
-  __shared__ int s_g, s_stage, s_idx, s_exit;
+  __shared__ int s_g, s_stage, s_idx, s_exit, s_close;
   __shared__ double red[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const SweepParams P = *sp;
-  WarpTable t = carve_table(smem, cap, warp);
-  init_table(t, lane);
+  group_tabs_init<false>(smem, slots);
   unsigned idle = 0;
   unsigned rot = blockIdx.x * 13u;
   for (;;) {
@@ -177,55 +178,36 @@ __global__ void __launch_bounds__(kBThreads, 2)
     int* n_cur = gr.n_moved + ((gen - 1u) & 1u);
     switch (stg.x) {
       case kEval: {
-        const int4 bt = gr.batches[stg.y];
-        if (idx < stg.w) {   // a chunk of light vertices
-          const int* verts = gr.order + bt.x;
-          const int a = idx * gr.chunk;
-          const int end = min(a + gr.chunk, bt.y);
-          unsigned long long c_visit = 0, c_moved = 0, c_acc = 0;
-          for (int i = a + warp; i < end; i += kBWarps) {
-            const int v = verts[i];
-            const uint4 x =
-                draw_record(gr.rng, (uint32_t)v, (uint32_t)gr.sweep, 0u, (long long)gr.sweep * gr.g.V + v, status);
-            int r, k_out, k_in;
-            const EvalResult res = evaluate_vertex<Store::kDense>(gr.g, gr.bm, v, x, t, lane, status, &r, &k_out, &k_in);
-            c_visit++;
-            if (res.s != r) c_moved++;
-            if (res.accepted) {
-              c_acc++;
-              if (lane == 0) {
-                gr.prop[v] = res.s;
-                gr.moved[atomicAdd(n_cur, 1)] = v;
-              }
-            }
-            table_reset(t, lane);
+        const BatchDesc bt = gr.batches[stg.y];
+        const bool light = idx < stg.w;
+        if (light || warp == 0) {   // a task per warp, or one heavy vertex on warp 0 with the CTA's whole table
+          const GroupTask k = group_task(bt, gr.gmin, light ? idx * kBWarps + warp : idx - stg.w, light);
+          const Lanes L(32 >> k.lg, lane);
+          const int sub = lane >> (5 - k.lg), share = kRegionSlots >> k.lg;
+          const GroupTab<false> T =
+              group_tab<false>(smem, slots, light ? warp * kRegionSlots + sub * share : 0, light ? share : slots);
+          const bool valid = k.first + sub < k.end;
+          const int4 rec = valid ? __ldg(gr.recs + (light ? bt.light_begin : bt.heavy_begin) + k.first + sub)
+                                 : make_int4(0, 0, 0, 0);
+          uint4 x = make_uint4(0, 0, 0, 0);
+          if (valid)
+            x = draw_record(gr.rng, (uint32_t)rec.x, (uint32_t)gr.sweep, 0u, (long long)gr.sweep * gr.g.V + rec.x, status);
+          const GroupEval e =
+              group_evaluate<false, Store::kDense, true>(gr.g, gr.bm, T, valid, rec, false, x, L, status);
+          const bool head = valid && L.gl == 0;
+          if (head && e.accepted) {
+            gr.prop[e.v] = e.s;
+            gr.moved[atomicAdd(n_cur, 1)] = e.v;
           }
+          T.clear(e.n, L);
+          const unsigned c_visit = __popc(__ballot_sync(kFull, head)),
+                         c_moved = __popc(__ballot_sync(kFull, head && e.s != e.r)),
+                         c_acc = __popc(__ballot_sync(kFull, head && e.accepted));
           if (lane == 0 && c_visit) {
-            atomicAdd(gr.counters + 0, c_visit);
-            atomicAdd(gr.counters + 1, c_moved);
-            atomicAdd(gr.counters + 2, c_acc);
+            atomicAdd(gr.counters + 0, (unsigned long long)c_visit);
+            atomicAdd(gr.counters + 1, (unsigned long long)c_moved);
+            atomicAdd(gr.counters + 2, (unsigned long long)c_acc);
           }
-        } else {             // one heavy vertex on warp 0, its table over the whole shared memory
-          if (warp == 0) {
-            WarpTable big = carve_table(smem, P.heavy_cap, 0);
-            init_table(big, lane);
-            const int v = gr.order[bt.z + (idx - stg.w)];
-            const uint4 x =
-                draw_record(gr.rng, (uint32_t)v, (uint32_t)gr.sweep, 0u, (long long)gr.sweep * gr.g.V + v, status);
-            int r, k_out, k_in;
-            const EvalResult res = evaluate_vertex<Store::kDense>(gr.g, gr.bm, v, x, big, lane, status, &r, &k_out, &k_in);
-            if (lane == 0) {
-              atomicAdd(gr.counters + 0, 1ull);
-              if (res.s != r) atomicAdd(gr.counters + 1, 1ull);
-              if (res.accepted) {
-                atomicAdd(gr.counters + 2, 1ull);
-                gr.prop[v] = res.s;
-                gr.moved[atomicAdd(n_cur, 1)] = v;
-              }
-            }
-          }
-          __syncthreads();
-          init_table(t, lane);   // the per-warp tables under the big one are empty again
         }
         break;
       }
@@ -251,27 +233,43 @@ __global__ void __launch_bounds__(kBThreads, 2)
         }
         break;
       }
-      case kMdlFinal: {
-        const double v = mdl_final_value(gr.partial, gr.mdl_ctas, gr.g.V, gr.g.E, gr.bm.B, red);
-        if (tid == 0) *gr.mdl_out = v;
-        break;
-      }
       default:
         break;
     }
     __threadfence();
     __syncthreads();
+    Queue& q = queue[gi];
     if (tid == 0) {
-      Queue& q = queue[gi];
       const int prev = atomicAdd(&q.done, 1);
-      if (prev + 1 == stg.z) {   // last item of the stage: open the next one
+      s_close = prev + 1 == stg.z;   // last item of the stage
+      __threadfence();
+    }
+    __syncthreads();
+    if (s_close) {
+      int next = s_stage + 1;
+      if (stg.x == kApply) {
+        const int n = *(volatile int*)n_cur;
+        if (n <= kFusedFinish) {
+          if (tid == 0) gr.n_moved[gen & 1u] = 0;   // the next batch's slot
+          for (int i = tid; i < n; i += kBThreads)
+            finish_moved_vertex<Store::kDense>(gr.bm, gr.moved[i], gr.prop, gr.qr, gr.qs, gr.last, gen);
+          next++;
+        }
+      } else if (stg.x == kMdlPart) {
+        const double v = mdl_final_value(gr.partial, gr.mdl_ctas, gr.g.V, gr.g.E, gr.bm.B, red);
+        if (tid == 0) *gr.mdl_out = v;
+        next++;
+      }
+      __threadfence();
+      __syncthreads();
+      if (tid == 0) {   // open the next stage
         atomicExch(&q.done, 0);
         __threadfence();
-        if (s_stage + 1 >= gr.nstages) {
+        if (next >= gr.nstages) {
           atomicExch(&q.finished, 1);
           atomicAdd(nfinished, 1);
         } else {
-          atomicExch(&q.ctr, (unsigned long long)(s_stage + 1) << 32);
+          atomicExch(&q.ctr, (unsigned long long)next << 32);
         }
       }
     }
@@ -283,10 +281,10 @@ __global__ void __launch_bounds__(kBThreads, 2)
 // Autotuner: candidate item shapes, the choice cached per workload shape.
 // ------------------------------------------------------------------------------------------
 struct Shape {
-  int chunk;         // light vertices per evaluation item
+  int chunk;         // vertices of the smallest groups per evaluation item: 8, 16 or 32 of 32, 16 or 8 lanes
   int ctas_per_sm;   // persistent CTAs per SM
 };
-const Shape kCandidates[] = {{8, 2}, {16, 2}, {32, 2}, {64, 2}, {16, 1}, {64, 1}};
+const Shape kCandidates[] = {{8, 2}, {16, 2}, {32, 2}, {8, 1}, {16, 1}, {32, 1}};
 constexpr int kNumCandidates = sizeof(kCandidates) / sizeof(kCandidates[0]);
 std::map<unsigned long long, Shape> g_tuned;   // workload key -> shape
 
@@ -302,18 +300,17 @@ bool batchable(const SbpBlockmodel& bm, const SbpGraph& g) {
   return !bm.sparse && g.light_cap <= kLightCapMax && g.heavy_cap <= 4096 && bm.B > 1;
 }
 
-// The stages of one sweep of a graph with the given plan and chunk.
-std::vector<int4> sweep_stages(const BatchPlan& p, int chunk, int mdl_ctas) {
+// The stages of one sweep of a graph with the given plan and smallest group.
+std::vector<int4> sweep_stages(const BatchPlan& p, int gmin, int mdl_ctas) {
   std::vector<int4> st;
   for (size_t b = 0; b < p.light_n.size(); ++b) {
-    const int lc = (p.light_n[b] + chunk - 1) / chunk;
+    const int lc = (group_tasks(p.desc[b], gmin) + kBWarps - 1) / kBWarps;
     st.push_back(make_int4(kEval, (int)b, lc + p.heavy_n[b], lc));
     const int stripes = std::max(1, (p.light_n[b] + p.heavy_n[b] + kApplyPerStripe - 1) / kApplyPerStripe);
     st.push_back(make_int4(kApply, (int)b, stripes, 0));
     st.push_back(make_int4(kFinish, (int)b, stripes, 0));
   }
   st.push_back(make_int4(kMdlPart, 0, (mdl_ctas + kMdlCtasPerItem - 1) / kMdlCtasPerItem, 0));
-  st.push_back(make_int4(kMdlFinal, 0, 1, 0));
   return st;
 }
 
@@ -334,7 +331,7 @@ struct Slot {
   int sweep = 0;
   int stage_chunk = -1, stage_mdl = -1;   // what the uploaded stages were made for
   std::chrono::steady_clock::time_point t0;
-  DevBuf<int4> batches, stages;
+  DevBuf<int4> stages;
   DevBuf<unsigned long long> counters;
   DevBuf<double> partial;
 };
@@ -424,14 +421,14 @@ class StepPool {
 static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const SbpOptions& opt, SbpBatchInfo& info) {
   Context& c = Context::get();
   const int n = (int)slots.size();
-  int cap = kLightCap, heavy_cap = 512;
+  int distinct = 1;   // of a heavy vertex's neighbour blocks, at most
   long long vertices = 0;
   for (auto& s : slots) {
-    cap = std::max(cap, std::min(s->g->light_cap, kLightCapMax));
-    if (s->g->heavy_cap <= 4096) heavy_cap = std::max(heavy_cap, s->g->heavy_cap);
+    if (s->g->heavy_cap <= 4096) distinct = std::max(distinct, s->g->max_k);
     vertices += s->g->V;
   }
-  const size_t smem = std::max((size_t)kBWarps * table_ints(cap), (size_t)table_ints(heavy_cap)) * sizeof(int);
+  const int table = std::max(kBWarps * kRegionSlots, pow2_at_least(2 * distinct));
+  const size_t smem = group_smem_bytes(false, table);
   set_smem_limit((const void*)k_batched_sweep, smem);
   int max_per_sm = 0;
   SBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_per_sm, k_batched_sweep, kBThreads, smem));
@@ -493,17 +490,9 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
     std::memset(&s.fs, 0, sizeof s.fs);
     s.fs.num_blocks = bm.B;
     s.plan = &s.g->plan(SBP_ASYNC_GIBBS, s.fo.batches);
-    if (!s.batches.p) {   // the plan is the graph's, the same in every round
-      std::vector<int4> bt(s.plan->light_n.size());
-      for (size_t b = 0; b < bt.size(); ++b)
-        bt[b] = make_int4(s.plan->light_begin[b], s.plan->light_n[b], s.plan->heavy_begin[b], s.plan->heavy_n[b]);
-      s.batches.reserve(std::max<size_t>(bt.size(), 1));
-      if (!bt.empty())
-        SBP_CUDA(SBP_COPY_ASYNC(s.batches.p, bt.data(), bt.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream));
-      s.stages.reserve(3 * bt.size() + 2);
-      s.counters.reserve(3);
-      s.partial.reserve(c.npartial);
-    }
+    s.stages.reserve(3 * s.plan->desc.size() + 1);
+    s.counters.reserve(3);
+    s.partial.reserve(c.npartial);
     SBP_CUDA(cudaMemsetAsync(s.counters.p, 0, 3 * sizeof(unsigned long long), c.stream));
     bm.overall_entropy = (float)mdl(bm, *s.g);
     s.initial = bm.overall_entropy;
@@ -595,7 +584,7 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
     for (Slot* s : act) {
       const int mdl_ctas = mdl_grid(s->ps->bm, *s->g);
       if (s->stage_chunk != shape.chunk || s->stage_mdl != mdl_ctas) {
-        const std::vector<int4> st = sweep_stages(*s->plan, shape.chunk, mdl_ctas);
+        const std::vector<int4> st = sweep_stages(*s->plan, 256 / shape.chunk, mdl_ctas);
         SBP_CUDA(SBP_COPY_ASYNC(s->stages.p, st.data(), st.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream));
         s->stage_chunk = shape.chunk;
         s->stage_mdl = mdl_ctas;
@@ -604,8 +593,8 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
       SbpBlockmodel& bm = s->ps->bm;
       b.g = s->g->view();
       b.bm = bm.view();
-      b.order = s->plan->order.p;
-      b.batches = s->batches.p;
+      b.recs = s->plan->recs.p;
+      b.batches = s->plan->desc_dev.p;
       b.stages = s->stages.p;
       b.out_src = s->g->out_src.p;
       b.prop = bm.prop.p;
@@ -623,14 +612,13 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
       b.rng.call = s->fo.call;
       b.sweep = s->sweep;
       b.gen0 = bm.gen;
-      b.nstages = (int)(3 * s->plan->light_n.size() + 2);
-      b.chunk = shape.chunk;
+      b.nstages = (int)(3 * s->plan->desc.size() + 1);
+      b.gmin = 256 / shape.chunk;
       b.mdl_cells = mdl_cell_form(bm, *s->g) ? 1 : 0;
       b.mdl_ctas = mdl_grid(bm, *s->g);
     }
     for (size_t k = 0; k < act.size(); ++k) hList[k] = act[k]->index;
     hP->ngraphs = (int)act.size();
-    hP->heavy_cap = heavy_cap;
     hP->wait_limit = (unsigned)g_batched_wait_limit;
     // fault injection for the failure-detection test: the stalled graph's first stage starts
     // with every item taken, so it never completes and no stage of that graph opens again
@@ -650,7 +638,7 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
       cudaMemcpyAsync(dP.p, hP, sizeof(SweepParams), cudaMemcpyHostToDevice, c.stream);
       cudaMemcpyAsync(dQ.p, hQ, n * sizeof(Queue), cudaMemcpyHostToDevice, c.stream);
       cudaMemsetAsync(dSync.p, 0, 2 * sizeof(int), c.stream);
-      k_batched_sweep<<<grid, kBThreads, smem, c.stream>>>(dG.p, dList.p, dQ.p, dSync.p, dSync.p + 1, dP.p, cap,
+      k_batched_sweep<<<grid, kBThreads, smem, c.stream>>>(dG.p, dList.p, dQ.p, dSync.p, dSync.p + 1, dP.p, table,
                                                            c.status);
       cudaMemcpyAsync(hMdl, dMdl.p, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream);
       cudaMemcpyAsync(hStatus, c.status, sizeof(int), cudaMemcpyDeviceToHost, c.stream);

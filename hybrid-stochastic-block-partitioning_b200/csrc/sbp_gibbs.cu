@@ -54,27 +54,21 @@ __device__ __forceinline__ void eval_batch(const EvalArgs& a, BatchDesc b, int s
                                            EvalCounts& cnt) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wid = blockIdx.x * kGroupWarps + warp, nw = gridDim.x * kGroupWarps;
-  const int n = b.light_n;
-  const int c32 = a.gmin >= 32 ? n : b.n32;
-  const int c16 = a.gmin >= 32 ? 0 : a.gmin >= 16 ? n - c32 : b.n16;
-  const int t16 = (c16 + 1) >> 1, t8 = (n - c32 - c16 + 3) >> 2;
   // Two passes over one body: the heavy vertices, each by one warp with the whole CTA's table (any
   // degree fits a direct-indexed histogram, so there by any warp), then the light ones.
 #pragma unroll 1
   for (int light = b.heavy_n > 0 ? 0 : 1; light < 2; ++light) {
     const bool whole = !kDirect && !light;
     const int first_task = whole ? (warp == 0 ? (int)blockIdx.x : b.heavy_n) : wid, step = whole ? (int)gridDim.x : nw;
-    const int tasks = light ? c32 + t16 + t8 : b.heavy_n;
+    const int tasks = light ? group_tasks(b, a.gmin) : b.heavy_n;
 #pragma unroll 1
     for (int task = first_task; task < tasks; task += step) {
-      const int lg = !light || task < c32 ? 0 : task < c32 + t16 ? 1 : 2;   // log2 of the vertices of the task
-      const int first = lg == 0 ? task : lg == 1 ? c32 + 2 * (task - c32) : c32 + c16 + 4 * (task - c32 - t16);
-      const int end = !light ? tasks : lg == 0 ? c32 : lg == 1 ? c32 + c16 : n;
-      const Lanes L(32 >> lg, lane);
-      const int sub = lane >> (5 - lg), share = kRegionSlots >> lg;
+      const GroupTask k = group_task(b, a.gmin, task, light);
+      const Lanes L(32 >> k.lg, lane);
+      const int sub = lane >> (5 - k.lg), share = kRegionSlots >> k.lg;
       const GroupTab<kDirect> T = group_tab<kDirect>(smem, a.slots, whole ? 0 : warp * kRegionSlots + sub * share,
                                                      whole ? a.slots : share);
-      eval_task<kDirect, ST>(a, T, (light ? b.light_begin : b.heavy_begin) + first + sub, first + sub < end, sweep,
+      eval_task<kDirect, ST>(a, T, (light ? b.light_begin : b.heavy_begin) + k.first + sub, k.first + sub < k.end, sweep,
                              n_moved, L, cnt, smem + group_smem_bytes(kDirect, a.slots) / sizeof(int) + 32 * warp);
     }
     if (whole) __syncthreads();

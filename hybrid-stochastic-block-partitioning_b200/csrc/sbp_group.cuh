@@ -20,6 +20,13 @@
 
 namespace sbpb {
 
+// One batch of an asynchronous-Gibbs plan: its light vertices, by degree descending, and its
+// heavy ones; n32 / n16 of the light ones are too large for a group of 16 / 8 lanes.
+struct BatchDesc {
+  int light_begin, light_n, heavy_begin, heavy_n;
+  int n32, n16;
+};
+
 constexpr int kRegionSlots = 512;   // table slots of one warp, shared by its groups
 constexpr int kGroupWarps = 8;      // warps per CTA
 constexpr int kGroupThreads = 32 * kGroupWarps;
@@ -245,7 +252,8 @@ __device__ __forceinline__ bool accept_move(double dS, double fwd, double bwd, b
 // step are all in flight together: the classes of group_max_k give a group four neighbours a lane
 // at most (a vertex beyond the largest class takes several rounds).  Row r of the entries is
 // fetched before the walk, which does not depend on it.
-template <bool kDirect, Store ST>
+// kAnyB: hash tables with either walk, for a kernel that serves blockmodels of any size.
+template <bool kDirect, Store ST, bool kAnyB = false>
 __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const BlockView& bm, const GroupTab<kDirect>& T,
                                                     bool valid, int4 rec, bool given, uint4 x, const Lanes& L,
                                                     int* status, int* bins = nullptr) {
@@ -365,7 +373,8 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
         if (L.gbase == first) found = at;
       }
     } else {
-      found = kDirect ? walk_row<ST>(bm, t, in_col, tg, walk, L) : walk_tree<ST>(bm, t, in_col, tg, walk, L);
+      if (kDirect || (kAnyB && B <= kSmallB)) found = walk_row<ST>(bm, t, in_col, tg, walk, L);
+      else found = walk_tree<ST>(bm, t, in_col, tg, walk, L);
     }
     if (walk) {
       s = found;
@@ -530,5 +539,27 @@ __device__ __forceinline__ GroupEval group_evaluate(const GraphView& g, const Bl
 
 // Largest degree of the class of G lanes: four neighbours a lane, a quarter of its slots.
 __host__ __device__ constexpr int group_max_k(int G) { return 4 * G; }
+
+// Tasks of a batch: one warp each, 32 / G vertices of one class, the largest degrees first; with
+// groups of at least gmin lanes.
+struct GroupTask {
+  int lg;           // log2 of the vertices of the task
+  int first, end;   // its vertices from `first`, those below `end` of the batch's light (heavy) list
+};
+__host__ __device__ inline int group_tasks(const BatchDesc& b, int gmin) {
+  const int n = b.light_n;
+  const int c32 = gmin >= 32 ? n : b.n32, c16 = gmin >= 32 ? 0 : gmin >= 16 ? n - c32 : b.n16;
+  return c32 + ((c16 + 1) >> 1) + ((n - c32 - c16 + 3) >> 2);
+}
+__device__ __forceinline__ GroupTask group_task(const BatchDesc& b, int gmin, int task, bool light) {
+  const int n = b.light_n;
+  const int c32 = gmin >= 32 ? n : b.n32, c16 = gmin >= 32 ? 0 : gmin >= 16 ? n - c32 : b.n16;
+  const int t16 = (c16 + 1) >> 1;
+  GroupTask k;
+  k.lg = !light || task < c32 ? 0 : task < c32 + t16 ? 1 : 2;
+  k.first = k.lg == 0 ? task : k.lg == 1 ? c32 + 2 * (task - c32) : c32 + c16 + 4 * (task - c32 - t16);
+  k.end = !light ? b.heavy_n : k.lg == 0 ? c32 : k.lg == 1 ? c32 + c16 : n;
+  return k;
+}
 
 }  // namespace sbpb

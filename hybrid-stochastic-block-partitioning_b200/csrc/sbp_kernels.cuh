@@ -7,12 +7,6 @@ namespace sbpb {
 constexpr int kProposalsPerBlock = 10;   // block_merge::NUM_AGG_PROPOSALS_PER_BLOCK (include/block_merge.hpp:24)
 constexpr int kMaxIterations = 100;      // finetune::MAX_NUM_ITERATIONS (include/finetune.hpp:56)
 
-// One batch of an asynchronous-Gibbs plan: its light vertices, by degree descending, and its
-// heavy ones; n32 / n16 of the light ones are too large for a group of 16 / 8 lanes.
-struct BatchDesc {
-  int light_begin, light_n, heavy_begin, heavy_n;
-  int n32, n16;
-};
 // Polls of a persistent kernel's grid barrier before it gives up (about 0.7 us each).
 constexpr unsigned kGridWaitLimit = 1u << 23;
 // What a whole finetune call in one kernel reports.
