@@ -104,43 +104,36 @@ struct SortScratch {
 };
 static thread_local SortScratch g_sort;   // per host thread (the batched partitioner merges on several)
 
-// 0..n-1 ordered by key ascending, equal keys by index: the order of std::stable_sort on the
-// indices with `key[a] < key[b]`, from an LSD radix sort (16-bit digits) of order-preserving
-// 64-bit images of the keys (-0.0 taken as +0.0, which compares equal).  With a NaN key (no
-// strict weak order) it is std::stable_sort itself.  A 200,000-key sort takes a few ms instead
-// of about 20.
+// 0..n-1 ordered by merge score ascending, equal scores by index: the order of std::stable_sort on
+// the indices with `key[a] < key[b]`.  Scores are multiples of 2^-20 (merge_score), so as long as
+// they all fit, their 32-bit integer images sort the same: an LSD radix sort of two 16-bit
+// digits.  (Four digits of the doubles' images took 4.1 ms for 200,000 blocks.)
 static std::vector<int> stable_order_by(const std::vector<double>& key) {
   const size_t n = key.size();
   std::vector<int> order(n);
   std::iota(order.begin(), order.end(), 0);
-  std::vector<unsigned long long> img(n);
+  std::vector<uint32_t> img(n);
+  std::vector<unsigned> count(1u << 17, 0u);   // both digits' counts
   for (size_t i = 0; i < n; ++i) {
-    double x = key[i];
-    if (std::isnan(x)) {
+    const double x = key[i] * 1048576.0;
+    if (!(std::fabs(x) < 2147483648.0) || x != std::nearbyint(x)) {   // out of range, or not such a multiple (NaN too)
       std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key[a] < key[b]; });
       return order;
     }
-    if (x == 0.0) x = 0.0;
-    unsigned long long bits;
-    std::memcpy(&bits, &x, sizeof bits);
-    img[i] = (bits >> 63) ? ~bits : (bits | (1ull << 63));
+    img[i] = (uint32_t)(int32_t)x ^ 0x80000000u;
+    count[img[i] & 0xffffu]++;
+    count[(1u << 16) + (img[i] >> 16)]++;
   }
   std::vector<int> tmp(n);
-  std::vector<unsigned> count(1u << 16);
-  for (int shift = 0; shift < 64; shift += 16) {
-    std::fill(count.begin(), count.end(), 0u);
-    for (size_t i = 0; i < n; ++i) count[(img[i] >> shift) & 0xffff]++;
-    if (n > 0 && count[(img[0] >> shift) & 0xffff] == n) continue;   // one digit value: order unchanged
+  for (int d = 0; d < 2; ++d) {
+    unsigned* c = count.data() + ((size_t)d << 16);
     unsigned run = 0;
-    for (auto& c : count) {
-      const unsigned k = c;
-      c = run;
+    for (size_t i = 0; i < (1u << 16); ++i) {
+      const unsigned k = c[i];
+      c[i] = run;
       run += k;
     }
-    for (size_t i = 0; i < n; ++i) {
-      const int o = order[i];
-      tmp[count[(img[o] >> shift) & 0xffff]++] = o;
-    }
+    for (int o : order) tmp[c[(img[o] >> (16 * d)) & 0xffffu]++] = o;
     order.swap(tmp);
   }
   return order;
@@ -579,22 +572,23 @@ struct MergeScratch {
 
 // block_map of the reference's carry-out loops: block_map[x] is the current name of x's group,
 // and merging `from` into `to` renames every entry equal to `from` (src/blockmodel/blockmodel.cpp:
-// 61-66).  Member lists make a rename cost the size of the renamed group instead of O(B).
+// 61-66).  A group's blocks are a linked list through `next`, so a rename costs the size of the
+// renamed group instead of O(B), and the map is four arrays (a vector per block took 14 of the
+// 50 ms of a merge of 200,000 blocks, and 4 more to free).
 struct GroupMap {
-  std::vector<int> name;                    // block -> group name
-  std::vector<std::vector<int>> members;    // group name -> blocks carrying it
-  explicit GroupMap(int B) : name(B), members(B) {
-    for (int i = 0; i < B; ++i) {
-      name[i] = i;
-      members[i].push_back(i);
-    }
+  std::vector<int> name;               // block -> group name
+  std::vector<int> head, tail, next;   // group name -> first and last block; block -> next of its group
+  explicit GroupMap(int B) : name(B), head(B), tail(B), next(B, -1) {
+    std::iota(name.begin(), name.end(), 0);
+    head = tail = name;
   }
   void rename(int from, int to) {
-    auto& src = members[from];
-    auto& dst = members[to];
-    for (int x : src) name[x] = to;
-    dst.insert(dst.end(), src.begin(), src.end());
-    std::vector<int>().swap(src);
+    if (from == to || head[from] < 0) return;
+    for (int x = head[from]; x >= 0; x = next[x]) name[x] = to;
+    if (head[to] < 0) head[to] = head[from];
+    else next[tail[to]] = head[from];
+    tail[to] = tail[from];
+    head[from] = tail[from] = -1;
   }
 };
 
@@ -842,15 +836,16 @@ Snapshot snapshot(SbpBlockmodel& bm) {
   x.empty = false;
   x.B = bm.B;
   x.entropy = bm.overall_entropy;
-  x.b.resize(bm.V);
-  SBP_CUDA(SBP_COPY_ASYNC(x.b.data(), bm.b.p, bm.V * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  auto b = std::make_shared<std::vector<int>>(bm.V);
+  SBP_CUDA(SBP_COPY_ASYNC(b->data(), bm.b.p, bm.V * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
   c.sync();
+  x.b = std::move(b);
   return x;
 }
 
 void restore(SbpBlockmodel& bm, SbpGraph& g, const Snapshot& x) {
   Context& c = Context::get();
-  SBP_CUDA(SBP_COPY_ASYNC(bm.b.p, x.b.data(), bm.V * sizeof(int), cudaMemcpyHostToDevice, c.stream));
+  SBP_CUDA(SBP_COPY_ASYNC(bm.b.p, x.b->data(), bm.V * sizeof(int), cudaMemcpyHostToDevice, c.stream));
   bm.set_blocks(x.B);
   bm.overall_entropy = x.entropy;
   rebuild(bm, g);
@@ -933,9 +928,7 @@ void partition_begin(PartitionState& ps, SbpGraph& g) {
   std::memset(&ps.st, 0, sizeof ps.st);
   SbpBlockmodel& bm = ps.bm;
   bm.init_vertex_scratch(g.V);
-  std::vector<int> ident(g.V);
-  std::iota(ident.begin(), ident.end(), 0);
-  SBP_CUDA(SBP_COPY_ASYNC(bm.b.p, ident.data(), g.V * sizeof(int), cudaMemcpyHostToDevice, c.stream));
+  SBP_CUDA(SBP_COPY_ASYNC(bm.b.p, g.identity.p, g.V * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   bm.set_blocks(g.V);
   bm.num_blocks_to_merge = (int)(g.V * 0.5f);
   rebuild(bm, g);
@@ -974,9 +967,10 @@ void partition_finish_round(PartitionState& ps, SbpGraph& g, const SbpStats& fs,
   ++ps.call;
   st.outer_iterations++;
   int to_merge = 0;
-  const Snapshot nxt = ps.t.next(snapshot(ps.bm), &to_merge);
+  const Snapshot now = snapshot(ps.bm);
+  const Snapshot nxt = ps.t.next(now, &to_merge);
   if (ps.t.optimal) {
-    std::memcpy(out, nxt.b.data(), g.V * sizeof(int));
+    std::memcpy(out, nxt.b->data(), g.V * sizeof(int));
     st.mdl = nxt.entropy;
     st.num_blocks = nxt.B;
     ps.done = true;
@@ -986,7 +980,15 @@ void partition_finish_round(PartitionState& ps, SbpGraph& g, const SbpStats& fs,
     }
     return;
   }
-  restore(ps.bm, g, nxt);
+  // The search goes on from the state at hand: its dense counts stand, d starts afresh.  (Row-hashed
+  // storage is laid out anew: its rows have filled up with cells that are zero again.)
+  if (nxt.b == now.b && !ps.bm.sparse) {
+    Context& c = Context::get();
+    k_rebuild_degrees<<<grid_for(ps.bm.B, 256, 1 << 20), 256, 0, c.stream>>>(ps.bm.view());
+    SBP_CHECK_LAUNCH();
+  } else {
+    restore(ps.bm, g, nxt);
+  }
   ps.bm.num_blocks_to_merge = to_merge;
 }
 

@@ -664,13 +664,14 @@ struct SbpBlockmodel {
     // dense only while it takes at most 60 % of the free device memory; cudaMemGetInfo can
     // stall the host for tens of milliseconds, so it is asked only for a matrix above 5 % of
     // the device's memory
-    if (!sparse && dense_bytes > 0.05 * (double)device_memory_bytes()) {
+    const double held = (double)P.n * sizeof(int2) + (double)DeviceCache::get().cached_bytes();
+    if (!sparse && dense_bytes > 0.05 * (double)device_memory_bytes() &&
+        dense_bytes > 0.01 * g_dense_max_memory_pct * held) {   // else dense whatever else is free
       size_t free_b = 0, total_b = 0;
       if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
         // buffers this blockmodel already holds, and those the device cache keeps for reuse,
         // count as free
-        const size_t have = P.n * sizeof(int2) + DeviceCache::get().cached_bytes();
-        if (dense_bytes > 0.01 * g_dense_max_memory_pct * (double)(free_b + have)) sparse = true;
+        if (dense_bytes > 0.01 * g_dense_max_memory_pct * ((double)free_b + held)) sparse = true;
       } else {
         cudaGetLastError();
       }
@@ -767,7 +768,7 @@ struct ReplayDev {
 // ------------------------------------------------------------------------------------------
 struct Snapshot {
   bool empty = true;
-  std::vector<int> b;
+  std::shared_ptr<const std::vector<int>> b;   // never changed once taken: snapshots of a state share it
   int B = 0;
   float entropy = 0.f;
 };
