@@ -78,25 +78,33 @@ __device__ __forceinline__ void slot_features(int co, int ci, float kf, long lon
   f[3] = is_cur ? 1.f : 0.f;
 }
 
+__device__ __forceinline__ float own_block_share(int c_cur, float kf) { return (float)c_cur / kf; }
+
 __device__ __forceinline__ void global_features(int k_out, int k_in, int B, int nvalid, int c_cur, float kf, int self,
                                                 long long dtot_cur, float inv, float* f) {
   f[0] = log1pf((float)k_out) / 5.f;
   f[1] = log1pf((float)k_in) / 5.f;
   f[2] = logf((float)B) / 10.f;
   f[3] = (float)nvalid / 14.f;
-  f[4] = (float)c_cur / kf;
+  f[4] = own_block_share(c_cur, kf);
   f[5] = self ? 1.f : 0.f;
   f[6] = feat_degree(dtot_cur, inv);
   f[7] = 1.f;
 }
 
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long y = __shfl_xor_sync(kFull, x, o);
-    x = y > x ? y : x;
+// This lane's best candidate below `prev`: (edge count, block id descending) of its table entries
+// i = lane, lane + 32, ... with a nonzero count; 0: none.
+__device__ __forceinline__ unsigned long long lane_candidate(const WarpTable& t, int n, int lane,
+                                                             unsigned long long prev) {
+  unsigned long long best = 0ull;
+  for (int i = lane; i < n; i += kWarp) {
+    const int h = t.list[i];
+    const int c = t.cout[h] + t.cin[h];
+    if (c <= 0) continue;
+    const unsigned long long P = ((unsigned long long)(unsigned)c << 32) | (0xFFFFFFFFu - (unsigned)t.keys[h]);
+    if (P < prev && P > best) best = P;
   }
-  return x;
+  return best;
 }
 
 // Features of v against the current state, written as one BF16 row; the candidate slots
@@ -110,22 +118,18 @@ __device__ __forceinline__ void vertex_features(const BlockView& bm, const WarpT
   const int k = k_out + k_in;
   const float kf = (float)(k > 0 ? k : 1);
   // top-14 (count desc, block asc) among entries with a nonzero count (the self loop's block
-  // enters the table with zero counts and never becomes a candidate)
-  unsigned long long mine = 0ull, prev = ~0ull;
+  // enters the table with zero counts and never becomes a candidate).  Every lane holds the best
+  // of its own entries, a slot is two warp maxima (count, then block), and only the lane that
+  // gave it looks at its entries again.
+  unsigned long long mine = 0ull, best = lane_candidate(t, n, lane, ~0ull);
   int nvalid = 0;
   for (int j = 0; j < kFeatSlots; ++j) {
-    unsigned long long best = 0ull;
-    for (int i = lane; i < n; i += kWarp) {
-      const int h = t.list[i];
-      const int c = t.cout[h] + t.cin[h];
-      if (c <= 0) continue;
-      const unsigned long long P = ((unsigned long long)(unsigned)c << 32) | (0xFFFFFFFFu - (unsigned)t.keys[h]);
-      if (P < prev && P > best) best = P;
-    }
-    best = warp_max_u64(best);
-    if (best == 0ull) break;
-    if (lane == j) mine = best;
-    prev = best;
+    const unsigned hi = __reduce_max_sync(kFull, (unsigned)(best >> 32));
+    if (hi == 0u) break;
+    const unsigned lo = __reduce_max_sync(kFull, (unsigned)(best >> 32) == hi ? (unsigned)best : 0u);
+    const unsigned long long top = ((unsigned long long)hi << 32) | lo;
+    if (lane == j) mine = top;
+    if (best == top) best = n > kWarp ? lane_candidate(t, n, lane, top) : 0ull;
     nvalid = j + 1;
   }
   int u = -1, co = 0, ci = 0;
@@ -204,83 +208,141 @@ __global__ void k_learn_features(GraphView g, BlockView bm, const int* __restric
   }
 }
 
-// q(target | logits) of the mixture; slot = candidate slot of the target block or -1.
-__device__ __forceinline__ double learned_q(const float* L, int nvalid, int slot, float eps, int B) {
-  float mx = L[kMlpEscape];
-  for (int j = 0; j < nvalid; ++j) mx = fmaxf(mx, L[j]);
-  double S = exp((double)(L[kMlpEscape] - mx));
-  for (int j = 0; j < nvalid; ++j) S += exp((double)(L[j] - mx));
-  const double esc = exp((double)(L[kMlpEscape] - mx)) / S;
+// The mixture over one row's logits, by a group of 16 lanes (half a warp): lane j holds slot j's
+// exponential, lane 14 the escape's.  The FP64 exponentials and divisions run side by side; the
+// sum is added in the order escape, slot 0, 1, ... by every lane, so q has the bits of the serial
+// form.  (One thread a row took 29 us for a batch of 2,000 vertices of the 20,000-vertex graph,
+// 30 exponentials one after the other.)
+constexpr int kRowLanes = 16;
+struct SlotMix {
+  double e;   // exp(logit - max) of this lane's slot, 0 beyond nvalid
+  double p;   // (1 - eps) pi of this lane's slot
+  double esc_q;   // probability of a block that is no slot
+};
+
+__device__ __forceinline__ double lane16(double x, int src) { return __shfl_sync(kFull, x, src, kRowLanes); }
+
+__device__ __forceinline__ SlotMix slot_mix(float L, int nvalid, float eps, int B, int j) {
+  const bool on = j < nvalid || j == kMlpEscape;
+  float mx = on ? L : -INFINITY;
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+  SlotMix m;
+  m.e = on ? exp((double)(L - mx)) : 0.0;
+  double S = lane16(m.e, kMlpEscape);
+#pragma unroll
+  for (int q = 0; q < kFeatSlots; ++q) S += lane16(m.e, q);   // slots beyond nvalid add 0
   const double w = 1.0 - (double)eps;
-  double q = (w * esc + (double)eps) / (double)B;
-  if (slot >= 0) q += w * exp((double)(L[slot] - mx)) / S;
-  return q;
+  m.p = w * m.e / S;
+  const double esc = lane16(m.e, kMlpEscape) / S;
+  m.esc_q = (w * esc + (double)eps) / (double)B;
+  return m;
+}
+
+// q of a block: its slot (or -1), the same for the 16 lanes.
+__device__ __forceinline__ double mix_q(const SlotMix& m, int slot) {
+  const double p = lane16(m.p, slot >= 0 ? slot : 0);
+  return slot >= 0 ? m.esc_q + p : m.esc_q;
+}
+
+// The slot of block `target` among the 16 lanes' slots (blk of lane j, j < nvalid), or -1.
+__device__ __forceinline__ int find_slot(int blk, int target, int nvalid, int j) {
+  const unsigned half = (__ballot_sync(kFull, j < nvalid && blk == target) >> (threadIdx.x & 16)) & 0xffffu;
+  return half ? __ffs(half) - 1 : -1;
 }
 
 // Draw s for vertex v (row i) from the forward logits, store q(s), and build the reverse-state
-// features.  One thread.
-__device__ __forceinline__ void propose_row(int i, int v, const BlockView& bm, BatchBufs bb, LearnedParams lp,
-                                            const RngParams& rng, int sweep, long long V, int* status) {
-  const uint4 x = draw_record(rng, (uint32_t)v, (uint32_t)sweep, 0u, (long long)sweep * V + v, status);
-  const int4 inf = bb.info[i];
+// features.  16 lanes a row (both halves of the warp call; `live` 0: the half has no row).
+__device__ __forceinline__ void propose_row(int i, int v, bool live, const BlockView& bm, BatchBufs bb,
+                                            LearnedParams lp, const RngParams& rng, int sweep, long long V,
+                                            int* status) {
+  const int j = threadIdx.x & (kRowLanes - 1);
+  uint4 x = make_uint4(0, 0, 0, 0);
+  int4 inf = make_int4(0, 0, 0, 0);
+  float L = 0.f;
+  int2 sl = make_int2(-1, 0);
+  uint2 f = make_uint2(0, 0);
+  if (live) {
+    x = draw_record(rng, (uint32_t)v, (uint32_t)sweep, 0u, (long long)sweep * V + v, status);
+    inf = bb.info[i];
+    L = bb.L1[(size_t)i * kMlpOut + j];
+    if (j < kFeatSlots) sl = bb.slot[(size_t)i * kFeatSlots + j];
+    f = *reinterpret_cast<const uint2*>(bb.F1 + (size_t)i * kMlpIn + 4 * j);
+  }
   const int r = inf.x, k_out = inf.y, k_in = inf.z, self = inf.w & 1, nvalid = inf.w >> 1;
   const int B = bm.B;
-  const float* L = bb.L1 + (size_t)i * kMlpOut;
-  const int2* sl = bb.slot + (size_t)i * kFeatSlots;
+  const SlotMix m = slot_mix(L, nvalid, lp.eps, B, j);
   // categorical draw over the slots and the escape
-  float mx = L[kMlpEscape];
-  for (int j = 0; j < nvalid; ++j) mx = fmaxf(mx, L[j]);
-  double S = exp((double)(L[kMlpEscape] - mx));
-  for (int j = 0; j < nvalid; ++j) S += exp((double)(L[j] - mx));
-  const double w = 1.0 - (double)lp.eps;
   const double u = (double)x.x * 0x1p-32;
   double acc = 0.0;
   int pick = -1;
-  for (int j = 0; j < nvalid; ++j) {
-    acc += w * exp((double)(L[j] - mx)) / S;
-    if (u < acc) {
-      pick = j;
-      break;
-    }
+#pragma unroll
+  for (int q = 0; q < kFeatSlots; ++q) {
+    acc += lane16(m.p, q);
+    if (pick < 0 && q < nvalid && u < acc) pick = q;
   }
-  const int s = pick >= 0 ? sl[pick].x : (int)scale32(x.y, (long long)B);
-  bb.s_prop[i] = s;
+  const int blk = __shfl_sync(kFull, sl.x, pick >= 0 ? pick : 0, kRowLanes);
+  const int s = pick >= 0 ? blk : (int)scale32(x.y, (long long)B);
+  const int slot_s = find_slot(sl.x, s, nvalid, j);
+  const double q = mix_q(m, slot_s);
+  const int cnt = __shfl_sync(kFull, sl.y, slot_s >= 0 ? slot_s : 0, kRowLanes);
+  if (!live) return;
+  if (j == 0) bb.s_prop[i] = s;
   if (s == r) return;
-  int slot_s = -1;
-  for (int j = 0; j < nvalid; ++j)
-    if (sl[j].x == s) slot_s = j;
-  bb.qf[i] = learned_q(L, nvalid, slot_s, lp.eps, B);
-  // reverse state: v in s; dtot of r and s change by k_out + k_in + self
-  const int k = k_out + k_in;
-  const float kf = (float)(k > 0 ? k : 1);
+  if (j == 0) bb.qf[i] = q;
+  // reverse state: v in s; dtot of r and s change by k_out + k_in + self.  Lane j holds features
+  // 4j .. 4j + 3: its slot's, lane 14 56..59, lane 15 60..63.
   const long long mv = (long long)k_out + k_in + self;
   const long long dt_r = (long long)bm.d_out[r] + bm.d_in[r] - mv;
   const long long dt_s = (long long)bm.d_out[s] + bm.d_in[s] + mv;
-  const __nv_bfloat16* f1 = bb.F1 + (size_t)i * kMlpIn;
-  __nv_bfloat16* f2 = bb.F2 + (size_t)i * kMlpIn;
-  for (int q = 0; q < kMlpIn; ++q) f2[q] = f1[q];
-  for (int j = 0; j < nvalid; ++j) {
-    const int uj = sl[j].x;
-    if (uj != r && uj != s) continue;
-    f2[4 * j + 2] = __float2bfloat16_rn(feat_degree(uj == r ? dt_r : dt_s, lp.inv_log2E));
-    f2[4 * j + 3] = __float2bfloat16_rn(uj == s ? 1.f : 0.f);
+  __nv_bfloat162 lo = *reinterpret_cast<__nv_bfloat162*>(&f.x), hi = *reinterpret_cast<__nv_bfloat162*>(&f.y);
+  if (j < nvalid && (sl.x == r || sl.x == s)) {
+    hi.x = __float2bfloat16_rn(feat_degree(sl.x == r ? dt_r : dt_s, lp.inv_log2E));
+    hi.y = __float2bfloat16_rn(sl.x == s ? 1.f : 0.f);
+  } else if (j == kRowLanes - 1) {
+    const int k = k_out + k_in;
+    lo.x = __float2bfloat16_rn(own_block_share(slot_s >= 0 ? cnt : 0, (float)(k > 0 ? k : 1)));
+    hi.x = __float2bfloat16_rn(feat_degree(dt_s, lp.inv_log2E));
   }
-  float g[8];
-  const int c_s = slot_s >= 0 ? sl[slot_s].y : 0;
-  global_features(k_out, k_in, B, nvalid, c_s, kf, self, dt_s, lp.inv_log2E, g);
-  f2[56 + 4] = __float2bfloat16_rn(g[4]);
-  f2[56 + 6] = __float2bfloat16_rn(g[6]);
+  f.x = *reinterpret_cast<const unsigned*>(&lo);
+  f.y = *reinterpret_cast<const unsigned*>(&hi);
+  *reinterpret_cast<uint2*>(bb.F2 + (size_t)i * kMlpIn + 4 * j) = f;
 }
 
 // Draw s from the forward logits, store q(s), and build the reverse-state features.
 __global__ void k_learn_propose(const int* __restrict__ verts, int n, BlockView bm, BatchBufs bb, LearnedParams lp,
                                 RngParams rng, int sweep, long long V, int* status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  propose_row(i, verts[i], bm, bb, lp, rng, sweep, V, status);
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kRowLanes;
+  propose_row(i, i < n ? verts[i] : 0, i < n, bm, bb, lp, rng, sweep, V, status);
 }
 
-// Delta-MDL of the drawn move, the exact Hastings factor from the reverse logits, accept.
+// Delta-MDL of the drawn move r -> s of vertex v (row `row` of the batch buffers), the exact
+// Hastings factor from the reverse logits, accept.  One warp; the table is left filled.  The
+// logits' load and their FP64 exponentials (one a lane) run while the neighbour blocks' cells are
+// on their way.
+template <Store ST>
+__device__ __forceinline__ int learned_accept(const GraphView& g, const BlockView& bm, int v, int row, int r, int s,
+                                              int k_out, int k_in, int self, int nvalid, int o0, int i0,
+                                              const BatchBufs& bb, LearnedParams lp, const RngParams& rng, int sweep,
+                                              const WarpTable& t, int lane, int* status, double* dS, double* H) {
+  const int j = lane & (kRowLanes - 1);
+  const float L = bb.L2[(size_t)row * kMlpOut + j];
+  const int blk = j < nvalid ? bb.slot[(size_t)row * kFeatSlots + j].x : -1;
+  const double qf = bb.qf[row];
+  const uint4 x = draw_record(rng, (uint32_t)v, (uint32_t)sweep, 0u, (long long)sweep * g.V + v, status);
+  gather_neighbour_blocks(g, bm, v, r, o0, k_out, i0, k_out + k_in, self, -1, t, lane, status);
+  NbPrefetch pre;
+  prefetch_nb<ST>(bm, r, t, lane, &pre);
+  const double qr = mix_q(slot_mix(L, nvalid, lp.eps, bm.B, j), find_slot(blk, r, nvalid, j));
+  double Hp;
+  *dS = move_delta<ST>(g, bm, r, s, k_out, k_in, self, t, lane, &Hp, &pre);
+  *H = qr / qf;
+  double ap = exp(-3.0 * *dS) * *H;
+  ap = ap >= 1.0 ? 1.0 : ap;
+  return (u53(x.z, x.w) <= ap) ? 1 : 0;
+}
+
+template <Store ST>
 __global__ void k_learn_eval(GraphView g, BlockView bm, const int* __restrict__ verts, int n, int row0,
                              BatchBufs bb, LearnedParams lp, RngParams rng, int sweep, int* prop, int* moved_list,
                              int* n_moved, unsigned long long* counters, double* out_dS, double* out_H, int cap,
@@ -290,30 +352,22 @@ __global__ void k_learn_eval(GraphView g, BlockView bm, const int* __restrict__ 
   const int wpb = blockDim.x >> 5;
   WarpTable t = carve_table(smem, cap, warp);
   init_table(t, lane);
-  unsigned long long c_visit = 0, c_moved = 0, c_acc = 0;
+  // one set of counters a CTA (three atomics a warp on the same words cost 2 us of a batch)
+  __shared__ int s_count[2];
+  if (threadIdx.x < 2) s_count[threadIdx.x] = 0;
+  __syncthreads();
+  int c_moved = 0, c_acc = 0;
   for (int i = blockIdx.x * wpb + warp; i < n; i += gridDim.x * wpb) {
     const int row = row0 + i;
     const int v = verts[i];
-    c_visit++;
     const int4 inf = bb.info[row];
     const int r = inf.x, k_out = inf.y, k_in = inf.z, self = inf.w & 1, nvalid = inf.w >> 1;
     const int s = bb.s_prop[row];
     if (s == r) continue;
     c_moved++;
-    const uint4 x = draw_record(rng, (uint32_t)v, (uint32_t)sweep, 0u, (long long)sweep * g.V + v, status);
-    const int o0 = g.out_ptr[v], i0 = g.in_ptr[v];
-    gather_neighbour_blocks(g, bm, v, r, o0, k_out, i0, k_out + k_in, self, -1, t, lane, status);
-    double Hp;
-    const double dS = move_delta(g, bm, r, s, k_out, k_in, self, t, lane, &Hp);
-    int slot_r = -1;
-    const int2* sl = bb.slot + (size_t)row * kFeatSlots;
-    for (int j = 0; j < nvalid; ++j)
-      if (sl[j].x == r) slot_r = j;
-    const double qr = learned_q(bb.L2 + (size_t)row * kMlpOut, nvalid, slot_r, lp.eps, bm.B);
-    const double H = qr / bb.qf[row];
-    double ap = exp(-3.0 * dS) * H;
-    ap = ap >= 1.0 ? 1.0 : ap;
-    const int accepted = (u53(x.z, x.w) <= ap) ? 1 : 0;
+    double dS, H;
+    const int accepted = learned_accept<ST>(g, bm, v, row, r, s, k_out, k_in, self, nvalid, g.out_ptr[v],
+                                            g.in_ptr[v], bb, lp, rng, sweep, t, lane, status, &dS, &H);
     if (lane == 0) {
       if (out_dS) out_dS[row] = dS;
       if (out_H) out_H[row] = H;
@@ -325,10 +379,15 @@ __global__ void k_learn_eval(GraphView g, BlockView bm, const int* __restrict__ 
     c_acc += accepted;
     table_reset(t, lane);
   }
-  if (lane == 0 && c_visit) {
-    atomicAdd(counters + 0, c_visit);
-    atomicAdd(counters + 1, c_moved);
-    atomicAdd(counters + 2, c_acc);
+  if (lane == 0 && c_moved) {
+    atomicAdd(s_count + 0, c_moved);
+    atomicAdd(s_count + 1, c_acc);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (blockIdx.x == 0) atomicAdd(counters + 0, (unsigned long long)n);
+    if (s_count[0]) atomicAdd(counters + 1, (unsigned long long)s_count[0]);
+    if (s_count[1]) atomicAdd(counters + 2, (unsigned long long)s_count[1]);
   }
 }
 
@@ -371,10 +430,10 @@ __global__ void k_learn_mh_features(GraphView g, BlockView bm, const int* __rest
 __global__ void k_learn_mh_propose(const int* __restrict__ verts, int n, const int* __restrict__ pos_ptr, int W,
                                    BlockView bm, BatchBufs bb, LearnedParams lp, RngParams rng, int sweep,
                                    long long V, int* status) {
-  const int w = threadIdx.x;
+  const int w = threadIdx.x / kRowLanes;
   const int i = *pos_ptr + w;
-  if (w >= W || i >= n) return;
-  propose_row(w, verts[i], bm, bb, lp, rng, sweep, V, status);
+  const bool live = w < W && i < n;
+  propose_row(w, live ? verts[i] : 0, live, bm, bb, lp, rng, sweep, V, status);
 }
 
 __global__ void __launch_bounds__(kMhRoundMaxWarps * 32)
@@ -403,21 +462,13 @@ __global__ void __launch_bounds__(kMhRoundMaxWarps * 32)
     k_in = inf.z;
     const int self = inf.w & 1, nvalid = inf.w >> 1;
     s = bb.s_prop[warp];
-    gather_neighbour_blocks(g, bm, v, r, g.out_ptr[v], k_out, g.in_ptr[v], k_out + k_in, self, -1, t, lane, status);
-    if (s != r) {
-      const uint4 x = draw_record(rng, (uint32_t)v, (uint32_t)sweep, 0u, (long long)sweep * g.V + v, status);
-      double Hp;
-      dS = move_delta(g, bm, r, s, k_out, k_in, self, t, lane, &Hp);
-      int slot_r = -1;
-      const int2* sl = bb.slot + (size_t)warp * kFeatSlots;
-      for (int j = 0; j < nvalid; ++j)
-        if (sl[j].x == r) slot_r = j;
-      const double qr = learned_q(bb.L2 + (size_t)warp * kMlpOut, nvalid, slot_r, lp.eps, bm.B);
-      const double H = qr / bb.qf[warp];
-      double ap = exp(-3.0 * dS) * H;
-      ap = ap >= 1.0 ? 1.0 : ap;
-      acc = (u53(x.z, x.w) <= ap) ? 1 : 0;
-    }
+    const int o0 = g.out_ptr[v], i0 = g.in_ptr[v];
+    double H;
+    if (s != r)
+      acc = learned_accept<Store::kAny>(g, bm, v, warp, r, s, k_out, k_in, self, nvalid, o0, i0, bb, lp, rng, sweep, t, lane,
+                           status, &dS, &H);
+    else   // the commit rule reads the table of every window vertex
+      gather_neighbour_blocks(g, bm, v, r, o0, k_out, i0, k_out + k_in, self, -1, t, lane, status);
   }
   if (lane == 0) {
     s_acc[warp] = acc;
@@ -493,14 +544,14 @@ __global__ void k_learn_collect(GraphView g, BlockView bm, const int* __restrict
 
 // q(target | v, state) of the forward path for given target blocks.
 __global__ void k_learn_q(const int* __restrict__ targets, int n, BatchBufs bb, LearnedParams lp, int B, double* q) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int nvalid = bb.info[i].w >> 1;
-  const int2* sl = bb.slot + (size_t)i * kFeatSlots;
-  int slot = -1;
-  for (int j = 0; j < nvalid; ++j)
-    if (sl[j].x == targets[i]) slot = j;
-  q[i] = learned_q(bb.L1 + (size_t)i * kMlpOut, nvalid, slot, lp.eps, B);
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / kRowLanes, j = threadIdx.x & (kRowLanes - 1);
+  const bool live = i < n;
+  const int nvalid = live ? bb.info[i].w >> 1 : 0;
+  const float L = live ? bb.L1[(size_t)i * kMlpOut + j] : 0.f;
+  const int blk = j < nvalid ? bb.slot[(size_t)i * kFeatSlots + j].x : -1;
+  const int slot = find_slot(blk, live ? targets[i] : -1, nvalid, j);
+  const double x = mix_q(slot_mix(L, nvalid, lp.eps, B, j), slot);
+  if (live && j == 0) q[i] = x;
 }
 
 __global__ void k_gather_rows(const __nv_bfloat16* __restrict__ X, const int* __restrict__ target,
@@ -616,7 +667,8 @@ static MhResult learned_mh_pass(SbpBlockmodel& bm, const SbpGraph& g, const int*
       SBP_CHECK_LAUNCH();
       mlp_forward(bb.F1, W, mlp.weights(), bb.L1, c.status, c.num_sms, c.stream);
       SBP_CHECK_LAUNCH();
-      k_learn_mh_propose<<<1, 32, 0, c.stream>>>(verts, n, pos, W, bm.view(), bb, lp, rng, sweep, g.V, c.status);
+      k_learn_mh_propose<<<1, kMhRoundMaxWarps * kRowLanes, 0, c.stream>>>(verts, n, pos, W, bm.view(), bb, lp, rng,
+                                                                           sweep, g.V, c.status);
       SBP_CHECK_LAUNCH();
       mlp_forward(bb.F2, W, mlp.weights(), bb.L2, c.status, c.num_sms, c.stream);
       SBP_CHECK_LAUNCH();
@@ -669,18 +721,19 @@ static void learned_batch(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan&
                  c.status);
   mlp_forward(bb.F1, n, mlp.weights(), bb.L1, c.status, c.num_sms, c.stream);
   SBP_CHECK_LAUNCH();
-  k_learn_propose<<<grid_for(n, 128, 1 << 20), 128, 0, c.stream>>>(verts, n, bm.view(), bb, lp, rng, sweep, g.V,
-                                                                    c.status);
+  k_learn_propose<<<grid_for(n, 128 / kRowLanes, 1 << 28), 128, 0, c.stream>>>(verts, n, bm.view(), bb, lp, rng,
+                                                                                sweep, g.V, c.status);
   SBP_CHECK_LAUNCH();
   mlp_forward(bb.F2, n, mlp.weights(), bb.L2, c.status, c.num_sms, c.stream);
   SBP_CHECK_LAUNCH();
   int* n_cur = bm.n_moved.p + (bm.gen & 1);
   double* no_out = nullptr;
+  const auto eval = bm.sparse ? k_learn_eval<Store::kHashed> : k_learn_eval<Store::kDenseFrozen>;
   if (nl > 0)
-    launch_warps(k_learn_eval, nl, g.light_cap, kLightWarps, g.view(), bm.view(), verts, nl, 0, bb, lp, rng, sweep,
+    launch_warps(eval, nl, g.light_cap, kLightWarps, g.view(), bm.view(), verts, nl, 0, bb, lp, rng, sweep,
                  bm.prop.p, bm.moved.p, n_cur, c.counters, no_out, no_out, g.light_cap, c.status);
   if (nh > 0)
-    launch_warps(k_learn_eval, nh, g.heavy_cap, 1, g.view(), bm.view(), verts + nl, nh, nl, bb, lp, rng, sweep,
+    launch_warps(eval, nh, g.heavy_cap, 1, g.view(), bm.view(), verts + nl, nh, nl, bb, lp, rng, sweep,
                  bm.prop.p, bm.moved.p, n_cur, c.counters, no_out, no_out, g.heavy_cap, c.status);
   gibbs_apply(bm, g, n);
 }
@@ -1164,13 +1217,14 @@ SbpStatus sbp_learned_evaluate(const SbpBlockmodel* cbm, const SbpGraph* g, cons
   launch_warps(k_learn_features, n, cap, 1, g->view(), bm->view(), verts.p, n, 0, bb, lp, cap, c.status);
   mlp_forward(bb.F1, n, m->weights(), bb.L1, c.status, c.num_sms, c.stream);
   SBP_CHECK_LAUNCH();
-  k_learn_propose<<<grid_for(n, 128, 1 << 20), 128, 0, c.stream>>>(verts.p, n, bm->view(), bb, lp, rng, 0, g->V,
-                                                                    c.status);
+  k_learn_propose<<<grid_for(n, 128 / kRowLanes, 1 << 28), 128, 0, c.stream>>>(verts.p, n, bm->view(), bb, lp,
+                                                                                rng, 0, g->V, c.status);
   SBP_CHECK_LAUNCH();
   mlp_forward(bb.F2, n, m->weights(), bb.L2, c.status, c.num_sms, c.stream);
   SBP_CHECK_LAUNCH();
   SBP_CUDA(cudaMemsetAsync(c.counters, 0, 8 * sizeof(unsigned long long), c.stream));
-  launch_warps(k_learn_eval, n, cap, 1, g->view(), bm->view(), verts.p, n, 0, bb, lp, rng, 0, bm->prop.p, moved.p,
+  const auto eval = bm->sparse ? k_learn_eval<Store::kHashed> : k_learn_eval<Store::kDenseFrozen>;
+  launch_warps(eval, n, cap, 1, g->view(), bm->view(), verts.p, n, 0, bb, lp, rng, 0, bm->prop.p, moved.p,
                nm.p, c.counters, dS.p, H.p, cap, c.status);
   std::vector<int> sp(n), pr(g->V), bh(g->V);
   std::vector<double> qf(n);
@@ -1218,7 +1272,7 @@ SbpStatus sbp_learned_q(const SbpBlockmodel* cbm, const SbpGraph* g, const SbpMl
   launch_warps(k_learn_features, n, cap, 1, g->view(), bm->view(), verts.p, n, 0, bb, lp, cap, c.status);
   mlp_forward(bb.F1, n, m->weights(), bb.L1, c.status, c.num_sms, c.stream);
   SBP_CHECK_LAUNCH();
-  k_learn_q<<<grid_for(n, 128, 1 << 20), 128, 0, c.stream>>>(tg.p, n, bb, lp, bm->B, qd.p);
+  k_learn_q<<<grid_for(n, 128 / kRowLanes, 1 << 28), 128, 0, c.stream>>>(tg.p, n, bb, lp, bm->B, qd.p);
   SBP_CHECK_LAUNCH();
   SBP_CUDA(SBP_COPY_ASYNC(q, qd.p, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
   check_tensor_status();

@@ -122,6 +122,27 @@ __device__ __forceinline__ void load_kmajor(unsigned char* dst, const __nv_bfloa
   }
 }
 
+// The same, without waiting: 16-byte asynchronous copies of the calling thread (rows beyond
+// `valid` read as zero).  Consecutive threads write consecutive 16 bytes of the tile (eight rows,
+// then the next eight columns), free of bank conflicts.  async_copies_wait, then async_fence and
+// a barrier, before the MMA.
+__device__ __forceinline__ void copy_kmajor(unsigned char* dst, const __nv_bfloat16* src, int rows, int K,
+                                            long long valid) {
+  const int chunks = rows * (K / 8);
+  for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
+    const int r = c / K * 8 + (c & 7), kc = (c % K) & ~7;   // K chunks in a group of eight rows
+    const int bytes = r < valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + kmaj(r, kc, K))),
+                 "l"(src + (size_t)(r < valid ? r : 0) * K + kc), "r"(bytes)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void async_copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void async_copies_wait() {   // all but the last kLeft groups have arrived
+  asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
+}
+
 // Transposed weight tile: dst[N = cols][K = rows] from a row-major [rows][cols] matrix.
 __device__ __forceinline__ void load_transposed(unsigned char* dst, const __nv_bfloat16* src, int rows, int cols) {
   for (int i = threadIdx.x; i < rows * cols; i += blockDim.x) {
@@ -167,9 +188,16 @@ __global__ void __launch_bounds__(128, 1)
   const int tid = threadIdx.x, warp = tid >> 5;
   float* sb = reinterpret_cast<float*>(sm + kFwdBias);
   const uint32_t bar = smem_u32(sm + kFwdBar);
-  load_kmajor(sm + kFwdW1, w.W1, kMlpHid, kMlpIn);
-  load_kmajor(sm + kFwdW2, w.W2, kMlpHid, kMlpHid);
-  load_kmajor(sm + kFwdW3, w.W3, kMlpOut, kMlpHid);
+  // A batch of the chain is 2,000 rows: 16 tiles, one a CTA, so the time is that of one tile from
+  // launch to store.  Everything it reads is asked for at once, the first layer's operands ahead.
+  const long long tiles = (n + kMlpTile - 1) / kMlpTile;
+  copy_kmajor(sm + kFwdW1, w.W1, kMlpHid, kMlpIn, kMlpHid);
+  copy_kmajor(sm + kFwdX, X + (long long)blockIdx.x * kMlpTile * kMlpIn, kMlpTile, kMlpIn,
+              n - (long long)blockIdx.x * kMlpTile);
+  async_copies_commit();
+  copy_kmajor(sm + kFwdW2, w.W2, kMlpHid, kMlpHid, kMlpHid);
+  copy_kmajor(sm + kFwdW3, w.W3, kMlpOut, kMlpHid, kMlpOut);
+  async_copies_commit();
   for (int i = tid; i < 272; i += blockDim.x) sb[i] = i < 128 ? w.b1[i] : i < 256 ? w.b2[i - 128] : w.b3[i - 256];
   if (tid == 0) mbar_init(bar);
   if (warp == 0) tmem_alloc(smem_u32(sm + kFwdSlot), 512);
@@ -180,15 +208,9 @@ __global__ void __launch_bounds__(128, 1)
   const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
   uint32_t phase = 0;
   int ok = 1;
-  const long long tiles = (n + kMlpTile - 1) / kMlpTile;
   for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
     const long long row0 = tile * kMlpTile;
-    for (int c = tid; c < kMlpTile * 8; c += blockDim.x) {
-      const int r = c >> 3, kc = (c & 7) * 8;
-      const long long gr = row0 + r;
-      const uint4 val = gr < n ? *reinterpret_cast<const uint4*>(X + gr * kMlpIn + kc) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(sm + kFwdX + kmaj(r, kc, kMlpIn)) = val;
-    }
+    async_copies_wait<1>();   // the tile's rows (and W1); the group behind may be in flight
     async_fence();
     tc_before();
     __syncthreads();
@@ -202,9 +224,17 @@ __global__ void __launch_bounds__(128, 1)
     if (!ok) break;
     tc_after();
     epilogue_relu(tm + lane_off + 0, sb, sm + kFwdH1, nullptr, tid);
+    async_copies_wait<0>();   // W2, W3
     async_fence();
     tc_before();
     __syncthreads();
+    // the first layer has read X: the next tile's rows, and an empty group behind them
+    if (tile + gridDim.x < tiles) {
+      const long long next = (tile + gridDim.x) * kMlpTile;
+      copy_kmajor(sm + kFwdX, X + next * kMlpIn, kMlpTile, kMlpIn, n - next);
+    }
+    async_copies_commit();
+    async_copies_commit();
     if (tid == 0) {
       tc_after();
       gemm(tm + 128, smem_u32(sm + kFwdH1), smem_u32(sm + kFwdW2), kMlpHid, kMlpHid, false);
@@ -240,6 +270,7 @@ __global__ void __launch_bounds__(128, 1)
     tc_before();
     __syncthreads();
   }
+  async_copies_wait<0>();
   if (!ok) {
     if (tid == 0) atomicOr(status, kErrTensorWait);
     mbar_wait(bar, phase ^ 1);   // the phase that gave up: let an MMA still in flight finish
