@@ -102,14 +102,16 @@ __device__ __forceinline__ double dxlogx(double a, double b) {
 // the counts are close or not (measured worst 1.9e-16; the (a - b) log a + b log(a / b) form
 // from a table of logs that it replaced: 3e-16).  Two loads and three additions: that form's
 // division, series and two-sided branch were most of the FP64 instructions of a visit.  Counts
-// beyond the table go through dxlogx.
+// beyond the table go through dxlogx (a call: inline at five places it was most of the code of the
+// kernels that evaluate one vertex a warp).
 constexpr int kXlogxTable = 1 << 20;
+static __device__ __noinline__ double dxlogx_far(int a, int b) { return dxlogx((double)a, (double)b); }
 __device__ __forceinline__ double dxlogx_int(const double2* __restrict__ gt, int a, int b) {
   if ((unsigned)a < (unsigned)kXlogxTable && (unsigned)b < (unsigned)kXlogxTable) {
     const double2 ga = __ldg(gt + a), gb = __ldg(gt + b);
     return (ga.x - gb.x) + (ga.y - gb.y);
   }
-  return dxlogx((double)a, (double)b);
+  return dxlogx_far(a, b);
 }
 
 // Merge delta-MDLs are rounded to a multiple of 2^-20 (about 1e-6) before merges are ranked:
@@ -470,17 +472,20 @@ __device__ __forceinline__ int walk_row(const BlockView& bm, int t, bool col, in
 
 // Same walk over a compressed list (idx[i], val[i]), i in [0, n).
 __device__ __forceinline__ int warp_select_sparse(const int* __restrict__ idx, const int* __restrict__ val, int n,
-                                                  long long target, int skip, int lane) {
+                                                  int target, int skip, int lane) {
   for (int base = 0; base < n; base += kWarp) {
     const int i = base + lane;
-    int c = -1;
-    long long v = 0;
+    int c = -1, incl = 0;   // a row's counts sum to at most E < 2^31
     if (i < n) {
       c = idx[i];
-      v = (c != skip) ? (long long)val[i] : 0;
+      incl = c != skip ? val[i] : 0;
     }
-    const long long incl = warp_incl_scan(v, lane);
-    const long long tot = __shfl_sync(kFull, incl, 31);
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+      const int y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int tot = __shfl_sync(kFull, incl, 31);
     if (target < tot) {
       const unsigned hit = __ballot_sync(kFull, incl > target);
       return __shfl_sync(kFull, c, __ffs(hit) - 1);
@@ -713,6 +718,11 @@ __device__ __forceinline__ bool maybe_zero_delta(double dS, int dout_r, int dout
   return fabsf((float)dS) <= 0x1.1p-40f * bound * (float)log_E;
 }
 
+// The double count of a net-zero Delta cell, m (log1p(a / b) + log1p(c / d)); rare, so out of line.
+static __device__ __noinline__ double net_zero_term(int m, int a, int b, int c, int d) {
+  return (double)m * (log1p((double)a / (double)b) + log1p((double)c / (double)d));
+}
+
 // Delta-MDL of moving v from r to s (s != r) against the current state, with the gathered
 // table of v's neighbour blocks, and the reference's Hastings correction (*H).
 //  - One load round over the distinct neighbour blocks (lane i: table entries i, i+32, ...)
@@ -794,11 +804,9 @@ __device__ __forceinline__ double move_delta(const GraphView& g, const BlockView
     const bool q_rs = (mc.co_s > 0 || mc.ci_r > 0) && d_rs == 0 && M_rs > 0;
     const bool q_sr = (mc.co_r > 0 || mc.ci_s > 0) && d_sr == 0 && M_sr > 0;
     const int qm = lane == 8 ? (q_rs ? M_rs : 0) : lane == 9 ? (q_sr ? M_sr : 0) : 0;
-    if (qm) {
-      const double x1 = lane == 8 ? (double)kin_self / (double)din_s : -(double)kin_self / (double)din_r;
-      const double x2 = lane == 8 ? -(double)k_out / (double)dout_r : (double)k_out / (double)dout_s;
-      dS += (double)qm * (log1p(x1) + log1p(x2));
-    }
+    if (qm)
+      dS += net_zero_term(qm, lane == 8 ? kin_self : -kin_self, lane == 8 ? din_s : din_r,
+                          lane == 8 ? -k_out : k_out, lane == 8 ? dout_r : dout_s);
   }
   fwd = warp_sum(fwd);
   bwd = warp_sum(bwd);

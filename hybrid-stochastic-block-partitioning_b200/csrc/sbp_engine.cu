@@ -449,8 +449,8 @@ void gibbs_apply(SbpBlockmodel& bm, const SbpGraph& g, int batch) {
   int* n_next = bm.n_moved.p + (slot ^ 1);
   const unsigned gen = ++bm.gen;
   const int gw = grid_for((long long)batch * 32, 256, 64 * c.num_sms);
-  k_apply_edges<<<gw, 256, 0, c.stream>>>(g.view(), bm.view(), bm.moved.p, n_cur, bm.prop.p, bm.qr.p, bm.qs.p,
-                                          bm.last.p, gen);
+  apply_edges_kernel(bm.sparse)<<<gw, 256, 0, c.stream>>>(g.view(), bm.view(), bm.moved.p, n_cur, bm.prop.p, bm.qr.p,
+                                                          bm.qs.p, bm.last.p, gen);
   SBP_CHECK_LAUNCH();
   if (bm.sparse) {
     int ovf = 0;
@@ -754,8 +754,8 @@ void merge_blocks(SbpBlockmodel& bm, SbpGraph& g, const SbpMergeOptions& opt, co
   ms.best_s.reserve(B);
   ms.best_dS.reserve(B);
   SBP_CUDA(cudaMemsetAsync(c.counters, 0, 8 * sizeof(unsigned long long), c.stream));
-  k_merge_propose<<<gw, 256, 0, c.stream>>>(bm.view(), rows, cols, rng, ms.best_s.p, ms.best_dS.p, c.counters,
-                                            c.status);
+  merge_propose_kernel(bm.sparse)<<<gw, 256, 0, c.stream>>>(bm.view(), rows, cols, rng, ms.best_s.p, ms.best_dS.p,
+                                                            c.counters, c.status);
   SBP_CHECK_LAUNCH();
   ms.sizes.reserve(B);
   SBP_CUDA(cudaMemsetAsync(ms.sizes.p, 0, B * sizeof(int), c.stream));
@@ -1532,8 +1532,9 @@ SbpStatus sbp_evaluate_vertices(const SbpBlockmodel* cbm, const SbpGraph* g, int
   dr.reserve(n);
   SBP_CUDA(SBP_COPY_ASYNC(dv.p, vertices, n * sizeof(int), cudaMemcpyHostToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(dr.p, records, n * sizeof(uint4), cudaMemcpyHostToDevice, c.stream));
-  set_smem_limit((const void*)k_eval_list, per_warp * W);
-  k_eval_list<<<grid_for(n, W, 64 * c.num_sms), W * 32, per_warp * W, c.stream>>>(
+  const EvalListKernel eval = eval_list_kernel(bm.sparse);
+  set_smem_limit((const void*)eval, per_warp * W);
+  eval<<<grid_for(n, W, 64 * c.num_sms), W * 32, per_warp * W, c.stream>>>(
       g->view(), bm.view(), dv.p, n, dr.p, cap, ds.p, dd.p, dh.p, da.p, c.status);
   SBP_CHECK_LAUNCH();
   SBP_CUDA(SBP_COPY_ASYNC(proposal, ds.p, n * sizeof(int), cudaMemcpyDeviceToHost, c.stream));

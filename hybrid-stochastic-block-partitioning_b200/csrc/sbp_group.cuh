@@ -204,18 +204,14 @@ __device__ __forceinline__ int2 row_pair(const RowRef<ST>& row, const BlockView&
   return m[0];
 }
 
-// Rare terms, out of line to keep the evaluation's code small: a count beyond the table, and the
-// double count of a net-zero Delta cell, m (log1p(a / b) + log1p(c / d)).
-static __device__ __noinline__ double dxlogx_far(int a, int b) { return dxlogx((double)a, (double)b); }
+// A difference of table entries that may lie beyond the table, out of line to keep the evaluation's
+// code small.
 static __device__ __noinline__ double dxlogx_wide(const double2* __restrict__ gt, int a, int b) {
   if ((unsigned)a < (unsigned)kXlogxTable && (unsigned)b < (unsigned)kXlogxTable) {
     const double2 ga = __ldg(gt + a), gb = __ldg(gt + b);
     return (ga.x - gb.x) + (ga.y - gb.y);
   }
   return dxlogx_far(a, b);
-}
-static __device__ __noinline__ double net_zero_term(int m, int a, int b, int c, int d) {
-  return (double)m * (log1p((double)a / (double)b) + log1p((double)c / (double)d));
 }
 
 // Accept test u <= min(1, exp(-3 dS) H), H = bwd / fwd (1 for a vertex without neighbours).  A

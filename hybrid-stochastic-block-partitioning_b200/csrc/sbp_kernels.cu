@@ -73,13 +73,17 @@ __global__ void k_rebuild_degrees(BlockView bm) {
 // result equals the reference's one-by-one application.  qr/qs keep the reference's diagonal
 // delta of each move as seen at its turn in vertex order, which Blockmodel::move_vertex folds
 // into d[r], d[s] (blockmodel.cpp:348-359); last[x] keeps (batch generation, last mover of x).
+template <Store ST>
 __global__ void k_apply_edges(GraphView g, BlockView bm, const int* moved_list, const int* n_moved, const int* prop,
                               int* qr, int* qs, unsigned long long* last, unsigned gen) {
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const int n = *n_moved;
-  for (int i = wid; i < n; i += nw) apply_moved_vertex(g, bm, moved_list[i], prop, qr, qs, last, gen, lane);
+  for (int i = wid; i < n; i += nw) apply_moved_vertex<ST>(g, bm, moved_list[i], prop, qr, qs, last, gen, lane);
+}
+ApplyEdgesKernel apply_edges_kernel(bool sparse) {
+  return sparse ? k_apply_edges<Store::kHashed> : k_apply_edges<Store::kDense>;
 }
 
 // d[r], d[s] from the last mover of each block, then the new assignment; clears the other
@@ -148,8 +152,9 @@ __global__ void k_mdl_cells_list_final(const double* partial, int n, int V, long
 // random record of a visit depends only on (vertex, sweep), so re-evaluation is idempotent.
 // out: [0] visits [1] proposals_moved [2] accepted (as doubles), [3] sum of accepted dS.
 // ------------------------------------------------------------------------------------------
-__global__ void k_mh(GraphView g, BlockView bm, const int* __restrict__ verts, int n, int start, RngParams rng,
-                     int sweep, int cap, double* out, int* status) {
+__global__ void __launch_bounds__(512)
+    k_mh(GraphView g, BlockView bm, const int* __restrict__ verts, int n, int start, RngParams rng, int sweep,
+         int cap, double* out, int* status) {
   extern __shared__ int smem[];
   __shared__ int s_acc[32], s_moved[32], s_r[32], s_s[32], s_t[32], s_commit[32];
   __shared__ double s_dS[32];
@@ -269,6 +274,7 @@ __global__ void k_move_vertex(GraphView g, BlockView bm, int v, int s, int cap, 
 }
 
 // Evaluate (without moving) a list of vertices with caller-supplied records.
+template <Store ST>
 __global__ void k_eval_list(GraphView g, BlockView bm, const int* verts, int n, const uint4* records, int cap,
                             int* out_s, double* out_dS, double* out_H, int* out_acc, int* status) {
   extern __shared__ int smem[];
@@ -279,7 +285,7 @@ __global__ void k_eval_list(GraphView g, BlockView bm, const int* verts, int n, 
   for (int i = blockIdx.x * wpb + warp; i < n; i += gridDim.x * wpb) {
     const int v = verts[i];
     int r, k_out, k_in;
-    const EvalResult res = evaluate_vertex(g, bm, v, records[i], t, lane, status, &r, &k_out, &k_in);
+    const EvalResult res = evaluate_vertex<ST>(g, bm, v, records[i], t, lane, status, &r, &k_out, &k_in);
     if (lane == 0) {
       out_s[i] = res.s;
       out_dS[i] = res.dS;
@@ -288,6 +294,9 @@ __global__ void k_eval_list(GraphView g, BlockView bm, const int* verts, int n, 
     }
     table_reset(t, lane);
   }
+}
+EvalListKernel eval_list_kernel(bool sparse) {
+  return sparse ? k_eval_list<Store::kHashed> : k_eval_list<Store::kDenseFrozen>;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -368,47 +377,73 @@ __global__ void k_row_fill(const int2* P, int col_side, int B, int ld, const int
 //      + sum_{c not in r,s} [g(M[c,s]) - g(M[c,s]+M[c,r])] + g(M[s,s]) - g(M[s,s]+M[r,r]+M[r,s]+M[s,r])
 //      - [g(do_r)+g(do_s)-g(do_r+do_s)] - [g(di_r)+g(di_s)-g(di_r+di_s)]
 // which equals entropy::block_merge_delta_mdl (src/entropy.cpp:127-180).
-__device__ double merge_delta(const BlockView& bm, const Csr& rows, const Csr& cols, int r, int s, int lane) {
-  double dS = 0.0;
-  for (int j = rows.ptr[r] + lane; j < rows.ptr[r + 1]; j += kWarp) {
-    const int c = rows.idx[j], m = rows.val[j];
-    dS += xlogx((double)m);
-    if (c != r && c != s) {
-      const int msc = bm_get(bm, s, c);
-      dS += dxlogx((double)msc, (double)(msc + m));
-    }
+//
+// Bound by instruction issue: a block scores ten proposals and FP64 logarithms are most of it.  So
+// a logarithm stands in one place and is called (the kernel was 56 KB of code with fourteen of
+// them inline), the six degree terms and the four corner cells take a lane each instead of every
+// lane all of them, and the terms that are exactly 0 are left out: counts of 1, of which most
+// cells are while the blocks are many, against an empty cell.  What is added, and in which
+// order, is as before, to the bit: equal scores decide merges.
+static __device__ __noinline__ double xlogx_call(double x) { return xlogx(x); }
+static __device__ __noinline__ double dxlogx_call(double a, double b) { return dxlogx(a, b); }
+
+// g(m) + [g(a) - g(a + m)] added to dS, m > 0 (pair: whether the second term counts).
+__device__ __forceinline__ void merge_term(double& dS, int m, int a, bool pair) {
+  if (m > 1) dS += xlogx_call((double)m);
+  if (pair && a + m > 1) dS += dxlogx_call((double)a, (double)(a + m));
+}
+
+template <Store ST>
+__device__ __forceinline__ double merge_delta(const BlockView& bm, const Csr& rows, const Csr& cols, int r, int s,
+                                              int lane) {
+  const int r0 = rows.ptr[r], r1 = rows.ptr[r + 1], c0 = cols.ptr[r], c1 = cols.ptr[r + 1];
+  // lanes 0..3: M_rr, M_rs, M_sr, M_ss; lanes 8..13: the degrees and their sums
+  int corner = 0;
+  if (lane < 4) corner = bm_get<ST>(bm, lane < 2 ? r : s, (lane & 1) ? s : r);
+  double deg = 0.0;
+  if (lane >= 8 && lane < 14) {
+    const int* d = lane < 11 ? bm.d_out : bm.d_in;
+    const int q = lane < 11 ? lane - 8 : lane - 11;
+    const double dr = q == 1 ? 0.0 : (double)d[r], ds = q == 0 ? 0.0 : (double)d[s];
+    deg = dr + ds;
   }
-  for (int j = cols.ptr[r] + lane; j < cols.ptr[r + 1]; j += kWarp) {
+  double dS = 0.0;
+  for (int j = r0 + lane; j < r1; j += kWarp) {
+    const int c = rows.idx[j], m = rows.val[j];
+    const bool pair = c != r && c != s;
+    merge_term(dS, m, pair ? bm_get<ST>(bm, s, c) : 0, pair);
+  }
+  for (int j = c0 + lane; j < c1; j += kWarp) {
     const int c = cols.idx[j], m = cols.val[j];
     if (c == r) continue;
-    dS += xlogx((double)m);
-    if (c != s) {
-      const int mcs = bm_getT(bm, s, c);
-      dS += dxlogx((double)mcs, (double)(mcs + m));
-    }
+    merge_term(dS, m, c != s ? bm_getT<ST>(bm, s, c) : 0, c != s);
   }
+  __syncwarp();
   dS = warp_sum(dS);
-  const int M_rr = bm_get(bm, r, r), M_rs = bm_get(bm, r, s);
-  const int M_sr = bm_get(bm, s, r), M_ss = bm_get(bm, s, s);
-  dS += dxlogx((double)M_ss, (double)(M_ss + M_rr + M_rs + M_sr));
-  const double dor = bm.d_out[r], dos = bm.d_out[s], dir = bm.d_in[r], dis = bm.d_in[s];
-  dS -= xlogx(dor) + xlogx(dos) - xlogx(dor + dos);
-  dS -= xlogx(dir) + xlogx(dis) - xlogx(dir + dis);
+  const double g = xlogx_call(deg);
+  const int M_ss = __shfl_sync(kFull, corner, 3), merged = warp_sum_int(corner);
+  if (merged > 1 && merged != M_ss) dS += dxlogx_call((double)M_ss, (double)merged);   // warp-uniform
+  dS -= __shfl_sync(kFull, g, 8) + __shfl_sync(kFull, g, 9) - __shfl_sync(kFull, g, 10);
+  dS -= __shfl_sync(kFull, g, 11) + __shfl_sync(kFull, g, 12) - __shfl_sync(kFull, g, 13);
   return dS;
 }
 
+template <Store ST>
 __global__ void k_merge_propose(BlockView bm, Csr rows, Csr cols, RngParams rng, int* best_s, double* best_dS,
                                 unsigned long long* counters, int* status) {
+  __shared__ int s_avoided;
+  if (threadIdx.x == 0) s_avoided = 0;
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   const int B = bm.B;
+  int avoided = 0;
   for (int r = wid; r < B; r += nw) {
-    int seen[kProposalsPerBlock];
+    int seen = -1;   // lane j: the j-th distinct proposal
     int nseen = 0;
     int best = -1;
     double bdS = 1.79769313486231570815e+308;
-    int avoided = 0;
     const long long k_out = bm.d_out[r], k = k_out + bm.d_in[r];
     for (int i = 0; i < kProposalsPerBlock; ++i) {
       const uint4 x = draw_record(rng, (uint32_t)r, (uint32_t)i, 1u, (long long)r * kProposalsPerBlock + i, status);
@@ -422,42 +457,44 @@ __global__ void k_merge_propose(BlockView bm, Csr rows, Csr cols, RngParams rng,
       } else if (k == 0) {
         s = random_block(r, B, x.y);
       } else {
+        // a neighbour block t of r by edges, then a block of t's row or column, r left out
         const long long target = scale32(x.x, k);
-        int t;
-        if (target < k_out) t = warp_select_sparse(rows.idx + rows.ptr[r], rows.val + rows.ptr[r],
-                                                   rows.ptr[r + 1] - rows.ptr[r], target, -1, lane);
-        else t = warp_select_sparse(cols.idx + cols.ptr[r], cols.val + cols.ptr[r], cols.ptr[r + 1] - cols.ptr[r],
-                                    target - k_out, -1, lane);
-        if (t < 0) {
-          if (lane == 0) atomicOr(status, kErrScan);
-          t = r;
-        }
-        const long long m_tr = bm_get(bm, t, r), m_rt = bm_get(bm, r, t);
-        const long long rowpart = (long long)bm.d_out[t] - m_tr;
-        const long long total = rowpart + (long long)bm.d_in[t] - m_rt;
-        if (total == 0) {
-          s = random_block(r, B, x.y);
-        } else {
-          const long long tg = scale32(x.y, total);
-          if (tg < rowpart) s = warp_select_sparse(rows.idx + rows.ptr[t], rows.val + rows.ptr[t],
-                                                   rows.ptr[t + 1] - rows.ptr[t], tg, r, lane);
-          else s = warp_select_sparse(cols.idx + cols.ptr[t], cols.val + cols.ptr[t], cols.ptr[t + 1] - cols.ptr[t],
-                                      tg - rowpart, r, lane);
-          if (s < 0) {
-            if (lane == 0) atomicOr(status, kErrScan);
-            s = random_block(r, B, x.y);
+        int t = -1;
+        s = -1;
+        bool uniform = false;
+        for (int step = 0; step < 2 && !uniform; ++step) {   // one code site for both walks
+          const int row = step == 0 ? r : t;
+          long long split = k_out, tg = target;
+          if (step == 1) {
+            int m = 0;   // lane 0: M[t, r], lane 1: M[r, t]
+            if (lane < 2) m = bm_get<ST>(bm, lane == 0 ? t : r, lane == 0 ? r : t);
+            split = (long long)bm.d_out[t] - __shfl_sync(kFull, m, 0);
+            const long long total = split + (long long)bm.d_in[t] - __shfl_sync(kFull, m, 1);
+            if (total == 0) {
+              uniform = true;
+              break;
+            }
+            tg = scale32(x.y, total);
           }
+          const bool in_row = tg < split;
+          const Csr& from = in_row ? rows : cols;
+          const int p0 = from.ptr[row];
+          const int u = warp_select_sparse(from.idx + p0, from.val + p0, from.ptr[row + 1] - p0,
+                                           (int)(in_row ? tg : tg - split), step == 0 ? -1 : r, lane);
+          if (u < 0 && lane == 0) atomicOr(status, kErrScan);
+          if (step == 0) t = u < 0 ? r : u;
+          else s = u;
         }
+        if (s < 0) s = random_block(r, B, x.y);
       }
-      bool dup = false;
-      for (int j = 0; j < nseen; ++j) dup |= (seen[j] == s);
-      if (dup) {
+      if (__any_sync(kFull, lane < nseen && seen == s)) {
         avoided++;
         continue;
       }
-      seen[nseen++] = s;
+      if (lane == nseen) seen = s;
+      nseen++;
       // same value for r->s and s->r; one fixed orientation makes mutual pairs tie exactly
-      const double dS = merge_score(merge_delta(bm, rows, cols, min(r, s), max(r, s), lane));
+      const double dS = merge_score(merge_delta<ST>(bm, rows, cols, min(r, s), max(r, s), lane));
       if (dS < bdS) {
         bdS = dS;
         best = s;
@@ -466,10 +503,17 @@ __global__ void k_merge_propose(BlockView bm, Csr rows, Csr cols, RngParams rng,
     if (lane == 0) {
       best_s[r] = best;
       best_dS[r] = bdS;
-      atomicAdd(counters + 0, (unsigned long long)kProposalsPerBlock);
-      atomicAdd(counters + 1, (unsigned long long)avoided);
     }
   }
+  if (lane == 0 && avoided) atomicAdd(&s_avoided, avoided);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (blockIdx.x == 0) atomicAdd(counters + 0, (unsigned long long)B * kProposalsPerBlock);
+    if (s_avoided) atomicAdd(counters + 1, (unsigned long long)s_avoided);
+  }
+}
+MergeProposeKernel merge_propose_kernel(bool sparse) {
+  return sparse ? k_merge_propose<Store::kHashed> : k_merge_propose<Store::kDenseFrozen>;
 }
 
 __global__ void k_block_sizes(const int* b, int V, int* size) {

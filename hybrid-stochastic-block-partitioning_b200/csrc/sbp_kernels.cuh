@@ -34,21 +34,25 @@ __global__ void k_mdl_cells_list(const int* __restrict__ rows, const int* __rest
 __global__ void k_mdl_cells_list_final(const double* partial, int n, int V, long long E, int B, double* out);
 __global__ void k_mdl(GraphView g, BlockView bm, const int* __restrict__ out_src, int cells, double* partial,
                       unsigned* done, double* out);
-__global__ void k_apply_edges(GraphView g, BlockView bm, const int* moved_list, const int* n_moved, const int* prop,
+// One instantiation per storage: the other's code is not in the instruction stream.
+using ApplyEdgesKernel = void (*)(GraphView g, BlockView bm, const int* moved_list, const int* n_moved, const int* prop,
                               int* qr, int* qs, unsigned long long* last, unsigned gen);
+ApplyEdgesKernel apply_edges_kernel(bool sparse);
 __global__ void k_apply_finish(BlockView bm, const int* moved_list, const int* n_moved, int* next_n_moved, int* prop,
                                const int* qr, const int* qs, const unsigned long long* last, unsigned gen);
 __global__ void k_mh(GraphView g, BlockView bm, const int* __restrict__ verts, int n, int start, RngParams rng,
                      int sweep, int cap, double* out, int* status);
 __global__ void k_move_vertex(GraphView g, BlockView bm, int v, int s, int cap, int* status);
-__global__ void k_eval_list(GraphView g, BlockView bm, const int* verts, int n, const uint4* records, int cap,
+using EvalListKernel = void (*)(GraphView g, BlockView bm, const int* verts, int n, const uint4* records, int cap,
                             int* out_s, double* out_dS, double* out_H, int* out_acc, int* status);
+EvalListKernel eval_list_kernel(bool sparse);
 __global__ void k_row_nnz(const int2* P, int col_side, int B, int ld, int* cnt);
 __global__ void k_excl_scan(const int* in, int* out, int n);
 __global__ void k_row_fill(const int2* P, int col_side, int B, int ld, const int* ptr, int* idx, int* val);
 __global__ void k_pairs_to_dense(const int2* __restrict__ P, int B, int ld, int row0, int rows, int* dense);
-__global__ void k_merge_propose(BlockView bm, Csr rows, Csr cols, RngParams rng, int* best_s, double* best_dS,
+using MergeProposeKernel = void (*)(BlockView bm, Csr rows, Csr cols, RngParams rng, int* best_s, double* best_dS,
                                 unsigned long long* counters, int* status);
+MergeProposeKernel merge_propose_kernel(bool sparse);
 __global__ void k_block_sizes(const int* b, int V, int* size);
 // Integer block statistics: out[0] = sum_b M[b,b], out[1] = sum_b d_in[b], out[2] = sum_b
 // d_out[b] * d_in[b] (the interblock-edge fraction and the modularity of a partition).
