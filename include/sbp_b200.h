@@ -114,12 +114,12 @@ int32_t sbp_device_count(void);
  * is faster wherever it fits).  "dense_max_memory_pct" (default 60, range 1-90): a dense matrix
  * that would take more than this percentage of the free device memory is row-hashed instead.
  * Both apply to blockmodels whose block count is set after the call.  "group_kernel" (default
- * 1): asynchronous-Gibbs and Metropolis-Hastings evaluation with a group of 8 lanes per vertex
- * on dense blockmodels of at most 128 blocks; 2: at every block count (vertices of degree up to
- * 128); 0: one warp per vertex everywhere (same results).  "hashed_row_factor" (default 4, range 2-64): a rebuilt hashed row gets room
+ * 1): lanes per vertex of the asynchronous-Gibbs and Metropolis-Hastings evaluation on dense
+ * storage, chosen from the batch and the vertex's degree; 2: as few as its degree allows
+ * (asynchronous Gibbs); 0: a warp per vertex (same results).  "hashed_row_factor" (default 4, range 2-64): a rebuilt hashed row gets room
  * for factor x its cells, at most 2 x for rows of more than 128 cells (larger: rows fill up and
  * are regrown less often; smaller: less memory and a cheaper walk of the row).  "graph_sweeps" (default 1): an
- * asynchronous-Gibbs finetune on dense storage runs as one CUDA graph launch whose sweep loop and
+ * asynchronous-Gibbs finetune on dense storage runs as one persistent launch whose sweep loop and
  * early stop are decided on the GPU; 0 drives every sweep from the host (same results).
  * "batched_wait_limit" (default 2^22, range 16-2^30): idle claim attempts (about 0.25 us each) of a
  * persistent CTA of sbp_partition_batched before its launch gives up and the call fails with

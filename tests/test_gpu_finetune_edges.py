@@ -1,0 +1,137 @@
+"""The finetune kernels at the sizes where their splits change, against the CPU oracle: vertex degrees on both sides of
+what a lane, a group of 8, 16 or 32 lanes and a warp hold, batches of 128 and 129 vertices (one cluster or the whole
+device), block counts on both sides of the walk's levels (none up to 128 blocks, sums of 64, sums of 64 of those), and
+the row-hashed storage.  Integer state is equal; the MDL is stored as a float on both sides (relative 1e-7)."""
+import numpy as np
+import pytest
+
+from conftest import random_assignment, random_graph
+from test_gpu_parity import assert_same_state
+
+pytestmark = pytest.mark.gpu
+
+# out + in degrees of the first vertices, one each
+DEGREES = [0, 1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 300, 511, 513, 700]
+
+
+def graph_of_degrees(V, seed):
+    """Vertex i < len(DEGREES) has DEGREES[i] edges (about half each way, no two alike) to the vertices after a third
+    of the rest, which have a few edges among themselves; some vertices have a self loop and some edges come twice."""
+    rng = np.random.default_rng(seed)
+    h = len(DEGREES)
+    src, dst = [], []
+    for i, k in enumerate(DEGREES):
+        out = k // 2
+        src += [i] * out
+        dst += rng.choice(np.arange(h, V), out, replace=False).tolist()
+        dst += [i] * (k - out)
+        src += rng.choice(np.arange(h, V), k - out, replace=False).tolist()
+    n = 5 * V
+    src += rng.integers(h, V, n).tolist()
+    dst += (h + (rng.integers(0, V - h, n) * rng.random(n)).astype(int)).tolist()
+    src += [3, 20, h + 5] + src[:40]
+    dst += [3, 20, h + 5] + dst[:40]
+    return np.array(src, np.int32), np.array(dst, np.int32)
+
+
+def run_both(S, O, V, s, d, B, seed, algo, batches, sweeps):
+    a = random_assignment(V, B, seed)
+    g, og = S.Graph(V, s, d), O.Graph(V, s, d)
+    assert g.E == og.E
+    bm, obm = S.Blockmodel(g, B, a), O.Blockmodel(og, B, a)
+    st = S.finetune.run(bm, algo, batches=batches, seed=seed, call=1, max_sweeps=sweeps)
+    ost = obm.finetune(algo, batches=batches, seed=seed, call=1, max_sweeps=sweeps)
+    assert_same_state(bm, obm)
+    for k in ("sweeps", "visits", "accepted", "proposals_moved"):
+        assert st[k] == ost[k], k
+    assert st["mdl"] == pytest.approx(ost["mdl"], rel=1e-7)
+
+
+@pytest.mark.parametrize("algo", [0, 1, 2])
+@pytest.mark.parametrize("B", [2, 127, 128, 129, 500])
+@pytest.mark.parametrize("storage", ["dense", "hashed"])
+def test_degrees_and_blocks(S, O, storage, B, algo):
+    V = 1200
+    s, d = graph_of_degrees(V, B)
+    S.set_option("dense_max_blocks", 131072 if storage == "dense" else 1)
+    try:
+        run_both(S, O, V, s, d, B, B + algo, algo, 5, 3)
+    finally:
+        S.set_option("dense_max_blocks", 131072)
+
+
+@pytest.mark.parametrize("algo", [0, 1])
+@pytest.mark.parametrize("B", [4095, 4096, 4097])   # 64 sums of 64 columns; beyond, a second level
+def test_walk_levels(S, O, B, algo):
+    V = 4600
+    s, d = graph_of_degrees(V, B)
+    run_both(S, O, V, s, d, B, B, algo, 3, 2)
+
+
+@pytest.mark.parametrize("per_batch", [1, 127, 128, 129])
+@pytest.mark.parametrize("device_sweeps", [1, 0])
+def test_batch_sizes(S, O, per_batch, device_sweeps):
+    batches = 4
+    V = per_batch * batches if per_batch > 1 else 60
+    V, s, d, _ = random_graph(V, 4, per_batch)
+    S.set_option("graph_sweeps", device_sweeps)
+    try:
+        run_both(S, O, V, s, d, min(30, V // 2), per_batch, 1, batches if per_batch > 1 else V, 5)
+    finally:
+        S.set_option("graph_sweeps", 1)
+
+
+@pytest.mark.parametrize("group", [0, 1, 2])
+def test_group_widths(S, O, group):
+    V = 1200
+    s, d = graph_of_degrees(V, 3)
+    S.set_option("group_kernel", group)
+    try:
+        for B in (40, 300):
+            run_both(S, O, V, s, d, B, 5, 1, 4, 3)
+    finally:
+        S.set_option("group_kernel", 1)
+
+
+@pytest.mark.parametrize("n", [1, 4095, 4096, 4097, 12289])   # edges a pass of the sort takes: 4,096
+def test_ingest_sorts(S, O, n):
+    """Duplicates and self loops in, in any order; the graph the oracle builds."""
+    rng = np.random.default_rng(n)
+    V = max(2, n // 6)
+    s, d = rng.integers(0, V, n).astype(np.int32), rng.integers(0, V, n).astype(np.int32)
+    g, og = S.Graph(V, s, d), O.Graph(V, s, d)
+    assert g.E == og.E
+    a = random_assignment(V, min(V, 20), n)
+    assert_same_state(S.Blockmodel(g, min(V, 20), a), O.Blockmodel(og, min(V, 20), a))
+
+
+@pytest.mark.parametrize("B", [2, 33, 1200])
+@pytest.mark.parametrize("storage", ["dense", "hashed"])
+def test_merge_scores(S, O, storage, B):
+    """Scores are rounded to 2^-20 on both sides: equal, or one step apart where the sums' last bits fall on either
+    side of a rounding boundary."""
+    V = 1200
+    s, d = graph_of_degrees(V, B)
+    a = random_assignment(V, B, B) if B < V else np.arange(V, dtype=np.int32)
+    S.set_option("dense_max_blocks", 131072 if storage == "dense" else 1)
+    try:
+        bm, obm = S.Blockmodel(S.Graph(V, s, d), B, a), O.Blockmodel(O.Graph(V, s, d), B, a)
+        got = S.block_merge.merge_blocks(bm, seed=2)
+        ref = obm.merge_blocks(seed=2)
+    finally:
+        S.set_option("dense_max_blocks", 131072)
+    assert np.abs(got["dS"] - ref["dS"]).max() <= 2.0**-20
+    assert (got["best"] == ref["best"]).mean() > 0.99
+
+
+def test_batched_many_moves(S):
+    """Batches in which more vertices move than the CTA that ends a stage finishes by itself (2,048)."""
+    V, s, d, _ = random_graph(9000, 6, 8)
+    graphs = [S.Graph(V, s, d) for _ in range(2)]
+    outs, stats, info = S.batched.stochastic_block_partition(graphs, batches=2, seed=3)
+    assert info["batched_finetunes"] > 0
+    one, st = S.sbp.stochastic_block_partition(graphs[0], batches=2, seed=3)
+    for a, sb in zip(outs, stats):
+        assert np.array_equal(a, one)
+        for k in ("num_blocks", "mdl", "sweeps", "accepted"):
+            assert sb[k] == st[k], k
