@@ -597,6 +597,7 @@ struct SbpBlockmodel {
   DevBuf<double> inv_d;
   DevBuf<int2> P;                            // dense counts of both directions (BlockView::P)
   DevBuf<int> prop, qr, qs, moved, n_moved;   // n_moved: two slots, alternating per batch
+  DevBuf<int4> moves;                         // a batch's accepted moves in the finetune kernel (EvalArgs::moves)
   DevBuf<unsigned long long> last;           // (batch generation << 32 | last mover) per block
   unsigned gen = 0;                          // batch generation
   int nch = 0, ncs = 0, nss = 0;

@@ -12,8 +12,9 @@ struct EvalCounts {
   unsigned visit = 0, moved = 0, acc = 0;
 };
 
-// Everything one batch's evaluation needs; `store_index`: the moved list gets plan indices
-// (records are looked up again by the apply), else vertex ids.
+// Everything one batch's evaluation needs.  Accepted moves go to `moved` (vertex ids) or, where it is
+// given, to `moves`: the vertex's record, then (r, s, -, -), so that the apply and the degree step
+// find all they need in one load by position.
 struct EvalArgs {
   GraphView g;
   BlockView bm;
@@ -21,16 +22,15 @@ struct EvalArgs {
   RngParams rng;
   int* prop;
   int* moved;
+  int4* moves;           // [2 * batch] or null
   int* status;
   int gmin;              // smallest group
   int slots;             // table slots of the CTA (kGroupWarps regions, or more for a heavy vertex)
-  int store_index;
 };
 
 template <bool kDirect, Store ST>
-__device__ __forceinline__ void eval_task(const EvalArgs& a, const GroupTab<kDirect>& T, int index, bool valid, int sweep,
+__device__ __forceinline__ void eval_task(const EvalArgs& a, const GroupTab<kDirect>& T, int4 rec, bool valid, int sweep,
                                           int* n_moved, const Lanes& L, EvalCounts& cnt, int* bins) {
-  const int4 rec = valid ? __ldg(a.recs + index) : make_int4(0, 0, 0, 0);
   uint4 x = make_uint4(0, 0, 0, 0);
   if (valid)
     x = draw_record(a.rng, (uint32_t)rec.x, (uint32_t)sweep, 0u, (long long)sweep * a.g.V + rec.x, a.status);
@@ -41,10 +41,24 @@ __device__ __forceinline__ void eval_task(const EvalArgs& a, const GroupTab<kDir
     if (e.accepted) {
       cnt.acc++;
       a.prop[e.v] = e.s;
-      a.moved[atomicAdd(n_moved, 1)] = a.store_index ? index : e.v;
+      const int i = atomicAdd(n_moved, 1);
+      if (a.moves) {
+        a.moves[2 * i] = rec;
+        a.moves[2 * i + 1] = make_int4(e.r, e.s, 0, 0);
+      } else {
+        a.moved[i] = e.v;
+      }
     }
   }
   T.clear(e.n, L);
+}
+
+// The record of this lane's vertex in task `task` of a batch (zeros: none).
+__device__ __forceinline__ int4 task_record(const EvalArgs& a, const BatchDesc& b, const GroupTask& k, int light,
+                                            int lane, bool* valid) {
+  const int i = k.first + (lane >> (5 - k.lg));
+  *valid = i < k.end;
+  return *valid ? __ldg(a.recs + (light ? b.light_begin : b.heavy_begin) + i) : make_int4(0, 0, 0, 0);
 }
 
 // One batch: tasks of 32 / G vertices, a warp each, the largest degrees first.  Strided over the
@@ -68,8 +82,10 @@ __device__ __forceinline__ void eval_batch(const EvalArgs& a, BatchDesc b, int s
       const int sub = lane >> (5 - k.lg), share = kRegionSlots >> k.lg;
       const GroupTab<kDirect> T = group_tab<kDirect>(smem, a.slots, whole ? 0 : warp * kRegionSlots + sub * share,
                                                      whole ? a.slots : share);
-      eval_task<kDirect, ST>(a, T, (light ? b.light_begin : b.heavy_begin) + k.first + sub, k.first + sub < k.end, sweep,
-                             n_moved, L, cnt, smem + group_smem_bytes(kDirect, a.slots) / sizeof(int) + 32 * warp);
+      bool valid;
+      const int4 rec = task_record(a, b, k, light, lane, &valid);
+      eval_task<kDirect, ST>(a, T, rec, valid, sweep, n_moved, L, cnt,
+                             smem + group_smem_bytes(kDirect, a.slots) / sizeof(int) + 32 * warp);
     }
     if (whole) __syncthreads();
   }
@@ -121,8 +137,6 @@ struct SweepsArgs {
   int cluster;              // 1: the grid is one cluster
   unsigned gen0;            // batch generation before the call
   unsigned wait_limit;      // polls of a barrier before it gives up
-  int* qr;
-  int* qs;
   unsigned long long* last;
   const int* out_src;
   double* partial;
@@ -195,11 +209,17 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_gibbs_sweeps(const __grid_
         const int n = *(volatile int*)n_cur;
         ++gen;
         if (n == 0) continue;   // the same for the whole grid
-        for (int i = wid; i < n; i += nw)
-          apply_moved_record<Store::kDense>(g, bm, __ldg(a.e.recs + a.e.moved[i]), a.e.prop, a.qr, a.qs, a.last, gen, lane);
+        for (int i = wid; i < n; i += nw) {
+          const int4 rec = a.e.moves[2 * i], mv = a.e.moves[2 * i + 1];
+          const MoveQuirks q = apply_moved_record<Store::kDense>(g, bm, rec, mv.x, mv.y, a.e.prop, a.last, gen, lane);
+          if (lane == 0) a.e.moves[2 * i + 1] = make_int4(mv.x, mv.y, q.qr, q.qs);
+        }
         if (!sync_grid(a, &target, &s_abort)) return;
-        for (int i = blockIdx.x * kGroupThreads + tid; i < n; i += gridDim.x * kGroupThreads)
-          finish_moved_vertex<Store::kDense>(bm, __ldg(&a.e.recs[a.e.moved[i]].x), a.e.prop, a.qr, a.qs, a.last, gen);
+        for (int i = blockIdx.x * kGroupThreads + tid; i < n; i += gridDim.x * kGroupThreads) {
+          const int v = a.e.moves[2 * i].x;
+          const int4 mv = a.e.moves[2 * i + 1];
+          finish_move<Store::kDense>(bm, v, mv.x, mv.y, {mv.z, mv.w}, a.e.prop, a.last, gen);
+        }
         if (!sync_grid(a, &target, &s_abort)) return;
       }
     }
@@ -255,12 +275,12 @@ EvalArgs eval_args(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& plan, 
   a.rng = rng;
   a.prop = bm.prop.p;
   a.moved = bm.moved.p;
+  a.moves = nullptr;
   a.status = Context::get().status;
   // a heavy vertex needs a slot for each of its distinct neighbour blocks, of which there are at
   // most B; twice that many while they fit
   const int distinct = std::min(g.max_k, bm.B);
   a.slots = std::max(kGroupWarps * kRegionSlots, std::min(kMaxCap, pow2_at_least(2 * distinct)));
-  a.store_index = 0;
   a.gmin = 8;
   return a;
 }
@@ -297,7 +317,8 @@ SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan&
   Context& c = Context::get();
   SweepsArgs a;
   a.e = eval_args(g, bm, plan, rng);
-  a.e.store_index = 1;
+  bm.moves.reserve(2 * (size_t)plan.max_batch);
+  a.e.moves = bm.moves.p;
   a.batches = plan.desc_dev.p;
   a.nbatches = (int)plan.desc.size();
   a.max_sweeps = max_sweeps;
@@ -306,8 +327,6 @@ SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan&
   a.mdl_ctas = mdl_grid(bm, g);
   a.gen0 = bm.gen;
   a.wait_limit = kGridWaitLimit;
-  a.qr = bm.qr.p;
-  a.qs = bm.qs.p;
   a.last = bm.last.p;
   a.out_src = g.out_src.p;
   a.partial = c.partial;

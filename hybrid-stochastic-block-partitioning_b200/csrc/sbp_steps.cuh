@@ -152,18 +152,22 @@ __device__ __forceinline__ void mh_apply_move(const GraphView& g, const BlockVie
   }
 }
 
-// Apply of one accepted move v: r -> prop[v] (Blockmodel::move_vertex, src/blockmodel/
+// The quirk terms of d[r] and d[s] that the apply of a move hands to its degree step.
+struct MoveQuirks {
+  int qr, qs;
+};
+
+// Apply of one accepted move v: r -> s (Blockmodel::move_vertex, src/blockmodel/
 // blockmodel.cpp:344-360, for a batch of simultaneous moves): the counts and chunk sums by edge,
 // d_out / d_in, the quirk terms qr/qs of d[r], d[s] (the neighbours that are counted in the
 // reference's sequential apply) and the batch's last mover of r and s.  One warp per vertex;
 // lanes whose edges change the same cell add their count with one atomic.
 template <Store ST = Store::kAny>
-__device__ __forceinline__ void apply_moved_record(const GraphView& g, const BlockView& bm, int4 rec, const int* prop,
-                                                   int* qr, int* qs, unsigned long long* last, unsigned gen,
-                                                   int lane) {
+__device__ __forceinline__ MoveQuirks apply_moved_record(const GraphView& g, const BlockView& bm, int4 rec, int r,
+                                                         int s, const int* prop, unsigned long long* last,
+                                                         unsigned gen, int lane) {
   const int v = rec.x, k_out = rec.z, k_in = rec.w >> 1, self = rec.w & 1, k = k_out + k_in;
   const int* nbr = g.adj + (unsigned)rec.y;
-  const int r = bm.b[v], s = prop[v];
   int cr = 0, cs = 0;
   // One pass over the joint neighbour list (out-edges, then in-edges), two elements per lane
   // in flight.  Out-edge v -> u (not the self loop): (r, b_u) -= 1 and (s, b'_u) += 1, b'_u the
@@ -222,30 +226,40 @@ __device__ __forceinline__ void apply_moved_record(const GraphView& g, const Blo
     atomicAdd(bm.d_out + s, k_out);
     atomicAdd(bm.d_in + r, -k_in_self);
     atomicAdd(bm.d_in + s, k_in_self);
-    qr[v] = -(cr + self);
-    qs[v] = cs + self;
     const unsigned long long key = ((unsigned long long)gen << 32) | (unsigned)v;
     atomicMax(last + r, key);
     atomicMax(last + s, key);
   }
+  return {-(cr + self), cs + self};
 }
 template <Store ST = Store::kAny>
 __device__ __forceinline__ void apply_moved_vertex(const GraphView& g, const BlockView& bm, int v, const int* prop,
                                                    int* qr, int* qs, unsigned long long* last, unsigned gen,
                                                    int lane) {
-  apply_moved_record<ST>(g, bm, vertex_record(g, v), prop, qr, qs, last, gen, lane);
+  const MoveQuirks q = apply_moved_record<ST>(g, bm, vertex_record(g, v), bm.b[v], prop[v], prop, last, gen, lane);
+  if (lane == 0) {
+    qr[v] = q.qr;
+    qs[v] = q.qs;
+  }
 }
 
-// d[r], d[s] from the last mover of each block, then the new assignment of v.
+// d[r], d[s] from the last mover of each block, then the new assignment of v.  Every load is issued
+// before the first test.
+template <Store ST = Store::kAny>
+__device__ __forceinline__ void finish_move(const BlockView& bm, int v, int r, int s, MoveQuirks q, int* prop,
+                                            const unsigned long long* last, unsigned gen) {
+  const unsigned long long key = ((unsigned long long)gen << 32) | (unsigned)v, last_r = last[r], last_s = last[s];
+  const int d_r = bm.d_out[r] + bm.d_in[r] - bm_get<ST>(bm, r, r) - q.qr;
+  const int d_s = bm.d_out[s] + bm.d_in[s] - bm_get<ST>(bm, s, s) - q.qs;
+  if (last_r == key) set_degree(bm, r, d_r);
+  if (last_s == key) set_degree(bm, s, d_s);
+  bm.b[v] = s;
+  prop[v] = -1;
+}
 template <Store ST = Store::kAny>
 __device__ __forceinline__ void finish_moved_vertex(const BlockView& bm, int v, int* prop, const int* qr,
                                                     const int* qs, const unsigned long long* last, unsigned gen) {
-  const int r = bm.b[v], s = prop[v];
-  const unsigned long long key = ((unsigned long long)gen << 32) | (unsigned)v;
-  if (last[r] == key) set_degree(bm, r, bm.d_out[r] + bm.d_in[r] - bm_get<ST>(bm, r, r) - qr[v]);
-  if (last[s] == key) set_degree(bm, s, bm.d_out[s] + bm.d_in[s] - bm_get<ST>(bm, s, s) - qs[v]);
-  bm.b[v] = s;
-  prop[v] = -1;
+  finish_move<ST>(bm, v, bm.b[v], prop[v], {qr[v], qs[v]}, prop, last, gen);
 }
 
 // MDL: L = sum_cells g(M) - sum g(d_out) - sum g(d_in); mdl = E h(B^2/E) + V log B - L.
