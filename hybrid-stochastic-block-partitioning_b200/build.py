@@ -17,9 +17,6 @@ HEADERS = ["sbp_device.cuh", "sbp_kernels.cuh", "sbp_sort.cuh", "sbp_engine.cuh"
 LIB = os.path.join(HERE, "libsbp_b200.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC"]
-# The batched persistent kernel reads blockmodel state that other CTAs of the same launch
-# update: its global loads go to L2 (cache-global), never a possibly stale L1 line.
-FILE_FLAGS = {"sbp_batched.cu": ["-Xptxas", "-dlcm=cg"]}
 
 
 def _stale():
@@ -38,7 +35,7 @@ def build(force=False, verbose=False):
 
     def compile_one(src):
         obj = os.path.join(OBJ, src.replace(".cu", ".o"))
-        cmd = [nvcc] + NVCC_FLAGS + FILE_FLAGS.get(src, []) + ["-c", os.path.join(CSRC, src), "-o", obj]
+        cmd = [nvcc] + NVCC_FLAGS + ["-c", os.path.join(CSRC, src), "-o", obj]
         if verbose:
             print(" ".join(cmd), file=sys.stderr)
         subprocess.check_call(cmd)

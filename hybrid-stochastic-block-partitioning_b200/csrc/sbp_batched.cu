@@ -11,11 +11,11 @@
 //     sum).  The CTA that ends a short apply does the degree step itself, and the one that ends the
 //     MDL's partial sums the final sum: a stage's hand-over costs more than they do;
 //   * a CTA claims the next item of any graph whose current stage still has unclaimed items
-//     (one 64-bit atomic: stage << 32 | next item); the CTA finishing a stage's last item opens
+//     (one 64-bit atomic on the queue's word); the CTA finishing a stage's last item opens
 //     the graph's next stage.  No CTA ever waits while holding an item, so one graph's stages
 //     stay in order while the other graphs keep the GPU busy;
 //   * the per-element work is the single-graph kernels' own code (group_evaluate,
-//     apply_moved_vertex, finish_moved_vertex, the MDL parts with the same virtual grid), so
+//     apply_moved_record, finish_move, the MDL parts with the same virtual grid), so
 //     every graph's chain and MDL are those of sbp_partition, bit for bit;
 //   * each sweep's launch (parameter upload, queue reset, kernel, result read-back) is a
 //     captured CUDA graph, replayed once per sweep;
@@ -53,10 +53,8 @@ struct BGraph {   // one graph of the batch (device side)
   const int4* stages;        // the sweep's stages
   const int* out_src;
   int* prop;
-  int* moved;
+  int4* moves;               // a batch's accepted moves: the vertex's record, then (r, s, qr, qs)
   int* n_moved;              // two slots, alternating per batch
-  int* qr;
-  int* qs;
   unsigned long long* last;
   unsigned long long* counters;   // visits, proposals moved, accepted
   double* partial;           // MDL partial sums, one per virtual CTA
@@ -70,10 +68,24 @@ struct BGraph {   // one graph of the batch (device side)
   int mdl_ctas;              // its virtual grid
 };
 
+// A queue's state in one word, so that one load says whether there is work and one atomic claims it:
+// stage << 44 | items of the stage << 22 | next item.  A claim that comes too late leaves `next`
+// beyond `items` (by at most the CTAs of the launch).
+constexpr int kItemBits = 22;
+constexpr unsigned kItemMask = (1u << kItemBits) - 1u;
+constexpr int kMaxItems = 1 << (kItemBits - 1);      // of a stage
+constexpr int kMaxStages = 1 << (64 - 2 * kItemBits);
+__host__ __device__ inline unsigned long long queue_word(int stage, int items) {
+  return (unsigned long long)stage << (2 * kItemBits) | (unsigned long long)items << kItemBits;
+}
+__device__ __forceinline__ bool queue_open(unsigned long long c) {
+  return ((unsigned)c & kItemMask) < ((unsigned)(c >> kItemBits) & kItemMask);
+}
+
 struct Queue {                 // per graph, reset before every launch
-  unsigned long long ctr;      // stage << 32 | next item
+  unsigned long long ctr;      // queue_word + next item
   int done;                    // items of the current stage finished
-  int finished;                // 1 once the last stage is done
+  int pad;
 };
 
 struct SweepParams {
@@ -84,8 +96,8 @@ struct SweepParams {
 constexpr int kBWarps = 8;
 constexpr int kBThreads = kBWarps * 32;
 constexpr int kErrBatchWait = 16;        // no claimable work for too long
-constexpr int kMdlCtasPerItem = 16;
-constexpr int kApplyPerStripe = 256;     // moved vertices per apply / finish stripe (bound)
+constexpr int kMdlCtasPerItem = 2;       // 16: 232 ms of sweeps for 16 graphs of 1,000 to 4,000 vertices, 2: 215
+constexpr int kApplyPerStripe = 256;     // moved vertices per apply stripe (bound)
 constexpr int kFusedFinish = 2048;       // moved vertices up to which the CTA that ends an apply runs the degree step
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
@@ -94,12 +106,22 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
   return v;
 }
 
+__device__ __forceinline__ void finish_moves(const BGraph& gr, int n, unsigned gen, int t, int nt) {
+  for (int i = t; i < n; i += nt) {
+    const int v = gr.moves[2 * i].x;
+    const int4 mv = gr.moves[2 * i + 1];
+    finish_move<Store::kDense>(gr.bm, v, mv.x, mv.y, {mv.z, mv.w}, gr.prop, gr.last, gen);
+  }
+}
+
 __global__ void __launch_bounds__(kBThreads, 2)
     k_batched_sweep(const BGraph* __restrict__ G, const int* __restrict__ glist, Queue* queue, int* nfinished,
                     int* abort_flag, const SweepParams* __restrict__ sp, int slots, int* status) {
   extern __shared__ int smem[];
   __shared__ int s_g, s_stage, s_idx, s_exit, s_close;
   __shared__ double red[32];
+  __shared__ __align__(16) unsigned char graph_bytes[sizeof(BGraph)];
+  int have = -1;   // the graph in graph_bytes
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const SweepParams P = *sp;
   group_tabs_init<false>(smem, slots);
@@ -116,11 +138,7 @@ __global__ void __launch_bounds__(kBThreads, 2)
         if (k < P.ngraphs) {
           g = glist[(k + rot) % P.ngraphs];
           const Queue& q = queue[g];
-          if (!*(volatile const int*)&q.finished) {
-            const unsigned long long c = ld_relaxed_u64(&q.ctr);
-            const int st = (int)(c >> 32), idx = (int)(c & 0xffffffffu);
-            avail = st < G[g].nstages && idx < G[g].stages[st].z;
-          }
+          avail = queue_open(ld_relaxed_u64(&q.ctr));
         }
         unsigned m = __ballot_sync(kFull, avail);
         while (m && cg < 0) {
@@ -129,9 +147,9 @@ __global__ void __launch_bounds__(kBThreads, 2)
           int got = 0, gst = 0, gidx = 0;
           if (lane == l) {
             const unsigned long long old = atomicAdd(&queue[g].ctr, 1ull);
-            gst = (int)(old >> 32);
-            gidx = (int)(old & 0xffffffffu);
-            got = gst < G[g].nstages && gidx < G[g].stages[gst].z;
+            gst = (int)(old >> (2 * kItemBits));
+            gidx = (int)((unsigned)old & kItemMask);
+            got = queue_open(old);
           }
           got = __shfl_sync(kFull, got, l);
           if (got) {
@@ -171,8 +189,18 @@ __global__ void __launch_bounds__(kBThreads, 2)
       continue;
     }
     __threadfence();
-    const BGraph& gr = G[gi];
-    const int4 stg = gr.stages[s_stage];
+    if (gi != have) {   // the graph's pointers and constants, the same for the whole launch
+      for (int i = tid; i < (int)(sizeof(BGraph) / sizeof(int)); i += kBThreads)
+        reinterpret_cast<int*>(graph_bytes)[i] = reinterpret_cast<const int*>(G + gi)[i];
+      have = gi;
+      __syncthreads();
+    }
+    const BGraph& gr = *reinterpret_cast<const BGraph*>(graph_bytes);
+    const int4 stg = __ldg(gr.stages + s_stage);
+    int after[2] = {0, 0};   // thread 0: items of the next two stages (0: none)
+    if (tid == 0)
+      for (int q = 0; q < 2; ++q)
+        if (s_stage + 1 + q < gr.nstages) after[q] = __ldg(&gr.stages[s_stage + 1 + q].z);
     const int idx = s_idx;
     const unsigned gen = gr.gen0 + (unsigned)stg.y + 1u;   // gibbs_apply's ++bm.gen of batch stg.y
     int* n_cur = gr.n_moved + ((gen - 1u) & 1u);
@@ -197,7 +225,9 @@ __global__ void __launch_bounds__(kBThreads, 2)
           const bool head = valid && L.gl == 0;
           if (head && e.accepted) {
             gr.prop[e.v] = e.s;
-            gr.moved[atomicAdd(n_cur, 1)] = e.v;
+            const int i = atomicAdd(n_cur, 1);
+            gr.moves[2 * i] = rec;
+            gr.moves[2 * i + 1] = make_int4(e.r, e.s, 0, 0);
           }
           T.clear(e.n, L);
           const unsigned c_visit = __popc(__ballot_sync(kFull, head)),
@@ -213,15 +243,17 @@ __global__ void __launch_bounds__(kBThreads, 2)
       }
       case kApply: {
         const int n = *(volatile int*)n_cur;
-        for (int i = idx * kBWarps + warp; i < n; i += stg.z * kBWarps)
-          apply_moved_vertex<Store::kDense>(gr.g, gr.bm, gr.moved[i], gr.prop, gr.qr, gr.qs, gr.last, gen, lane);
+        for (int i = idx * kBWarps + warp; i < n; i += stg.z * kBWarps) {
+          const int4 rec = gr.moves[2 * i], mv = gr.moves[2 * i + 1];
+          const MoveQuirks q = apply_moved_record<Store::kDense>(gr.g, gr.bm, rec, mv.x, mv.y, gr.prop, gr.last, gen, lane);
+          if (lane == 0) gr.moves[2 * i + 1] = make_int4(mv.x, mv.y, q.qr, q.qs);
+        }
         break;
       }
       case kFinish: {
         const int n = *(volatile int*)n_cur;
         if (idx == 0 && tid == 0) gr.n_moved[gen & 1u] = 0;   // the next batch's slot
-        for (int i = idx * kBThreads + tid; i < n; i += stg.z * kBThreads)
-          finish_moved_vertex<Store::kDense>(gr.bm, gr.moved[i], gr.prop, gr.qr, gr.qs, gr.last, gen);
+        finish_moves(gr, n, gen, idx * kBThreads + tid, stg.z * kBThreads);
         break;
       }
       case kMdlPart: {
@@ -251,8 +283,7 @@ __global__ void __launch_bounds__(kBThreads, 2)
         const int n = *(volatile int*)n_cur;
         if (n <= kFusedFinish) {
           if (tid == 0) gr.n_moved[gen & 1u] = 0;   // the next batch's slot
-          for (int i = tid; i < n; i += kBThreads)
-            finish_moved_vertex<Store::kDense>(gr.bm, gr.moved[i], gr.prop, gr.qr, gr.qs, gr.last, gen);
+          finish_moves(gr, n, gen, tid, kBThreads);
           next++;
         }
       } else if (stg.x == kMdlPart) {
@@ -265,12 +296,8 @@ __global__ void __launch_bounds__(kBThreads, 2)
       if (tid == 0) {   // open the next stage
         atomicExch(&q.done, 0);
         __threadfence();
-        if (next >= gr.nstages) {
-          atomicExch(&q.finished, 1);
-          atomicAdd(nfinished, 1);
-        } else {
-          atomicExch(&q.ctr, (unsigned long long)next << 32);
-        }
+        if (next >= gr.nstages) atomicAdd(nfinished, 1);   // the queue stays without open items
+        else atomicExch(&q.ctr, queue_word(next, next == s_stage + 1 ? after[0] : after[1]));
       }
     }
     __syncthreads();
@@ -300,15 +327,24 @@ bool batchable(const SbpBlockmodel& bm, const SbpGraph& g) {
   return !bm.sparse && g.light_cap <= kLightCapMax && g.heavy_cap <= 4096 && bm.B > 1;
 }
 
+// Whether a sweep's stages and their items fit a queue's word (all but graphs of millions of
+// vertices or hundreds of thousands of batches).
+bool fits_queue(const BatchPlan& p) {
+  if (3 * (long long)p.desc.size() + 1 >= kMaxStages) return false;
+  for (const BatchDesc& b : p.desc)
+    if ((long long)b.light_n / kBWarps + 1 + b.heavy_n > kMaxItems) return false;
+  return true;
+}
+
 // The stages of one sweep of a graph with the given plan and smallest group.
 std::vector<int4> sweep_stages(const BatchPlan& p, int gmin, int mdl_ctas) {
   std::vector<int4> st;
   for (size_t b = 0; b < p.light_n.size(); ++b) {
     const int lc = (group_tasks(p.desc[b], gmin) + kBWarps - 1) / kBWarps;
     st.push_back(make_int4(kEval, (int)b, lc + p.heavy_n[b], lc));
-    const int stripes = std::max(1, (p.light_n[b] + p.heavy_n[b] + kApplyPerStripe - 1) / kApplyPerStripe);
-    st.push_back(make_int4(kApply, (int)b, stripes, 0));
-    st.push_back(make_int4(kFinish, (int)b, stripes, 0));
+    const int n = p.light_n[b] + p.heavy_n[b];
+    st.push_back(make_int4(kApply, (int)b, std::max(1, (n + kApplyPerStripe - 1) / kApplyPerStripe), 0));
+    st.push_back(make_int4(kFinish, (int)b, std::max(1, (n + kBThreads - 1) / kBThreads), 0));
   }
   st.push_back(make_int4(kMdlPart, 0, (mdl_ctas + kMdlCtasPerItem - 1) / kMdlCtasPerItem, 0));
   return st;
@@ -330,6 +366,7 @@ struct Slot {
   std::vector<double> deltas;
   int sweep = 0;
   int stage_chunk = -1, stage_mdl = -1;   // what the uploaded stages were made for
+  int first_items = 0;                    // items of the first stage
   std::chrono::steady_clock::time_point t0;
   DevBuf<int4> stages;
   DevBuf<unsigned long long> counters;
@@ -526,7 +563,8 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
     if (s.state == kEnded) end_finetune(s);
     if (s.state != kNeedMerge) return;
     const int algo = partition_merge(*s.ps, *s.g, opt, &s.fo);
-    if (algo == SBP_ASYNC_GIBBS && batchable(s.ps->bm, *s.g)) {
+    if (algo == SBP_ASYNC_GIBBS && batchable(s.ps->bm, *s.g) &&
+        fits_queue(s.g->plan(SBP_ASYNC_GIBBS, s.fo.batches))) {
       start_finetune(s);
       n_batched++;
     } else {
@@ -586,6 +624,7 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
       if (s->stage_chunk != shape.chunk || s->stage_mdl != mdl_ctas) {
         const std::vector<int4> st = sweep_stages(*s->plan, 256 / shape.chunk, mdl_ctas);
         SBP_CUDA(SBP_COPY_ASYNC(s->stages.p, st.data(), st.size() * sizeof(int4), cudaMemcpyHostToDevice, c.stream));
+        s->first_items = st[0].z;
         s->stage_chunk = shape.chunk;
         s->stage_mdl = mdl_ctas;
       }
@@ -598,10 +637,9 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
       b.stages = s->stages.p;
       b.out_src = s->g->out_src.p;
       b.prop = bm.prop.p;
-      b.moved = bm.moved.p;
+      bm.moves.reserve(2 * (size_t)s->plan->max_batch);
+      b.moves = bm.moves.p;
       b.n_moved = bm.n_moved.p;
-      b.qr = bm.qr.p;
-      b.qs = bm.qs.p;
       b.last = bm.last.p;
       b.counters = s->counters.p;
       b.partial = s->partial.p;
@@ -625,7 +663,8 @@ static void partition_batched(std::vector<std::unique_ptr<Slot>>& slots, const S
     for (Slot* s : act) {
       Queue& q = hQ[s->index];
       std::memset(&q, 0, sizeof q);
-      if (g_batched_stall_graph == s->index) q.ctr = 1ull << 20;   // stage 0, item 2^20: beyond every stage
+      q.ctr = queue_word(0, s->first_items);
+      if (g_batched_stall_graph == s->index) q.ctr += kMaxItems;   // beyond every stage
     }
     const int reserve = waiting ? std::min(g_batched_overlap, shape.ctas_per_sm * c.num_sms / 2) : 0;
     const int grid = shape.ctas_per_sm * c.num_sms - reserve;
