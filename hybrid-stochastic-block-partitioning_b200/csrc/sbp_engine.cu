@@ -326,7 +326,7 @@ static bool regrow_hashed(SbpBlockmodel& bm, const SbpGraph& g) {
   if (h[3]) k_regrow_clear<<<4 * c.num_sms, 256, 0, c.stream>>>(g_regrow_list.p + B, (int)h[3], bm.cbase.p,
                                                                  bm.cmask.p, bm.cslot.p);
   if (g.E > 0)
-    k_regrow_fill<<<grid_for(g.E, 256, 16 * c.num_sms), 256, 0, c.stream>>>(g.view(), bm.view(), g.out_src.p);
+    k_regrow_fill<<<grid_for(g.V, 256, 16 * c.num_sms), 256, 0, c.stream>>>(g.view(), bm.view());
   SBP_CHECK_LAUNCH();
   SBP_CUDA(cudaMemsetAsync(bm.overflow.p, 0, (1 + 2 * (size_t)B) * sizeof(int), c.stream));
   return true;

@@ -80,7 +80,7 @@ __global__ void k_regrow_alloc(const int* __restrict__ full, const int* __restri
                                int* mask, int* list, unsigned long long* no_room);
 __global__ void k_regrow_clear(const int* __restrict__ list, int n, const long long* __restrict__ base,
                                const int* __restrict__ mask, int2* slot);
-__global__ void k_regrow_fill(GraphView g, BlockView bm, const int* __restrict__ out_src);
+__global__ void k_regrow_fill(GraphView g, BlockView bm);
 // sbp_ingest.cu
 __global__ void k_ingest_first(const int* __restrict__ src, const int* __restrict__ dst, long long n, int V,
                                unsigned long long* keys, int* first, int tbits, int* bad);
