@@ -61,9 +61,8 @@ def args_parse():
     ap.add_argument("--no-batched", action="store_true", help="skip the batched 64-graph comparison")
     ap.add_argument("--no-mh", action="store_true", help="skip the Metropolis-Hastings / hybrid partitions")
     ap.add_argument("--host-sweeps", action="store_true",
-                    help="drive every finetune sweep from the host (same kernels and results) instead of one CUDA "
-                         "graph per finetune call; for kernel profilers, which do not profile the kernel nodes of a "
-                         "graph with conditional nodes")
+                    help="drive every finetune sweep from the host (same evaluation and results) instead of one "
+                         "persistent launch per finetune call; for kernel profilers")
     ap.add_argument("--eval-case", type=int, default=0, metavar="PARTS",
                     help="a small case for kernel profilers instead of the bench: three host-driven asynchronous-"
                          "Gibbs sweeps from the planted partition split PARTS ways")
@@ -75,8 +74,8 @@ def args_parse():
 
 def eval_case(a, V, src, dst, truth):
     """Kernel-profiler case: the planted partition with each block split into `a.eval_case` random
-    parts, three asynchronous-Gibbs sweeps driven from the host, so that every evaluation launch is
-    a plain kernel launch (ncu does not profile the kernel nodes of the graph-run finetune)."""
+    parts, three asynchronous-Gibbs sweeps driven from the host, so that every batch's evaluation is
+    a launch of its own."""
     import numpy as np
     import sbp_b200 as S
     S.load()
@@ -98,7 +97,8 @@ def split_planted(truth, parts):
 
 
 def eval_load_model(V, src, dst, truth, parts):
-    """Loads of one visit of the evaluation kernel on dense storage (evaluate_vertex), counted on
+    """Loads of one visit by a warp over counts and their transpose in separate matrices, an upper
+    bound for the pair layout (whose cells share sectors two by two), counted on
     the host from the de-duplicated graph and the profiler case's assignment, averaged over all
     vertices.  Per visit of v (block r, k = k_out + k_in neighbours, nb distinct neighbour
     blocks u, proposed block s, walk block t):
@@ -432,7 +432,7 @@ def main():
               "blocks_planted": int(truth.max()) + 1, "algorithm": a.algorithm, "batches": a.batches,
               "merge": "approximate", "step": "one full stochastic_block_partition (B = V -> final B)",
               "l2": "256 MB buffer written before every timed step (L2 flush)", "parallelism": f"replicas x{world}",
-              "sweep_driver": "host loop" if a.host_sweeps else "one CUDA graph per finetune call"}
+              "sweep_driver": "host loop" if a.host_sweeps else "one persistent launch per finetune call"}
     if a.eval_case:
         eval_case(a, V, src, dst, truth)
         return

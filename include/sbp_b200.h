@@ -116,11 +116,11 @@ int32_t sbp_device_count(void);
  * Both apply to blockmodels whose block count is set after the call.  "group_kernel" (default
  * 1): lanes per vertex of the asynchronous-Gibbs and Metropolis-Hastings evaluation on dense
  * storage, chosen from the batch and the vertex's degree; 2: as few as its degree allows
- * (asynchronous Gibbs); 0: a warp per vertex (same results).  "hashed_row_factor" (default 4, range 2-64): a rebuilt hashed row gets room
- * for factor x its cells, at most 2 x for rows of more than 128 cells (larger: rows fill up and
- * are regrown less often; smaller: less memory and a cheaper walk of the row).  "graph_sweeps" (default 1): an
- * asynchronous-Gibbs finetune on dense storage runs as one persistent launch whose sweep loop and
- * early stop are decided on the GPU; 0 drives every sweep from the host (same results).
+ * (asynchronous Gibbs); 0: a warp per vertex (same results).  "hashed_row_factor" (default 4,
+ * range 2-64): a rebuilt hashed row gets room for factor x its cells, at most 2 x for rows of more
+ * than 128 cells (larger: rows fill up and are regrown less often; smaller: less memory and a
+ * cheaper walk of the row).  "graph_sweeps" (default 1): an asynchronous-Gibbs finetune on dense
+ * storage runs as one persistent launch whose sweep loop and early stop are decided on the GPU; 0 drives every sweep from the host (same results).
  * "batched_wait_limit" (default 2^22, range 16-2^30): idle claim attempts (about 0.25 us each) of a
  * persistent CTA of sbp_partition_batched before its launch gives up and the call fails with
  * SBP_ERR_DEVICE.  "batched_stall_graph" (default -1): fault injection for failure-detection
@@ -449,7 +449,7 @@ typedef struct {
     int32_t fallback_finetunes; /* finetune calls run by the single-graph path (row-hashed storage,
                                    Metropolis-Hastings or hybrid rounds, very large degrees) */
     int32_t sweep_launches;     /* persistent-kernel launches (one per sweep of a round) */
-    int32_t chunk;              /* light vertices per evaluation work item (autotuned) */
+    int32_t chunk;              /* vertices of the smallest groups per evaluation item (autotuned) */
     int32_t ctas_per_sm;        /* persistent CTAs per SM (autotuned) */
     int32_t tuned;              /* 1: this call ran the autotuner; 0: it used an earlier choice */
     int32_t candidates;         /* candidates timed */
