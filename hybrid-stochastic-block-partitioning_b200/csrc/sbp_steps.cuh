@@ -161,19 +161,21 @@ struct MoveQuirks {
 // blockmodel.cpp:344-360, for a batch of simultaneous moves): the counts and chunk sums by edge,
 // d_out / d_in, the quirk terms qr/qs of d[r], d[s] (the neighbours that are counted in the
 // reference's sequential apply) and the batch's last mover of r and s.  One warp per vertex;
-// lanes whose edges change the same cell add their count with one atomic.
+// lanes whose edges change the same cell add their count with one atomic.  A move may be shared by
+// `parts` warps: part p takes every parts-th 64 neighbours, part 0 what is not by edge; the quirk
+// terms are then the sums of the parts'.
 template <Store ST = Store::kAny>
 __device__ __forceinline__ MoveQuirks apply_moved_record(const GraphView& g, const BlockView& bm, int4 rec, int r,
                                                          int s, const int* prop, unsigned long long* last,
-                                                         unsigned gen, int lane) {
-  const int v = rec.x, k_out = rec.z, k_in = rec.w >> 1, self = rec.w & 1, k = k_out + k_in;
+                                                         unsigned gen, int lane, int part = 0, int parts = 1) {
+  const int v = rec.x, k_out = rec.z, k_in = rec.w >> 1, k = k_out + k_in, self = part == 0 ? rec.w & 1 : 0;
   const int* nbr = g.adj + (unsigned)rec.y;
   int cr = 0, cs = 0;
   // One pass over the joint neighbour list (out-edges, then in-edges), two elements per lane
   // in flight.  Out-edge v -> u (not the self loop): (r, b_u) -= 1 and (s, b'_u) += 1, b'_u the
   // block u moves to in this batch.  In-edge u -> v of a u that stays: (b_u, r) -= 1 and
   // (b_u, s) += 1 (a moving u's own out-edge covers the cell otherwise).
-  for (int base = 0; base < k; base += 2 * kWarp) {
+  for (int base = part * 2 * kWarp; base < k; base += parts * 2 * kWarp) {
     int u[2], bo[2], pu[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -216,7 +218,7 @@ __device__ __forceinline__ MoveQuirks apply_moved_record(const GraphView& g, con
   }
   cr = warp_sum_int(cr);
   cs = warp_sum_int(cs);
-  if (lane == 0) {
+  if (lane == 0 && part == 0) {
     if (self) {
       cell_add<ST>(bm, r, r, -1);
       cell_add<ST>(bm, s, s, 1);
