@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(128, 1)
   float* sb = reinterpret_cast<float*>(sm + kFwdBias);
   const uint32_t bar = smem_u32(sm + kFwdBar);
   // A batch of the chain is 2,000 rows: 16 tiles, one a CTA, so the time is that of one tile from
-  // launch to store.  Everything it reads is asked for at once, the first layer's operands ahead.
+  // launch to store.  Everything it reads is asked for at once, the first layer's operands ahead
+  // (12.9 -> 9.4 us; 27 dependent rounds of loads into conflicting rows before).
   const long long tiles = (n + kMlpTile - 1) / kMlpTile;
   copy_kmajor(sm + kFwdW1, w.W1, kMlpHid, kMlpIn, kMlpHid);
   copy_kmajor(sm + kFwdX, X + (long long)blockIdx.x * kMlpTile * kMlpIn, kMlpTile, kMlpIn,

@@ -60,6 +60,21 @@ def test_degrees_and_blocks(S, O, storage, B, algo):
         S.set_option("dense_max_blocks", 131072)
 
 
+@pytest.mark.parametrize("B", [40, 300])
+def test_regrown_rows_count_self_loops(S, O, B):
+    """Tight hashed rows run out of room; they are recounted from the out-lists, the in-lists and the self loops."""
+    V = 1200
+    s, d = graph_of_degrees(V, B)
+    loops = np.arange(0, V, 3, dtype=np.int32)
+    S.set_option("dense_max_blocks", 1)
+    S.set_option("hashed_row_factor", 2)
+    try:
+        run_both(S, O, V, np.concatenate([s, loops]), np.concatenate([d, loops]), B, B, 1, 4, 4)
+    finally:
+        S.set_option("hashed_row_factor", 4)
+        S.set_option("dense_max_blocks", 131072)
+
+
 @pytest.mark.parametrize("algo", [0, 1])
 @pytest.mark.parametrize("B", [4095, 4096, 4097])   # 64 sums of 64 columns; beyond, a second level
 def test_walk_levels(S, O, B, algo):
