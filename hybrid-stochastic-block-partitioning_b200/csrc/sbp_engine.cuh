@@ -596,7 +596,8 @@ struct SbpBlockmodel {
   DevBuf<int> b, CS, CST, SS, SST, d_out, d_in, d;
   DevBuf<double> inv_d;
   DevBuf<int2> P;                            // dense counts of both directions (BlockView::P)
-  DevBuf<int> prop, qr, qs, moved, n_moved;   // n_moved: two slots, alternating per batch
+  DevBuf<int> prop, qr, qs, moved;
+  DevBuf<int> n_moved;                        // two slots, alternating per batch: between calls slot gen & 1 is zero
   DevBuf<int4> moves;                         // a batch's accepted moves in the finetune kernel (EvalArgs::moves)
   DevBuf<unsigned long long> last;           // (batch generation << 32 | last mover) per block
   unsigned gen = 0;                          // batch generation

@@ -400,7 +400,10 @@ SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan&
   SBP_CUDA(SBP_COPY_ASYNC(&r, c.sweep_result, sizeof r, cudaMemcpyDeviceToHost, c.stream));
   c.sync();
   c.check_status();   // before the result is used: an aborted kernel leaves none
-  bm.gen += (unsigned)(a.nbatches * r.sweeps);
+  // The batches counted in words of their own, so the slot that the next launch per batch takes, gen & 1
+  // of bm.n_moved, has to be the one it would have taken before this call: that one is zero, the other
+  // keeps the last such batch's count.
+  bm.gen += ((unsigned)(a.nbatches * r.sweeps) + 1u) & ~1u;
   return r;
 }
 
