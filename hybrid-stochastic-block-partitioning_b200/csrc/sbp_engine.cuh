@@ -253,8 +253,7 @@ struct Context {
   double* partial = nullptr;             // MDL partial sums
   double* scalar = nullptr;              // MDL result
   double* mh_out = nullptr;              // MH sweep outputs [4]
-  int* sweep_words = nullptr;            // [8] moved counts and barrier words of the persistent finetune kernel
-  SweepsResult* sweep_result = nullptr;
+  SweepsState* sweeps = nullptr;         // of the persistent finetune kernel
   unsigned* done = nullptr;              // CTAs finished in the current k_mdl launch (0 between launches)
   double2* xlogxt = nullptr;             // [kXlogxTable] x log x as hi + lo doubles
   int npartial = 0;
@@ -274,8 +273,7 @@ struct Context {
     SBP_CUDA(cudaMalloc(&c->scalar, sizeof(double)));
     SBP_CUDA(cudaMalloc(&c->mh_out, 16 * sizeof(double)));
     SBP_CUDA(cudaMalloc(&c->done, sizeof(unsigned)));
-    SBP_CUDA(cudaMalloc(&c->sweep_words, 8 * sizeof(int)));
-    SBP_CUDA(cudaMalloc(&c->sweep_result, sizeof(SweepsResult)));
+    SBP_CUDA(cudaMalloc(&c->sweeps, sizeof(SweepsState)));
     SBP_CUDA(cudaMemset(c->status, 0, 8 * sizeof(int)));
     SBP_CUDA(cudaMemset(c->done, 0, sizeof(unsigned)));
     SBP_CUDA(cudaEventCreate(&c->ev0));

@@ -246,7 +246,6 @@ __global__ void __launch_bounds__(kGroupThreads, 2) k_gibbs_sweeps(const __grid_
       bool stop = false;
       if (it < 0) {
         initial = (double)(float)mdl;   // the reference stores the entropy as float
-        if (blockIdx.x == 0) a.result->initial = mdl;
       } else {
         const double d0 = mdl - initial;   // last_iteration_entropy is never updated
         if (d0 == 0.0) {
@@ -341,9 +340,9 @@ SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan&
   a.out_src = g.out_src.p;
   a.partial = c.partial;
   a.counters = c.counters;
-  a.n_moved = c.sweep_words;
-  a.bar = reinterpret_cast<unsigned*>(c.sweep_words + 4);
-  a.result = c.sweep_result;
+  a.n_moved = c.sweeps->n_moved;
+  a.bar = c.sweeps->bar;
+  a.result = &c.sweeps->result;
   const bool direct = bm.B <= kSmallB;
   const size_t smem = group_smem_bytes(direct, a.e.slots);
   const auto k = direct ? k_gibbs_sweeps<true> : k_gibbs_sweeps<false>;
@@ -393,17 +392,18 @@ SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan&
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
   }
-  SBP_CUDA(cudaMemsetAsync(c.sweep_words, 0, 8 * sizeof(int), c.stream));
+  SBP_CUDA(cudaMemsetAsync(c.sweeps, 0, sizeof(SweepsState), c.stream));
   SBP_CUDA(cudaLaunchKernelEx(&cfg, k, a));
   SBP_CHECK_LAUNCH();
   SweepsResult r;
-  SBP_CUDA(SBP_COPY_ASYNC(&r, c.sweep_result, sizeof r, cudaMemcpyDeviceToHost, c.stream));
+  SBP_CUDA(SBP_COPY_ASYNC(&r, a.result, sizeof r, cudaMemcpyDeviceToHost, c.stream));
   c.sync();
-  c.check_status();   // before the result is used: an aborted kernel leaves none
-  // The batches counted in words of their own, so the slot that the next launch per batch takes, gen & 1
-  // of bm.n_moved, has to be the one it would have taken before this call: that one is zero, the other
-  // keeps the last such batch's count.
+  // Before any error is thrown: bm.last holds the generations of the batches that ran.  They counted in
+  // words of their own, so the slot that the next launch per batch takes, gen & 1 of bm.n_moved, has to
+  // be the one it would have taken before this call: that one is zero, the other keeps the last such
+  // batch's count.
   bm.gen += ((unsigned)(a.nbatches * r.sweeps) + 1u) & ~1u;
+  c.check_status();   // before the result is used: a kernel that gave up leaves none
   return r;
 }
 

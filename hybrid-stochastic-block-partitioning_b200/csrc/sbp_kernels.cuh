@@ -11,9 +11,16 @@ constexpr int kMaxIterations = 100;      // finetune::MAX_NUM_ITERATIONS (includ
 constexpr unsigned kGridWaitLimit = 1u << 23;
 // What a whole finetune call in one kernel reports.
 struct SweepsResult {
-  double initial, mdl;   // MDL before the first sweep and after the last
-  int sweeps;
+  double mdl;            // after the last sweep
+  int sweeps;            // 0: the kernel gave up
   int pad;
+};
+// Its words in global memory, all zero at launch.
+struct SweepsState {
+  SweepsResult result;
+  int n_moved[3];        // moved counts of a batch, taken in turn
+  int pad;
+  unsigned bar[2];       // barrier: arrivals, abort flag
 };
 
 struct Csr {

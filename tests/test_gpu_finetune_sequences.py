@@ -4,7 +4,7 @@ finetunes, collected moves, host-driven sweeps and row-hashed rounds are launche
 import numpy as np
 import pytest
 
-from conftest import random_assignment, random_graph
+from conftest import random_assignment, random_graph, random_records
 from test_gpu_parity import assert_same_state
 
 pytestmark = pytest.mark.gpu
@@ -92,3 +92,18 @@ def test_partition_whose_search_crosses_the_storages(S, O, algo, dense_max):
     assert np.array_equal(out, ref)
     for k in ("num_blocks", "visits", "accepted"):
         assert st[k] == ost[k], k
+
+
+def test_finetune_after_one_that_reported_an_error(S):
+    """A replay stream that ends early: the call fails after its sweeps; the blockmodel keeps their state."""
+    V, s, d, _ = random_graph(1500, 8, 9)
+    g = S.Graph(V, s, d)
+    bm = S.Blockmodel(g, 80, random_assignment(V, 80, 1))
+    for call in range(3):
+        with pytest.raises(S.SbpError) as e:
+            S.finetune.run(bm, GIBBS, batches=5, replay=random_records(V + V // 2, call), max_sweeps=2)
+        assert e.value.code == 4
+        other = fresh(S, bm, g)
+        for m in (bm, other):
+            S.finetune.run(m, GIBBS, batches=5, seed=2, call=call, max_sweeps=3)
+        same(bm, other)
