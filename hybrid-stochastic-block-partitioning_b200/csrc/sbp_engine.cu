@@ -1120,6 +1120,9 @@ SbpStatus sbp_set_option(const char* name, int64_t value) {
   } else if (n == "graph_sweeps") {
     SBP_REQUIRE(value == 0 || value == 1, "graph_sweeps must be 0 or 1");
     g_graph_sweeps = (int)value;
+  } else if (n == "sweep_wait_limit") {
+    SBP_REQUIRE(value >= 1 && value <= (1LL << 30), "sweep_wait_limit must be in [1, 2^30]");
+    g_sweep_wait_limit = value;
   } else if (n == "dense_max_memory_pct") {
     SBP_REQUIRE(value >= 1 && value <= 90, "dense_max_memory_pct must be in [1, 90]");
     g_dense_max_memory_pct = (int)value;

@@ -413,6 +413,8 @@ inline int g_hashed_row_factor = 4;
 // 1: an asynchronous-Gibbs finetune on dense storage runs as one persistent kernel, its sweep loop
 // and early stop on the GPU; 0: one host-driven launch sequence per sweep (sbp_set_option).
 inline int g_graph_sweeps = 1;
+// Polls of that kernel's grid barrier (about 0.7 us each) before a CTA gives up (sbp_set_option).
+inline long long g_sweep_wait_limit = 1LL << 23;
 inline thread_local long long g_overflow_rebuilds = 0;   // rebuilds forced by a full hashed row (calling thread)
 // Lanes per vertex of the evaluation on dense blockmodels (sbp_set_option "group_kernel"): 1
 // (default) chosen from the batch or round and the vertex's degree, 2 as few as its degree allows

@@ -294,6 +294,15 @@ EvalArgs eval_args(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& plan, 
   return a;
 }
 
+// After a kernel that gave up somewhere in a batch: moves without their apply, counts half updated,
+// generations begun.  The assignment is sound at every moment (a vertex changes block by one store), so
+// the state is that assignment with everything else made anew.
+void recover(SbpBlockmodel& bm, const SbpGraph& g) {
+  bm.init_vertex_scratch(bm.V);
+  SBP_CUDA(cudaMemsetAsync(bm.last.p, 0, sizeof(unsigned long long) * bm.B, Context::get().stream));
+  rebuild(bm, g);
+}
+
 // Smallest group for a batch: eight lanes a vertex once that still gives every resident warp a
 // task, else as many lanes as the idle warps allow -- a visit's chain gets shorter with more lanes.
 int group_min(int batch, int warps) {
@@ -335,7 +344,7 @@ SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan&
   a.mdl_cells = mdl_cell_form(bm, g) ? 1 : 0;
   a.mdl_ctas = mdl_grid(bm, g);
   a.gen0 = bm.gen;
-  a.wait_limit = kGridWaitLimit;
+  a.wait_limit = (unsigned)g_sweep_wait_limit;
   a.last = bm.last.p;
   a.out_src = g.out_src.p;
   a.partial = c.partial;
@@ -403,6 +412,7 @@ SweepsResult gibbs_sweeps(SbpBlockmodel& bm, const SbpGraph& g, const BatchPlan&
   // be the one it would have taken before this call: that one is zero, the other keeps the last such
   // batch's count.
   bm.gen += ((unsigned)(a.nbatches * r.sweeps) + 1u) & ~1u;
+  if (r.sweeps == 0) recover(bm, g);
   c.check_status();   // before the result is used: a kernel that gave up leaves none
   return r;
 }

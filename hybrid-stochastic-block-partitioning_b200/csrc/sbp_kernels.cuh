@@ -7,8 +7,6 @@ namespace sbpb {
 constexpr int kProposalsPerBlock = 10;   // block_merge::NUM_AGG_PROPOSALS_PER_BLOCK (include/block_merge.hpp:24)
 constexpr int kMaxIterations = 100;      // finetune::MAX_NUM_ITERATIONS (include/finetune.hpp:56)
 
-// Polls of a persistent kernel's grid barrier before it gives up (about 0.7 us each).
-constexpr unsigned kGridWaitLimit = 1u << 23;
 // What a whole finetune call in one kernel reports.
 struct SweepsResult {
   double mdl;            // after the last sweep

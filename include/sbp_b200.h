@@ -120,7 +120,10 @@ int32_t sbp_device_count(void);
  * range 2-64): a rebuilt hashed row gets room for factor x its cells, at most 2 x for rows of more
  * than 128 cells (larger: rows fill up and are regrown less often; smaller: less memory and a
  * cheaper walk of the row).  "graph_sweeps" (default 1): an asynchronous-Gibbs finetune on dense
- * storage runs as one persistent launch whose sweep loop and early stop are decided on the GPU; 0 drives every sweep from the host (same results).
+ * storage runs as one persistent launch whose sweep loop and early stop are decided on the GPU; 0
+ * drives every sweep from the host (same results).  "sweep_wait_limit" (default 2^23, range 1-2^30):
+ * polls (about 0.7 us each) of that launch's barrier before a CTA gives up and the call fails with
+ * SBP_ERR_DEVICE; the blockmodel then holds the assignment reached, with counts and degrees recounted.
  * "batched_wait_limit" (default 2^22, range 16-2^30): idle claim attempts (about 0.25 us each) of a
  * persistent CTA of sbp_partition_batched before its launch gives up and the call fails with
  * SBP_ERR_DEVICE.  "batched_stall_graph" (default -1): fault injection for failure-detection

@@ -107,3 +107,25 @@ def test_finetune_after_one_that_reported_an_error(S):
         for m in (bm, other):
             S.finetune.run(m, GIBBS, batches=5, seed=2, call=call, max_sweeps=3)
         same(bm, other)
+
+
+def test_a_barrier_wait_that_runs_out(S):
+    """Failure detection without a GPU fault: with the shortest limit the first CTAs at a barrier of the persistent
+    finetune give up, every CTA leaves, the call fails and the blockmodel is left sound."""
+    V, s, d, _ = random_graph(20_000, 12, 3)
+    g = S.Graph(V, s, d)
+    bm = S.Blockmodel(g, 500, random_assignment(V, 500, 1))
+    for call in range(3):
+        S.set_option("sweep_wait_limit", 1)
+        try:
+            with pytest.raises(S.SbpError) as e:
+                S.finetune.run(bm, GIBBS, batches=4, seed=1, call=call, max_sweeps=5)
+        finally:
+            S.set_option("sweep_wait_limit", 1 << 23)
+        assert e.value.code == 5 and "grid barrier wait" in str(e.value)
+        other = S.Blockmodel(g, 500, bm.block_assignment())
+        same(bm, other)
+        for algo in (GIBBS, HYBRID):
+            for m in (bm, other):
+                S.finetune.run(m, algo, batches=4, seed=2, call=call, max_sweeps=2)
+            same(bm, other)

@@ -85,6 +85,16 @@ def test_engine_options_are_checked_on_the_host():
         assert name in S.last_error() or "option" in S.last_error()
 
 
+def test_sweep_wait_limit_is_an_option():
+    import sbp_b200 as S
+    assert '"sweep_wait_limit"' in open(os.path.join(ROOT, "include", "sbp_b200.h")).read()
+    for bad in (0, (1 << 30) + 1):
+        with pytest.raises(S.SbpError) as e:
+            S.set_option("sweep_wait_limit", bad)
+        assert e.value.code == 1
+    S.set_option("sweep_wait_limit", 1 << 23)
+
+
 def test_release_cached_memory_needs_no_device():
     import sbp_b200 as S
     S.release_cached_memory()   # nothing cached: no CUDA call
