@@ -488,6 +488,9 @@ void finetune(SbpBlockmodel& bm, SbpGraph& g, int algo, const SbpFinetuneOptions
     st.mdl = bm.overall_entropy;
     return;
   }
+  // Threads with handles of their own may finetune at once: without the lock one call's clear of the sweep
+  // words falls between another's clear and its launch, whose barriers then let every CTA through.
+  std::lock_guard<std::mutex> one(c.finetuning);
   SBP_CUDA(cudaEventRecord(c.ev0, c.stream));
   ReplayDev rp;
   rp.upload(replay);

@@ -258,6 +258,7 @@ struct Context {
   double2* xlogxt = nullptr;             // [kXlogxTable] x log x as hi + lo doubles
   int npartial = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  std::mutex finetuning;                 // one finetune at a time: it uses the words, counters and events above
 
   // A context: its own stream and scratch; the x log x table is shared when given.
   static Context* create(double2* xlogxt) {

@@ -1,6 +1,8 @@
 """Several calls on one blockmodel: what a call leaves behind in the blockmodel's scratch must not reach the next one,
 whichever kernels the calls take.  A dense asynchronous-Gibbs finetune is one persistent kernel; hybrid and learned
 finetunes, collected moves, host-driven sweeps and row-hashed rounds are launches per batch."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -129,3 +131,32 @@ def test_a_barrier_wait_that_runs_out(S):
             for m in (bm, other):
                 S.finetune.run(m, algo, batches=4, seed=2, call=call, max_sweeps=2)
             same(bm, other)
+
+
+@pytest.mark.parametrize("algo", [GIBBS, HYBRID])
+def test_finetunes_of_two_threads(S, algo):
+    """Threads with handles of their own: states and counts are those of the calls one after the other."""
+    def build():
+        out = []
+        for V, B, seed in ((20_000, 300, 1), (1001, 40, 2), (6_000, 130, 3)):
+            V, s, d, _ = random_graph(V, 8, seed)
+            out.append(S.Blockmodel(S.Graph(V, s, d), B, random_assignment(V, B, seed)))
+        return out
+
+    def work(bm, got):
+        for call in range(8):
+            st = S.finetune.run(bm, algo, batches=10, seed=4, call=call, max_sweeps=2)
+            got.append([st[k] for k in ("visits", "accepted", "proposals_moved", "sweeps", "mdl")])
+
+    alone, together = build(), build()
+    want, got = [[] for _ in alone], [[] for _ in alone]
+    for bm, w in zip(alone, want):
+        work(bm, w)
+    threads = [threading.Thread(target=work, args=x) for x in zip(together, got)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert got == want
+    for a, b in zip(alone, together):
+        same(a, b)
