@@ -164,8 +164,7 @@ static long long unique_cells(long long E, int B, unsigned long long* keys) {
     c.sync();
     nu = lastpos + lastflag;
   }
-  k_unique_rows<<<grid_for(nu + 1, 256, 16 * c.num_sms), 256, 0, c.stream>>>(g_sort.ukeys.p, nu, B, bits,
-                                                                            g_sort.rowptr.p);
+  k_unique_rows<<<grid_for(B, 256, 16 * c.num_sms), 256, 0, c.stream>>>(g_sort.ukeys.p, nu, B, bits, g_sort.rowptr.p);
   SBP_CHECK_LAUNCH();
   return nu;
 }

@@ -16,16 +16,24 @@ __global__ void k_edge_keys(GraphView g, const int* __restrict__ b, const int* _
   }
 }
 
-// First unique key of every row: the unique keys are sorted, so the thread that sees a row change
-// writes the offsets of the rows it opens (empty rows before it included).  rowptr has B + 1 entries.
+// First unique key of every row, by a search of the sorted keys: neighbouring rows search nearly the same
+// places.  (A thread a key that writes the offsets of the rows it opens leaves a run of empty rows to one
+// thread: a blockmodel of 600,000 blocks of which 570,000 have no edge took 6.4 ms to create, with the search
+// 1.25; 10 million keys and no empty row: the same.)  rowptr has B + 1 entries.
 __global__ void k_unique_rows(const unsigned long long* __restrict__ ukeys, long long n, int B, int bits,
                               long long* rowptr) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j <= n; j += stride) {
-    const int row = j < n ? (int)(ukeys[j] >> bits) : B;
-    const int before = j > 0 ? (int)(ukeys[j - 1] >> bits) : -1;
-    for (int r = before + 1; r <= row; ++r) rowptr[r] = j;
+  const int stride = gridDim.x * blockDim.x;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < B; r += stride) {
+    const unsigned long long first = (unsigned long long)r << bits;
+    long long lo = 0, hi = n;
+    while (lo < hi) {
+      const long long mid = (lo + hi) >> 1;
+      if (ukeys[mid] < first) lo = mid + 1;
+      else hi = mid;
+    }
+    rowptr[r] = lo;
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) rowptr[B] = n;
 }
 
 // Row capacity: a power of two of at least factor * cells + 4 factor slots (room to grow: at

@@ -150,3 +150,25 @@ def test_batched_many_moves(S):
         assert np.array_equal(a, one)
         for k in ("num_blocks", "mdl", "sweeps", "accepted"):
             assert sb[k] == st[k], k
+
+
+@pytest.mark.parametrize("first,last", [(0, 3000), (0, 40), (2960, 3000), (1500, 1501), (0, 0)])
+@pytest.mark.parametrize("storage", ["dense", "hashed"])
+def test_runs_of_empty_rows(S, O, storage, first, last):
+    """Blocks with edges only from first to last: the offsets of the empty rows around them, in the storage's rows and
+    in the merge's."""
+    V = 3000
+    rng = np.random.default_rng(last)
+    n = 4000 if last > first else 0
+    s, d = (rng.integers(first, max(last, 1), n).astype(np.int32) for _ in range(2))
+    a = np.arange(V, dtype=np.int32)
+    S.set_option("dense_max_blocks", 131072 if storage == "dense" else 1)
+    try:
+        bm, obm = S.Blockmodel(S.Graph(V, s, d), V, a), O.Blockmodel(O.Graph(V, s, d), V, a)
+        assert_same_state(bm, obm)
+        if n:
+            got, ref = S.block_merge.merge_blocks(bm, seed=1), obm.merge_blocks(seed=1)
+            assert np.array_equal(got["best"], ref["best"])
+            assert_same_state(bm, obm)
+    finally:
+        S.set_option("dense_max_blocks", 131072)
