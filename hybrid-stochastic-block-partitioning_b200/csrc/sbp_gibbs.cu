@@ -26,6 +26,7 @@ struct EvalArgs {
   int* status;
   int gmin;              // smallest group
   int slots;             // table slots of the CTA (kGroupWarps regions, or more for a heavy vertex)
+  int heavy;             // those of a heavy vertex: a warp's region, twice that, ..., all of them
 };
 
 template <bool kDirect, Store ST>
@@ -67,27 +68,28 @@ template <bool kDirect, Store ST>
 __device__ __forceinline__ void eval_batch(const EvalArgs& a, BatchDesc b, int sweep, int* n_moved, int* smem,
                                            EvalCounts& cnt) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wid = blockIdx.x * kGroupWarps + warp, nw = gridDim.x * kGroupWarps;
-  // Two passes over one body: the heavy vertices, each by one warp with the whole CTA's table (any
-  // degree fits a direct-indexed histogram, so there by any warp), then the light ones.
+  const int wid = blockIdx.x * kGroupWarps + warp;
+  // Two passes over one body: the heavy vertices, a warp each, then the light ones.  As many warps of a
+  // CTA take heavy ones as its table has shares large enough for any of them (with a histogram by block:
+  // all); few as they are, they go to all CTAs before a second warp takes one.
 #pragma unroll 1
   for (int light = b.heavy_n > 0 ? 0 : 1; light < 2; ++light) {
-    const bool whole = !kDirect && !light;
-    const int first_task = whole ? (warp == 0 ? (int)blockIdx.x : b.heavy_n) : wid, step = whole ? (int)gridDim.x : nw;
+    const int at_once = kDirect || light ? kGroupWarps : min(kGroupWarps, a.slots / a.heavy);
     const int tasks = light ? group_tasks(b, a.gmin) : b.heavy_n;
+    const int first_task = light ? wid : warp < at_once ? warp * (int)gridDim.x + (int)blockIdx.x : tasks;
 #pragma unroll 1
-    for (int task = first_task; task < tasks; task += step) {
+    for (int task = first_task; task < tasks; task += at_once * (int)gridDim.x) {
       const GroupTask k = group_task(b, a.gmin, task, light);
       const Lanes L(32 >> k.lg, lane);
-      const int sub = lane >> (5 - k.lg), share = kRegionSlots >> k.lg;
-      const GroupTab<kDirect> T = group_tab<kDirect>(smem, a.slots, whole ? 0 : warp * kRegionSlots + sub * share,
-                                                     whole ? a.slots : share);
+      const int sub = lane >> (5 - k.lg), share = kDirect || light ? kRegionSlots >> k.lg : a.heavy;
+      const GroupTab<kDirect> T =
+          group_tab<kDirect>(smem, a.slots, warp * (kDirect || light ? kRegionSlots : a.heavy) + sub * share, share);
       bool valid;
       const int4 rec = task_record(a, b, k, light, lane, &valid);
       eval_task<kDirect, ST>(a, T, rec, valid, sweep, n_moved, L, cnt,
                              smem + group_smem_bytes(kDirect, a.slots) / sizeof(int) + 32 * warp);
     }
-    if (whole) __syncthreads();
+    if (!kDirect && !light) __syncthreads();   // the shares lie across the regions
   }
 }
 
@@ -290,6 +292,10 @@ EvalArgs eval_args(const SbpGraph& g, SbpBlockmodel& bm, const BatchPlan& plan, 
   // most B; twice that many while they fit
   const int distinct = std::min(g.max_k, bm.B);
   a.slots = std::max(kGroupWarps * kRegionSlots, std::min(kMaxCap, pow2_at_least(2 * distinct)));
+  // A share for a heavy vertex: at most three quarters full, or all there is.  6,000 vertices of 670
+  // neighbours, three sweeps: 1.15 ms at 300 blocks (a share a warp), 1.38 at 500 (four a CTA), 2.66 at
+  // 3,000 (two), where one warp a CTA with the whole table took 3.30, 2.23 and 2.87.
+  a.heavy = std::min(a.slots, std::max(kRegionSlots, pow2_at_least(distinct + (distinct + 2) / 3)));
   a.gmin = 8;
   return a;
 }

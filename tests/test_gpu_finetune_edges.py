@@ -172,3 +172,27 @@ def test_runs_of_empty_rows(S, O, storage, first, last):
             assert_same_state(bm, obm)
     finally:
         S.set_option("dense_max_blocks", 131072)
+
+
+@pytest.mark.parametrize("top", [384, 385, 768, 769, 1536, 1537, 3200])   # distinct neighbour blocks a share takes
+@pytest.mark.parametrize("storage", ["dense", "hashed"])
+def test_shares_of_heavy_vertices(S, O, storage, top):
+    """Every vertex its own block, so a vertex has as many neighbour blocks as neighbours; 20 of them heavy."""
+    V = 3300
+    rng = np.random.default_rng(top)
+    s, d = rng.integers(20, V, 3 * V), rng.integers(20, V, 3 * V)
+    for i in range(20):
+        k = max(257, top - 37 * i)
+        u = rng.choice(np.arange(20, V), k, replace=False)
+        out = rng.random(k) < 0.5
+        s, d = np.concatenate([s, np.where(out, i, u)]), np.concatenate([d, np.where(out, u, i)])
+    s, d = s.astype(np.int32), d.astype(np.int32)
+    S.set_option("dense_max_blocks", 131072 if storage == "dense" else 1)
+    try:
+        g, og = S.Graph(V, s, d), O.Graph(V, s, d)
+        bm, obm = S.Blockmodel(g, V, np.arange(V)), O.Blockmodel(og, V, np.arange(V))
+        S.finetune.run(bm, 1, batches=3, seed=1, call=1, max_sweeps=2)
+        obm.finetune(1, batches=3, seed=1, call=1, max_sweeps=2)
+        assert_same_state(bm, obm)
+    finally:
+        S.set_option("dense_max_blocks", 131072)
