@@ -196,3 +196,31 @@ def test_shares_of_heavy_vertices(S, O, storage, top):
         assert_same_state(bm, obm)
     finally:
         S.set_option("dense_max_blocks", 131072)
+
+
+def carried_out(best, dS, merges):
+    """Blockmodel::carry_out_best_merges of one vertex a block: block pairs by score, equal scores by index."""
+    name = np.arange(len(best))
+    groups = {i: [i] for i in range(len(best))}
+    for x in np.argsort(dS, kind="stable"):
+        if merges == 0:
+            break
+        to = name[best[x]]
+        if best[x] >= 0 and to != x:
+            moved = groups.pop(x, [])
+            name[moved] = to
+            groups[to] = groups.get(to, []) + moved
+            merges -= 1
+    return np.unique(name, return_inverse=True)[1]
+
+
+@pytest.mark.parametrize("hub", [3, 900, 2500])   # merges of two hubs of 2,500 neighbours score beyond +-2,048
+def test_order_of_the_carried_out_merges(S, hub):
+    V, hubs = 50_040, 40
+    rng = np.random.default_rng(hub)
+    s = np.repeat(np.arange(hubs), hub).astype(np.int32)
+    d = np.concatenate([hubs + rng.permutation(V - hubs)[:hub] for _ in range(hubs)]).astype(np.int32)
+    bm = S.Blockmodel(S.Graph(V, s, d), V, np.arange(V))
+    got = S.block_merge.merge_blocks(bm, seed=1)
+    assert (got["dS"].max() > 2048) == (hub == 2500)
+    assert np.array_equal(bm.block_assignment(), carried_out(got["best"], got["dS"], V - bm.B))
