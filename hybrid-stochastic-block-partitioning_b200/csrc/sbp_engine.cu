@@ -287,14 +287,7 @@ void rebuild(SbpBlockmodel& bm, const SbpGraph& g, bool recompute_d) {
   Context& c = Context::get();
   const size_t cells = (size_t)bm.B * (size_t)bm.ld;
   SBP_CUDA(cudaMemsetAsync(bm.P.p, 0, cells * sizeof(int2), c.stream));
-  if (bm.B > kSmallB) {
-    SBP_CUDA(cudaMemsetAsync(bm.CS.p, 0, (size_t)bm.B * bm.ncs * sizeof(int), c.stream));
-    SBP_CUDA(cudaMemsetAsync(bm.CST.p, 0, (size_t)bm.B * bm.ncs * sizeof(int), c.stream));
-    if (bm.nss) {
-      SBP_CUDA(cudaMemsetAsync(bm.SS.p, 0, (size_t)bm.B * bm.nss * sizeof(int), c.stream));
-      SBP_CUDA(cudaMemsetAsync(bm.SST.p, 0, (size_t)bm.B * bm.nss * sizeof(int), c.stream));
-    }
-  }
+  if (bm.B > kSmallB) SBP_CUDA(cudaMemsetAsync(bm.sums.p, 0, bm.sum_words() * sizeof(int), c.stream));
   SBP_CUDA(cudaMemsetAsync(bm.d_out.p, 0, bm.B * sizeof(int), c.stream));
   SBP_CUDA(cudaMemsetAsync(bm.d_in.p, 0, bm.B * sizeof(int), c.stream));
   if (g.V > 0) {
@@ -1382,17 +1375,8 @@ SbpStatus sbp_blockmodel_copy(const SbpBlockmodel* src, SbpBlockmodel** out) {
   const size_t cells = (size_t)src->B * src->ld;
   SBP_CUDA(SBP_COPY_ASYNC(bm->b.p, src->b.p, src->V * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->P.p, src->P.p, cells * sizeof(int2), cudaMemcpyDeviceToDevice, c.stream));
-  if (src->B > kSmallB) {
-    auto sums = [&](DevBuf<int>& to, const DevBuf<int>& from, int stride) {
-      SBP_CUDA(SBP_COPY_ASYNC(to.p, from.p, (size_t)src->B * stride * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
-    };
-    sums(bm->CS, src->CS, src->ncs);
-    sums(bm->CST, src->CST, src->ncs);
-    if (src->nss) {
-      sums(bm->SS, src->SS, src->nss);
-      sums(bm->SST, src->SST, src->nss);
-    }
-  }
+  if (src->B > kSmallB)
+    SBP_CUDA(SBP_COPY_ASYNC(bm->sums.p, src->sums.p, src->sum_words() * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->d_out.p, src->d_out.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->d_in.p, src->d_in.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));
   SBP_CUDA(SBP_COPY_ASYNC(bm->d.p, src->d.p, src->B * sizeof(int), cudaMemcpyDeviceToDevice, c.stream));

@@ -594,7 +594,8 @@ struct SbpGraph {
 struct SbpBlockmodel {
   int V = 0, B = 0, ld = 0;
   const SbpGraph* graph = nullptr;   // the graph the blockmodel was created on (must outlive it)
-  DevBuf<int> b, CS, CST, SS, SST, d_out, d_in, d;
+  DevBuf<int> b, d_out, d_in, d;
+  DevBuf<int> sums;                          // BlockView::CS, CST, SS, SST one after the other
   DevBuf<double> inv_d;
   DevBuf<int2> P;                            // dense counts of both directions (BlockView::P)
   DevBuf<int> prop, qr, qs, moved;
@@ -629,10 +630,10 @@ struct SbpBlockmodel {
     v.nch = nch;
     v.ncs = ncs;
     v.nss = nss;
-    v.SS = SS.p;
-    v.SST = SST.p;
-    v.CS = CS.p;
-    v.CST = CST.p;
+    v.CS = sums.p;
+    v.CST = v.CS + (size_t)B * ncs;
+    v.SS = v.CST + (size_t)B * ncs;
+    v.SST = v.SS + (size_t)B * nss;
     v.b = b.p;
     v.P = P.p;
     v.d_out = d_out.p;
@@ -658,6 +659,9 @@ struct SbpBlockmodel {
     SBP_CUDA(cudaMemsetAsync(prop.p, 0xff, sizeof(int) * V, c.stream));
     SBP_CUDA(cudaMemsetAsync(n_moved.p, 0, 2 * sizeof(int), c.stream));
   }
+
+  // Words of `sums` in use (dense, more than kSmallB blocks).
+  size_t sum_words() const { return 2 * (size_t)B * (size_t)(ncs + nss); }
 
   void set_blocks(int nb) {
     Context& c = Context::get();
@@ -692,14 +696,7 @@ struct SbpBlockmodel {
     } else {
       const size_t cells = (size_t)B * (size_t)ld;
       P.reserve(cells);
-      if (B > kSmallB) {
-        CS.reserve((size_t)B * ncs);
-        CST.reserve((size_t)B * ncs);
-        if (nss) {
-          SS.reserve((size_t)B * nss);
-          SST.reserve((size_t)B * nss);
-        }
-      }
+      if (B > kSmallB) sums.reserve(sum_words());
     }
     d_out.reserve(B);
     d_in.reserve(B);

@@ -160,3 +160,17 @@ def test_finetunes_of_two_threads(S, algo):
     assert got == want
     for a, b in zip(alone, together):
         same(a, b)
+
+
+@pytest.mark.parametrize("B", [100, 300, 4096, 4200])   # no sums, one level of them, two
+def test_a_copy_finetunes_as_its_source(S, B):
+    V, s, d, _ = random_graph(4600, 8, 5)
+    g = S.Graph(V, s, d)
+    bm = S.Blockmodel(g, B, random_assignment(V, B, 1))
+    S.finetune.run(bm, GIBBS, batches=3, seed=1, call=1, max_sweeps=1)
+    twin = bm.copy()
+    same(bm, twin)
+    for m in (bm, twin):
+        S.finetune.run(m, GIBBS, batches=3, seed=1, call=2, max_sweeps=2)
+        S.finetune.run(m, 0, seed=1, call=3, max_sweeps=1)
+    same(bm, twin)
