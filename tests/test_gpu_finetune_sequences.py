@@ -174,3 +174,13 @@ def test_a_copy_finetunes_as_its_source(S, B):
         S.finetune.run(m, GIBBS, batches=3, seed=1, call=2, max_sweeps=2)
         S.finetune.run(m, 0, seed=1, call=3, max_sweeps=1)
     same(bm, twin)
+
+
+@pytest.mark.parametrize("B", [1, 2, 63, 64, 65, 128, 129])
+def test_block_matrix_readback(S, B):
+    V, s, d, _ = random_graph(400, 5, 2)
+    a = random_assignment(V, B, 1)
+    pairs = np.unique(s.astype(np.int64) * V + d)
+    M = np.zeros((B, B), np.int32)
+    np.add.at(M, (a[pairs // V], a[pairs % V]), 1)
+    assert np.array_equal(S.Blockmodel(S.Graph(V, s, d), B, a).blockmatrix(), M)
