@@ -16,12 +16,14 @@
 //
 // A round is one chain of dependent loads (a few microseconds) whatever its width, and a pass is
 // the rounds its accepted moves force: the round's width W = warps * 32 / G trades against the
-// length of the chain, which grows as a group has fewer lanes.  G is chosen round by round from the
-// positions that recent rounds got through.  The commit issues atomics and stores only; every
+// length of the chain, which grows as a group has fewer lanes.  G is chosen round by round from how far
+// recent rounds got before a dependence stopped them.  The commit issues atomics and stores only; every
 // value it needs was read by the evaluation.
 #include "sbp_engine.cuh"
 #include "sbp_group.cuh"
 #include "sbp_steps.cuh"
+
+#include <limits>
 
 namespace sbpb {
 namespace {
@@ -37,29 +39,10 @@ struct MhArgs {
   RngParams rng;
   int sweep;
   int region;           // table slots of a warp
-  int kref;             // typical degree of the list
-  int min_lanes;        // smallest group
+  float m16, m8;        // groups of 16 (8) lanes from this many positions between dependences on
   double* out;          // [0] visits [1] proposals moved [2] accepted [3] sum of accepted delta-MDL in list order
   int* status;
 };
-
-// Lanes per vertex for the next round: most positions decided per unit of time, when a round is
-// expected to get through `expect` positions and its chain is a fixed part and a part per four
-// neighbours of a lane (measured at 32 blocks: about 4 to 1).
-__device__ __forceinline__ int mh_group_lanes(float expect, int warps, int kref) {
-  int best = 32;
-  float rate = 0.f;
-#pragma unroll
-  for (int G = 8; G <= 32; G *= 2) {
-    const float passes = (float)((kref + 4 * G - 1) / (4 * G));
-    const float r = fminf(expect, (float)(warps * (32 / G))) / (4.f + passes);
-    if (r > rate) {
-      rate = r;
-      best = G;
-    }
-  }
-  return best;
-}
 
 template <bool kDirect>
 __global__ void __launch_bounds__(kMhWarps * 32, 1) k_mh_dense(const __grid_constant__ MhArgs a) {
@@ -76,10 +59,10 @@ __global__ void __launch_bounds__(kMhWarps * 32, 1) k_mh_dense(const __grid_cons
   __syncthreads();
   long long visits = 0, moved = 0, accepted = 0;   // warp 0; sum_dS its first lane
   double sum_dS = 0.0;
-  float expect = 16.f;
+  float decided = 16.f, stops = 1.f;   // of recent rounds: positions got through, dependences met
   bool whole_warp = false;   // the next vertex does not fit a smaller group's table
   for (int pos = 0; pos < a.n;) {
-    const int G = whole_warp ? 32 : max(a.min_lanes, mh_group_lanes(expect, warps, a.kref));
+    const int G = whole_warp || decided < a.m16 * stops ? 32 : decided < a.m8 * stops ? 16 : 8;
     const Lanes L(G, lane);
     const int lg = G == 32 ? 0 : G == 16 ? 1 : 2, per = 1 << lg, W = warps * per;   // groups of a warp, of the CTA
     const int w = warp * per + (lane >> (5 - lg));
@@ -187,7 +170,8 @@ __global__ void __launch_bounds__(kMhWarps * 32, 1) k_mh_dense(const __grid_cons
     T.clear(e.n, L);
     __syncthreads();
     whole_warp = stop == 0;   // only a vertex that did not fit stops a round at its start
-    if (stop > 0) expect = 0.75f * expect + 0.25f * (stop >= W ? 2.f * (float)W : (float)stop);
+    decided = 0.9375f * decided + (float)stop;
+    stops = 0.9375f * stops + (stop < W ? 1.f : 0.f);
     pos += stop;
   }
   if (threadIdx.x == 0) {
@@ -211,8 +195,6 @@ MhResult mh_pass_dense(SbpBlockmodel& bm, const SbpGraph& g, const VertexList& l
   a.sweep = sweep;
   a.out = c.mh_out;
   a.status = c.status;
-  a.kref = std::max(1, (int)std::ceil(1.5 * list.mean_k));
-  a.min_lanes = g_group_kernel == 0 ? 32 : 8;
   const bool direct = bm.B <= kSmallB;
   if (!direct) mh_cap(list.max_k);   // the degree limit of the row-hashed and the learned pass
   // a whole warp's table holds every distinct neighbour block of the largest vertex
@@ -220,6 +202,30 @@ MhResult mh_pass_dense(SbpBlockmodel& bm, const SbpGraph& g, const VertexList& l
   a.region = direct ? kRegionSlots : std::max(kRegionSlots, pow2_at_least(distinct + distinct / 3));
   const int warps = (int)std::min<size_t>(kMhWarps, kSmemBudget / group_smem_bytes(direct, a.region));
   if (warps < 1) throw Error(SBP_ERR_UNSUPPORTED, "vertex degree too large for the Metropolis-Hastings kernel");
+  // Microseconds of a round, to about a fifth (graphs of 2,000 to 20,000 vertices, 4 to 200 neighbours, 8 to
+  // 1,900 blocks): a fixed part, a part per four neighbours of a lane, and what the dependence tests of
+  // 64 or 32 positions add, more with hash tables, whose look-ups are chains.  With 300 blocks and 20
+  // neighbours 16.3, 8.7 and 6.9; taken for equal, as they were, widths that dependences did not let
+  // commit were evaluated: two sweeps of 20,000 vertices at 129 blocks 174 ms against 70.
+  const int kref = std::max(1, (int)std::ceil(1.5 * list.mean_k));   // typical degree of the list
+  const float wide[3] = {direct ? 2.6f : 9.f, direct ? 0.9f : 3.f, 0.f};
+  float cost[3];   // groups of 8, 16 and 32 lanes
+  for (int i = 0; i < 3; ++i) {
+    const int four_g = 4 * (8 << i);
+    cost[i] = 5.f + (direct ? 1.f : 2.5f) * (float)((kref + four_g - 1) / four_g) + wide[i];
+  }
+  // When a dependence comes after m positions on average, a round of width W gets through m (1 - exp(-W / m))
+  // of them: the wider round is the better one from some m on.
+  auto from = [&](int i, int j) {
+    for (float m = 1.f; m < 4096.f; m *= 1.05f)
+      if ((1.f - std::exp(-(float)(warps << (2 - i)) / m)) * cost[j] >
+          (1.f - std::exp(-(float)(warps << (2 - j)) / m)) * cost[i])
+        return m;
+    return std::numeric_limits<float>::infinity();
+  };
+  a.m16 = std::min(from(1, 2), from(0, 2));
+  a.m8 = std::max(from(0, 1), from(0, 2));
+  if (g_group_kernel == 0) a.m16 = std::numeric_limits<float>::infinity();
   const size_t smem = group_smem_bytes(direct, a.region * warps);
   const auto k = direct ? k_mh_dense<true> : k_mh_dense<false>;
   set_smem_limit((const void*)k, smem);

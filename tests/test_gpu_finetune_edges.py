@@ -224,3 +224,21 @@ def test_order_of_the_carried_out_merges(S, hub):
     got = S.block_merge.merge_blocks(bm, seed=1)
     assert (got["dS"].max() > 2048) == (hub == 2500)
     assert np.array_equal(bm.block_assignment(), carried_out(got["best"], got["dS"], V - bm.B))
+
+
+@pytest.mark.parametrize("split,moved", [(1, 0.0), (1, 0.1), (12, 0.0), (12, 0.5), (60, 0.1)])
+def test_widths_of_metropolis_hastings_rounds(S, O, split, moved):
+    """Few and many accepted moves: rounds of 64, 32 and 16 positions, with histograms by block and with hash tables."""
+    V, s, d, truth = random_graph(5000, 12, split, kmin=6, kmax=60)
+    rng = np.random.default_rng(split)
+    a = truth * split + rng.integers(0, split, V)
+    some = rng.random(V) < moved
+    a[some] = rng.integers(0, 12 * split, some.sum())
+    a = np.unique(a, return_inverse=True)[1].astype(np.int32)
+    B = int(a.max()) + 1
+    bm, obm = S.Blockmodel(S.Graph(V, s, d), B, a), O.Blockmodel(O.Graph(V, s, d), B, a)
+    st = S.finetune.run(bm, 0, seed=1, call=1, max_sweeps=4)
+    ost = obm.finetune(0, seed=1, call=1, max_sweeps=4)
+    assert_same_state(bm, obm)
+    for k in ("sweeps", "visits", "accepted", "proposals_moved"):
+        assert st[k] == ost[k], k
