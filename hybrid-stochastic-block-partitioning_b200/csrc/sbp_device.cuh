@@ -162,6 +162,7 @@ constexpr int kRowPad = 128;   // rows of P are padded to a multiple of this man
 // blocks read 2.5 KB in six dependent steps and took a third of a visit).
 constexpr int kChunk = 64;
 constexpr int kFan = 64;
+constexpr int kMaxDense = kChunk * kFan * kFan;   // blocks that three levels reach (their matrix: 550 GB)
 constexpr int kSmallB = 128;   // up to this many blocks: no sums, and direct-indexed histograms
 
 struct BlockView {
@@ -181,7 +182,7 @@ struct BlockView {
   int ld;                 // row stride of P (multiple of kRowPad pairs)
   int nch;                // chunks per row = ceil(B / kChunk)
   int ncs;                // row stride of CS and CST: nch rounded up to kFan, the rest zero
-  int nss;                // row stride of SS and SST: spans rounded up to kFan; 0 up to kFan chunks
+  int nss;                // row stride of SS and SST: kFan; 0 up to kFan chunks
   int* CS;                // [B*ncs] CS[row*ncs+c] = sum of M[row, c*kChunk .. c*kChunk+kChunk)
   int* CST;               // [B*ncs] the same over the columns of M
   int* SS;                // [B*nss] sums of kFan chunk sums of CS
@@ -392,28 +393,7 @@ template <Store ST>
 __device__ __forceinline__ int walk_tree(const BlockView& bm, int t, bool col, int tg, bool on, const Lanes& L) {
   bool ok = on;
   int span = 0;
-  if (bm.nss) {
-    const int* ss = (col ? bm.SST : bm.SS) + (size_t)t * bm.nss;
-    if (bm.nss == kFan) {
-      span = walk_sums<ST>(ss, &tg, &ok, L);
-    } else {   // more than kFan spans: window by window
-      bool found = false;
-      for (int w = 0; w < bm.nss; w += kFan) {
-        int rest = tg, tot = 0;
-        bool here = on && !found;
-        const int at = walk_sums<ST>(ss + w, &rest, &here, L);
-        if (!found && on && !here)
-          for (int j = 0; j < kFan; ++j) tot += ldi<ST>(ss + w + j);
-        if (here) {
-          found = true;
-          span = w + at;
-          tg = rest;
-        }
-        if (!found) tg -= tot;
-      }
-      ok = on && found;
-    }
-  }
+  if (bm.nss) span = walk_sums<ST>((col ? bm.SST : bm.SS) + (size_t)t * bm.nss, &tg, &ok, L);
   const int chunk = span * kFan + walk_sums<ST>((col ? bm.CST : bm.CS) + (size_t)t * bm.ncs + (ok ? span : 0) * kFan,
                                                 &tg, &ok, L);
   ok = ok && chunk < bm.nch;

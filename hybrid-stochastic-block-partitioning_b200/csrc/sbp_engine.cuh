@@ -666,7 +666,7 @@ struct SbpBlockmodel {
   void set_blocks(int nb) {
     Context& c = Context::get();
     B = nb;
-    sparse = B > g_dense_max_blocks;
+    sparse = B > std::min(g_dense_max_blocks, kMaxDense);
     const double dense_bytes = 2.0 * (double)B * (double)(((B + kRowPad - 1) / kRowPad) * kRowPad) * sizeof(int);
     // dense only while it takes at most 60 % of the free device memory; cudaMemGetInfo can
     // stall the host for tens of milliseconds, so it is asked only for a matrix above 5 % of
@@ -686,7 +686,7 @@ struct SbpBlockmodel {
     ld = ((B + kRowPad - 1) / kRowPad) * kRowPad;
     nch = (B + kChunk - 1) / kChunk;
     ncs = (nch + kFan - 1) / kFan * kFan;
-    nss = nch > kFan ? (ncs / kFan + kFan - 1) / kFan * kFan : 0;
+    nss = nch > kFan ? kFan : 0;
     if (sparse) {
       rbase.reserve(B);
       cbase.reserve(B);
