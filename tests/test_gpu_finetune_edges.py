@@ -242,3 +242,60 @@ def test_widths_of_metropolis_hastings_rounds(S, O, split, moved):
     assert_same_state(bm, obm)
     for k in ("sweeps", "visits", "accepted", "proposals_moved"):
         assert st[k] == ost[k], k
+
+
+@pytest.mark.parametrize("B", [300, 600, 900])   # rows that start with few cells
+def test_regrown_rows_do_regrow(S, O, B):
+    V = 1200
+    s, d = graph_of_degrees(V, B)
+    loops = np.arange(0, V, 3, dtype=np.int32)
+    s, d = np.concatenate([s, loops]), np.concatenate([d, loops])
+    a = random_assignment(V, B, B)
+    S.set_option("dense_max_blocks", 1)
+    S.set_option("hashed_row_factor", 2)
+    try:
+        bm, obm = S.Blockmodel(S.Graph(V, s, d), B, a), O.Blockmodel(O.Graph(V, s, d), B, a)
+        st = S.finetune.run(bm, 1, batches=4, seed=B, call=1, max_sweeps=4)
+        obm.finetune(1, batches=4, seed=B, call=1, max_sweeps=4)
+        assert st["overflow_rebuilds"] > 0
+        assert_same_state(bm, obm)
+    finally:
+        S.set_option("hashed_row_factor", 4)
+        S.set_option("dense_max_blocks", 131072)
+
+
+def test_batched_degree_step_as_a_stage(S):
+    """Batches of which more than 2,048 vertices move, so that the degree step is a stage of its own."""
+    V, s, d, _ = random_graph(20_000, 6, 8)
+    g = S.Graph(V, s, d)
+    first = S.Blockmodel(g, V, np.arange(V))   # the partition's first round
+    S.block_merge.merge_blocks(first, seed=3)
+    assert S.finetune.run(first, 1, batches=2, seed=3, max_sweeps=1)["accepted"] > 2 * 2048
+    outs, stats, info = S.batched.stochastic_block_partition([g, S.Graph(V, s, d)], batches=2, seed=3)
+    assert info["batched_finetunes"] > 0
+    one, st = S.sbp.stochastic_block_partition(g, batches=2, seed=3)
+    for a, sb in zip(outs, stats):
+        assert np.array_equal(a, one)
+        for k in ("num_blocks", "mdl", "sweeps", "accepted"):
+            assert sb[k] == st[k], k
+
+
+@pytest.mark.parametrize("storage,algo", [("dense", 0), ("dense", 1), ("hashed", 1)])   # (hashed, 0): refused, the degrees
+@pytest.mark.parametrize("share", [(0.5, 0.5), (0.55, 0.4, 0.03, 0.02)])   # corners alone, cells beside them
+def test_counts_beyond_the_table(S, O, storage, share, algo):
+    """Six million edges between a few blocks: counts and degrees beyond the 2^20 entries of the x log x table."""
+    V, B = 3000, len(share)
+    rng = np.random.default_rng(B)
+    s, d = (x.astype(np.int32) for x in np.nonzero(rng.random((V, V)) < 0.67))
+    a = rng.choice(B, V, p=share).astype(np.int32)
+    S.set_option("dense_max_blocks", 131072 if storage == "dense" else 1)
+    try:
+        bm, obm = S.Blockmodel(S.Graph(V, s, d), B, a), O.Blockmodel(O.Graph(V, s, d), B, a)
+        M = bm.blockmatrix()
+        assert M[0, 1] > 1 << 20
+        st = S.finetune.run(bm, algo, batches=4, seed=1, call=1, max_sweeps=1)
+        ost = obm.finetune(algo, batches=4, seed=1, call=1, max_sweeps=1)
+        assert st["accepted"] == ost["accepted"] > 0
+        assert_same_state(bm, obm)
+    finally:
+        S.set_option("dense_max_blocks", 131072)
