@@ -84,9 +84,9 @@ inline size_t device_memory_bytes() {
 cudaStream_t engine_stream();
 
 struct DeviceCache {
-  // at most half the device's memory (at least 32 GB) stays cached: the dense block matrix of a
-  // 100,000-block finetune (two 40 GB buffers) is reused by the next partition instead of being
-  // freed and allocated again
+  // at most half the device's memory (at least 32 GB; 96 GB here) stays cached: the dense block matrix of
+  // a 100,000-block finetune (one buffer of 80 GB) is reused by the next partition instead of being
+  // freed and allocated again; one of more than 109,000 blocks is not kept
   static size_t cap_bytes() {
     static const size_t cap = std::max<size_t>(32ull << 30, device_memory_bytes() / 2);
     return cap;

@@ -4,7 +4,8 @@
  * Plain pointers and sizes only; no exceptions cross this boundary.  Every function returns
  * an SbpStatus; sbp_last_error() gives a message for the last failure on the calling thread.
  * Device memory is owned by the handles; the caller owns every host buffer.  Calls on the
- * same handle are not thread-safe.  There is no CPU fallback: without a usable CUDA device
+ * same handle are not thread-safe; finetunes of different handles may come from several threads
+ * and run one at a time.  There is no CPU fallback: without a usable CUDA device
  * every compute call fails with SBP_ERR_CUDA.
  *
  * Each entry point names the reference interface it replaces
